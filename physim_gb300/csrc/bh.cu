@@ -11,7 +11,8 @@
 //                octree 21 levels x 3 bits = 63 bits, quadtree 31 x 2 = 62.
 //                Bodies within a rounding margin of a cell boundary re-derive
 //                q by replaying the reference's f64 centre arithmetic.
-//   3. sort      stable LSD radix sort of (key, body) pairs, 9-bit digits.
+//   3. sort      stable radix sort of (key, body) pairs, 9-bit digits.
+//                Up to 1.2M bodies steps 1-3 are one launch (tree_sort_kernel).
 //   4. tree      not path-compressed (as the reference's pointer tree): a
 //                cell with more than leaf_size bodies that are not all at
 //                one key splits into its non-empty children; breadth-first
@@ -128,25 +129,44 @@ __global__ void extent_kernel(const double *__restrict__ x, const double *__rest
 // Cell index of coordinate p at the finest level D: the reference descends
 // from centre 0 / half-width X deciding `p > centre` at every level.
 // u = (p + X) * 2^(D-1) / X is the position in finest-cell units; unless u is
-// within 2^-mbits (mbits = 40 - D) of a cell boundary, the cell is floor(u),
-// read off u's bits with integer instructions (two f64 operations per axis).
-// Close to a boundary, or for u < 1, the reference's centre arithmetic is
-// replayed in f64.
-__device__ __forceinline__ uint32_t axis_cell(double p, double X, double scale, int D, int mbits)
+// within 2^-mbits of a cell boundary, the cell is floor(u), read off u's bits
+// with integer instructions (two f64 operations per axis).  Close to a
+// boundary, or for u < 1, the reference's centre arithmetic is replayed in
+// f64.  The margin: u carries three roundings (< 2^(D-51)), the reference's
+// centres at most D of 2^-53 X each (< 2^(D-49) of a cell), together under
+// 2^(D-48); mbits = 46 - D leaves a factor of four.  A replay is a chain of D
+// dependent f64 steps (3 us for the one body that needs it, and its whole sort
+// waits), so a margin as wide as 2^(D-40) was felt at 100,000 bodies, where it
+// caught about one body per step.
+__host__ __device__ inline int key_margin_bits(int D) { return 46 - D; }
+
+// axis_cell_fast reads the cell off u, or sets `replay` where that may not be
+// the reference's cell.
+__device__ __forceinline__ uint32_t axis_cell_fast(double p, double X, double scale, int D,
+                                                   int mbits, bool &replay)
 {
     const uint32_t lim = (1u << D) - 1u;
     const double u = __dmul_rn(__dadd_rn(p, X), scale);
     const unsigned long long bits = (unsigned long long)__double_as_longlong(u);
     const int ex = (int)((bits >> 52) & 0x7ff) - 1023;
     if (ex == 1024) return 0;  // NaN (or infinite) coordinate
-    if (ex >= 0 && ex <= 52 - mbits) {
-        const unsigned long long mant = (bits & 0xfffffffffffffull) | (1ull << 52);
-        const int fb = 52 - ex;  // fraction bits of u
-        const unsigned long long ip = mant >> fb;
-        const unsigned long long top = (mant >> (fb - mbits)) & ((1ull << mbits) - 1ull);
-        if (top != 0ull && top != (1ull << mbits) - 1ull)
-            return ip > lim ? lim : (uint32_t)ip;
-    }
+    const unsigned long long mant = (bits & 0xfffffffffffffull) | (1ull << 52);
+    const int fb = 52 - ex;  // fraction bits of u
+    // (shift counts outside 0..63 are only formed where `replay` discards the result)
+    const unsigned long long ip = mant >> (fb & 63);
+    const unsigned long long top = (mant >> ((fb - mbits) & 63)) & ((1ull << mbits) - 1ull);
+    const bool inside = ex >= 0 && ex <= 52 - mbits && top != 0ull && top != (1ull << mbits) - 1ull;
+    replay = replay || !inside;
+    return ip > lim ? lim : (uint32_t)ip;
+}
+
+__device__ __noinline__ uint32_t axis_cell_replay(double p, double X, int D)
+{
+    // The body that sets the extent sits on a boundary in every state: every
+    // centre lies strictly between -X and X (D <= 31 halvings of a normal X
+    // round to at most X (1 - 2^-D)), so p = X is above and p = -X below all.
+    const unsigned long long xb = (unsigned long long)__double_as_longlong(X);
+    if (abs_bits(p) == xb && (xb >> 52) > 64) return p > 0.0 ? (1u << D) - 1u : 0u;
     double c = 0.0, ext = X;
     uint32_t q = 0;
     for (int d = 0; d < D; ++d) {
@@ -181,6 +201,24 @@ __device__ __forceinline__ uint64_t spread2(uint32_t v)
     return x;
 }
 
+// Morton key of a body (X > 0; scale = 2^(D-1) / X).
+__device__ __forceinline__ uint64_t body_key(double x, double y, double z, double X, double scale,
+                                             int nchild)
+{
+    const int D = tree_levels(nchild), mbits = key_margin_bits(D);
+    bool rx = false, ry = false, rz = false;
+    uint32_t qx = axis_cell_fast(x, X, scale, D, mbits, rx);
+    uint32_t qy = axis_cell_fast(y, X, scale, D, mbits, ry);
+    uint32_t qz = nchild == 8 ? axis_cell_fast(z, X, scale, D, mbits, rz) : 0u;
+    if (rx || ry || rz) {
+        if (rx) qx = axis_cell_replay(x, X, D);
+        if (ry) qy = axis_cell_replay(y, X, D);
+        if (rz) qz = axis_cell_replay(z, X, D);
+    }
+    if (nchild != 8) return spread2(qx) | (spread2(qy) << 1);
+    return spread3(qx) | (spread3(qy) << 1) | (spread3(qz) << 2);
+}
+
 // Keys, plus the histograms of all 7 radix digits of all keys (block-local in
 // shared memory, then one global atomic per non-empty bucket), for the
 // one-sweep sort.  ghist [7][512] must be zero on entry.  Block 0 also resets
@@ -207,19 +245,8 @@ keys_kernel(const double *__restrict__ x, const double *__restrict__ y,
     }
     __syncthreads();
     const double scale = s_scale;
-    const int mbits = 40 - D;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint64_t key = 0;
-        if (X > 0.0) {
-            const uint32_t qx = axis_cell(x[i], X, scale, D, mbits);
-            const uint32_t qy = axis_cell(y[i], X, scale, D, mbits);
-            if (nchild == 8) {
-                const uint32_t qz = axis_cell(z[i], X, scale, D, mbits);
-                key = spread3(qx) | (spread3(qy) << 1) | (spread3(qz) << 2);
-            } else {
-                key = spread2(qx) | (spread2(qy) << 1);
-            }
-        }
+        const uint64_t key = X > 0.0 ? body_key(x[i], y[i], z[i], X, scale, nchild) : 0ull;
         keys[i] = key;
         vals[i] = (uint32_t)i;
 #pragma unroll
@@ -533,6 +560,382 @@ radix_sort_kernel(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, int n,
         if (pass + 1 < kSortPasses &&
             !sort_grid_barrier(bar, (uint32_t)(pass + 1) * gridDim.x, flags, spin_limit, &s_ok))
             return;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Extent, keys and sort in one launch, for states whose sort tiles are all
+// resident (one block per tile, at most one per SM: up to 1.2M bodies).
+// ---------------------------------------------------------------------------
+// The sort's cost is latency: a pass moves 24 B a key through L2, but each is
+// a chain of load, rank, exchange of the tiles' digit counts, scatter.  So:
+//   * tiles of kSortThreads x ITEMS keys, ITEMS the smallest that keeps every
+//     tile resident: a small state's passes are spread over more SMs;
+//   * the tiles exchange counts through one grid barrier (a tile adds its
+//     counts to its group of kSortGroup tiles, then sums the groups and the
+//     group's tiles before it: at most 10 + 15 loads in flight together)
+//     instead of a look-back's dependent reads;
+//   * the passes cover only the top kSortTopPasses digits (36 bits), then
+//     every key finds its place among the few that share those bits (a run)
+//     by comparing whole keys in shared memory.  If some run has more than
+//     kFixRun keys that are not all equal, every block learns it at the last
+//     barrier and all seven passes run over the order reached so far, which
+//     holds equal keys in body order: the result is the same stable order;
+//   * the extent and the keys are computed in the same launch (the keys go
+//     from registers into the first pass), and the digits' places come from
+//     the counts exchanged anyway, so no histogram pass is needed.
+// Measured against extent, keys and the look-back sort of all seven digits in
+// three launches (us, whole state): 8,195 bodies 96 -> 30, 100,003 bodies
+// 110 -> 37, 1,048,580 bodies 160 -> 92, of which the f64 pipe takes 17 for
+// the keys (2 f64 operations an axis) and each pass 15.  Beyond the resident
+// sizes the look-back sort, whose blocks take several tiles, stays.
+constexpr int kSortTopPasses = 4;
+constexpr int kSortGroup = 16;   // tiles per count group
+constexpr int kFixRun = 64;      // keys either side that share the top digits
+constexpr uint32_t kBarPoison = 0x40000000u;  // the barrier's "a wait gave up" bit
+
+struct TreeSortArgs {
+    const double *x, *y, *z;
+    int n, nchild;
+    unsigned long long *extent_bits;  // out
+    unsigned long long *blockmax;     // one per block
+    uint64_t *k0, *k1;                // the sorted keys end in k1
+    uint32_t *v0, *v1;
+    uint32_t *tile_cnt;  // [tiles][512]
+    uint32_t *grp;       // [2][groups][512]
+    uint32_t *bar;       // [0] barrier count, [1] blocks that left, [2] a run was too long
+    uint32_t *flags;
+    int spin_limit, stall_tile;
+};
+
+// Grid barrier of the resident sort: the count must reach `target`.  A wait
+// that exceeds the limit raises the sort's error flag and sets the poison bit,
+// which ends every other wait.  False: some wait gave up.
+__device__ __forceinline__ bool tree_sort_barrier(const TreeSortArgs &a, uint32_t target,
+                                                  int *s_ok)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> bar(*a.bar);
+        bar.fetch_add(1u, cuda::memory_order_release);
+        // the test hook's tile waits for a count that nothing reaches
+        const uint32_t want = (int)blockIdx.x == a.stall_tile ? kBarPoison : target;
+        int spins = 0;
+        uint32_t v;
+        while ((v = bar.load(cuda::memory_order_acquire)) < want) {
+            if (++spins > a.spin_limit) {
+                atomicOr(&a.flags[kFlagSort], 1u);
+                v = bar.fetch_or(kBarPoison, cuda::memory_order_relaxed) | kBarPoison;
+                break;
+            }
+        }
+        *s_ok = v < kBarPoison;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
+template <int ITEMS>
+struct TreeSortShared {
+    uint32_t h[kSortWarps][kRadixBuckets];
+    uint32_t digit_off[kRadixBuckets];
+    uint32_t local_start[kRadixBuckets];
+    unsigned long long wm[kSortWarps];
+    uint32_t ws[33];
+    int ok;
+};
+
+// One pass over digit `pass`: this block's tile (keys in kk / vv) goes to its
+// place in keys_out / vals_out.  Ends with the grid barrier after the writes.
+template <int ITEMS>
+__device__ __forceinline__ bool tree_sort_pass(const TreeSortArgs &a, int pass, int seq,
+                                               uint32_t &target, const uint64_t (&kk)[ITEMS],
+                                               const uint32_t (&vv)[ITEMS], uint64_t *keys_out,
+                                               uint32_t *vals_out, TreeSortShared<ITEMS> &sh,
+                                               uint64_t *skeys)
+{
+    constexpr int kTile = kSortThreads * ITEMS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int shift = kRadixBits * pass;
+    const int tile = blockIdx.x, tiles = gridDim.x;
+    const int groups = (tiles + kSortGroup - 1) / kSortGroup;
+    const int base = tile * kTile + warp * (ITEMS * 32);
+    uint32_t *svals = reinterpret_cast<uint32_t *>(skeys + kTile);
+    uint32_t *grp = a.grp + (size_t)(seq & 1) * groups * kRadixBuckets;
+    // the other half of the group counts is free (read before the last
+    // barrier): cleared for the next pass
+    {
+        uint32_t *nxt = a.grp + (size_t)((seq & 1) ^ 1) * groups * kRadixBuckets;
+        for (int k = tile * kSortThreads + threadIdx.x; k < groups * kRadixBuckets;
+             k += tiles * kSortThreads)
+            nxt[k] = 0u;
+    }
+    for (int k = threadIdx.x; k < kSortWarps * kRadixBuckets; k += kSortThreads)
+        (&sh.h[0][0])[k] = 0;
+    __syncthreads();
+    uint32_t rank[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = base + r * 32 + lane < a.n;
+        const uint32_t d = valid ? (uint32_t)(kk[r] >> shift) & (kRadixBuckets - 1) : 0u;
+        uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < kRadixBits; ++b) {
+            const uint32_t bit = (d >> b) & 1u;
+            const uint32_t vote = __ballot_sync(0xffffffffu, bit);
+            peers &= bit ? vote : ~vote;
+        }
+        const uint32_t before = __popc(peers & lanemask_lt());
+        uint32_t cur = 0;
+        if (valid) cur = sh.h[warp][d];
+        __syncwarp();
+        if (valid && before == 0) sh.h[warp][d] = cur + __popc(peers);
+        __syncwarp();
+        rank[r] = cur + before;
+    }
+    __syncthreads();
+    const int d = threadIdx.x;  // one digit per thread
+    uint32_t count = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t c = sh.h[w][d];
+        sh.h[w][d] = count;
+        count += c;
+    }
+    a.tile_cnt[(size_t)tile * kRadixBuckets + d] = count;
+    if (count) atomicAdd(&grp[(size_t)(tile / kSortGroup) * kRadixBuckets + d], count);
+    {
+        uint32_t total;
+        sh.local_start[d] = block_exclusive_scan(count, sh.ws, total);
+    }
+    __syncthreads();
+    // the tile in digit order in shared memory
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        if (base + r * 32 + lane >= a.n) continue;
+        const uint32_t dg = (uint32_t)(kk[r] >> shift) & (kRadixBuckets - 1);
+        const uint32_t lp = sh.local_start[dg] + sh.h[warp][dg] + rank[r];
+        skeys[lp] = kk[r];
+        svals[lp] = vv[r];
+    }
+    target += tiles;
+    if (!tree_sort_barrier(a, target, &sh.ok)) return false;
+    // this digit's keys in lower tiles, and in the whole state
+    uint32_t before = 0, all = 0;
+    for (int g = 0; g < groups; ++g) {
+        const uint32_t c = __ldcg(&grp[(size_t)g * kRadixBuckets + d]);
+        all += c;
+        if (g < tile / kSortGroup) before += c;
+    }
+#pragma unroll 4
+    for (int t = tile / kSortGroup * kSortGroup; t < tile; ++t)
+        before += __ldcg(&a.tile_cnt[(size_t)t * kRadixBuckets + d]);
+    {
+        uint32_t total;
+        sh.digit_off[d] = block_exclusive_scan(all, sh.ws, total) + before - sh.local_start[d];
+    }
+    __syncthreads();
+    const int cnt = min(kTile, a.n - tile * kTile);
+    for (int j = threadIdx.x; j < cnt; j += kSortThreads) {
+        const uint64_t key = skeys[j];
+        const uint32_t dg = (uint32_t)(key >> shift) & (kRadixBuckets - 1);
+        const uint32_t pos = sh.digit_off[dg] + (uint32_t)j;
+        keys_out[pos] = key;
+        vals_out[pos] = svals[j];
+    }
+    target += tiles;
+    return tree_sort_barrier(a, target, &sh.ok);
+}
+
+template <int ITEMS>
+__device__ __forceinline__ void tree_sort_body(const TreeSortArgs &a, TreeSortShared<ITEMS> &sh,
+                                               uint64_t *skeys)
+{
+    constexpr int kTile = kSortThreads * ITEMS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = blockIdx.x, tiles = gridDim.x;
+    const int base = tile * kTile + warp * (ITEMS * 32);
+    uint32_t target = 0;
+    // positions in batches whose loads are in flight together (a batch is a
+    // thread's whole share up to 4 keys: then the keys need no second read)
+    constexpr int kBatch = ITEMS < 4 ? ITEMS : 4;
+    double px[kBatch], py[kBatch], pz[kBatch];
+    auto load_positions = [&](int r0) {
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const int i = base + (r0 + r) * 32 + lane;
+            const bool valid = r0 + r < ITEMS && i < a.n;
+            px[r] = valid ? a.x[i] : 0.0;
+            py[r] = valid ? a.y[i] : 0.0;
+            pz[r] = valid ? a.z[i] : 0.0;
+        }
+    };
+    // extent: the tiles' maxima, and the first pass's group counts cleared
+    {
+        const int groups = (tiles + kSortGroup - 1) / kSortGroup;
+        for (int k = tile * kSortThreads + threadIdx.x; k < groups * kRadixBuckets;
+             k += tiles * kSortThreads)
+            a.grp[k] = 0u;
+        if (tile == 0 && threadIdx.x == 0) a.bar[2] = 0u;
+        unsigned long long m = 0;
+#pragma unroll 1
+        for (int r0 = 0; r0 < ITEMS; r0 += kBatch) {
+            load_positions(r0);
+#pragma unroll
+            for (int r = 0; r < kBatch; ++r)
+                m = max(max(m, abs_bits(px[r])), max(abs_bits(py[r]), abs_bits(pz[r])));
+        }
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) sh.wm[warp] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kSortWarps; ++w) m = max(m, sh.wm[w]);
+            a.blockmax[tile] = m;
+        }
+    }
+    target += tiles;
+    if (!tree_sort_barrier(a, target, &sh.ok)) return;
+    {
+        unsigned long long m = 0;
+        for (int t = threadIdx.x; t < tiles; t += kSortThreads)
+            m = max(m, __ldcg(&a.blockmax[t]));
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) sh.wm[warp] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kSortWarps; ++w) m = max(m, sh.wm[w]);
+            sh.wm[0] = m;
+            if (tile == 0) *a.extent_bits = m;
+        }
+        __syncthreads();
+    }
+    const double X = __longlong_as_double((long long)sh.wm[0]);
+    uint64_t kk[ITEMS];
+    uint32_t vv[ITEMS];
+    {
+        const int D = tree_levels(a.nchild);
+        __shared__ double s_scale;
+        if (threadIdx.x == 0) s_scale = X > 0.0 ? __ddiv_rn(ldexp(1.0, D - 1), X) : 0.0;
+        __syncthreads();
+        const double scale = s_scale;
+        // through shared memory: the loop stays rolled (unrolled over all keys
+        // its code outgrows the instruction cache) and the keys in registers
+#pragma unroll 1
+        for (int r0 = 0; r0 < ITEMS; r0 += kBatch) {
+            if (ITEMS > kBatch) load_positions(r0);
+#pragma unroll
+            for (int r = 0; r < kBatch; ++r) {
+                if (r0 + r >= ITEMS) break;
+                const int i = base + (r0 + r) * 32 + lane;
+                skeys[i - tile * kTile] =
+                    i < a.n && X > 0.0 ? body_key(px[r], py[r], pz[r], X, scale, a.nchild) : 0ull;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int i = base + r * 32 + lane;  // written by this thread
+            kk[r] = skeys[i - tile * kTile];
+            vv[r] = (uint32_t)i;
+        }
+    }
+    int seq = 0;
+    uint64_t *kin = a.k0, *kout = a.k1;
+    uint32_t *vin = a.v0, *vout = a.v1;
+    auto load = [&]() {
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int i = base + r * 32 + lane;
+            kk[r] = i < a.n ? __ldcg(&kin[i]) : 0ull;
+            vv[r] = i < a.n ? __ldcg(&vin[i]) : 0u;
+        }
+    };
+    auto swap = [&]() {
+        uint64_t *tk = kin;
+        kin = kout;
+        kout = tk;
+        uint32_t *tv = vin;
+        vin = vout;
+        vout = tv;
+    };
+    static_assert(kSortTopPasses % 2 == 0 && kSortPasses % 2 == 1, "the order ends in k1, v1");
+#pragma unroll 1
+    for (int pass = kSortPasses - kSortTopPasses; pass < kSortPasses; ++pass) {
+        if (seq > 0) load();
+        if (!tree_sort_pass<ITEMS>(a, pass, seq, target, kk, vv, kout, vout, sh, skeys)) return;
+        ++seq;
+        swap();
+    }
+    // kin (k0) is in order of the top digits; each key's place among those
+    // that share them, into k1
+    {
+        const int shift = kRadixBits * (kSortPasses - kSortTopPasses);
+        const int t0 = tile * kTile;
+#pragma unroll 4  // loads in flight together
+        for (int t = threadIdx.x; t < kTile + 2 * kFixRun; t += kSortThreads) {
+            const int i = t0 - kFixRun + t;
+            skeys[t] = i >= 0 && i < a.n ? __ldcg(&kin[i]) : ~0ull;  // no key has bit 63
+        }
+        uint32_t *sv = reinterpret_cast<uint32_t *>(skeys + kTile + 2 * kFixRun);
+#pragma unroll 4
+        for (int t = threadIdx.x; t < kTile; t += kSortThreads)
+            sv[t] = t0 + t < a.n ? __ldcg(&vin[t0 + t]) : 0u;
+        __syncthreads();
+        bool too_long = false;
+#pragma unroll 1
+        for (int t = threadIdx.x; t < kTile && t0 + t < a.n; t += kSortThreads) {
+            const uint64_t *p = skeys + kFixRun + t;
+            const uint64_t k = p[0];
+            int left = 0, right = 0, rank = 0;
+            bool differ = false;
+            while (left < kFixRun) {
+                const uint64_t o = p[-(left + 1)];
+                if ((o ^ k) >> shift) break;
+                ++left;
+                rank += o <= k;
+                differ |= o != k;
+            }
+            while (right < kFixRun) {
+                const uint64_t o = p[right + 1];
+                if ((o ^ k) >> shift) break;
+                ++right;
+                rank += o < k;
+                differ |= o != k;
+            }
+            too_long |= differ && (left == kFixRun || right == kFixRun);
+            const int at = t0 + t;
+            const int to = at - left + rank;  // within the run: always in [0, n)
+            kout[to] = k;
+            vout[to] = sv[t];
+        }
+        if (__syncthreads_or(too_long) && threadIdx.x == 0) atomicOr(&a.bar[2], 1u);
+    }
+    target += tiles;
+    if (!tree_sort_barrier(a, target, &sh.ok)) return;
+    if (__ldcg(&a.bar[2]) == 0u) return;
+#pragma unroll 1
+    for (int pass = 0; pass < kSortPasses; ++pass) {
+        load();
+        if (!tree_sort_pass<ITEMS>(a, pass, seq, target, kk, vv, kout, vout, sh, skeys)) return;
+        ++seq;
+        swap();
+    }
+}
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, 1) tree_sort_kernel(TreeSortArgs a)
+{
+    static_assert(kSortThreads == kRadixBuckets, "one thread per digit");
+    __shared__ TreeSortShared<ITEMS> sh;
+    extern __shared__ uint64_t skeys_dyn[];
+    tree_sort_body<ITEMS>(a, sh, skeys_dyn);
+    // the last block to leave resets the barrier for the next build
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {
+            a.bar[0] = 0u;
+            a.bar[1] = 0u;
+        }
     }
 }
 
@@ -1737,6 +2140,56 @@ namespace {
 // single-launch sort an SM holds (0 = one launch per pass)
 std::atomic<bool> g_sort_ready[64];
 std::atomic<int> g_sort_coop_per_sm[64];
+
+constexpr int kTreeSortItems[] = {1, 2, 4, 6, 8, 10, 12, 14, 16};
+
+const void *tree_sort_fn(int items)
+{
+    switch (items) {
+    case 1: return (const void *)tree_sort_kernel<1>;
+    case 2: return (const void *)tree_sort_kernel<2>;
+    case 4: return (const void *)tree_sort_kernel<4>;
+    case 6: return (const void *)tree_sort_kernel<6>;
+    case 8: return (const void *)tree_sort_kernel<8>;
+    case 10: return (const void *)tree_sort_kernel<10>;
+    case 12: return (const void *)tree_sort_kernel<12>;
+    case 14: return (const void *)tree_sort_kernel<14>;
+    default: return (const void *)tree_sort_kernel<16>;
+    }
+}
+
+size_t tree_sort_smem(int items)
+{
+    // the staged tile; its runs are placed with kFixRun keys either side
+    return (size_t)kSortThreads * items * (sizeof(uint64_t) + sizeof(uint32_t)) +
+           2 * kFixRun * sizeof(uint64_t);
+}
+
+int tree_sort_attributes()
+{
+    for (int items : kTreeSortItems)
+        PG_CUDA(cudaFuncSetAttribute(tree_sort_fn(items),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)tree_sort_smem(items)));
+    return PHYSIM_OK;
+}
+
+// Keys per thread of the resident sort of n bodies: the fewest that give
+// every tile a block of its own on `blocks` resident blocks (0: none does).
+int resident_items(size_t n, int blocks)
+{
+    for (int items : kTreeSortItems)
+        if (((n + (size_t)kSortThreads * items - 1) / ((size_t)kSortThreads * items)) <=
+            (size_t)blocks)
+            return items;
+    return 0;
+}
+
+// Tiles that the resident sort of up to n bodies can need.
+int resident_tiles(size_t n, int blocks)
+{
+    return (int)std::min<size_t>((n + kSortThreads - 1) / kSortThreads, (size_t)blocks);
+}
 }  // namespace
 
 struct BhWorkspace {
@@ -1750,6 +2203,10 @@ struct BhWorkspace {
     // sort_status: look-back words, tiles x digits
     uint32_t *sort_meta = nullptr;
     unsigned long long *sort_status = nullptr;
+    // the resident sort: tiles' digit counts, their groups' counts (two
+    // halves), blocks' extents, and barrier words
+    uint32_t *tile_cnt = nullptr, *tile_grp = nullptr, *tree_bar = nullptr;
+    unsigned long long *blockmax = nullptr;
     float4 *sbody = nullptr;
     uint8_t *lcp = nullptr;        // L(k): leading digits keys[k-1] and keys[k] share
     uint32_t *mask = nullptr;      // level mask of each sorted body
@@ -1780,7 +2237,8 @@ static void ws_release(BhWorkspace *ws)
                  ws->nd.count,    ws->nd.child,   ws->nd.nchild,  ws->nd.level,
                  ws->nd.c64,      ws->nd.geo,     ws->nd.com,     ws->lv,
                  ws->extent_bits, ws->flags,      ws->nd.meta,    ws->stats,
-                 ws->nd.parent,   ws->nd.quad_a,  ws->nd.quad_b,  ws->nd.arrivals};
+                 ws->nd.parent,   ws->nd.quad_a,  ws->nd.quad_b,  ws->nd.arrivals,
+                 ws->tile_cnt,    ws->tile_grp,   ws->tree_bar,   ws->blockmax};
     for (void *q : p) dev_free(q, ws->stream);
 }
 
@@ -1808,6 +2266,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
         PG_CUDA(cudaFuncSetAttribute(radix_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kSortSmem));
         int coop = 0, per_sm = 0;
+        PG_TRY(tree_sort_attributes());
         PG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
         if (coop)
             PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, radix_sort_kernel,
@@ -1822,6 +2281,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
     const size_t cap = n < 64 ? 64 : n;
     w->cap_n = cap;
     const int tiles = cdiv((long long)cap, kSortTile);
+    const int resident_blocks = device_sm_count(device);
     const size_t tree_blocks = (size_t)cdiv((long long)cap, kTreeBlock);
     // Node capacity: leaves hold about leaf/4 bodies on average, so 8N/leaf
     // (at most 4N) nodes hold every non-degenerate distribution; deeper
@@ -1837,6 +2297,11 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
     PG_WA(w->vals[1], cap);
     PG_WA(w->sort_meta, (size_t)kSortPasses * kRadixBuckets + kSortPasses + 2);
     PG_WA(w->sort_status, (size_t)kRadixBuckets * tiles);
+    const size_t rtiles = (size_t)resident_tiles(cap, resident_blocks);
+    PG_WA(w->tile_cnt, rtiles * kRadixBuckets);
+    PG_WA(w->tile_grp, 2 * ((rtiles + kSortGroup - 1) / kSortGroup) * kRadixBuckets);
+    PG_WA(w->blockmax, rtiles);
+    PG_WA(w->tree_bar, 4);
     PG_WA(w->sbody, cap);
     PG_WA(w->lcp, cap);
     PG_WA(w->mask, cap);
@@ -1869,6 +2334,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
         (cudaMemsetAsync(w->flags, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->nd.arrivals, 0, ncap * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->lv, 0, sizeof(LevelInfo), stream) != cudaSuccess ||
+         cudaMemsetAsync(w->tree_bar, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->sort_meta, 0,
                          ((size_t)kSortPasses * kRadixBuckets + kSortPasses + 2) * sizeof(uint32_t),
                          stream) != cudaSuccess ||
@@ -1956,12 +2422,43 @@ int wait_limit()
 }
 }  // namespace
 
-static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, cudaStream_t st)
+// Extent, keys and sort of a state whose tiles are all resident.
+static int launch_tree_sort(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, int n,
+                            int items, cudaStream_t st)
 {
-    const int n = (int)b.n;
-    int launches = 0;
+    TreeSortArgs a;
+    a.x = b.x;
+    a.y = b.y;
+    a.z = b.z;
+    a.n = n;
+    a.nchild = p.nchild;
+    a.extent_bits = ws->extent_bits;
+    a.blockmax = ws->blockmax;
+    a.k0 = ws->keys[0];
+    a.k1 = ws->keys[1];
+    a.v0 = ws->vals[0];
+    a.v1 = ws->vals[1];
+    a.tile_cnt = ws->tile_cnt;
+    a.grp = ws->tile_grp;
+    a.bar = ws->tree_bar;
+    a.flags = ws->flags;
+    a.spin_limit = wait_limit();
+    a.stall_tile = (int)g_stall_tile.load();
+    void *args[] = {&a};
+    PG_CUDA(cudaLaunchCooperativeKernel(tree_sort_fn(items),
+                                        dim3((unsigned)cdiv(n, kSortThreads * items)),
+                                        dim3(kSortThreads), args, tree_sort_smem(items), st));
+    return PHYSIM_OK;
+}
+
+// The same as separate launches: extent, keys with the digits' histograms, and
+// the one-sweep radix sort of all seven digits, in one cooperative launch
+// where the device allows it (blocks then sort several tiles), else one launch
+// per pass.
+static int launch_split_sort(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, int n,
+                             int per_sm, int sms, cudaStream_t st, int *cur_out, int *launches)
+{
     PG_CUDA(cudaMemsetAsync(ws->extent_bits, 0, sizeof(unsigned long long), st));
-    const int sms = device_sm_count(ws->device);
     extent_kernel<<<sms * 2, 256, 0, st>>>(b.x, b.y, b.z, n, ws->extent_bits);
     uint32_t *ghist = ws->sort_meta;
     uint32_t *tile_ctr = ws->sort_meta + kSortPasses * kRadixBuckets;
@@ -1971,11 +2468,10 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
     keys_kernel<<<std::min(cdiv(n, 256), sms * 8), 256, 0, st>>>(
         b.x, b.y, b.z, n, p.nchild, ws->extent_bits, ws->keys[0], ws->vals[0], ghist, tile_ctr,
         epoch, sort_bar);
-    launches += 2;
+    *launches += 2;
     // one-sweep radix sort over 9-bit digits: all passes in one cooperative
     // launch where the device allows it, else one launch per pass
     const int tiles = cdiv(n, kSortTile);
-    const int per_sm = ws->device >= 0 && ws->device < 64 ? g_sort_coop_per_sm[ws->device].load() : 0;
     int cur = 0;
     if (g_sort_single.load() && per_sm > 0) {
         cudaLaunchConfig_t cfg = {};
@@ -1993,7 +2489,7 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
                                    (const uint32_t *)epoch, ws->flags, wait_limit(),
                                    (int)g_stall_tile.load(), sort_bar));
         cur = kSortPasses & 1;
-        launches += 1;
+        *launches += 1;
     } else {
         for (int pass = 0; pass < kSortPasses; ++pass) {
             radix_pass_kernel<<<tiles, kSortThreads, kSortSmem, st>>>(
@@ -2001,8 +2497,27 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
                 ws->vals[cur ^ 1], n, pass, ghist, tile_ctr, ws->sort_status, epoch, ws->flags,
                 wait_limit(), g_stall_tile.load());
             cur ^= 1;
-            launches += 1;
+            *launches += 1;
         }
+    }
+    *cur_out = cur;
+    return PHYSIM_OK;
+}
+
+static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, cudaStream_t st)
+{
+    const int n = (int)b.n;
+    int launches = 0;
+    const int sms = device_sm_count(ws->device);
+    const int per_sm = ws->device >= 0 && ws->device < 64 ? g_sort_coop_per_sm[ws->device].load() : 0;
+    const int items = per_sm > 0 ? resident_items((size_t)n, sms) : 0;
+    int cur = 0;
+    if (g_sort_single.load() && items > 0) {
+        PG_TRY(launch_tree_sort(ws, b, p, n, items, st));
+        cur = 1;
+        launches += 1;
+    } else {
+        PG_TRY(launch_split_sort(ws, b, p, n, per_sm, sms, st, &cur, &launches));
     }
     ws->sorted = cur;
     // the tree: boundaries (+ sorted f32 bodies), level masks, one scan, node
