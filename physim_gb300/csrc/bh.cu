@@ -21,8 +21,9 @@
 //                key-prefix boundaries (section 4).  Geometric centres are
 //                computed exactly as the reference does (child = parent +-
 //                extent/2, octree.rs:167-215).
-//   5. moments   mass, centre of mass (double-float sums) and optionally
-//                second moments (f32) of every cell, bottom up in one launch.
+//   5. cells     geometry, mass, centre of mass (double-float sums) and optionally
+//                second moments (f32) of every cell, all cells at once from
+//                sums over groups of consecutive sorted bodies.
 //   6. traversal one warp per 32 consecutive sorted bodies, DFS with a shared
 //                stack, the reference's opening rule extent/|x - centre| < theta
 //                (octree.rs:137-144).  EXACT: every body keeps its own
@@ -945,18 +946,54 @@ __global__ void __launch_bounds__(kSortThreads, 1) tree_sort_kernel(TreeSortArgs
 struct NodeArrays {
     int32_t *begin, *count, *child;
     uint8_t *nchild, *level;
-    double *c64;   // 4 x cap: cx, cy, cz, extent
-    float4 *geo;   // cx, cy, cz, extent (f32)
+    float4 *geo;     // cx, cy, cz, extent (f32)
+    float4 *geo_lo;  // the centre's f64 value less its f32 one (exact traversal only)
     float4 *com;   // x, y, z, mass (f32)
     int4 *meta;    // (id | nchild << 28, first child, first body, body count)
     int32_t *parent;   // parent node, -1 for the root
-    float4 *msum_hi;   // mass and mass-weighted position sums (M, Mx, My, Mz) as
-    float4 *msum_lo;   //   double-float pairs (hi + lo)
     float4 *quad_a;    // second moments about the centre of mass: Sxx, Syy, Szz, trace
     float4 *quad_b;    // Sxy, Sxz, Syz, 0
-    uint32_t *arrivals;  // children finished, for the bottom-up moment pass (kept at 0)
     int cap;
 };
+
+// ---------------------------------------------------------------------------
+// double-float helpers
+// ---------------------------------------------------------------------------
+// (ah, al) + (bh, bl) as a normalised double-float pair.
+__device__ __forceinline__ void df_add(float &ah, float &al, float bh, float bl)
+{
+    float s, e;
+    two_sum(ah, bh, s, e);
+    e += al + bl;
+    ah = s + e;
+    al = e - (ah - s);
+}
+
+// f32 rounding of (sh + sl) / (mh + ml): an f32 quotient corrected once with
+// its exact residual (TwoProduct by FMA).
+__device__ __forceinline__ float df_div(float sh, float sl, float mh, float ml)
+{
+    const float q = sh / mh;
+    const float p = q * mh;
+    const float pe = fmaf(q, mh, -p);
+    const float r = fmaf(-q, ml, ((sh - p) - pe) + sl);
+    return q + r / mh;
+}
+
+__device__ __forceinline__ float4 df_com(const float4 h, const float4 l, float4 geo)
+{
+    if (h.x == 0.f && l.x == 0.f) return make_float4(geo.x, geo.y, geo.z, 0.f);
+    return make_float4(df_div(h.y, l.y, h.x, l.x), df_div(h.z, l.z, h.x, l.x),
+                       df_div(h.w, l.w, h.x, l.x), h.x + l.x);
+}
+
+// m * p added exactly-rounded into the double-float (hi, lo)
+__device__ __forceinline__ void df_add_prod(float &hi, float &lo, float m, float p)
+{
+    const float pr = m * p;
+    const float pe = fmaf(m, p, -pr);
+    df_add(hi, lo, pr, pe);
+}
 
 // ---------------------------------------------------------------------------
 // 4. tree build (flat: a few launches for all levels)
@@ -999,25 +1036,291 @@ __device__ __forceinline__ bool sort_failed(const uint32_t *flags)
     return *(volatile const uint32_t *)&flags[kFlagSort] != 0u;
 }
 
-// L(k) for k >= 1 (the number of leading digits keys[k-1] and keys[k] share,
-// D for equal keys), and the sorted f32 bodies.
-__global__ void boundary_kernel(const uint64_t *__restrict__ keys,
-                                const uint32_t *__restrict__ order, int n, int nchild,
-                                const float4 *__restrict__ body4, float4 *__restrict__ sbody,
-                                uint8_t *__restrict__ lcp, const uint32_t *__restrict__ flags)
+// Sums over groups of consecutive sorted bodies, from which cell_kernel reads
+// any cell's moments without waiting for its children: level k holds groups of
+// kSegBase 2^k bodies, complete groups only, level after level.  A group keeps
+// its mass and mass-weighted position sums (M, Mx, My, Mz) as double-float
+// pairs (hi + lo) and, for quadrupole builds, its f32 centre of mass and second
+// moments about it.  Sums are additions of sub-sums only (no differences of
+// prefixes), so a cell is as exact beside a heavy neighbour as alone.
+constexpr int kSegBase = 4;
+constexpr int kSegLevels = 30;
+constexpr int kSegBlock = 1024;                   // bodies whose groups one block sums
+constexpr int kSegBlockLevel = 8;                 // kSegBase << 8 = kSegBlock
+
+struct Segments {
+    float4 *hi, *lo;
+    float4 *com, *qa, *qb;  // quadrupole builds
+    int n;                  // bodies
+    int off[kSegLevels];    // first group of each level
+    __host__ __device__ int groups(int level) const { return n / kSegBase >> level; }
+};
+
+struct GroupSum {
+    float4 h, l;
+};
+
+__device__ __forceinline__ void df_add4(GroupSum &a, const GroupSum &b)
 {
-    if (sort_failed(flags)) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int D = tree_levels(nchild), B = level_bits(nchild);
-    sbody[k] = body4[order[k]];
-    int L = 0;
-    if (k > 0) {
-        const uint64_t x = keys[k - 1] ^ keys[k];
-        // keys use the low B * D bits: 64 - B * D leading bits are always 0
-        L = x == 0 ? D : (__clzll((long long)x) - (64 - B * D)) / B;
+    df_add(a.h.x, a.l.x, b.h.x, b.l.x);
+    df_add(a.h.y, a.l.y, b.h.y, b.l.y);
+    df_add(a.h.z, a.l.z, b.h.z, b.l.z);
+    df_add(a.h.w, a.l.w, b.h.w, b.l.w);
+}
+
+__device__ __forceinline__ void df_add_body(GroupSum &a, float4 p)
+{
+    df_add(a.h.x, a.l.x, p.w, 0.f);
+    df_add_prod(a.h.y, a.l.y, p.w, p.x);
+    df_add_prod(a.h.z, a.l.z, p.w, p.y);
+    df_add_prod(a.h.w, a.l.w, p.w, p.z);
+}
+
+__device__ __forceinline__ GroupSum group_zero()
+{
+    GroupSum g;
+    g.h = g.l = make_float4(0.f, 0.f, 0.f, 0.f);
+    return g;
+}
+
+// Second moments: xx, yy, zz, xy, xz, yz.
+struct Quad6 {
+    float v[6];
+};
+
+// q += m d d^T + s (s about its own centre, d from the new centre to it)
+__device__ __forceinline__ void quad_shift_add(Quad6 &q, const Quad6 &s, float m, float dx,
+                                               float dy, float dz)
+{
+    q.v[0] += fmaf(m * dx, dx, s.v[0]);
+    q.v[1] += fmaf(m * dy, dy, s.v[1]);
+    q.v[2] += fmaf(m * dz, dz, s.v[2]);
+    q.v[3] += fmaf(m * dx, dy, s.v[3]);
+    q.v[4] += fmaf(m * dx, dz, s.v[4]);
+    q.v[5] += fmaf(m * dy, dz, s.v[5]);
+}
+
+__device__ __forceinline__ void quad_body_add(Quad6 &q, float4 p, float4 com)
+{
+    const float dx = p.x - com.x, dy = p.y - com.y, dz = p.z - com.z;
+    q.v[0] = fmaf(p.w * dx, dx, q.v[0]);
+    q.v[1] = fmaf(p.w * dy, dy, q.v[1]);
+    q.v[2] = fmaf(p.w * dz, dz, q.v[2]);
+    q.v[3] = fmaf(p.w * dx, dy, q.v[3]);
+    q.v[4] = fmaf(p.w * dx, dz, q.v[4]);
+    q.v[5] = fmaf(p.w * dy, dz, q.v[5]);
+}
+
+__device__ __forceinline__ Quad6 quad_load(const Segments &sg, int at)
+{
+    const float4 a = sg.qa[at], b = sg.qb[at];
+    return {{a.x, a.y, a.z, b.x, b.y, b.z}};
+}
+
+__device__ __forceinline__ void group_store(const Segments &sg, int at, const GroupSum &g)
+{
+    sg.hi[at] = g.h;
+    sg.lo[at] = g.l;
+}
+
+__device__ __forceinline__ void group_store_quad(const Segments &sg, int at, float4 com,
+                                                 const Quad6 &q)
+{
+    sg.com[at] = com;
+    sg.qa[at] = make_float4(q.v[0], q.v[1], q.v[2], q.v[0] + q.v[1] + q.v[2]);
+    sg.qb[at] = make_float4(q.v[3], q.v[4], q.v[5], 0.f);
+}
+
+// A group and its quadrupole from its two halves.
+template <bool kQuad>
+__device__ __forceinline__ void group_join(GroupSum &g, float4 &com, Quad6 &q, const GroupSum &o,
+                                           float4 ocom, const Quad6 &oq)
+{
+    df_add4(g, o);
+    if (kQuad) {
+        const float4 c = df_com(g.h, g.l, com);
+        Quad6 t = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+        quad_shift_add(t, q, com.w, com.x - c.x, com.y - c.y, com.z - c.z);
+        quad_shift_add(t, oq, ocom.w, ocom.x - c.x, ocom.y - c.y, ocom.z - c.z);
+        com = c;
+        q = t;
     }
-    lcp[k] = (uint8_t)L;
+}
+
+__device__ __forceinline__ float4 shfl_down4(float4 v, int o)
+{
+    return make_float4(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o),
+                       __shfl_down_sync(0xffffffffu, v.z, o),
+                       __shfl_down_sync(0xffffffffu, v.w, o));
+}
+
+// Sums of the next levels over the block's threads (thread t holds group
+// first + t of `level`, complete where first + t < groups(level)), by shuffles
+// within a warp and then over the warps' sums in shared memory; each complete
+// group is stored.
+template <bool kQuad>
+__device__ __forceinline__ void block_groups(const Segments &sg, int level, int first,
+                                             GroupSum g, float4 com, Quad6 q,
+                                             GroupSum *warp_sum, float4 *warp_com,
+                                             Quad6 *warp_quad)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto fold = [&](int at, int lanes) {  // `at`: this thread's group of `level`
+        for (int o = 1; o < lanes; o <<= 1) {
+            GroupSum p;
+            p.h = shfl_down4(g.h, o);
+            p.l = shfl_down4(g.l, o);
+            float4 pc = com;
+            Quad6 pq = q;
+            if (kQuad) {
+                pc = shfl_down4(com, o);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) pq.v[c] = __shfl_down_sync(0xffffffffu, q.v[c], o);
+            }
+            ++level;
+            at >>= 1;
+            if (lane < lanes && (lane & (2 * o - 1)) == 0) {
+                group_join<kQuad>(g, com, q, p, pc, pq);
+                if (level < kSegLevels && at < sg.groups(level)) {
+                    group_store(sg, sg.off[level] + at, g);
+                    if (kQuad) group_store_quad(sg, sg.off[level] + at, com, q);
+                }
+            }
+        }
+    };
+    fold(first + (int)threadIdx.x, 32);
+    if (lane == 0) {
+        warp_sum[warp] = g;
+        if (kQuad) {
+            warp_com[warp] = com;
+            warp_quad[warp] = q;
+        }
+    }
+    __syncthreads();
+    const int warps = (int)(blockDim.x >> 5);
+    if (warp == 0) {
+        const int w = lane < warps ? lane : 0;
+        g = warp_sum[w];
+        if (kQuad) {
+            com = warp_com[w];
+            q = warp_quad[w];
+        }
+        fold((first >> 5) + lane, warps);
+    }
+}
+
+// L(k) for k >= 1 (the number of leading digits keys[k-1] and keys[k] share,
+// D for equal keys), the sorted f32 bodies (with kExact what f32 dropped of
+// their f64 positions), and the group sums of up to kSegBlock bodies.  Four
+// bodies a thread: the keys and the order come as 16-byte words and a thread's
+// bodies are its first group.
+template <bool kQuad, bool kExact>
+__global__ void __launch_bounds__(kSegBlock / kSegBase)
+boundary_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ order, int n,
+                int nchild, const float4 *__restrict__ body4, const double *__restrict__ bx,
+                const double *__restrict__ by, const double *__restrict__ bz,
+                float4 *__restrict__ sbody, float4 *__restrict__ sbody_lo,
+                uint8_t *__restrict__ lcp, Segments sg, const uint32_t *__restrict__ flags)
+{
+    static_assert(kSegBase == 4, "a thread's bodies are one 16-byte word of the order");
+    if (sort_failed(flags)) return;
+    __shared__ GroupSum warp_sum[kSegBlock / kSegBase / 32];
+    __shared__ float4 warp_com[kSegBlock / kSegBase / 32];
+    __shared__ Quad6 warp_quad[kSegBlock / kSegBase / 32];
+    const int first = blockIdx.x * (kSegBlock / kSegBase);
+    const int g0 = first + (int)threadIdx.x;  // this thread's group
+    const int k0 = g0 * kSegBase;
+    const int D = tree_levels(nchild), B = level_bits(nchild);
+    const int cnt = max(0, min(kSegBase, n - k0));
+    uint64_t key[kSegBase] = {0, 0, 0, 0};
+    uint32_t ord[kSegBase] = {0, 0, 0, 0};
+    if (cnt == kSegBase) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(keys + k0);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(keys + k0 + 2);
+        const uint4 o = *reinterpret_cast<const uint4 *>(order + k0);
+        key[0] = a.x;
+        key[1] = a.y;
+        key[2] = b.x;
+        key[3] = b.y;
+        ord[0] = o.x;
+        ord[1] = o.y;
+        ord[2] = o.z;
+        ord[3] = o.w;
+    } else {
+#pragma unroll
+        for (int u = 0; u < kSegBase; ++u)
+            if (u < cnt) {
+                key[u] = keys[k0 + u];
+                ord[u] = order[k0 + u];
+            }
+    }
+    uint64_t prev = k0 > 0 && cnt > 0 ? keys[k0 - 1] : 0ull;
+    float4 p[kSegBase];
+#pragma unroll
+    for (int u = 0; u < kSegBase; ++u)
+        p[u] = u < cnt ? body4[ord[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+    GroupSum g = group_zero();
+#pragma unroll
+    for (int u = 0; u < kSegBase; ++u) {
+        if (u >= cnt) continue;
+        const uint64_t x = prev ^ key[u];
+        prev = key[u];
+        // keys use the low B * D bits: 64 - B * D leading bits are always 0
+        const int L = x == 0 ? D : (__clzll((long long)x) - (64 - B * D)) / B;
+        lcp[k0 + u] = (uint8_t)(k0 + u == 0 ? 0 : L);
+        sbody[k0 + u] = p[u];
+        if (kExact) {
+            const uint32_t i = ord[u];
+            sbody_lo[k0 + u] = make_float4((float)(bx[i] - (double)p[u].x),
+                                           (float)(by[i] - (double)p[u].y),
+                                           (float)(bz[i] - (double)p[u].z), 0.f);
+        }
+        df_add_body(g, p[u]);
+    }
+    float4 com = p[0];
+    Quad6 q = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+    if (kQuad) {
+        com = df_com(g.h, g.l, p[0]);
+#pragma unroll
+        for (int u = 0; u < kSegBase; ++u)
+            if (u < cnt) quad_body_add(q, p[u], com);
+    }
+    if (g0 < sg.groups(0)) {
+        group_store(sg, sg.off[0] + g0, g);
+        if (kQuad) group_store_quad(sg, sg.off[0] + g0, com, q);
+    }
+    block_groups<kQuad>(sg, 0, first, g, com, q, warp_sum, warp_com, warp_quad);
+}
+
+// The group sums of more than kSegBlock bodies, by one block of 1,024 threads
+// (ten levels per round).
+template <bool kQuad>
+__device__ __forceinline__ void top_groups(const Segments &sg)
+{
+    __shared__ GroupSum warp_sum[32];
+    __shared__ float4 warp_com[32];
+    __shared__ Quad6 warp_quad[32];
+    for (int level = kSegBlockLevel; level < kSegLevels && sg.groups(level) > 1; level += 10) {
+        const int m = sg.groups(level);
+        for (int first = 0; first < m; first += 1024) {
+            const int at = first + (int)threadIdx.x;
+            GroupSum g = group_zero();
+            float4 com = make_float4(0.f, 0.f, 0.f, 0.f);
+            Quad6 q = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+            if (at < m) {
+                g.h = __ldcg(&sg.hi[sg.off[level] + at]);
+                g.l = __ldcg(&sg.lo[sg.off[level] + at]);
+                if (kQuad) {
+                    com = __ldcg(&sg.com[sg.off[level] + at]);
+                    const float4 a = __ldcg(&sg.qa[sg.off[level] + at]);
+                    const float4 b = __ldcg(&sg.qb[sg.off[level] + at]);
+                    q = {{a.x, a.y, a.z, b.x, b.y, b.z}};
+                }
+            }
+            block_groups<kQuad>(sg, level, first, g, com, q, warp_sum, warp_com, warp_quad);
+            __syncthreads();  // the warps' sums serve the next chunk, the groups the next round
+        }
+    }
 }
 
 // First index j in [lo, n) with keys[j] != keys[i] (keys sorted), or n.
@@ -1039,8 +1342,7 @@ __device__ __forceinline__ int next_key_change(const uint64_t *__restrict__ keys
 // Level masks of the bodies (bit l: a node at level l starts at this body),
 // per-block counts of every level (blk_cnt[l * nblk + block]) and the body
 // count of the leaf starting at each body (the deepest run it starts; 0: no
-// node starts here, kLongLeaf: longer than the shared tile reaches); also
-// zeroes the child counters.  The questions about L near a body (the minimum
+// node starts here, kLongLeaf: longer than the shared tile reaches).  The questions about L near a body (the minimum
 // over the next `leaf` boundaries; how many consecutive boundaries either side,
 // or after the body, are at or below a level) are answered from tables of
 // window minima over 1, 2, 4, ..., 64 boundaries of the block's tile: the
@@ -1056,16 +1358,13 @@ static_assert(kMaxLeaf <= (1 << (kMinTables - 1)) && kMaxLeaf + 1 < kTreeHalo,
 __global__ void __launch_bounds__(kTreeBlock)
 mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, int n,
             int nchild, int leaf, uint32_t *__restrict__ mask, uint32_t *__restrict__ blk_cnt,
-            int nblk, uint8_t *__restrict__ leafcnt, uint32_t *__restrict__ nchild32, int cap,
-            const uint32_t *__restrict__ flags)
+            int nblk, uint8_t *__restrict__ leafcnt, const uint32_t *__restrict__ flags)
 {
     if (sort_failed(flags)) return;
     // sM[p][t]: minimum of L over boundaries t .. t + 2^p - 1 of the tile
     // (clipped at the tile's end; every query below stays inside it)
     __shared__ int8_t sM[kMinTables][kTreeTile];
     __shared__ uint32_t cnt[32];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cap; k += gridDim.x * blockDim.x)
-        nchild32[k] = 0u;
     const int D = tree_levels(nchild);
     const int base = blockIdx.x * kTreeBlock;
     // boundaries base - halo .. base + block + halo; -1 marks "no boundary
@@ -1159,17 +1458,25 @@ mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, 
     if (threadIdx.x < 32) blk_cnt[(size_t)threadIdx.x * nblk + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// One block: per level, the exclusive scan of the block counts (blk_off,
-// same layout as blk_cnt) and the level's first node.  Warp l scans row l,
+// Block 0: per level, the exclusive scan of the block counts (blk_off,
+// same layout as blk_cnt) and the level's first node; block 1: the group sums
+// of over kSegBlock bodies.  Warp l scans row l,
 // 32 blocks per step.  If the nodes do not fit the node arrays, the tree
 // stops at the deepest level that fits (its nodes become leaves: results
 // stay exact, slower) and flags[kFlagNodes] is raised.
 __global__ void __launch_bounds__(1024)
 level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
                   uint32_t *__restrict__ blk_off, LevelInfo *lv, int cap,
-                  uint32_t *__restrict__ flags)
+                  uint32_t *__restrict__ flags, Segments sg, int quad)
 {
     if (sort_failed(flags)) return;
+    if (blockIdx.x == 1) {
+        if (quad)
+            top_groups<true>(sg);
+        else
+            top_groups<false>(sg);
+        return;
+    }
     __shared__ uint32_t total_of[32];
     const int D = tree_levels(nchild);
     const int l = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1224,13 +1531,12 @@ level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
 
 // Node records: per body, one node per set bit of its mask.  Leaves get
 // their body count here; an internal node's count, its child count and its
-// traversal metadata are completed by the moment pass (children counted into
-// nchild32 here); the centres by centre_kernel.
+// traversal metadata, and every node's geometry and moments, are cell_kernel's.
 __global__ void __launch_bounds__(kTreeBlock)
 node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafcnt,
             const uint32_t *__restrict__ mask, const uint32_t *__restrict__ blk_off, int nblk,
             int n, int nchild, NodeArrays nd, const LevelInfo *__restrict__ lv,
-            uint32_t *__restrict__ nchild32, const uint32_t *__restrict__ flags)
+            const uint32_t *__restrict__ flags)
 {
     if (sort_failed(flags)) return;
     __shared__ uint32_t sbal[kTreeBlock / 32][32];  // per warp and level: lanes with that bit
@@ -1269,7 +1575,6 @@ node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafc
         if (l > 0) {
             // the last node of level l - 1 starting at or before body i
             parent = lbeg[l - 1] + (int)woff[warp][l - 1] + __popc(sbal[warp][l - 1] & le) - 1;
-            atomicAdd(&nchild32[parent], 1u);
         }
         const bool splits = l + 1 <= max_level && ((m >> (l + 1)) & 1u);
         const int first_child =
@@ -1303,15 +1608,6 @@ node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafc
     }
 }
 
-// Geometric centres and half-widths of the nodes.  For the exact traversal
-// (exact != 0) the f64 centres follow the reference's arithmetic from the
-// root down (child = parent +- half-width / 2 per level, octree.rs:167-215,
-// quadtree.rs:167-194; the traversal re-decides near-threshold openings with
-// them): thread x follows the digits of its node's first key.  The warp
-// traversal needs only the f32 geometry: X (2q + 1 - 2^l) / 2^l from the
-// cell index q, one f64 product per axis rounded to f32 (within an f32 ulp
-// of the f64 chain's value; the traversal's margins allow 3).  Node-parallel,
-// so consecutive threads hold nodes of one level (equal chain lengths).
 __device__ __forceinline__ uint32_t compact3(uint64_t x)
 {
     x &= 0x1249249249249249ull;
@@ -1334,196 +1630,199 @@ __device__ __forceinline__ uint32_t compact2(uint64_t x)
     return (uint32_t)x;
 }
 
-__global__ void centre_kernel(const uint64_t *__restrict__ keys, NodeArrays nd,
-                              const LevelInfo *__restrict__ lv, int nchild, int exact,
-                              const unsigned long long *__restrict__ extent_bits,
-                              const uint32_t *__restrict__ flags)
+// ---------------------------------------------------------------------------
+// 5. cells: geometry, counts, mass, centre of mass and (optionally) second
+//    moments of every node, one thread per node, all nodes at once
+// ---------------------------------------------------------------------------
+// Nothing is passed up the tree: a node's bodies are the range [begin, end) of
+// the sorted order, and its sums are those of the O(log count) complete groups
+// (Segments) that tile the range, with up to three bodies at either end.  The
+// end of an internal node is its next sibling's begin, or its parent's end if it
+// is the last child.  A bottom-up pass (each parent finished by its last child
+// to arrive) took 37 us at 8,195 bodies, 45 at 1,048,580 (leaf 16) and 124 at
+// 250,007 with one body per leaf: three dependent round trips to L2 per level of
+// the tree, whatever the size, after a centre pass of 6, 12 and 70 (the f64
+// chain of every centre).  This takes 14, 23 and 24 for both, and the group
+// sums add 1, 3 and 5 to the boundary pass.
+//
+// Each product m x is taken exactly (TwoProduct by FMA) and summed as
+// double-float (hi + lo f32) pairs -- FP32 arithmetic only, as GB300 issues f64
+// instructions at a small fraction of its f32 rate.  The f32 centre of mass
+// c = S / M is the double-float quotient rounded once.  A leaf whose bodies all
+// sit at one position keeps that exact position, so a body there cancels
+// against it as the reference's equal-centre skip does; a massless cell sits at
+// its geometric centre.  Second moments (kQuad) are f32, combined with the
+// parallel-axis rule S = sum [S_g + M_g (c_g - c)(c_g - c)^T] over the groups.
+//
+// Geometry: X (2q + 1 - 2^l) / 2^l from the cell index q, one f64 product per
+// axis rounded to f32 (geo), and for the exact traversal (kExact) what that
+// rounding dropped (geo_lo), within 2^-48 X of the reference's f64 centre; the
+// traversal replays the reference's own centre arithmetic (cell_centre) only
+// for the openings those bounds leave open.
+
+// The reference's f64 centre and half-width of the level-l cell with key `key`
+// (child = parent +- half-width / 2 per level, octree.rs:167-215,
+// quadtree.rs:167-194).
+__device__ __forceinline__ void cell_centre(uint64_t key, int l, int nchild, double X, double &cx,
+                                            double &cy, double &cz, double &ext)
+{
+    const int D = tree_levels(nchild), B = level_bits(nchild);
+    const uint32_t dmask = (uint32_t)nchild - 1u;
+    cx = cy = cz = 0.0;
+    ext = X;
+    for (int j = 1; j <= l; ++j) {
+        const uint32_t q = (uint32_t)(key >> (B * (D - j))) & dmask;
+        const double h = __dmul_rn(ext, 0.5);  // ext / 2, exact
+        cx = (q & 1) ? __dadd_rn(cx, h) : __dsub_rn(cx, h);
+        cy = (q & 2) ? __dadd_rn(cy, h) : __dsub_rn(cy, h);
+        if (nchild == 8) cz = (q & 4) ? __dadd_rn(cz, h) : __dsub_rn(cz, h);
+        ext = h;
+    }
+}
+
+// The centres of a tree snapshot: planes cx, cy, cz, half-width of m entries.
+__global__ void snapshot_centre_kernel(const uint64_t *__restrict__ keys, NodeArrays nd, int m,
+                                       int nchild,
+                                       const unsigned long long *__restrict__ extent_bits,
+                                       double *__restrict__ out)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= m) return;
+    double c[4];
+    cell_centre(keys[nd.begin[x]], nd.level[x], nchild,
+                __longlong_as_double((long long)*extent_bits), c[0], c[1], c[2], c[3]);
+    for (int p = 0; p < 4; ++p) out[(size_t)p * m + x] = c[p];
+}
+
+// Calls body(p) for the bodies of [b, e) outside complete groups and
+// group(a, left, z, right) for the groups, each once; loads go out together,
+// three bodies or two groups at a time.
+template <typename Body, typename Group>
+__device__ __forceinline__ void range_pieces(const Segments &sg, const float4 *__restrict__ sbody,
+                                             int b, int e, Body body, Group group)
+{
+    auto bodies = [&](int from, int to) {
+        for (int j = from; j < to; j += 3) {
+            float4 p[3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) p[u] = sbody[min(j + u, to - 1)];
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+                if (j + u < to) body(p[u]);
+        }
+    };
+    int lo = (b + kSegBase - 1) / kSegBase, hi = e / kSegBase;
+    bodies(b, lo < hi ? lo * kSegBase : e);
+    if (lo >= hi) return;
+    bodies(hi * kSegBase, e);
+    for (int k = 0; lo < hi; ++k, lo >>= 1, hi >>= 1) {
+        const bool left = lo & 1, right = hi & 1;
+        group(sg.off[k] + lo, left, sg.off[k] + hi - 1, right);
+        lo += left;
+        hi -= right;
+    }
+}
+
+template <bool kQuad, bool kExact>
+__global__ void __launch_bounds__(256)
+cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody, NodeArrays nd,
+            const LevelInfo *__restrict__ lv, int nchild, Segments sg,
+            const unsigned long long *__restrict__ extent_bits,
+            const uint32_t *__restrict__ flags)
 {
     if (sort_failed(flags)) return;
     const int total = lv->total;
     const int D = tree_levels(nchild), B = level_bits(nchild);
-    const uint32_t dmask = (uint32_t)nchild - 1u;
     const double X = __longlong_as_double((long long)*extent_bits);
-    const size_t cap = nd.cap;
     for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += gridDim.x * blockDim.x) {
-        const int l = nd.level[x];
-        const uint64_t key = keys[nd.begin[x]];
-        if (exact) {
-            double cx = 0.0, cy = 0.0, cz = 0.0, ext = X;
-            for (int j = 1; j <= l; ++j) {
-                const uint32_t q = (uint32_t)(key >> (B * (D - j))) & dmask;
-                const double h = __dmul_rn(ext, 0.5);  // ext / 2, exact
-                cx = (q & 1) ? __dadd_rn(cx, h) : __dsub_rn(cx, h);
-                cy = (q & 2) ? __dadd_rn(cy, h) : __dsub_rn(cy, h);
-                if (nchild == 8) cz = (q & 4) ? __dadd_rn(cz, h) : __dsub_rn(cz, h);
-                ext = h;
-            }
-            nd.c64[x] = cx;
-            nd.c64[cap + x] = cy;
-            nd.c64[2 * cap + x] = cz;
-            nd.c64[3 * cap + x] = ext;
-            nd.geo[x] = make_float4((float)cx, (float)cy, (float)cz, (float)ext);
+        const int l = nd.level[x], b = nd.begin[x], fc = nd.child[x];
+        const uint64_t key = keys[b];
+        int e;
+        if (fc < 0) {
+            e = b + nd.count[x];
         } else {
-            const uint64_t pre = l == 0 ? 0ull : key >> (B * (D - l));
-            const double h = X * pow2d(-l);  // the half-width, exact
-            const long long span = 1ll << l;
-            const uint32_t qx = nchild == 8 ? compact3(pre) : compact2(pre);
-            const uint32_t qy = nchild == 8 ? compact3(pre >> 1) : compact2(pre >> 1);
-            const float gx = (float)(h * (double)(2ll * qx + 1 - span));
-            const float gy = (float)(h * (double)(2ll * qy + 1 - span));
-            const float gz =
-                nchild == 8 ? (float)(h * (double)(2ll * compact3(pre >> 2) + 1 - span)) : 0.f;
-            nd.geo[x] = make_float4(gx, gy, gz, (float)h);
+            // siblings are consecutive: the next sibling's begin, or the parent's end
+            int s = x, par = nd.parent[x];
+            for (;;) {
+                if (par < 0) {
+                    e = sg.n;
+                    break;
+                }
+                if (s + 1 < total && nd.parent[s + 1] == par) {
+                    e = nd.begin[s + 1];
+                    break;
+                }
+                s = par;
+                par = nd.parent[s];
+            }
+            int nc = 1;  // the nodes from fc on whose parent this is
+#pragma unroll
+            for (int k = 1; k < 8; ++k)
+                nc += k < nchild && fc + k < total && nd.parent[fc + k] == x;
+            nd.count[x] = e - b;
+            nd.nchild[x] = (uint8_t)nc;
+            nd.meta[x] = make_int4(x | (nc << 28), fc, b, e - b);
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// 5. moments: mass, centre of mass and (optionally) second moments of every
-//    cell, bottom up in one launch
-// ---------------------------------------------------------------------------
-// Each leaf sums its own bodies: mass and mass-weighted positions as
-// double-float (hi + lo f32) pairs, each product m x taken exactly (TwoProduct
-// by FMA) -- FP32 arithmetic only, as GB300 issues f64 instructions at a small
-// fraction of its f32 rate.  A parent is finished by the thread of its last
-// child to arrive (an acquire-release count of arrivals; nothing waits),
-// which adds the children's pairs in child order -- so results do not depend
-// on the arrival order -- and continues upwards; it also completes the
-// parent's body count, child count and traversal metadata.  The f32 centre
-// of mass c = S / M is the double-float quotient rounded once.  A leaf whose
-// bodies all sit at one position keeps that exact position, so a body there
-// cancels against it as the reference's equal-centre skip does; a massless
-// cell sits at its geometric centre.  Second moments (quad) are f32,
-// combined with the parallel-axis rule S = sum_c [S_c + M_c (c_c - c)(c_c - c)^T].
-__device__ __forceinline__ void store_quad(const NodeArrays &nd, int i, const float s[6])
-{
-    nd.quad_a[i] = make_float4(s[0], s[1], s[2], s[0] + s[1] + s[2]);
-    nd.quad_b[i] = make_float4(s[3], s[4], s[5], 0.f);
-}
-
-// (ah, al) + (bh, bl) as a normalised double-float pair.
-__device__ __forceinline__ void df_add(float &ah, float &al, float bh, float bl)
-{
-    float s, e;
-    two_sum(ah, bh, s, e);
-    e += al + bl;
-    ah = s + e;
-    al = e - (ah - s);
-}
-
-// f32 rounding of (sh + sl) / (mh + ml): an f32 quotient corrected once with
-// its exact residual (TwoProduct by FMA).
-__device__ __forceinline__ float df_div(float sh, float sl, float mh, float ml)
-{
-    const float q = sh / mh;
-    const float p = q * mh;
-    const float pe = fmaf(q, mh, -p);
-    const float r = fmaf(-q, ml, ((sh - p) - pe) + sl);
-    return q + r / mh;
-}
-
-__device__ __forceinline__ float4 df_com(const float4 h, const float4 l, float4 geo)
-{
-    if (h.x == 0.f && l.x == 0.f) return make_float4(geo.x, geo.y, geo.z, 0.f);
-    return make_float4(df_div(h.y, l.y, h.x, l.x), df_div(h.z, l.z, h.x, l.x),
-                       df_div(h.w, l.w, h.x, l.x), h.x + l.x);
-}
-
-// m * p added exactly-rounded into the double-float (hi, lo)
-__device__ __forceinline__ void df_add_prod(float &hi, float &lo, float m, float p)
-{
-    const float pr = m * p;
-    const float pe = fmaf(m, p, -pr);
-    df_add(hi, lo, pr, pe);
-}
-
-__global__ void moments_kernel(NodeArrays nd, const LevelInfo *__restrict__ lv,
-                               const float4 *__restrict__ sbody, int quad,
-                               const uint32_t *__restrict__ nchild32,
-                               const uint32_t *__restrict__ flags)
-{
-    if (sort_failed(flags)) return;
-    const int total = lv->total;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        if (nd.child[i] >= 0) continue;
-        const int b = nd.begin[i], e = b + nd.count[i];
+        // geometry
+        const uint64_t pre = l == 0 ? 0ull : key >> (B * (D - l));
+        const double h = X * pow2d(-l);  // the half-width, exact
+        const long long span = 1ll << l;
+        const uint32_t qx = nchild == 8 ? compact3(pre) : compact2(pre);
+        const uint32_t qy = nchild == 8 ? compact3(pre >> 1) : compact2(pre >> 1);
+        const double dx = h * (double)(2ll * qx + 1 - span);
+        const double dy = h * (double)(2ll * qy + 1 - span);
+        const double dz =
+            nchild == 8 ? h * (double)(2ll * compact3(pre >> 2) + 1 - span) : 0.0;
+        const float4 geo = make_float4((float)dx, (float)dy, (float)dz, (float)h);
+        nd.geo[x] = geo;
+        if (kExact)
+            nd.geo_lo[x] = make_float4((float)(dx - (double)geo.x), (float)(dy - (double)geo.y),
+                                       (float)(dz - (double)geo.z), 0.f);
+        // moments
+        GroupSum g = group_zero();
+        range_pieces(
+            sg, sbody, b, e, [&](float4 p) { df_add_body(g, p); },
+            [&](int a, bool left, int z, bool right) {
+                GroupSum p = group_zero(), r = p;
+                if (left) {
+                    p.h = sg.hi[a];
+                    p.l = sg.lo[a];
+                }
+                if (right) {
+                    r.h = sg.hi[z];
+                    r.l = sg.lo[z];
+                }
+                if (left) df_add4(g, p);
+                if (right) df_add4(g, r);
+            });
+        bool same = fc < 0;  // a leaf's bodies all at one position
         const float4 p0 = sbody[b];
-        float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-        bool same = true;
-        for (int j = b; j < e; ++j) {
+        for (int j = b + 1; same && j < e; ++j) {
             const float4 p = sbody[j];
-            df_add(h.x, l.x, p.w, 0.f);
-            df_add_prod(h.y, l.y, p.w, p.x);
-            df_add_prod(h.z, l.z, p.w, p.y);
-            df_add_prod(h.w, l.w, p.w, p.z);
-            same = same && p.x == p0.x && p.y == p0.y && p.z == p0.z;
+            same = p.x == p0.x && p.y == p0.y && p.z == p0.z;
         }
-        nd.msum_hi[i] = h;
-        nd.msum_lo[i] = l;
-        const float4 com = same ? make_float4(p0.x, p0.y, p0.z, h.x + l.x)
-                                : df_com(h, l, nd.geo[i]);
-        nd.com[i] = com;
-        if (quad) {
-            float q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const float4 com = same ? make_float4(p0.x, p0.y, p0.z, g.h.x + g.l.x)
+                                : df_com(g.h, g.l, geo);
+        nd.com[x] = com;
+        if (kQuad) {
+            Quad6 q = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
             if (!same)
-                for (int j = b; j < e; ++j) {
-                    const float4 p = sbody[j];
-                    const float dx = p.x - com.x, dy = p.y - com.y, dz = p.z - com.z;
-                    q[0] = fmaf(p.w * dx, dx, q[0]);
-                    q[1] = fmaf(p.w * dy, dy, q[1]);
-                    q[2] = fmaf(p.w * dz, dz, q[2]);
-                    q[3] = fmaf(p.w * dx, dy, q[3]);
-                    q[4] = fmaf(p.w * dx, dz, q[4]);
-                    q[5] = fmaf(p.w * dy, dz, q[5]);
-                }
-            store_quad(nd, i, q);
-        }
-        int node = i;
-        for (;;) {
-            const int par = nd.parent[node];
-            if (par < 0) break;
-            const int nc = (int)nchild32[par];
-            // release: this child's sums are visible before its arrival
-            // counts; acquire: the last arriver sees every sibling's
-            cuda::atomic_ref<uint32_t, cuda::thread_scope_device> arrivals(nd.arrivals[par]);
-            const uint32_t arrived = arrivals.fetch_add(1u, cuda::memory_order_acq_rel);
-            if (arrived + 1u != (uint32_t)nc) break;
-            nd.arrivals[par] = 0u;  // ready for the next build
-            const int fc = nd.child[par];
-            float4 ph = __ldcg(&nd.msum_hi[fc]), pl = __ldcg(&nd.msum_lo[fc]);
-            int count = __ldcg(&nd.count[fc]);
-            for (int k = fc + 1; k < fc + nc; ++k) {
-                const float4 ch = __ldcg(&nd.msum_hi[k]), cl = __ldcg(&nd.msum_lo[k]);
-                df_add(ph.x, pl.x, ch.x, cl.x);
-                df_add(ph.y, pl.y, ch.y, cl.y);
-                df_add(ph.z, pl.z, ch.z, cl.z);
-                df_add(ph.w, pl.w, ch.w, cl.w);
-                count += __ldcg(&nd.count[k]);
-            }
-            nd.msum_hi[par] = ph;
-            nd.msum_lo[par] = pl;
-            nd.count[par] = count;
-            nd.nchild[par] = (uint8_t)nc;
-            nd.meta[par] = make_int4(par | (nc << 28), fc, nd.begin[par], count);
-            const float4 cp = df_com(ph, pl, nd.geo[par]);
-            nd.com[par] = cp;
-            if (quad) {
-                float t[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                for (int k = fc; k < fc + nc; ++k) {
-                    const float4 cc = __ldcg(&nd.com[k]);
-                    const float4 qa = __ldcg(&nd.quad_a[k]);
-                    const float4 qb = __ldcg(&nd.quad_b[k]);
-                    const float dx = cc.x - cp.x, dy = cc.y - cp.y, dz = cc.z - cp.z;
-                    t[0] += fmaf(cc.w * dx, dx, qa.x);
-                    t[1] += fmaf(cc.w * dy, dy, qa.y);
-                    t[2] += fmaf(cc.w * dz, dz, qa.z);
-                    t[3] += fmaf(cc.w * dx, dy, qb.x);
-                    t[4] += fmaf(cc.w * dx, dz, qb.y);
-                    t[5] += fmaf(cc.w * dy, dz, qb.z);
-                }
-                store_quad(nd, par, t);
-            }
-            node = par;
+                range_pieces(
+                    sg, sbody, b, e, [&](float4 p) { quad_body_add(q, p, com); },
+                    [&](int a, bool left, int z, bool right) {
+                        if (left) {
+                            const float4 c = sg.com[a];
+                            quad_shift_add(q, quad_load(sg, a), c.w, c.x - com.x, c.y - com.y,
+                                           c.z - com.z);
+                        }
+                        if (right) {
+                            const float4 c = sg.com[z];
+                            quad_shift_add(q, quad_load(sg, z), c.w, c.x - com.x, c.y - com.y,
+                                           c.z - com.z);
+                        }
+                    });
+            nd.quad_a[x] = make_float4(q.v[0], q.v[1], q.v[2], q.v[0] + q.v[1] + q.v[2]);
+            nd.quad_b[x] = make_float4(q.v[3], q.v[4], q.v[5], 0.f);
         }
     }
 }
@@ -1534,6 +1833,9 @@ __global__ void moments_kernel(NodeArrays nd, const LevelInfo *__restrict__ lv,
 struct TravArgs {
     NodeArrays nd;
     const float4 *sbody;
+    const float4 *sbody_lo;      // f64 positions less their f32 values (exact traversal)
+    const uint64_t *keys;
+    int nchild;
     const double *bx, *by, *bz;  // the f64 state, unsorted (body order[k] is sorted body k)
     const uint32_t *order;
     const LevelInfo *lv;
@@ -1586,30 +1888,39 @@ __device__ __forceinline__ float4 scaled2(float4 q, float f)
     return make_float4(q.x * f, q.y * f, q.z * f, q.w * f);
 }
 
-// The reference's opening rule `extent / r < theta` (octree.rs:137-144):
+// The reference's opening rule `extent / r < theta` (octree.rs:137-144) in
 // FP32, re-evaluated in f64 with the reference's arithmetic near the edge.
-__device__ __forceinline__ bool accept_cell(const TravArgs &a, int node, float4 geo, float qx,
-                                            float qy, float qz, int k)
+// ql / gl: what f32 dropped of the body's position and the cell's centre.
+__device__ __forceinline__ bool accept_cell(const TravArgs &a, int node, float4 geo, float4 gl,
+                                            float4 q, float4 ql, int k)
 {
-    const float dx = qx - geo.x, dy = qy - geo.y, dz = qz - geo.z;
+    const float dx = (q.x - geo.x) + (ql.x - gl.x);
+    const float dy = (q.y - geo.y) + (ql.y - gl.y);
+    const float dz = (q.z - geo.z) + (ql.z - gl.z);
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const float inv = rsqrt_approx(r2);
     const float ratio = geo.w * inv;
     // Bound on the relative error of `ratio` against the reference's f64
-    // value: rounding positions and centres (|.| <= X) to f32 perturbs each
-    // difference by <= 3 * 2^-24 * X, i.e. r by <= 3.1e-7 X; rsqrt.approx and
-    // the f32 extent add ~3e-7.  Decisions inside twice that band are redone
-    // in f64 with the reference's operations.
-    const float band = fabsf(a.theta) * (6.4e-7f * a.extent * inv + 1e-6f) + 1e-30f;
+    // value.  Each difference is the f64 one to a relative 3 * 2^-24 (the f32
+    // difference rounds once, the sum with the dropped parts once) and to an
+    // absolute 2^-45 X (the dropped parts round at 2^-24 of themselves, the
+    // centre is within 2^-48 X of the reference's); the squares, rsqrt.approx
+    // and the f32 extent add 4e-7.  Decisions inside twice that band are redone
+    // in f64 with the reference's operations.  (From f32 positions alone the
+    // band is 6.4e-7 X / r wide: at a cell of level 15 two percent of theta, so
+    // most warps had a lane that took the f64 branch.)
+    const float band = fabsf(a.theta) * (1e-13f * a.extent * inv + 1.5e-6f) + 1e-30f;
     if (fabsf(ratio - a.theta) > band && ratio == ratio && r2 > 1e-30f)
         return ratio < a.theta;
-    const size_t cap = a.nd.cap;
     const uint32_t i = a.order[k];
-    const double d0 = a.bx[i] - a.nd.c64[node];
-    const double d1 = a.by[i] - a.nd.c64[cap + node];
-    const double d2 = a.bz[i] - a.nd.c64[2 * cap + node];
+    double cx, cy, cz, ext;
+    cell_centre(a.keys[a.nd.begin[node]], a.nd.level[node], a.nchild,
+                __longlong_as_double((long long)*a.extent_bits), cx, cy, cz, ext);
+    const double d0 = a.bx[i] - cx;
+    const double d1 = a.by[i] - cy;
+    const double d2 = a.bz[i] - cz;
     const double r64 = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-    return a.nd.c64[3 * cap + node] / r64 < a.theta64;
+    return ext / r64 < a.theta64;
 }
 
 __device__ __forceinline__ void pair_acc(float qx, float qy, float qz, float4 b, float e,
@@ -1741,6 +2052,7 @@ traverse_exact_kernel(TravArgs a_in)
 {
     __shared__ StackEntry stack[kTravWarps][kStack];
     __shared__ float4 child_geo[kTravWarps][8];  // the children being tested
+    __shared__ float4 child_lo[kTravWarps][8];
     __shared__ int4 child_meta[kTravWarps][8];
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
@@ -1756,6 +2068,7 @@ traverse_exact_kernel(TravArgs a_in)
     const bool valid = k < a.n;
     const uint32_t active = __ballot_sync(0xffffffffu, valid);
     const float4 q = valid ? a.sbody[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 ql = valid ? a.sbody_lo[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 qs = scaled(q, a.sc, a.msc);
     float ax = 0.f, ay = 0.f, az = 0.f, hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
     int sp = 0;
@@ -1766,11 +2079,11 @@ traverse_exact_kernel(TravArgs a_in)
     // accepted lanes take the cell's monopole (and quadrupole); the lanes that
     // open a leaf take its bodies here; an internal cell opened by any lane
     // goes on the stack with those lanes, to have its children tested.
-    auto visit = [&](int node, uint32_t mask, float4 geo, int4 meta) {
+    auto visit = [&](int node, uint32_t mask, float4 geo, float4 gl, int4 meta) {
         const bool in = (mask >> lane) & 1u;
         bool acc = false;
         if (in) {
-            acc = accept_cell(a, node, geo, q.x, q.y, q.z, k);
+            acc = accept_cell(a, node, geo, gl, q, ql, k);
             if (acc && a.com_theta > 0.f) acc = com_guard(a, geo, a.nd.com[node], q.x, q.y, q.z);
         }
         const uint32_t open = mask & ~__ballot_sync(0xffffffffu, acc);
@@ -1807,7 +2120,7 @@ traverse_exact_kernel(TravArgs a_in)
             since_fold = 0;
         }
     };
-    visit(0, active, a.nd.geo[0], a.nd.meta[0]);
+    visit(0, active, a.nd.geo[0], a.nd.geo_lo[0], a.nd.meta[0]);
     while (sp > 0 && !overflow) {
         __syncwarp();
         const StackEntry top = stack[warp][sp - 1];
@@ -1818,13 +2131,14 @@ traverse_exact_kernel(TravArgs a_in)
         // the children's records, one lane each, loaded together
         if (lane < nc) {
             child_geo[warp][lane] = a.nd.geo[fc + lane];
+            child_lo[warp][lane] = a.nd.geo_lo[fc + lane];
             child_meta[warp][lane] = a.nd.meta[fc + lane];
         }
         __syncwarp();
         // last child first, as the reference pops them (octree.rs:152-154)
 #pragma unroll 1
         for (int c = nc - 1; c >= 0; --c)
-            visit(fc + c, top.mask, child_geo[warp][c], child_meta[warp][c]);
+            visit(fc + c, top.mask, child_geo[warp][c], child_lo[warp][c], child_meta[warp][c]);
     }
     if (overflow && lane == 0) atomicOr(&a.flags[kFlagStack], 1u);
     fold(hx, lx, ax);
@@ -2213,7 +2527,8 @@ struct BhWorkspace {
     uint8_t *leafcnt = nullptr;    // bodies of the leaf starting at each sorted body
     uint32_t *blk_cnt = nullptr;   // per level and tree block: nodes starting in it
     uint32_t *blk_off = nullptr;   // ... and the level's nodes before the block
-    uint32_t *nchild32 = nullptr;  // children of each node (counted by the node kernel)
+    float4 *sbody_lo = nullptr;    // what f32 dropped of the sorted positions
+    Segments sg = {};              // group sums (n and off are set per build)
     NodeArrays nd = {};
     LevelInfo *lv = nullptr;
     unsigned long long *extent_bits = nullptr;
@@ -2223,6 +2538,8 @@ struct BhWorkspace {
     // which key/val buffer holds the sorted result
     int sorted = 0;
     int leaf_min = 1;  // smallest leaf size the node capacity was sized for
+    int nchild = 8;     // of the last build
+    bool exact = false;
     // optional events around the traversal kernel (recorded into graphs too)
     bool profiling = false;
     cudaEvent_t trav_ev[2] = {nullptr, nullptr};
@@ -2233,11 +2550,12 @@ static void ws_release(BhWorkspace *ws)
     void *p[] = {ws->keys[0],     ws->keys[1],    ws->vals[0],    ws->vals[1],
                  ws->sort_meta,   ws->sort_status, ws->sbody,     ws->lcp,
                  ws->mask,        ws->leafcnt,    ws->blk_cnt,    ws->blk_off,
-                 ws->nchild32,    ws->nd.msum_hi, ws->nd.msum_lo, ws->nd.begin,
+                 ws->sbody_lo,    ws->sg.hi,      ws->sg.lo,      ws->nd.begin,
                  ws->nd.count,    ws->nd.child,   ws->nd.nchild,  ws->nd.level,
-                 ws->nd.c64,      ws->nd.geo,     ws->nd.com,     ws->lv,
+                 ws->nd.geo_lo,   ws->nd.geo,     ws->nd.com,     ws->lv,
                  ws->extent_bits, ws->flags,      ws->nd.meta,    ws->stats,
-                 ws->nd.parent,   ws->nd.quad_a,  ws->nd.quad_b,  ws->nd.arrivals,
+                 ws->nd.parent,   ws->nd.quad_a,  ws->nd.quad_b,  ws->sg.com,
+                 ws->sg.qa,       ws->sg.qb,
                  ws->tile_cnt,    ws->tile_grp,   ws->tree_bar,   ws->blockmax};
     for (void *q : p) dev_free(q, ws->stream);
 }
@@ -2308,22 +2626,25 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
     PG_WA(w->leafcnt, cap);
     PG_WA(w->blk_cnt, 32 * tree_blocks);
     PG_WA(w->blk_off, 32 * tree_blocks);
-    PG_WA(w->nchild32, ncap);
+    PG_WA(w->sbody_lo, cap);
+    const size_t groups = cap / 2 + kSegLevels;  // all levels of cap / 4, cap / 8, ...
+    PG_WA(w->sg.hi, groups);
+    PG_WA(w->sg.lo, groups);
+    PG_WA(w->sg.com, groups);
+    PG_WA(w->sg.qa, groups);
+    PG_WA(w->sg.qb, groups);
     PG_WA(w->nd.begin, ncap);
     PG_WA(w->nd.count, ncap);
     PG_WA(w->nd.child, ncap);
     PG_WA(w->nd.nchild, ncap);
     PG_WA(w->nd.level, ncap);
-    PG_WA(w->nd.c64, 4 * ncap);
+    PG_WA(w->nd.geo_lo, ncap);
     PG_WA(w->nd.geo, ncap);
     PG_WA(w->nd.com, ncap);
     PG_WA(w->nd.meta, ncap);
     PG_WA(w->nd.parent, ncap);
-    PG_WA(w->nd.msum_hi, ncap);
-    PG_WA(w->nd.msum_lo, ncap);
     PG_WA(w->nd.quad_a, ncap);
     PG_WA(w->nd.quad_b, ncap);
-    PG_WA(w->nd.arrivals, ncap);
     PG_WA(w->stats, 4);
     PG_WA(w->lv, 1);
     PG_WA(w->extent_bits, 1);
@@ -2332,7 +2653,6 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
     w->nd.cap = (int)ncap;
     if (rc == PHYSIM_OK &&
         (cudaMemsetAsync(w->flags, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
-         cudaMemsetAsync(w->nd.arrivals, 0, ncap * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->lv, 0, sizeof(LevelInfo), stream) != cudaSuccess ||
          cudaMemsetAsync(w->tree_bar, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->sort_meta, 0,
@@ -2520,31 +2840,40 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
         PG_TRY(launch_split_sort(ws, b, p, n, per_sm, sms, st, &cur, &launches));
     }
     ws->sorted = cur;
-    // the tree: boundaries (+ sorted f32 bodies), level masks, one scan, node
-    // records, centres, moments
-    boundary_kernel<<<cdiv(n, 256), 256, 0, st>>>(ws->keys[cur], ws->vals[cur], n, p.nchild,
-                                                  b.body4, ws->sbody, ws->lcp, ws->flags);
+    // the tree: boundaries, sorted bodies and group sums; level masks; one scan
+    // (and the top group sums); node records; cells
+    const uint64_t *keys = ws->keys[cur];
+    const bool quad = p.multipole == kMultipoleQuadrupole;
+    const bool exact = p.traversal == PHYSIM_TRAVERSAL_EXACT;
+    Segments &sg = ws->sg;
+    sg.n = n;
+    for (int k = 0, at = 0; k < kSegLevels; ++k) {
+        sg.off[k] = at;
+        at += sg.groups(k);
+    }
+    auto boundary = quad ? (exact ? boundary_kernel<true, true> : boundary_kernel<true, false>)
+                         : (exact ? boundary_kernel<false, true> : boundary_kernel<false, false>);
+    boundary<<<cdiv(n, kSegBlock), kSegBlock / kSegBase, 0, st>>>(
+        keys, ws->vals[cur], n, p.nchild, b.body4, b.x, b.y, b.z, ws->sbody, ws->sbody_lo, ws->lcp,
+        sg, ws->flags);
     const int tree_blocks = cdiv(n, kTreeBlock);
     PG_CHECK(p.leaf_size >= 1 && p.leaf_size <= kMaxLeaf, PHYSIM_ERR_ARGUMENT,
              "leaf size %d outside 1..%d", p.leaf_size, kMaxLeaf);
-    mask_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(ws->keys[cur], ws->lcp, n, p.nchild,
-                                                    p.leaf_size, ws->mask, ws->blk_cnt,
-                                                    tree_blocks, ws->leafcnt, ws->nchild32,
-                                                    ws->nd.cap, ws->flags);
-    level_scan_kernel<<<1, 1024, 0, st>>>(ws->blk_cnt, tree_blocks, p.nchild, ws->blk_off, ws->lv,
-                                          ws->nd.cap, ws->flags);
-    node_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(ws->keys[cur], ws->leafcnt, ws->mask,
-                                                    ws->blk_off, tree_blocks, n, p.nchild, ws->nd,
-                                                    ws->lv, ws->nchild32, ws->flags);
-    centre_kernel<<<sms * 8, 256, 0, st>>>(ws->keys[cur], ws->nd, ws->lv, p.nchild,
-                                           p.traversal == PHYSIM_TRAVERSAL_EXACT ? 1 : 0,
-                                           ws->extent_bits, ws->flags);
-    // one thread per node (the capacity bounds the count): a grid-stride loop
-    // would queue a second leaf's climb behind the first's on one thread
-    moments_kernel<<<cdiv(ws->nd.cap, 256), 256, 0, st>>>(
-        ws->nd, ws->lv, ws->sbody, p.multipole == kMultipoleQuadrupole ? 1 : 0, ws->nchild32,
-        ws->flags);
-    launches += 6;
+    mask_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(keys, ws->lcp, n, p.nchild, p.leaf_size,
+                                                    ws->mask, ws->blk_cnt, tree_blocks,
+                                                    ws->leafcnt, ws->flags);
+    level_scan_kernel<<<2, 1024, 0, st>>>(ws->blk_cnt, tree_blocks, p.nchild, ws->blk_off, ws->lv,
+                                          ws->nd.cap, ws->flags, sg, quad ? 1 : 0);
+    node_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(keys, ws->leafcnt, ws->mask, ws->blk_off,
+                                                    tree_blocks, n, p.nchild, ws->nd, ws->lv,
+                                                    ws->flags);
+    auto cells = quad ? (exact ? cell_kernel<true, true> : cell_kernel<true, false>)
+                      : (exact ? cell_kernel<false, true> : cell_kernel<false, false>);
+    cells<<<sms * 8, 256, 0, st>>>(keys, ws->sbody, ws->nd, ws->lv, p.nchild, sg, ws->extent_bits,
+                                   ws->flags);
+    launches += 5;
+    ws->nchild = p.nchild;
+    ws->exact = exact;
     PG_CUDA(cudaGetLastError());
     ws->launches = launches;
     return PHYSIM_OK;
@@ -2562,6 +2891,9 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
     TravArgs a;
     a.nd = ws->nd;
     a.sbody = ws->sbody;
+    a.sbody_lo = ws->sbody_lo;
+    a.keys = ws->keys[ws->sorted];
+    a.nchild = p.nchild;
     a.bx = b.x;
     a.by = b.y;
     a.bz = b.z;
@@ -2628,10 +2960,15 @@ int bh_snapshot(BhWorkspace *ws, size_t n, cudaStream_t st, PhysimTreeSnapshot *
     PG_TRY(cp(out->node_child, ws->nd.child, nn * sizeof(int32_t)));
     PG_TRY(cp(out->node_nchild, ws->nd.nchild, nn));
     PG_TRY(cp(out->node_level, ws->nd.level, nn));
-    if (out->node_centre)
-        for (int c = 0; c < 4; ++c)
-            PG_TRY(cp(out->node_centre + c * nn, ws->nd.c64 + (size_t)c * ws->nd.cap,
-                      nn * sizeof(double)));
+    if (out->node_centre && ws->exact && nn) {
+        double *c64 = nullptr;
+        PG_TRY(dev_alloc(c64, 4 * nn, st));
+        snapshot_centre_kernel<<<cdiv((long long)nn, 256), 256, 0, st>>>(
+            ws->keys[ws->sorted], ws->nd, (int)nn, ws->nchild, ws->extent_bits, c64);
+        const int rc = cp(out->node_centre, c64, 4 * nn * sizeof(double));
+        dev_free(c64, st);
+        PG_TRY(rc);
+    }
     PG_TRY(cp(out->node_com, ws->nd.com, nn * sizeof(float4)));
     if (out->node_quad) {
         PG_TRY(cp(out->node_quad, ws->nd.quad_a, nn * sizeof(float4)));
