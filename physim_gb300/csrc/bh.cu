@@ -2158,21 +2158,45 @@ traverse_exact_kernel(TravArgs a_in)
     }
 }
 
-// Warp traversal: the 32 bodies of a warp (consecutive in Morton order) walk
-// the tree together, and the lanes work on different cells.  Each iteration
-// takes up to 32 pending cells from the top of a shared stack, one per lane,
-// and tests each against the warp's bounding box: a cell is accepted when
+// Warp traversal: the 32 bodies of a group (consecutive in Morton order) walk
+// the tree together, and the lanes work on different cells.  Each round takes
+// pending cells from the top of a shared stack, one per lane, and tests each
+// against the group's bounding box: a cell is accepted when
 //     extent * (1 + 2e-6) < theta * (r_min - 6e-7 X),
-// r_min = distance from the cell centre to the box.  Every body of the warp
+// r_min = distance from the cell centre to the box.  Every body of the group
 // is at least r_min (less f32 rounding of positions and centres, <= 2.1e-7 X)
 // from the centre, so an accepted cell passes every body's own f64 reference
 // test extent / r < theta; cells that some body would open are opened.
 // Accepted cells and the bodies of opened leaves are queued (>= 0 body,
 // < 0 cell) and gathered 32 at a time into shared memory, where all lanes
 // evaluate them against their own body.
-constexpr int kGStack = 1024;                 // pending cells per warp
-constexpr int kGWide = kGStack - 256 - 8 * 22;  // above this, pop one cell at a time
-constexpr int kGQueue = 640;                  // queued interactions per warp
+//
+// A group is walked by a team of S warps: S x 32 lanes share the stack, the
+// queue and the rounds, and the queued tiles of 32 are dealt to the warps in
+// turn (so the sums do not depend on timing).  One warp per group is the least
+// work, but its walk is a chain of 15 to 60 rounds of L2 latency, 50 us at
+// 8,195 bodies and 540 at 100,003 with quadrupoles, with 2 to 20 warps an SM to
+// hide it; bh_team picks S.  A block is one team, so a warp's slot is free again
+// when its own walk ends (four groups to a block kept 22.8 of 28 warps running,
+// one 24.2).
+//
+// At 1,048,580 bodies and theta 0.5 the kernel is bound by instruction issue
+// (72%; FMA pipe 56%), half of it the walk's bookkeeping: 13 rounds and 334 cells
+// per group, 532 interactions per body.  397M -> 343M warp instructions and 472
+// -> 405 us came from testing squared distances, the sample bodies, the unrolled
+// pushes and four packed pairs in flight.
+constexpr int kTeamTake(int S) { return S == 1 ? 16 : 8; }  // bodies a lane queues at a time
+template <int S>
+struct TeamSize {
+    static constexpr int kLanes = 32 * S;                      // a block is a team
+    static constexpr int kStackCap = S == 1 ? 1024 : 512 * S;  // pending cells
+    // above this, pop one cell at a time (each level then adds at most 7)
+    static constexpr int kWide = kStackCap - 8 * kLanes - 8 * 22;
+    static constexpr int kFlush = S == 1 ? 256 : 128 * S;      // queued before evaluating
+    static constexpr int kQueue = S == 1 ? 640 : kFlush + kLanes * kTeamTake(S);
+    static_assert(kWide > 0, "a full round fits");
+};
+constexpr int kSamples = 4;  // bodies a rejected cell is tried against before all of them
 
 __device__ __forceinline__ int warp_exclusive_scan(int v, int lane, int &total)
 {
@@ -2188,24 +2212,52 @@ __device__ __forceinline__ int warp_exclusive_scan(int v, int lane, int &total)
 // kQuad: quadrupole corrections of accepted cells (the quadrupole tiles are
 // only sized in that instantiation, so the monopole kernel keeps its
 // registers and occupancy).
-template <bool kQuad>
-__global__ void __launch_bounds__(kTravWarps * 32)
+template <bool kQuad, int S>
+__global__ void __launch_bounds__(S * 32, kQuad || S > 1 ? 1 : 28)
 traverse_warp_kernel(TravArgs a_in)
 {
-    __shared__ int32_t gstack[kTravWarps][kGStack];
-    __shared__ int32_t queue[kTravWarps][kGQueue];
-    __shared__ float4 tile[kTravWarps][32];
-    __shared__ float4 tqa[kQuad ? kTravWarps : 1][32];
-    __shared__ float4 tqb[kQuad ? kTravWarps : 1][32];
+    using T = TeamSize<S>;
+    __shared__ int32_t stack[T::kStackCap];
+    __shared__ int32_t queue[T::kQueue];
+    __shared__ float4 tile[S][32];
+    __shared__ float4 tqa[kQuad ? S : 1][32];
+    __shared__ float4 tqb[kQuad ? S : 1][32];
+    __shared__ float4 sample_xy[kSamples / 2];  // negated (x, x', y, y')
+    __shared__ float2 sample_z[kSamples / 2];
+    __shared__ int warp_total[2][S];
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
     TravArgs a = a_in;
     a.extent = load_extent(a_in);
     set_pair_scale(a);
     const float sc = a.sc, msc = a.msc, sc2 = a.sc * a.sc * a.msc;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k0 = (blockIdx.x * kTravWarps + warp) * 32;
-    if (k0 >= a.n) return;
+    const int tw = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tl = threadIdx.x;  // lane within the team
+    const int k0 = blockIdx.x * 32;
+    auto team_sync = [&]() {
+        if (S == 1)
+            __syncwarp();
+        else
+            __syncthreads();
+    };
+    int scans = 0;
+    // exclusive scan over the team's lanes (S > 1: also a barrier of the team)
+    auto team_scan = [&](int v, int &total) {
+        int x = warp_exclusive_scan(v, lane, total);
+        if (S > 1) {
+            int *wt = warp_total[scans++ & 1];
+            if (lane == 0) wt[tw] = total;
+            __syncthreads();
+            total = 0;
+#pragma unroll
+            for (int w = 0; w < S; ++w) {
+                const int t = wt[w];
+                if (w < tw) x += t;
+                total += t;
+            }
+        }
+        return x;
+    };
     const int k = k0 + lane;
     const bool valid = k < a.n;
     const int nvalid = __popc(__ballot_sync(0xffffffffu, valid));
@@ -2220,49 +2272,76 @@ traverse_warp_kernel(TravArgs a_in)
         hi_z = fmaxf(hi_z, __shfl_xor_sync(0xffffffffu, hi_z, o));
     }
     // largest coordinate magnitude in the box: bounds the f32 rounding of the
-    // warp's positions
+    // group's positions
     const float bmax = fmaxf(fmaxf(fmaxf(fabsf(lo_x), fabsf(hi_x)), fmaxf(fabsf(lo_y), fabsf(hi_y))),
                              fmaxf(fabsf(lo_z), fabsf(hi_z)));
     const float pmax = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
     const float theta = a.theta;
+    const float need = (1.f + 2.8e-6f) / theta;
+    if (tw == 0) {
+        // four bodies spread over the group
+#pragma unroll
+        for (int u = 0; u < kSamples; ++u)
+            if (lane == u * 31 / (kSamples - 1)) {
+                float *xy = reinterpret_cast<float *>(&sample_xy[u >> 1]) + (u & 1);
+                xy[0] = -q.x;
+                xy[2] = -q.y;
+                reinterpret_cast<float *>(&sample_z[u >> 1])[u & 1] = -q.z;
+            }
+    }
     float ax = 0.f, ay = 0.f, az = 0.f, hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
     unsigned long long visits = 0, pairs = 0;
     int nq = 0;
     int sp = 1;
-    if (lane == 0) gstack[warp][0] = 0;
-    __syncwarp();
+    // The root is opened by every body when theta sqrt(3) < 1: no body is
+    // further than sqrt(3) X from its centre.
+    {
+        const int4 root = a.nd.meta[0];
+        if (root.y >= 0 && theta > 0.f && theta * 1.7320515f < 1.f) {
+            sp = (int)((uint32_t)root.x >> 28);
+            visits = 1;
+            if (tl < sp) stack[tl] = root.y + tl;
+        } else if (tl == 0) {
+            stack[0] = 0;
+        }
+    }
+    team_sync();
     // Bodies are queued from the front of the queue, accepted cells from the
     // back, so each is evaluated by its own loop: plain pairs for bodies,
     // pair + quadrupole (kQuad) for cells.
     int nc = 0;  // queued cells
     const float2 nqx = make_float2(-q.x * sc, -q.x * sc), nqy = make_float2(-q.y * sc, -q.y * sc);
     const float2 nqz = make_float2(-q.z * sc, -q.z * sc), e2 = make_float2(a.es, a.es);
-    // Evaluates `count` queued interactions whose (x, y, z, m) load(t) gives:
-    // entries 2k and 2k + 1 are staged interleaved as (x, x', y, y')(z, z', m, m'),
-    // so two 128-bit loads give the float2 operands of two interactions, which go
-    // through packed FADD2/FMUL2/FFMA2 (an odd count is padded with a massless
-    // entry, which adds exactly zero); the next tile is loaded while the current
-    // one is evaluated.
+    // Evaluates this warp's tiles of `count` queued interactions whose (x, y, z,
+    // m) load(t) gives: entries 2k and 2k + 1 are staged interleaved as (x, x',
+    // y, y')(z, z', m, m'), so two 128-bit loads give the float2 operands of two
+    // interactions, which go through packed FADD2/FMUL2/FFMA2 (a tile is padded
+    // to a multiple of eight with massless entries, which add exactly zero, so
+    // four pairs are in flight at a time); the next tile is loaded while the
+    // current one is evaluated.
     auto eval_packed = [&](int count, auto load) {
         float4 nb = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (lane < count) nb = load(lane);
-        for (int j0 = 0; j0 < count; j0 += 32) {
+        if (tw * 32 + lane < count) nb = load(tw * 32 + lane);
+        for (int j0 = tw * 32; j0 < count; j0 += T::kLanes) {
             const int m = min(32, count - j0);
             __syncwarp();
             const float4 bj = nb;
             nb = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j0 + 32 + lane < count) nb = load(j0 + 32 + lane);
-            float *pl = reinterpret_cast<float *>(&tile[warp][lane & ~1]) + (lane & 1);
+            if (j0 + T::kLanes + lane < count) nb = load(j0 + T::kLanes + lane);
+            float *pl = reinterpret_cast<float *>(&tile[tw][lane & ~1]) + (lane & 1);
             pl[0] = bj.x * sc;
             pl[2] = bj.y * sc;
             pl[4] = bj.z * sc;
             pl[6] = bj.w * msc;
             __syncwarp();
             float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
-            for (int jj = 0; jj < (m + 1) >> 1; ++jj) {
-                const float4 A = tile[warp][2 * jj], B = tile[warp][2 * jj + 1];
-                pair_acc2(nqx, nqy, nqz, make_float2(A.x, A.y), make_float2(A.z, A.w),
-                          make_float2(B.x, B.y), make_float2(B.z, B.w), e2, sx, sy, sz);
+            for (int jj = 0; jj < m; jj += 8) {
+#pragma unroll
+                for (int u = 0; u < 8; u += 2) {
+                    const float4 A = tile[tw][jj + u], B = tile[tw][jj + u + 1];
+                    pair_acc2(nqx, nqy, nqz, make_float2(A.x, A.y), make_float2(A.z, A.w),
+                              make_float2(B.x, B.y), make_float2(B.z, B.w), e2, sx, sy, sz);
+                }
             }
             ax += sx.x + sx.y;
             ay += sy.x + sy.y;
@@ -2270,37 +2349,38 @@ traverse_warp_kernel(TravArgs a_in)
         }
     };
     auto flush = [&]() {
+        team_sync();  // every lane's queue entries
         // leaf bodies, then accepted cells (monopoles packed like bodies;
         // with quadrupoles one cell per lane step)
-        eval_packed(nq, [&](int t) { return a.sbody[queue[warp][t]]; });
+        eval_packed(nq, [&](int t) { return a.sbody[queue[t]]; });
         if (!kQuad) {
-            eval_packed(nc, [&](int t) { return a.nd.com[-queue[warp][kGQueue - 1 - t] - 1]; });
+            eval_packed(nc, [&](int t) { return a.nd.com[-queue[T::kQueue - 1 - t] - 1]; });
         } else {
             // cells with quadrupoles, two per packed instruction: centre of
             // mass and both moment vectors staged interleaved like bodies
-            for (int j0 = 0; j0 < nc; j0 += 32) {
+            for (int j0 = tw * 32; j0 < nc; j0 += T::kLanes) {
                 const int m = min(32, nc - j0);
                 __syncwarp();
                 float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f), qa = c4, qb = c4;
                 if (lane < m) {
-                    const int c = -queue[warp][kGQueue - 1 - (j0 + lane)] - 1;
+                    const int c = -queue[T::kQueue - 1 - (j0 + lane)] - 1;
                     c4 = scaled(a.nd.com[c], sc, msc);
                     qa = scaled2(a.nd.quad_a[c], sc2);
                     qb = scaled2(a.nd.quad_b[c], sc2);
                 }
                 const int slot = lane & ~1, half = lane & 1;
-                float *pc = reinterpret_cast<float *>(&tile[warp][slot]) + half;
-                float *pa = reinterpret_cast<float *>(&tqa[warp][slot]) + half;
-                float *pb = reinterpret_cast<float *>(&tqb[warp][slot]) + half;
+                float *pc = reinterpret_cast<float *>(&tile[tw][slot]) + half;
+                float *pa = reinterpret_cast<float *>(&tqa[tw][slot]) + half;
+                float *pb = reinterpret_cast<float *>(&tqb[tw][slot]) + half;
                 pc[0] = c4.x; pc[2] = c4.y; pc[4] = c4.z; pc[6] = c4.w;
                 pa[0] = qa.x; pa[2] = qa.y; pa[4] = qa.z; pa[6] = qa.w;
                 pb[0] = qb.x; pb[2] = qb.y; pb[4] = qb.z; pb[6] = qb.w;
                 __syncwarp();
                 float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
                 for (int jj = 0; jj < (m + 1) >> 1; ++jj) {
-                    const float4 C0 = tile[warp][2 * jj], C1 = tile[warp][2 * jj + 1];
-                    const float4 A0 = tqa[warp][2 * jj], A1 = tqa[warp][2 * jj + 1];
-                    const float4 B0 = tqb[warp][2 * jj], B1 = tqb[warp][2 * jj + 1];
+                    const float4 C0 = tile[tw][2 * jj], C1 = tile[tw][2 * jj + 1];
+                    const float4 A0 = tqa[tw][2 * jj], A1 = tqa[tw][2 * jj + 1];
+                    const float4 B0 = tqb[tw][2 * jj], B1 = tqb[tw][2 * jj + 1];
                     cell_quad_acc2(nqx, nqy, nqz, make_float2(C0.x, C0.y), make_float2(C0.z, C0.w),
                                    make_float2(C1.x, C1.y), make_float2(C1.z, C1.w),
                                    make_float2(A0.x, A0.y), make_float2(A0.z, A0.w),
@@ -2319,31 +2399,31 @@ traverse_warp_kernel(TravArgs a_in)
         fold(hz, lz, az);
         nq = 0;
         nc = 0;
-        __syncwarp();
+        team_sync();  // the queue is free again
     };
     bool overflow = false;
     while (sp > 0) {
-        const int m = sp > kGWide ? 1 : min(32, sp);
+        const int m = sp > T::kWide ? 1 : min(T::kLanes, sp);
         int cell = 0;
-        if (lane < m) cell = gstack[warp][sp - m + lane];
-        __syncwarp();
+        if (tl < m) cell = stack[sp - m + tl];
+        if (S == 1) __syncwarp();  // (S > 1: the scan below is a barrier)
         sp -= m;
         visits += m;
         int qref = 0, qcnt = 0, nchild = 0, first_child = 0;
         float4 geo = make_float4(0.f, 0.f, 0.f, 0.f);
         bool acc = false, maybe = false;
-        if (lane < m) {
+        if (tl < m) {
             geo = a.nd.geo[cell];
             const int4 meta = a.nd.meta[cell];
             const float cmax = fmaxf(fmaxf(fabsf(geo.x), fabsf(geo.y)), fabsf(geo.z));
             const float dx = fmaxf(fmaxf(lo_x - geo.x, geo.x - hi_x), 0.f);
             const float dy = fmaxf(fmaxf(lo_y - geo.y, geo.y - hi_y), 0.f);
             const float dz = fmaxf(fmaxf(lo_z - geo.z, geo.z - hi_z), 0.f);
-            const float r = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
             // f32 rounding of positions and centre moves r by at most
-            // 1.1e-7 (|p| + |c|) + 3.5e-7 r against the reference's f64 value
-            const float rmin = r - (2e-7f * (bmax + cmax) + 5e-7f * r);
-            acc = theta > 0.f && rmin > 0.f && geo.w * (1.f + 2e-6f) < theta * rmin;
+            // 1.1e-7 (|p| + |c|) + 3.5e-7 r against the reference's f64 value:
+            // r - (2e-7 (bmax + cmax) + 5e-7 r) must exceed extent (1 + 2e-6) / theta
+            const float t = fmaf(geo.w, need, 2.000002e-7f * (bmax + cmax));
+            acc = theta > 0.f && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > t * t;
             if (acc && a.com_theta > 0.f) {
                 // centre-of-mass guard against the whole box (distance from c
                 // to the box is a lower bound of every body's |x - c|)
@@ -2370,7 +2450,23 @@ traverse_warp_kernel(TravArgs a_in)
             }
         }
         // Internal cells the box test rejects: accept them if every body of
-        // the warp passes its own test (with the same rounding margin).
+        // the group passes its own test (with the same rounding margin).  Most
+        // fail for some of four sample bodies, by more than the margin (r theta
+        // <= extent, f32 rounding under 2e-6), and are opened without asking
+        // the rest: of 60 such cells per group at theta 0.5, 1M bodies, 42 are
+        // opened, each asked of every body by four shuffles and a vote.
+        if (__any_sync(0xffffffffu, maybe)) {
+            const float t2 = theta * theta, w2 = geo.w * geo.w;
+#pragma unroll
+            for (int u = 0; u < kSamples / 2; ++u) {
+                const float4 xy = sample_xy[u];
+                const float2 dx = add2(make_float2(xy.x, xy.y), make_float2(geo.x, geo.x));
+                const float2 dy = add2(make_float2(xy.z, xy.w), make_float2(geo.y, geo.y));
+                const float2 dz = add2(sample_z[u], make_float2(geo.z, geo.z));
+                const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                maybe = maybe && !(t2 * r2.x <= w2) && !(t2 * r2.y <= w2);
+            }
+        }
         uint32_t pend = __ballot_sync(0xffffffffu, maybe);
         while (pend) {
             const int src = __ffs(pend) - 1;
@@ -2396,42 +2492,72 @@ traverse_warp_kernel(TravArgs a_in)
                 nchild = 0;
             }
         }
-        // push the children of opened cells
-        int ctotal;
-        const int coff = warp_exclusive_scan(nchild, lane, ctotal);
-        if (sp + ctotal > kGStack) {
+        // push the children of opened cells, queue the accepted ones (back)
+        const bool is_cell = qref < 0;
+        int total;
+        const int off = team_scan(nchild | (is_cell ? 1 << 16 : 0), total);
+        const int kids = total & 0xffff, cells = total >> 16;
+        if (sp + kids > T::kStackCap) {
             overflow = true;
             break;
         }
-        for (int c = 0; c < nchild; ++c) gstack[warp][sp + coff + c] = first_child + c;
-        sp += ctotal;
-        // queue leaf bodies (front) and cells (back), at most 16 entries per
-        // lane per round
-        while (__any_sync(0xffffffffu, qcnt > 0)) {
-            const int take = min(qcnt, 16);
-            const bool is_cell = qref < 0;
-            int btotal, ctotal;
-            const int boff = warp_exclusive_scan(is_cell ? 0 : take, lane, btotal);
-            const int coff = warp_exclusive_scan(is_cell ? take : 0, lane, ctotal);
-            if (nq + nc + btotal + ctotal > kGQueue) flush();
-            if (is_cell) {
-                if (take) queue[warp][kGQueue - 1 - (nc + coff)] = qref;
-            } else {
-                for (int j = 0; j < take; ++j) queue[warp][nq + boff + j] = qref + j;
-                qref += take;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if (c < nchild) stack[sp + (off & 0xffff) + c] = first_child + c;
+        sp += kids;
+        if (nq + nc + cells > T::kQueue) flush();
+        if (is_cell) {
+            queue[T::kQueue - 1 - (nc + (off >> 16))] = qref;
+            qcnt = 0;
+        }
+        nc += cells;
+        // queue leaf bodies (front), a bounded number per lane and turn
+        for (bool more = S > 1 || __any_sync(0xffffffffu, qcnt > 0); more;) {
+            const int take = min(qcnt, kTeamTake(S));
+            int btotal;
+            const int boff = team_scan(take | (qcnt > take ? 1 << 16 : 0), btotal) & 0xffff;
+            more = btotal >> 16;
+            btotal &= 0xffff;
+            if (nq + nc + btotal > T::kQueue) flush();
+            for (int j = 0; j < take; j += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (j + u < take) queue[nq + boff + j + u] = qref + j + u;
             }
+            qref += take;
             qcnt -= take;
             nq += btotal;
-            nc += ctotal;
         }
-        __syncwarp();
-        if (nq + nc >= 256) flush();
+        team_sync();  // the pushed cells
+        if (nq + nc >= T::kFlush) flush();
     }
     flush();
-    if (lane == 0) {
+    if (tl == 0) {
         if (overflow) atomicOr(&a.flags[kFlagStack], 1u);
         atomicAdd(&a.stats[0], visits);
         atomicAdd(&a.stats[1], pairs * (unsigned long long)nvalid);
+    }
+    if (S > 1) {
+        // the warps' sums, added in warp order (the stack is free: flush was a barrier)
+        float *part = reinterpret_cast<float *>(stack);
+        const float v[6] = {hx, hy, hz, lx, ly, lz};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) part[(tw * 6 + c) * 32 + lane] = v[c];
+        __syncthreads();
+        if (tw > 0) return;
+        for (int w = 1; w < S; ++w) {
+            const float *o = part + w * 6 * 32 + lane;
+            float s, err;
+            two_sum(hx, o[0], s, err);
+            hx = s;
+            lx += err + o[3 * 32];
+            two_sum(hy, o[32], s, err);
+            hy = s;
+            ly += err + o[4 * 32];
+            two_sum(hz, o[2 * 32], s, err);
+            hz = s;
+            lz += err + o[5 * 32];
+        }
     }
     if (valid) {
         const uint32_t i = a.order[k];
@@ -2566,10 +2692,14 @@ static int wsalloc(T *&p, size_t count, cudaStream_t st)
     return dev_alloc(p, count, st);
 }
 
-int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t stream)
+int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaStream_t stream)
 {
-    leaf = leaf < 1 ? 1 : leaf;
-    if (ws && n <= ws->cap_n && leaf >= ws->leaf_min) return PHYSIM_OK;
+    const int leaf = p.leaf_size < 1 ? 1 : p.leaf_size;
+    const bool quad = p.multipole == kMultipoleQuadrupole;
+    const bool exact = p.traversal != PHYSIM_TRAVERSAL_WARP;
+    if (ws && n <= ws->cap_n && leaf >= ws->leaf_min && (ws->nd.quad_a || !quad) &&
+        (ws->nd.geo_lo || !exact))
+        return PHYSIM_OK;
     if (ws) {
         ws_release(ws);
         delete ws;
@@ -2626,25 +2756,27 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, int leaf, cudaStream_t st
     PG_WA(w->leafcnt, cap);
     PG_WA(w->blk_cnt, 32 * tree_blocks);
     PG_WA(w->blk_off, 32 * tree_blocks);
-    PG_WA(w->sbody_lo, cap);
+    if (exact) PG_WA(w->sbody_lo, cap);
     const size_t groups = cap / 2 + kSegLevels;  // all levels of cap / 4, cap / 8, ...
     PG_WA(w->sg.hi, groups);
     PG_WA(w->sg.lo, groups);
-    PG_WA(w->sg.com, groups);
-    PG_WA(w->sg.qa, groups);
-    PG_WA(w->sg.qb, groups);
+    if (quad) {
+        PG_WA(w->sg.com, groups);
+        PG_WA(w->sg.qa, groups);
+        PG_WA(w->sg.qb, groups);
+        PG_WA(w->nd.quad_a, ncap);
+        PG_WA(w->nd.quad_b, ncap);
+    }
     PG_WA(w->nd.begin, ncap);
     PG_WA(w->nd.count, ncap);
     PG_WA(w->nd.child, ncap);
     PG_WA(w->nd.nchild, ncap);
     PG_WA(w->nd.level, ncap);
-    PG_WA(w->nd.geo_lo, ncap);
+    if (exact) PG_WA(w->nd.geo_lo, ncap);
     PG_WA(w->nd.geo, ncap);
     PG_WA(w->nd.com, ncap);
     PG_WA(w->nd.meta, ncap);
     PG_WA(w->nd.parent, ncap);
-    PG_WA(w->nd.quad_a, ncap);
-    PG_WA(w->nd.quad_b, ncap);
     PG_WA(w->stats, 4);
     PG_WA(w->lv, 1);
     PG_WA(w->extent_bits, 1);
@@ -2879,6 +3011,32 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
     return PHYSIM_OK;
 }
 
+// Warps per group of 32 bodies of the warp traversal.  A team of four shortens
+// each walk's chain of rounds but spends about 1.6 times the instructions, so it
+// pays while a walk is long (theta below 0.8, or the accuracy options) and the
+// groups are too few to hide it.  Step times, one warp vs four (us): theta 0.5,
+// Plummer, 8,195 bodies 116 vs 99, 20,011 127 vs 109, 50,021 141 vs 150; theta
+// 1.0, 20,011 bodies 87 vs 90; quadrupoles and com_theta 0.6, 20,011 bodies 291
+// vs 197, 100,003 673 vs 639, 300,007 1,538 vs 1,754.  (Teams of two and eight
+// were never the best by more than 1%.)
+static int bh_team(int n, const BhParams &p, int sms)
+{
+    const bool options = p.multipole == kMultipoleQuadrupole || p.com_theta > 0.0;
+    const long long groups_per_sm = cdiv(n, 32) / sms;
+    if (options) return groups_per_sm < 24 ? 4 : 1;
+    return p.theta < 0.8 && groups_per_sm < 8 ? 4 : 1;
+}
+
+template <bool kQuad>
+static void launch_traverse_warp(const TravArgs &a, int team, cudaStream_t st)
+{
+    const int groups = cdiv(a.n, 32);
+    if (team == 4)
+        traverse_warp_kernel<kQuad, 4><<<groups, 128, 0, st>>>(a);
+    else
+        traverse_warp_kernel<kQuad, 1><<<groups, 32, 0, st>>>(a);
+}
+
 int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, double *partial,
                      cudaStream_t st)
 {
@@ -2918,11 +3076,13 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
     // external records, so they also time the kernel when replayed from a graph
     if (ws->profiling)
         PG_CUDA(cudaEventRecordWithFlags(ws->trav_ev[0], st, cudaEventRecordExternal));
-    if (p.traversal == PHYSIM_TRAVERSAL_WARP && a.quad)
-        traverse_warp_kernel<true><<<blocks, kTravWarps * 32, 0, st>>>(a);
-    else if (p.traversal == PHYSIM_TRAVERSAL_WARP)
-        traverse_warp_kernel<false><<<blocks, kTravWarps * 32, 0, st>>>(a);
-    else
+    if (p.traversal == PHYSIM_TRAVERSAL_WARP) {
+        const int team = bh_team(n, p, device_sm_count(ws->device));
+        if (a.quad)
+            launch_traverse_warp<true>(a, team, st);
+        else
+            launch_traverse_warp<false>(a, team, st);
+    } else
         traverse_exact_kernel<<<blocks, kTravWarps * 32, 0, st>>>(a);
     PG_CUDA(cudaGetLastError());
     if (ws->profiling)
@@ -2970,7 +3130,7 @@ int bh_snapshot(BhWorkspace *ws, size_t n, cudaStream_t st, PhysimTreeSnapshot *
         PG_TRY(rc);
     }
     PG_TRY(cp(out->node_com, ws->nd.com, nn * sizeof(float4)));
-    if (out->node_quad) {
+    if (out->node_quad && ws->nd.quad_a) {
         PG_TRY(cp(out->node_quad, ws->nd.quad_a, nn * sizeof(float4)));
         PG_TRY(cp(out->node_quad + 4 * nn, ws->nd.quad_b, nn * sizeof(float4)));
     }

@@ -79,7 +79,6 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
                              el->partial, st));
     } else {
         PG_TRY(ensure_doubles(el->partial, el->partial_cap, 3 * n, st));
-        PG_TRY(bh_reserve(el->bh, n, el->device, el->leaf_size, st));
         BhParams p;
         p.nchild = el->kind == 1 ? 8 : 4;
         p.theta = el->theta;
@@ -88,6 +87,7 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
         p.traversal = el->traversal;
         p.multipole = el->multipole;
         p.com_theta = el->com_theta;
+        PG_TRY(bh_reserve(el->bh, n, el->device, p, st));
         PG_TRY(bh_accelerations(el->bh, el->bodies, p, el->partial, st));
     }
     PG_TRY(launch_accumulate_aos(el->bodies, el->partial, splits, acc_io, st));

@@ -73,15 +73,8 @@ namespace {
 
 using namespace pg;
 
-int sim_forces(PhysimSim *s, int *splits_out)
+BhParams bh_params(const PhysimSimConfig &c)
 {
-    const size_t n = s->n;
-    const PhysimSimConfig &c = s->cfg;
-    if (c.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO) {
-        *splits_out = s->plan.splits;
-        return launch_direct(s->plan, s->b.body4, (float)c.e, s->b.scale, s->partial, s->stream,
-                             s->profiling ? s->ev[3] : nullptr);
-    }
     BhParams p;
     p.nchild = c.gravity == PHYSIM_GRAVITY_ASTRO2 ? 8 : 4;
     p.theta = c.theta;
@@ -92,9 +85,19 @@ int sim_forces(PhysimSim *s, int *splits_out)
     p.multipole = c.multipole == PHYSIM_MULTIPOLE_QUADRUPOLE ? kMultipoleQuadrupole
                                                              : kMultipoleMonopole;
     p.com_theta = c.com_theta;
+    return p;
+}
+
+int sim_forces(PhysimSim *s, int *splits_out)
+{
+    const PhysimSimConfig &c = s->cfg;
+    if (c.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO) {
+        *splits_out = s->plan.splits;
+        return launch_direct(s->plan, s->b.body4, (float)c.e, s->b.scale, s->partial, s->stream,
+                             s->profiling ? s->ev[3] : nullptr);
+    }
     *splits_out = 1;
-    (void)n;
-    return bh_accelerations(s->bh, s->b, p, s->partial, s->stream);
+    return bh_accelerations(s->bh, s->b, bh_params(c), s->partial, s->stream);
 }
 
 // Captures the gravity phase into a graph.  If the stream cannot be captured
@@ -192,7 +195,7 @@ int physim_gpu_sim_create(const PhysimSimConfig *cfg, size_t n, PhysimSim **out)
         partial_elems = direct_partial_doubles(s->plan);
     }
     if (rc == PHYSIM_OK && cfg->gravity != PHYSIM_GRAVITY_SIMPLE_ASTRO)
-        rc = bh_reserve(s->bh, n, cfg->device, (int)cfg->leaf_size, s->stream);
+        rc = bh_reserve(s->bh, n, cfg->device, bh_params(*cfg), s->stream);
     if (rc == PHYSIM_OK) rc = dev_alloc(s->partial, partial_elems, s->stream);
     if (rc == PHYSIM_ERR_MEMORY && s->plan.symmetric) {
         // the symmetric plan's slot buffer did not fit: fall back to a one-pair plan
