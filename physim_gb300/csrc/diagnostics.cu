@@ -170,7 +170,7 @@ extern "C" int physim_gpu_energy_compute(PhysimEnergy *E, const Entity *state, s
     memset(out, 0, sizeof *out);
     if (n == 0) return PHYSIM_OK;
     PG_CUDA(cudaSetDevice(E->device));
-    PG_TRY(bodies_reserve(E->b, n, true, E->stream));
+    PG_TRY(bodies_reserve(E->b, n, true, false, E->stream));
     if (!E->d_out) PG_TRY(dev_alloc(E->d_out, 9, E->stream));
     PG_CUDA(cudaMemcpyAsync(E->b.aos, state, n * sizeof(Entity), cudaMemcpyHostToDevice,
                             E->stream));

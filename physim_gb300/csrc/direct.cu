@@ -34,81 +34,16 @@ namespace {
 template <int BLOCK, int IPT, bool COMP>
 __global__ void __launch_bounds__(BLOCK, 2)
 direct_forces_kernel(const float4 *__restrict__ body, int n, int n_jtiles, int chunk_tiles, float e,
-                     const PairScale *__restrict__ scale, double *__restrict__ partial)
+                     ScaleRef scale, double *__restrict__ partial)
 {
     __shared__ float4 tile[2][BLOCK][2];
     const int split = blockIdx.y;
     const int t0 = split * chunk_tiles;
     const int t1 = min(t0 + chunk_tiles, n_jtiles);
-    direct_tile<BLOCK, IPT, COMP>(body, n, blockIdx.x * BLOCK * IPT, t0, t1, e, scale->k,
-                                  scale->km, partial + (size_t)split * 3 * n, tile);
-}
-
-// Largest |coordinate| and |mass| of body4[0, n) (f32 bit patterns order
-// like the non-negative values; NaN and infinities skipped), reduced by the
-// last block to finish into ps->k and ps->km (see PairScale).
-__device__ __forceinline__ uint32_t finite_abs_bits(float v)
-{
-    const uint32_t b = __float_as_uint(v) & 0x7fffffffu;
-    return b < 0x7f800000u ? b : 0u;
-}
-
-__global__ void __launch_bounds__(256)
-pair_scale_kernel(const float4 *__restrict__ body, int n, float e, PairScale *ps)
-{
-    uint32_t m = 0, w = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 b = body[i];
-        m = max(m, max(finite_abs_bits(b.x), max(finite_abs_bits(b.y), finite_abs_bits(b.z))));
-        w = max(w, finite_abs_bits(b.w));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
-    }
-    __shared__ uint32_t wm[8], ww[8];
-    __shared__ bool last;
-    if ((threadIdx.x & 31) == 0) {
-        wm[threadIdx.x >> 5] = m;
-        ww[threadIdx.x >> 5] = w;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
-            m = max(m, wm[k]);
-            w = max(w, ww[k]);
-        }
-        ps->blockmax[blockIdx.x] = m;
-        ps->blockmass[blockIdx.x] = w;
-        __threadfence();
-        last = atomicAdd(&ps->arrivals, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    uint32_t t = 0, tw = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-        t = max(t, __ldcg(&ps->blockmax[b]));
-        tw = max(tw, __ldcg(&ps->blockmass[b]));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        t = max(t, __shfl_xor_sync(0xffffffffu, t, o));
-        tw = max(tw, __shfl_xor_sync(0xffffffffu, tw, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        wm[threadIdx.x >> 5] = t;
-        ww[threadIdx.x >> 5] = tw;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
-            t = max(t, wm[k]);
-            tw = max(tw, ww[k]);
-        }
-        ps->k = pair_scale_exp(__uint_as_float(t), e);
-        ps->km = mass_scale_exp(__uint_as_float(tw));
-        ps->arrivals = 0u;
-    }
+    direct_tile<BLOCK, IPT, COMP>(body, n, blockIdx.x * BLOCK * IPT, t0, t1, e,
+                                  pair_scale_exp(__uint_as_float(*scale.ext), e),
+                                  mass_scale_exp(__uint_as_float(*scale.mass)),
+                                  partial + (size_t)split * 3 * n, tile);
 }
 
 struct Shape {
@@ -182,12 +117,12 @@ static double wave_efficiency(long units, long slots)
 }
 
 // Bodies from which the heuristic plan evaluates each unordered pair once.
-// Measured on GB300 (best one-pair plan vs the symmetric plan, force pass):
-// 8,192 bodies 0.039 vs 0.105 ms (36 tile pairs cannot fill 152 SMs),
-// 16,384 0.120 vs 0.108 ms, 65,536 1.81 vs 1.20 ms, 1,048,580 428 vs 293 ms.
-constexpr int kSymmetricMinBodies = 20480;
+// Measured on GB300 (step of the best one-pair plan vs the symmetric plan):
+// 4,098 bodies 25 vs 37 us, 6,000 31 vs 39, 8,192 49 vs 38, 12,289 87 vs 73,
+// 16,387 139 vs 96, 65,536 1.81 vs 1.05 ms.
+constexpr int kSymmetricMinBodies = 7168;
 // Smallest size at which the autotuner also times the symmetric plan.
-constexpr int kSymmetricCandidateBodies = 12288;
+constexpr int kSymmetricCandidateBodies = 4096;
 
 // The symmetric plan's slot buffer grows as n^2 (12 B per body and 1,024-body
 // tile: 12.9 GB at 1,048,580 bodies, 51 GB at 2M).  It is planned only while
@@ -301,14 +236,6 @@ int record_event(cudaEvent_t ev, cudaStream_t stream)
     return PHYSIM_OK;
 }
 
-int launch_pair_scale(const float4 *body4, int n, float e, PairScale *ps, cudaStream_t stream)
-{
-    const int blocks = std::max(1, std::min(kScaleBlocks, (n + 2047) / 2048));
-    pair_scale_kernel<<<blocks, 256, 0, stream>>>(body4, n, e, ps);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
-}
-
 float max_abs_mass(const Entity *state, size_t n)
 {
     float m = 0.f;
@@ -332,22 +259,21 @@ float max_abs_coordinate(const Entity *state, size_t n)
     return m;
 }
 
-int launch_direct(const DirectPlan &plan, const float4 *body4, float e, PairScale *scale,
-                  double *partial, cudaStream_t stream, cudaEvent_t pairs_done)
+int launch_direct(const DirectPlan &plan, const float4 *body4, const float *mass256, float e,
+                  ScaleRef scale, double *partial, cudaStream_t stream, cudaEvent_t pairs_done)
 {
     if (plan.n <= 0) return PHYSIM_OK;
-    PG_CHECK(scale, PHYSIM_ERR_ARGUMENT, "no pair-scale workspace");
-    PG_TRY(launch_pair_scale(body4, plan.n, e, scale, stream));
+    PG_CHECK(scale.ext, PHYSIM_ERR_ARGUMENT, "no pair-scale workspace");
     if (plan.symmetric)
-        return launch_direct_symmetric(plan, body4, e, scale, partial, stream, pairs_done);
+        return launch_direct_symmetric(plan, body4, mass256, e, scale, partial, stream,
+                                       pairs_done);
     dim3 grid(plan.n_itiles, plan.splits);
     void *fn = shape_kernel(plan.block, plan.ipt, plan.compensated);
     PG_CHECK(fn != nullptr, PHYSIM_ERR_ARGUMENT, "no direct-sum kernel for block %d ipt %d",
              plan.block, plan.ipt);
     int n = plan.n, njt = plan.n_jtiles, ct = plan.chunk_tiles;
-    const PairScale *sc = scale;
     void *args[] = {(void *)&body4, (void *)&n, (void *)&njt, (void *)&ct, (void *)&e,
-                    (void *)&sc, (void *)&partial};
+                    (void *)&scale, (void *)&partial};
     PG_CUDA(cudaLaunchKernel(fn, grid, dim3(plan.block), args, 0, stream));
     if (pairs_done) PG_TRY(record_event(pairs_done, stream));
     return PHYSIM_OK;

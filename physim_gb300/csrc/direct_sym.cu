@@ -23,7 +23,8 @@
 //
 // Two schedules share that core.  With few tiles (one [3][n] f32 slot per
 // tile fits in kSymPairsSlotBytes) every tile pair (I, J), I <= J, is one
-// block (sym_tile_pair in direct_sym_tile.cuh): tile J's contribution to tile
+// block, or one cluster of up to eight that share out tile J (pair_parts;
+// sym_tile_pair in direct_sym_tile.cuh): tile J's contribution to tile
 // I goes to slot J, tile I's to tile J to slot I, and a reduce adds each
 // body's T slots.  That keeps every SM busy at any size and is the faster of
 // the two, but its slots grow as 12 T n bytes (12.9 GB at 1,048,580 bodies),
@@ -171,9 +172,8 @@ __device__ __forceinline__ void sym_reduce_tile(cg::cluster_group &cluster, int 
 // 64 threads of up to 255 registers (about 245 used), 54 KB of shared
 // memory: four blocks per SM.
 __global__ void __cluster_dims__(kSymCluster, 1, 1) __launch_bounds__(kSymThreads, 4)
-direct_sym_kernel(const float4 *__restrict__ body, int n, int T, float e,
-                  const PairScale *__restrict__ scale, float *__restrict__ Pi,
-                  float *__restrict__ Pj)
+direct_sym_kernel(const float4 *__restrict__ body, const float *__restrict__ mass256, int n, int T,
+                  float e, ScaleRef scale, float *__restrict__ Pi, float *__restrict__ Pj)
 {
     extern __shared__ float4 smem4[];
     float *smem = reinterpret_cast<float *>(smem4);
@@ -197,10 +197,13 @@ direct_sym_kernel(const float4 *__restrict__ body, int n, int T, float e,
     const bool have_i = I < T;
     const int warp = threadIdx.x >> 5;
     const int ib = warp * 32 + (threadIdx.x & 31);  // this thread's first body of tile I
-    const int sk = scale->k, skm = scale->km;
+    const int sk = pair_scale_exp(__uint_as_float(*scale.ext), e);
+    const int skm = mass_scale_exp(__uint_as_float(*scale.mass));
     const float sc = pow2f(-sk), msc = pow2f(-skm);
     const float es = e * pow2f(-2 * sk);
     const float2 e2 = make_float2(es, es);
+    float mi = 0.f;
+    const bool uni_i = have_i && common_mass(mass256, I * 4, I * 4 + 4, mi);
     float2 nx[kSymQ], ny[kSymQ], nz[kSymQ], nm[kSymQ], ax[kSymQ], ay[kSymQ], az[kSymQ];
 #pragma unroll
     for (int q = 0; q < kSymQ; ++q) {
@@ -220,10 +223,14 @@ direct_sym_kernel(const float4 *__restrict__ body, int n, int T, float e,
         // free: every block has read it (tile J - 3) before arriving for tile J - 2
         for (int x = threadIdx.x; x < 3 * kSymTile; x += kSymThreads) (&jw[0][0])[x] = 0.f;
         __syncthreads();
+        float mj = 0.f;
+        const bool uni = uni_i && common_mass(mass256, J * 4, J * 4 + 4, mj);
         if (have_i && I < J)
-            sym_pair_core<false, true>(body, J, sc, msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
+            sym_pair<false, true>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc, msc, e2, nx,
+                                  ny, nz, nm, ax, ay, az, jw);
         else if (have_i && I == J)
-            sym_pair_core<true>(body, J, sc, msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
+            sym_pair<true, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc, msc, e2, nx,
+                                  ny, nz, nm, ax, ay, az, jw);
         if (have_i && I <= J) {
             // this tile's partial sums into the compensated run sums
 #pragma unroll
@@ -271,11 +278,18 @@ direct_sym_kernel(const float4 *__restrict__ body, int n, int T, float e,
     cluster_wait();
 }
 
+// The factor that takes the scaled sums back: 2^(km - 2k).
+__device__ __forceinline__ double unscale(ScaleRef scale, float e)
+{
+    return pow2d(mass_scale_exp(__uint_as_float(*scale.mass)) -
+                 2 * pair_scale_exp(__uint_as_float(*scale.ext), e));
+}
+
 // out[c*n + k] = the sum of body k's slots (i-side by run, then j-side by
 // group), TwoSum-compensated f32, rounded once to f64 and unscaled
 // (x 2^(km - 2k)).
 __global__ void sym_reduce_kernel(const float *__restrict__ Pi, const float *__restrict__ Pj,
-                                  int n, int T, const PairScale *__restrict__ scale,
+                                  int n, int T, ScaleRef scale, float e,
                                   double *__restrict__ out)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -302,29 +316,31 @@ __global__ void sym_reduce_kernel(const float *__restrict__ Pi, const float *__r
         hi = s;
         lo += err;
     }
-    out[idx] = ((double)hi + (double)lo) * pow2d(scale->km - 2 * scale->k);
+    out[idx] = ((double)hi + (double)lo) * unscale(scale, e);
 }
 
-// The tile-pair schedule: block u takes tile pair (I, J) (unit_tiles).
-__global__ void __launch_bounds__(kSymThreads, 3)
-direct_sym_pairs_kernel(const float4 *__restrict__ body, int n, float e,
-                        const PairScale *__restrict__ scale, float *__restrict__ P)
+// The tile-pair schedule: `parts` consecutive blocks (a thread-block cluster)
+// take tile pair (I, J) (unit_tiles).
+__global__ void __launch_bounds__(kSymThreads, 4)
+direct_sym_pairs_kernel(const float4 *__restrict__ body, const float *__restrict__ mass256, int n,
+                        float e, ScaleRef scale, float *__restrict__ P, int parts)
 {
-    __shared__ float jacc[kSymWarps][kSymTile][3];
+    __shared__ float smem[kSymWarps * kSymTile * 3];
     int I, J;
-    unit_tiles(blockIdx.x, I, J);
-    const int sk = scale->k, skm = scale->km;
+    const int u = (int)blockIdx.x / parts, rank = (int)blockIdx.x - u * parts;
+    unit_tiles(u, I, J);
+    const int sk = pair_scale_exp(__uint_as_float(*scale.ext), e);
+    const int skm = mass_scale_exp(__uint_as_float(*scale.mass));
     if (I == J)
-        sym_tile_pair<true>(body, n, I, J, e, sk, skm, P, jacc);
+        sym_tile_pair<true>(body, mass256, n, I, J, e, sk, skm, P, smem, rank, parts);
     else
-        sym_tile_pair<false>(body, n, I, J, e, sk, skm, P, jacc);
+        sym_tile_pair<false>(body, mass256, n, I, J, e, sk, skm, P, smem, rank, parts);
 }
 
 // out[idx] = the sum of entry idx of the T slots P[t][3][n], in slot order,
 // TwoSum-compensated, rounded once to f64 and unscaled (x 2^(km - 2k)).
 __global__ void sym_pairs_reduce_kernel(const float *__restrict__ P, long long n3, int T,
-                                        const PairScale *__restrict__ scale,
-                                        double *__restrict__ out)
+                                        ScaleRef scale, float e, double *__restrict__ out)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n3) return;
@@ -338,7 +354,7 @@ __global__ void sym_pairs_reduce_kernel(const float *__restrict__ P, long long n
         hi = s;
         lo += err;
     }
-    out[idx] = ((double)hi + (double)lo) * pow2d(scale->km - 2 * scale->k);
+    out[idx] = ((double)hi + (double)lo) * unscale(scale, e);
 }
 
 }  // namespace
@@ -400,8 +416,37 @@ size_t direct_partial_doubles(const DirectPlan &p)
     return n3 + (sym_slot_floats(p.tiles, nullptr) + 1) / 2;
 }
 
-int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, float e,
-                            const PairScale *scale, double *partial, cudaStream_t stream,
+// Blocks per tile pair.  A block's two warps go to two of an SM's four
+// schedulers, so an SM's time is that of its blocks rounded up to an even
+// number, each 1 / parts of a tile pair; while more blocks than are resident at
+// once (four per SM) follow one another, the last ones run beside idle slots,
+// about one block's time more; and each doubling of the parts costs some 3%
+// (the cluster's exchange).  Force passes at 1 / 2 / 4 / 8 parts (us): 12,289
+// bodies 171 / 101 / 96 / 73, 16,387 169 / 100 / 96 / 101, 24,000 173 / 175 /
+// 187 / 181, 30,011 319 / 264 / 266 / 264, 50,000 731 / 690 / 668 / 679, 65,537
+// 1,053 / 1,073 / 1,109 / 1,125.
+static int pair_parts(int n, int sms)
+{
+    const double tiles = (double)n / kSymTile;
+    if (tiles > 60.0) return 1;
+    const double pairs = tiles * (tiles + 1.0) / 2.0;
+    int best = 1;
+    double best_time = 1e300;
+    for (int parts = 1, step = 0; parts <= 8; parts *= 2, ++step) {
+        const double blocks = pairs * parts;
+        double time = 2.0 * ceil(blocks / sms / 2.0);
+        if (blocks > 4.0 * sms) time += 1.0;
+        time *= (1.0 + 0.03 * step) / parts;
+        if (time < best_time) {
+            best_time = time;
+            best = parts;
+        }
+    }
+    return best;
+}
+
+int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const float *mass256,
+                            float e, ScaleRef scale, double *partial, cudaStream_t stream,
                             cudaEvent_t pairs_done)
 {
     if (plan.n <= 0) return PHYSIM_OK;
@@ -412,12 +457,24 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, float e
                  plan.n);
         const long long n3 = 3ll * plan.n;
         float *P = (float *)(partial + n3);
-        direct_sym_pairs_kernel<<<(unsigned)units, kSymThreads, 0, stream>>>(body4, plan.n, e,
-                                                                            scale, P);
-        PG_CUDA(cudaGetLastError());
+        int device = 0;
+        PG_CUDA(cudaGetDevice(&device));
+        const int parts = pair_parts(plan.n, device_sm_count(device));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(units * parts));
+        cfg.blockDim = dim3(kSymThreads);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)parts;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = parts > 1 ? 1 : 0;
+        PG_CUDA(cudaLaunchKernelEx(&cfg, direct_sym_pairs_kernel, body4, mass256, plan.n, e, scale,
+                                   P, parts));
         if (pairs_done) PG_TRY(record_event(pairs_done, stream));
         sym_pairs_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(
-            P, n3, (int)T, scale, partial);
+            P, n3, (int)T, scale, e, partial);
         PG_CUDA(cudaGetLastError());
         return PHYSIM_OK;
     }
@@ -430,12 +487,12 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, float e
     sym_slot_floats(T, &jside_at);
     float *Pi = (float *)(partial + n3);
     float *Pj = Pi + jside_at;
-    direct_sym_kernel<<<(unsigned)blocks, kSymThreads, kSymSmem, stream>>>(body4, plan.n, T, e,
-                                                                           scale, Pi, Pj);
+    direct_sym_kernel<<<(unsigned)blocks, kSymThreads, kSymSmem, stream>>>(
+        body4, mass256, plan.n, T, e, scale, Pi, Pj);
     PG_CUDA(cudaGetLastError());
     if (pairs_done) PG_TRY(record_event(pairs_done, stream));
     sym_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(Pi, Pj, plan.n, T,
-                                                                         scale, partial);
+                                                                         scale, e, partial);
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }

@@ -5,6 +5,8 @@
 // the slot-buffer layout are described in direct_sym.cu.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -57,17 +59,34 @@ __device__ __forceinline__ void red_shared_add(float *p, float v)
                  : "memory");
 }
 
-// Tile I (in registers) against tile J: a_i += the pairs' terms (scaled, see
-// sym_load_i); unless DIAG, tile J's reactions go to shared memory, jw[j][c]
-// for body j of tile J: stored (this warp's own slice), or with ADD added to
+// The mass that all bodies of 256-body blocks [b0, b1) have (DeviceBodies::
+// mass256); false where there is none.
+__device__ __forceinline__ bool common_mass(const float *__restrict__ mass256, int b0, int b1,
+                                            float &m)
+{
+    m = mass256[b0];
+    bool same = m == m;
+    for (int b = b0 + 1; b < b1; ++b) same = same && mass256[b] == m;
+    return same;
+}
+
+// Tile I (in registers) against groups [g0, g1) of 32 bodies of tile J: a_i +=
+// the pairs' terms (scaled, see sym_load_i); unless DIAG, tile J's reactions go
+// to shared memory, jw[j][c] for body j from group g0 on: stored (this warp's own slice), or with ADD added to
 // a slice that starts at zero and that both warps of the block add to (two
 // terms added onto zero round the same in either order, so the sum does not
 // depend on which warp comes first).  With DIAG (I == J) every ordered pair
 // of the tile is evaluated for a_i only (a body meets itself with d = 0,
 // which contributes 0 through the r^2 guard).
-template <bool DIAG, bool ADD = false>
-__device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, int J, float sc,
-                                              float msc, float2 e2, const float2 (&nx)[kSymQ],
+// With UNI the bodies of either tile all have one mass: the pairs' terms are
+// summed without masses (15 FMA-pipe operations and 9 shuffles per 16 pairs
+// instead of 17 and 10), the reactions leave multiplied by nmi (minus tile I's
+// scaled mass), and the caller multiplies a_i by tile J's.  One rounding per sum
+// takes the place of one per term.
+template <bool DIAG, bool ADD, bool UNI>
+__device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, int J, int g0,
+                                              int g1, float sc, float msc, float nmi, float2 e2,
+                                              const float2 (&nx)[kSymQ],
                                               const float2 (&ny)[kSymQ],
                                               const float2 (&nz)[kSymQ],
                                               const float2 (&nm)[kSymQ], float2 (&ax)[kSymQ],
@@ -79,11 +98,11 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
     const unsigned full = 0xffffffffu;
     const int src = (lane + 1) & 31;
 
-    float4 next = body[J * kSymTile + lane];
-    for (int g = 0; g < kSymGroups; ++g) {
+    float4 next = body[J * kSymTile + g0 * 32 + lane];
+    for (int g = g0; g < g1; ++g) {
         const float4 bj = next;
         // the next group's body is loaded while this group is evaluated
-        if (g + 1 < kSymGroups) next = body[J * kSymTile + (g + 1) * 32 + lane];
+        if (g + 1 < g1) next = body[J * kSymTile + (g + 1) * 32 + lane];
         float xj = bj.x * sc, yj = bj.y * sc, zj = bj.z * sc, mj = bj.w * msc;
         float2 jx = make_float2(0.f, 0.f), jy = jx, jz = jx;
 #pragma unroll 2
@@ -96,7 +115,7 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
             xj = __shfl_sync(full, xj, src);
             yj = __shfl_sync(full, yj, src);
             zj = __shfl_sync(full, zj, src);
-            mj = __shfl_sync(full, mj, src);
+            if (!UNI) mj = __shfl_sync(full, mj, src);
 #pragma unroll
             for (int q = 0; q < kSymQ; ++q) {
                 const float2 dx = add2(xj2, nx[q]);
@@ -109,12 +128,12 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
                 const float2 ww = mul2(w, w);
                 const float2 qv = fma2(r2, ww, g2);
                 const float2 inv = make_float2(rsqrt_approx(qv.x), rsqrt_approx(qv.y));
-                const float2 fi = mul2(mj2, inv);
+                const float2 fi = UNI ? inv : mul2(mj2, inv);
                 ax[q] = fma2(dx, fi, ax[q]);
                 ay[q] = fma2(dy, fi, ay[q]);
                 az[q] = fma2(dz, fi, az[q]);
                 if (!DIAG) {
-                    const float2 fj = mul2(nm[q], inv);
+                    const float2 fj = UNI ? inv : mul2(nm[q], inv);
                     jx = fma2(dx, fj, jx);
                     jy = fma2(dy, fj, jy);
                     jz = fma2(dz, fj, jz);
@@ -131,76 +150,160 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
         }
         if (!DIAG) {
             // after 32 rotations lane `lane` holds body g*32 + lane's reaction again
-            float *dst = jw[g * 32 + lane];
+            float *dst = jw[(g - g0) * 32 + lane];
+            const float f = UNI ? nmi : 1.f;
+            const float rx = (jx.x + jx.y) * f, ry = (jy.x + jy.y) * f, rz = (jz.x + jz.y) * f;
             if (ADD) {
-                red_shared_add(dst + 0, jx.x + jx.y);
-                red_shared_add(dst + 1, jy.x + jy.y);
-                red_shared_add(dst + 2, jz.x + jz.y);
+                red_shared_add(dst + 0, rx);
+                red_shared_add(dst + 1, ry);
+                red_shared_add(dst + 2, rz);
             } else {
-                dst[0] = jx.x + jx.y;
-                dst[1] = jy.x + jy.y;
-                dst[2] = jz.x + jz.y;
+                dst[0] = rx;
+                dst[1] = ry;
+                dst[2] = rz;
             }
         }
     }
 }
 
-// One tile pair (I, J) with its own slots (the ensemble's layout): tile J's
-// contribution to tile I's bodies goes to slot J, tile I's to tile J's
-// bodies to slot I, of P[T][3][n] (f32, left scaled: positions entering as
-// p 2^-sk, masses as m 2^-skm; the reduction multiplies by 2^(skm - 2sk) in
-// f64).
+// sym_pair_core with the variant that the tiles' masses allow.  uni: tile I's
+// scaled mass mi and the groups' mj are common.  a_i must enter as zero.
+template <bool DIAG, bool ADD>
+__device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
+                                         const float4 *__restrict__ body, int J, int g0, int g1,
+                                         float sc, float msc, float2 e2,
+                                         const float2 (&nx)[kSymQ], const float2 (&ny)[kSymQ],
+                                         const float2 (&nz)[kSymQ], const float2 (&nm)[kSymQ],
+                                         float2 (&ax)[kSymQ], float2 (&ay)[kSymQ],
+                                         float2 (&az)[kSymQ], float (*jw)[3])
+{
+    if (uni) {
+        sym_pair_core<DIAG, ADD, true>(body, J, g0, g1, sc, msc, -mi, e2, nx, ny, nz, nm, ax, ay,
+                                       az, jw);
+        const float2 m2 = make_float2(mj, mj);
+#pragma unroll
+        for (int q = 0; q < kSymQ; ++q) {
+            ax[q] = mul2(ax[q], m2);
+            ay[q] = mul2(ay[q], m2);
+            az[q] = mul2(az[q], m2);
+        }
+    } else {
+        sym_pair_core<DIAG, ADD, false>(body, J, g0, g1, sc, msc, 0.f, e2, nx, ny, nz, nm, ax, ay,
+                                        az, jw);
+    }
+}
+
+// Part `rank` of `parts` of one tile pair (I, J): tile I against that share of
+// tile J's groups.  Tile J's contribution to tile I's bodies goes to slot J,
+// tile I's to tile J's bodies to slot I, of P[T][3][n] (f32, left scaled:
+// positions entering as p 2^-sk, masses as m 2^-skm; the reduction multiplies by
+// 2^(skm - 2sk) in f64).  With parts > 1 the blocks of one thread-block cluster
+// take the parts: their sums for tile I are added through distributed shared
+// memory, ranks in order with TwoSum, each block adding and writing its share
+// of the bodies, so there is one slot per tile pair whatever the parts.
+// smem: 6 x 1,024 floats.
 template <bool DIAG>
-__device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body, int n, int I,
+__device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
+                                              const float *__restrict__ mass256, int n, int I,
                                               int J, float e, int sk, int skm,
-                                              float *__restrict__ P, float (*jacc)[kSymTile][3])
+                                              float *__restrict__ P, float *smem, int rank = 0,
+                                              int parts = 1)
 {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const size_t n3 = 3 * (size_t)n;
-    const int ib = I * kSymTile + warp * 32 + lane;
+    const int ib = warp * 32 + lane;
     const float sc = pow2f(-sk), msc = pow2f(-skm);
     const float es = e * pow2f(-2 * sk);
     const float2 e2 = make_float2(es, es);
+    // the groups of tile J that hold bodies, shared out over the parts
+    const int groups = min(kSymGroups, (n - J * kSymTile + 31) / 32);
+    const int g0 = rank * groups / parts, g1 = (rank + 1) * groups / parts;
+    const int rows = (g1 - g0) * 32;  // <= 512 with two parts or more
+    float (*jacc)[3] = reinterpret_cast<float (*)[3]>(smem);  // [kSymWarps][rows][3]
     float2 nx[kSymQ], ny[kSymQ], nz[kSymQ], nm[kSymQ], ax[kSymQ], ay[kSymQ], az[kSymQ];
     sym_load_i(body, I, sc, msc, nx, ny, nz, nm);
 #pragma unroll
     for (int q = 0; q < kSymQ; ++q) ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
-    sym_pair_core<DIAG>(body, J, sc, msc, e2, nx, ny, nz, nm, ax, ay, az, jacc[warp]);
-
+    if (rows > 0) {
+        float mi = 0.f, mj = 0.f;
+        bool uni = common_mass(mass256, I * 4, I * 4 + 4, mi);
+        uni = common_mass(mass256, J * 4 + g0 / 8, J * 4 + (g1 + 7) / 8, mj) && uni;
+        sym_pair<DIAG, false>(uni, mi * msc, mj * msc, body, J, g0, g1, sc, msc, e2, nx, ny, nz,
+                              nm, ax, ay, az, jacc + warp * rows);
+    }
     // tile J's contribution to tile I's bodies: slot J
     float *pi = P + (size_t)J * n3;
+    if (parts == 1) {
 #pragma unroll
-    for (int q = 0; q < kSymQ; ++q) {
-        const int i0 = ib + (2 * q) * kSymThreads;
-        const int i1 = i0 + kSymThreads;
-        if (i0 < n) {
-            pi[i0] = ax[q].x;
-            pi[(size_t)n + i0] = ay[q].x;
-            pi[2 * (size_t)n + i0] = az[q].x;
+        for (int q = 0; q < kSymQ; ++q) {
+            const int i0 = I * kSymTile + ib + (2 * q) * kSymThreads;
+            const int i1 = i0 + kSymThreads;
+            if (i0 < n) {
+                pi[i0] = ax[q].x;
+                pi[(size_t)n + i0] = ay[q].x;
+                pi[2 * (size_t)n + i0] = az[q].x;
+            }
+            if (i1 < n) {
+                pi[i1] = ax[q].y;
+                pi[(size_t)n + i1] = ay[q].y;
+                pi[2 * (size_t)n + i1] = az[q].y;
+            }
         }
-        if (i1 < n) {
-            pi[i1] = ax[q].y;
-            pi[(size_t)n + i1] = ay[q].y;
-            pi[2 * (size_t)n + i1] = az[q].y;
+        if (!DIAG) __syncthreads();
+    } else {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        float *mine = smem + 3 * kSymTile;  // [3][1,024], past the reactions
+#pragma unroll
+        for (int q = 0; q < kSymQ; ++q) {
+            const int b0 = ib + (2 * q) * kSymThreads, b1 = b0 + kSymThreads;
+            mine[b0] = ax[q].x;
+            mine[kSymTile + b0] = ay[q].x;
+            mine[2 * kSymTile + b0] = az[q].x;
+            mine[b1] = ax[q].y;
+            mine[kSymTile + b1] = ay[q].y;
+            mine[2 * kSymTile + b1] = az[q].y;
+        }
+        cluster.sync();
+        const int share = kSymTile / parts, first = rank * share;
+        for (int t = threadIdx.x; t < 3 * share; t += kSymThreads) {
+            const int c = t / share, b = first + t - c * share;
+            const int i = I * kSymTile + b;
+            if (i >= n) continue;
+            float v[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                v[r] = r < parts ? cluster.map_shared_rank(mine, r)[c * kSymTile + b] : 0.f;
+            float hi = 0.f, lo = 0.f;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                if (r >= parts) break;
+                float s, err;
+                two_sum(hi, v[r], s, err);
+                hi = s;
+                lo += err;
+            }
+            pi[(size_t)c * n + i] = hi + lo;
         }
     }
     if (!DIAG) {
         // tile I's contribution to tile J's bodies: slot I, warps added in order
-        __syncthreads();
         float *pj = P + (size_t)I * n3;
-        for (int j = threadIdx.x; j < kSymTile; j += kSymThreads) {
-            const int k = J * kSymTile + j;
+        for (int j = threadIdx.x; j < rows; j += kSymThreads) {
+            const int k = J * kSymTile + g0 * 32 + j;
             if (k >= n) break;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                float s = jacc[0][j][c];
+                float s = jacc[j][c];
 #pragma unroll
-                for (int w = 1; w < kSymWarps; ++w) s += jacc[w][j][c];
+                for (int w = 1; w < kSymWarps; ++w) s += jacc[w * rows + j][c];
                 pj[(size_t)c * n + k] = s;
             }
         }
     }
+    // every block's shared memory stays until the others have read it
+    if (parts > 1) cooperative_groups::this_cluster().sync();
 }
 
 }  // namespace pg

@@ -38,7 +38,7 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
     const bool tree = el->kind != 0;
     bool direct = false;
     PG_TRY(host_direct(el->device, &direct));
-    PG_TRY(bodies_reserve(el->bodies, n, tree, st));
+    PG_TRY(bodies_reserve(el->bodies, n, tree, !tree, st));
     Acceleration *acc_io = acc;  // DIRECT: the kernels read and write the caller's array
     const Entity *state_in = state;
     if (direct) {
@@ -75,8 +75,8 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
         }
         PG_TRY(rc);
         splits = el->plan.splits;
-        PG_TRY(launch_direct(el->plan, el->bodies.body4, (float)el->e, el->bodies.scale,
-                             el->partial, st));
+        PG_TRY(launch_direct(el->plan, el->bodies.body4, el->bodies.mass256, (float)el->e,
+                             el->bodies.scale_ref(), el->partial, st));
     } else {
         PG_TRY(ensure_doubles(el->partial, el->partial_cap, 3 * n, st));
         BhParams p;

@@ -41,14 +41,22 @@ constexpr float kPairGuard = 1.17549435e-38f;
 // to [-100, 100].  What remains: with e = 0, pairs closer than ~3e-6 of the
 // largest |coordinate| lose accuracy beyond 1e-5 relative, and closer than
 // ~5e-7 of it they contribute almost nothing (r'^6 underflows into the guard).
-constexpr int kScaleBlocks = 256;
+//
+// The maxima are kept as f32 bit patterns (NaN and infinities skipped) by the
+// kernels that write body4 -- unpack and the integrators -- so a force pass
+// needs no pass over the bodies of its own (it was 5 of 37 us per step at 4,098
+// bodies).  Each maximum has two halves: the kernel that writes a state adds its
+// bodies' maxima to the half that is not current, which is zero, and clears the
+// current one, which no later kernel on the stream reads; then the halves change
+// places (DeviceBodies::ext_half, mass_half).
 struct PairScale {
-    int32_t k;          // coordinate scale exponent of the current state
-    int32_t km;         // mass scale exponent
-    uint32_t arrivals;  // blocks of a running scale pass that finished (reset by the last)
-    uint32_t pad;
-    uint32_t blockmax[kScaleBlocks];   // per-block max |coordinate| (f32 bit patterns)
-    uint32_t blockmass[kScaleBlocks];  // per-block max |mass|
+    uint32_t ext[2];   // largest |coordinate|
+    uint32_t mass[2];  // largest |mass| (unpack only: integrators keep masses)
+};
+
+// A state's maxima, as the pair kernels take them.
+struct ScaleRef {
+    const uint32_t *ext = nullptr, *mass = nullptr;
 };
 
 // Exponent of the largest |coordinate| m: m = f 2^k, f in [0.5, 1) (0 for m = 0).
@@ -85,13 +93,8 @@ __host__ __device__ inline int mass_scale_exp(float m)
     return k < -100 ? -100 : (k > 100 ? 100 : k);
 }
 
-// Computes ps->k and ps->km for the n bodies of body4 (max over |x|, |y|,
-// |z| and over |m|; NaN and infinite values skipped) and easing e, on
-// `stream`: one launch whose last block to finish reduces the per-block
-// maxima.  ps->arrivals must be 0 before the first pass (it is left 0).
-int launch_pair_scale(const float4 *body4, int n, float e, PairScale *ps, cudaStream_t stream);
-// The coordinate pass over the members of an ensemble is done by its
-// integrator kernel; host-side values for a state being uploaded:
+// An ensemble's members keep their own (per member; its integrator kernel
+// updates the coordinates'); host-side values for a state being uploaded:
 float max_abs_coordinate(const Entity *state, size_t n);
 float max_abs_mass(const Entity *state, size_t n);
 
@@ -140,12 +143,14 @@ size_t direct_partial_doubles(const DirectPlan &plan);
 // s < plan.splits holds the partial sums.  pairs_done (optional) is recorded
 // on `stream` right after the pair kernel, before any reduction of its
 // output (as an external event node when the stream is being captured).
-// Before the pair kernel, launch_direct runs the scale pass of body4 into
-// `scale` (see PairScale); the partial sums come out unscaled.
-int launch_direct(const DirectPlan &plan, const float4 *body4, float e, PairScale *scale,
-                  double *partial, cudaStream_t stream, cudaEvent_t pairs_done = nullptr);
-int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, float e,
-                            const PairScale *scale, double *partial, cudaStream_t stream,
+// scale: body4's maxima (see PairScale); the partial sums come out unscaled.
+// mass256 (symmetric plans): the common mass of each 256 bodies (see
+// DeviceBodies).
+int launch_direct(const DirectPlan &plan, const float4 *body4, const float *mass256, float e,
+                  ScaleRef scale, double *partial, cudaStream_t stream,
+                  cudaEvent_t pairs_done = nullptr);
+int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const float *mass256,
+                            float e, ScaleRef scale, double *partial, cudaStream_t stream,
                             cudaEvent_t pairs_done);
 // Records `ev` on `stream`; inside a stream capture as an external event node.
 int record_event(cudaEvent_t ev, cudaStream_t stream);
@@ -164,7 +169,12 @@ struct DeviceBodies {
     double *radius = nullptr;
     uint64_t *id = nullptr;
     Entity *aos = nullptr;  // staging for host<->device copies
-    PairScale *scale = nullptr;  // pair-law scale of the direct-sum kernels
+    PairScale *scale = nullptr;  // pair-law maxima of the direct-sum kernels
+    int ext_half = 0, mass_half = 0;  // the current halves of *scale
+    // the mass that all of each 256 bodies have, as f32; NaN where they differ
+    // or padding is among them (direct-sum states only)
+    float *mass256 = nullptr;
+    ScaleRef scale_ref() const { return {&scale->ext[ext_half], &scale->mass[mass_half]}; }
 };
 
 // Stream-ordered device memory (cudaMallocAsync / cudaFreeAsync on the
@@ -181,7 +191,9 @@ inline int dev_alloc(T *&p, size_t count, cudaStream_t stream)
 }
 
 // `stream` orders the allocations (and frees) with the owner's work.
-int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, cudaStream_t stream);
+// with_scale: the direct sum's maxima and common masses are kept.
+int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, bool with_scale,
+                   cudaStream_t stream);
 void bodies_free(DeviceBodies &b, cudaStream_t stream);
 
 // True when calls on `device` hand the caller's host arrays to the kernels
@@ -198,7 +210,8 @@ int host_direct(int device, bool *direct);
 // populate (not host memory, an older kernel) is left to the GPU's faults.
 void host_prefault(const void *p, size_t bytes, bool write);
 
-// Unpacks an Entity array into the SoA arrays.  `aos` may be device memory
+// Unpacks an Entity array into the SoA arrays (with b.scale and b.mass256, the
+// direct-sum kernels' maxima and common masses too).  `aos` may be device memory
 // or, where host_direct() holds, the caller's host array: each block reads
 // its 256 entities as one contiguous run.
 int launch_unpack(DeviceBodies &b, const Entity *aos, size_t n, bool full_state,
@@ -214,7 +227,8 @@ int launch_accumulate_aos(const DeviceBodies &b, const double *partial, int spli
 int launch_combine_soa(const DeviceBodies &b, const double *partial, int splits,
                        double *acc_soa, cudaStream_t stream);
 // Verlet step (verlet.rs:24-82) fused with the combine of the partial sums,
-// updating the f64 state and the f32 body copy in place.
+// updating the f64 state and the f32 body copy in place (and, like the other
+// integrators, the largest |coordinate| where b.scale is kept).
 int launch_verlet(DeviceBodies &b, const double *partial, int splits, double dt, bool initial,
                   cudaStream_t stream);
 

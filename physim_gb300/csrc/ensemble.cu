@@ -86,13 +86,14 @@ ensemble_forces_kernel(const float4 *__restrict__ body4, const MemberInfo *__res
 }
 
 __global__ void __launch_bounds__(kSymThreads, 3)
-ensemble_sym_kernel(const float4 *__restrict__ body4, const MemberInfo *__restrict__ members,
+ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ mass256,
+                    const MemberInfo *__restrict__ members,
                     const SymUnit *__restrict__ units, int n_units,
                     const unsigned long long *__restrict__ remaining, int *__restrict__ counter,
                     const int32_t *__restrict__ member_kx, const int32_t *__restrict__ member_km,
                     float *__restrict__ slots)
 {
-    __shared__ float jacc[kSymWarps][kSymTile][3];
+    __shared__ float smem[kSymWarps * kSymTile * 3];
     __shared__ int next;
     for (;;) {
         if (threadIdx.x == 0) next = atomicAdd(counter, 1);
@@ -104,11 +105,11 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const MemberInfo *__restri
             const MemberInfo m = members[w.member];
             const int sk = pair_scale_from(member_kx[w.member], m.e), skm = member_km[w.member];
             if (w.I == w.J)
-                sym_tile_pair<true>(body4 + m.off, m.n, w.I, w.J, m.e, sk, skm, slots + m.soff,
-                                    jacc);
+                sym_tile_pair<true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
+                                    skm, slots + m.soff, smem);
             else
-                sym_tile_pair<false>(body4 + m.off, m.n, w.I, w.J, m.e, sk, skm, slots + m.soff,
-                                     jacc);
+                sym_tile_pair<false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
+                                     skm, slots + m.soff, smem);
         }
         __syncthreads();
     }
@@ -228,9 +229,14 @@ __global__ void ensemble_count_kernel(unsigned long long *remaining, unsigned lo
 __global__ void ensemble_unpack_kernel(const Entity *__restrict__ in, int n, int off, float4 *body4,
                                        uint8_t *fixed, double *x, double *y, double *z,
                                        double *vx, double *vy, double *vz, double *m,
-                                       double *radius, uint64_t *id)
+                                       double *radius, uint64_t *id, float *mass256)
 {
+    // whole tiles: a block fills one entry of mass256 (DeviceBodies::mass256)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const float mass = i < n ? (float)in[i].mass : 0.f;
+    const float m0 = (float)in[min((int)(blockIdx.x * blockDim.x), n - 1)].mass;
+    const bool same = __syncthreads_and(i < n && mass == m0 && fabsf(m0) <= 3.4028235e38f);
+    if (threadIdx.x == 0) mass256[off / 256 + blockIdx.x] = same ? m0 : __int_as_float(0x7fc00000);
     if (i >= n) return;
     const Entity en = in[i];
     const int s = off + i;
@@ -327,6 +333,7 @@ struct PhysimEnsemble {
     int slots = 0;
     // device state (concatenated, every member padded to kBodyPad slots)
     float4 *body4 = nullptr;
+    float *mass256 = nullptr;  // as DeviceBodies::mass256
     uint8_t *fixed = nullptr;
     double *x = nullptr, *y = nullptr, *z = nullptr, *vx = nullptr, *vy = nullptr, *vz = nullptr;
     double *px = nullptr, *py = nullptr, *pz = nullptr, *m = nullptr, *radius = nullptr;
@@ -483,7 +490,7 @@ int launch_forces(PhysimEnsemble *E)
 {
     if (E->n_sym_units > 0) {
         ensemble_sym_kernel<<<std::min(E->sym_grid, E->n_sym_units), kSymThreads, 0, E->stream>>>(
-            E->body4, E->d_members, E->d_sym_units, E->n_sym_units, E->remaining, E->counter + 1,
+            E->body4, E->mass256, E->d_members, E->d_sym_units, E->n_sym_units, E->remaining, E->counter + 1,
             E->member_kx, E->member_km, E->slot_sums);
         PG_CUDA(cudaGetLastError());
     }
@@ -514,7 +521,7 @@ int enqueue_step(PhysimEnsemble *E)
 void free_ensemble(PhysimEnsemble *E)
 {
     drop_graph(E);
-    void *p[] = {E->body4, E->fixed, E->x,  E->y,  E->z,  E->vx, E->vy, E->vz, E->px, E->py,
+    void *p[] = {E->body4, E->mass256, E->fixed, E->x,  E->y,  E->z,  E->vx, E->vy, E->vz, E->px, E->py,
                  E->pz,    E->m,     E->radius, E->id, E->slot_member, E->d_members, E->d_units,
                  E->remaining, E->done, E->counter, E->partial, E->staging,
                  E->d_sym_units, E->slot_sums, E->member_kx, E->member_km, E->member_ext};
@@ -577,6 +584,7 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
 #define EA(ptr, cnt)                                                                        \
     if (rc == PHYSIM_OK) rc = ealloc(E, ptr, cnt)
     EA(E->body4, slots);
+    EA(E->mass256, slots / 256);
     EA(E->fixed, slots);
     EA(E->x, slots);
     EA(E->y, slots);
@@ -651,9 +659,9 @@ int physim_gpu_ensemble_upload(PhysimEnsemble *E, size_t index, const Entity *st
     PG_CUDA(cudaMemcpyAsync(E->staging, state, n * sizeof(Entity), cudaMemcpyHostToDevice,
                             E->stream));
     const int off = E->members[index].off;
-    ensemble_unpack_kernel<<<cdiv((long long)n, 256), 256, 0, E->stream>>>(
+    ensemble_unpack_kernel<<<(int)(pad_bodies(n) / 256), 256, 0, E->stream>>>(
         E->staging, (int)n, off, E->body4, E->fixed, E->x, E->y, E->z, E->vx, E->vy, E->vz, E->m,
-        E->radius, E->id);
+        E->radius, E->id, E->mass256);
     PG_CUDA(cudaGetLastError());
     const unsigned long long zero = 0ull, all = ~0ull;
     // pair scale of the uploaded positions (the integrator keeps it current)

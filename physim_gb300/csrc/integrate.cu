@@ -52,23 +52,70 @@ __device__ __forceinline__ void block_copy(void *dst, const void *src, int bytes
     }
 }
 
+// |v| as f32 bits, 0 for NaN and infinities (bit patterns order like the
+// non-negative values).
+__device__ __forceinline__ uint32_t finite_abs_bits(float v)
+{
+    const uint32_t b = __float_as_uint(v) & 0x7fffffffu;
+    return b < 0x7f800000u ? b : 0u;
+}
+
+__device__ __forceinline__ uint32_t max_abs_bits(float4 b)
+{
+    return max(finite_abs_bits(b.x), max(finite_abs_bits(b.y), finite_abs_bits(b.z)));
+}
+
+// The half of a maximum (PairScale) that this kernel fills, and the one it
+// clears; null: the state keeps none.
+struct Track {
+    uint32_t *fill = nullptr, *clear = nullptr;
+};
+
+// Adds the block's largest `m` to the tracked maximum (every thread of the
+// block takes part).
+__device__ __forceinline__ void track_max(const Track &t, uint32_t m)
+{
+    if (!t.fill) return;
+    __shared__ uint32_t wm[kThreads / 32];
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max(m, wm[w]);
+        if (m) atomicMax(t.fill, m);
+        if (blockIdx.x == 0) *t.clear = 0u;
+    }
+    __syncthreads();  // wm may serve another maximum
+}
+
 __global__ void unpack_kernel(const Entity *__restrict__ in, int n, int n_pad, float4 *body4,
                               uint8_t *fixed, double *x, double *y, double *z, double *vx,
-                              double *vy, double *vz, double *m, double *radius, uint64_t *id)
+                              double *vy, double *vz, double *m, double *radius, uint64_t *id,
+                              Track ext, Track mass, float *mass256)
 {
+    static_assert(kThreads == 256, "a block fills one entry of mass256");
     __shared__ __align__(16) Entity s_in[kThreads];
     const int base = blockIdx.x * kThreads;
     const int count = min(kThreads, n - base);  // <= 0 for blocks of the padded tail
     if (count > 0) block_copy(s_in, in + base, count * (int)sizeof(Entity));
     __syncthreads();
-    const int i = base + threadIdx.x;
-    if (i >= n_pad) return;
-    if (i >= n) {
-        body4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
+    const int i = base + threadIdx.x;  // n_pad is a multiple of the block
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n) {
+        const Entity &en = s_in[threadIdx.x];
+        b4 = make_float4((float)en.x, (float)en.y, (float)en.z, (float)en.mass);
     }
+    body4[i] = b4;
+    if (ext.fill) {
+        track_max(ext, max_abs_bits(b4));
+        track_max(mass, finite_abs_bits(b4.w));
+        const float m0 = (float)s_in[0].mass;
+        const bool same = __syncthreads_and(i < n && b4.w == m0 && fabsf(m0) <= 3.4028235e38f);
+        if (threadIdx.x == 0 && mass256)
+            mass256[blockIdx.x] = same ? m0 : __int_as_float(0x7fc00000);
+    }
+    if (i >= n) return;
     const Entity en = s_in[threadIdx.x];
-    body4[i] = make_float4((float)en.x, (float)en.y, (float)en.z, (float)en.mass);
     fixed[i] = en.fixed ? 1 : 0;
     m[i] = en.mass;
     if (x) {
@@ -113,10 +160,24 @@ __device__ __forceinline__ void body_acc(const double *partial, int splits, int 
 {
     ax = ay = az = 0.0;
     if (fixed) return;
-    for (int s = 0; s < splits; ++s) {
-        ax += partial[(size_t)(s * 3 + 0) * n + i];
-        ay += partial[(size_t)(s * 3 + 1) * n + i];
-        az += partial[(size_t)(s * 3 + 2) * n + i];
+    // four splits' loads in flight together (summed in split order): one after
+    // another they were a chain of L2 round trips, 6 of 11 us at 17 splits
+    constexpr int kAhead = 4;
+    for (int s0 = 0; s0 < splits; s0 += kAhead) {
+        double p[kAhead][3];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (s0 + u < splits)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    p[u][c] = partial[(size_t)((s0 + u) * 3 + c) * n + i];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (s0 + u < splits) {
+                ax += p[u][0];
+                ay += p[u][1];
+                az += p[u][2];
+            }
     }
     if (mass == 0.0) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
 }
@@ -182,27 +243,39 @@ __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *
                               const double *partial,
                               int splits, int n, double *x, double *y, double *z, double *vx,
                               double *vy, double *vz, double *px, double *py, double *pz,
-                              double dt, int initial)
+                              double dt, int initial, Track ext)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 b = body4[i];
-    double ax, ay, az;
-    body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
-    const double dt2 = __dmul_rn(dt, dt);
-    double xi = x[i], yi = y[i], zi = z[i];
-    double vxi = vx[i], vyi = vy[i], vzi = vz[i];
-    double pxi = px[i], pyi = py[i], pzi = pz[i];
-    verlet_axis(xi, vxi, pxi, ax, dt, dt2, initial);
-    verlet_axis(yi, vyi, pyi, ay, dt, dt2, initial);
-    verlet_axis(zi, vzi, pzi, az, dt, dt2, initial);
-    x[i] = xi; y[i] = yi; z[i] = zi;
-    vx[i] = vxi; vy[i] = vyi; vz[i] = vzi;
-    px[i] = pxi; py[i] = pyi; pz[i] = pzi;
-    b.x = (float)xi;
-    b.y = (float)yi;
-    b.z = (float)zi;
-    body4[i] = b;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t top = 0;
+    if (i < n) {
+        float4 b = body4[i];
+        double xi = x[i], yi = y[i], zi = z[i];
+        double vxi = 0.0, vyi = 0.0, vzi = 0.0, pxi = 0.0, pyi = 0.0, pzi = 0.0;
+        if (initial) {  // the Taylor step reads the velocities, the others the positions before
+            vxi = vx[i];
+            vyi = vy[i];
+            vzi = vz[i];
+        } else {
+            pxi = px[i];
+            pyi = py[i];
+            pzi = pz[i];
+        }
+        double ax, ay, az;
+        body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
+        const double dt2 = __dmul_rn(dt, dt);
+        verlet_axis(xi, vxi, pxi, ax, dt, dt2, initial);
+        verlet_axis(yi, vyi, pyi, ay, dt, dt2, initial);
+        verlet_axis(zi, vzi, pzi, az, dt, dt2, initial);
+        x[i] = xi; y[i] = yi; z[i] = zi;
+        vx[i] = vxi; vy[i] = vyi; vz[i] = vzi;
+        px[i] = pxi; py[i] = pyi; pz[i] = pzi;
+        b.x = (float)xi;
+        b.y = (float)yi;
+        b.z = (float)zi;
+        body4[i] = b;
+        top = max_abs_bits(b);
+    }
+    track_max(ext, top);  // (every thread of the block)
 }
 
 __global__ void verlet_aos_kernel(const Entity *in, const Entity *prev, Entity *out, Entity *keep,
@@ -258,26 +331,30 @@ __global__ void verlet_aos_kernel(const Entity *in, const Entity *prev, Entity *
 // body has a = 0 (transforms skip it) and still drifts with its velocity.
 __global__ void euler_kernel(float4 *body4, const double *mass, const uint8_t *fixed,
                              const double *partial, int splits, int n, double *x, double *y,
-                             double *z, double *vx, double *vy, double *vz, double dt)
+                             double *z, double *vx, double *vy, double *vz, double dt, Track ext)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 b = body4[i];
-    double ax, ay, az;
-    body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
-    const double dt2 = __dmul_rn(dt, dt);
-    double xi = x[i], yi = y[i], zi = z[i];
-    double vxi = vx[i], vyi = vy[i], vzi = vz[i];
-    double unused = 0.0;
-    verlet_axis(xi, vxi, unused, ax, dt, dt2, true);
-    verlet_axis(yi, vyi, unused, ay, dt, dt2, true);
-    verlet_axis(zi, vzi, unused, az, dt, dt2, true);
-    x[i] = xi; y[i] = yi; z[i] = zi;
-    vx[i] = vxi; vy[i] = vyi; vz[i] = vzi;
-    b.x = (float)xi;
-    b.y = (float)yi;
-    b.z = (float)zi;
-    body4[i] = b;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t top = 0;
+    if (i < n) {
+        float4 b = body4[i];
+        double ax, ay, az;
+        body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
+        const double dt2 = __dmul_rn(dt, dt);
+        double xi = x[i], yi = y[i], zi = z[i];
+        double vxi = vx[i], vyi = vy[i], vzi = vz[i];
+        double unused = 0.0;
+        verlet_axis(xi, vxi, unused, ax, dt, dt2, true);
+        verlet_axis(yi, vyi, unused, ay, dt, dt2, true);
+        verlet_axis(zi, vzi, unused, az, dt, dt2, true);
+        x[i] = xi; y[i] = yi; z[i] = zi;
+        vx[i] = vxi; vy[i] = vyi; vz[i] = vzi;
+        b.x = (float)xi;
+        b.y = (float)yi;
+        b.z = (float)zi;
+        body4[i] = b;
+        top = max_abs_bits(b);
+    }
+    track_max(ext, top);  // (every thread of the block)
 }
 
 // One RK4 stage (rk4.rs:33-178) for body i, given the stage state q (x, y, z,
@@ -325,36 +402,40 @@ __device__ __forceinline__ void rk4_stage(int stage, const double q[6], const do
 __global__ void rk4_stage_kernel(float4 *body4, const double *mass, const uint8_t *fixed,
                                  const double *partial, int splits, int n, double *x, double *y,
                                  double *z, double *vx, double *vy, double *vz, double *save,
-                                 double *ksum, double dt, int stage)
+                                 double *ksum, double dt, int stage, Track ext)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const bool fx = fixed[i] != 0;
-    double a[3];
-    body_acc(partial, splits, n, i, fx, mass[i], a[0], a[1], a[2]);
-    double *st[6] = {x, y, z, vx, vy, vz};
-    double q[6], e[6], S[6], out[6];
-    for (int c = 0; c < 6; ++c) q[c] = st[c][i];
-    if (stage == 1) {
-        for (int c = 0; c < 6; ++c) {
-            e[c] = q[c];
-            save[(size_t)c * n + i] = q[c];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t top = 0;
+    if (i < n) {
+        const bool fx = fixed[i] != 0;
+        double a[3];
+        body_acc(partial, splits, n, i, fx, mass[i], a[0], a[1], a[2]);
+        double *st[6] = {x, y, z, vx, vy, vz};
+        double q[6], e[6], S[6], out[6];
+        for (int c = 0; c < 6; ++c) q[c] = st[c][i];
+        if (stage == 1) {
+            for (int c = 0; c < 6; ++c) {
+                e[c] = q[c];
+                save[(size_t)c * n + i] = q[c];
+            }
+        } else {
+            for (int c = 0; c < 6; ++c) {
+                e[c] = save[(size_t)c * n + i];
+                S[c] = ksum[(size_t)c * n + i];
+            }
         }
-    } else {
-        for (int c = 0; c < 6; ++c) {
-            e[c] = save[(size_t)c * n + i];
-            S[c] = ksum[(size_t)c * n + i];
-        }
+        rk4_stage(stage, q, a, e, S, fx, dt, out);
+        if (stage < 4)
+            for (int c = 0; c < 6; ++c) ksum[(size_t)c * n + i] = S[c];
+        for (int c = 0; c < 6; ++c) st[c][i] = out[c];
+        float4 b = body4[i];
+        b.x = (float)out[0];
+        b.y = (float)out[1];
+        b.z = (float)out[2];
+        body4[i] = b;
+        top = max_abs_bits(b);
     }
-    rk4_stage(stage, q, a, e, S, fx, dt, out);
-    if (stage < 4)
-        for (int c = 0; c < 6; ++c) ksum[(size_t)c * n + i] = S[c];
-    for (int c = 0; c < 6; ++c) st[c][i] = out[c];
-    float4 b = body4[i];
-    b.x = (float)out[0];
-    b.y = (float)out[1];
-    b.z = (float)out[2];
-    body4[i] = b;
+    track_max(ext, top);  // (every thread of the block)
 }
 
 __global__ void euler_aos_kernel(const Entity *in, Entity *out, const Acceleration *acc, int n,
@@ -464,15 +545,16 @@ int host_direct(int device, bool *direct)
 void bodies_free(DeviceBodies &b, cudaStream_t stream)
 {
     void *ptrs[] = {b.body4, b.fixed, b.x,  b.y,  b.z,      b.vx, b.vy,    b.vz,
-                    b.px,    b.py,    b.pz, b.m,  b.radius, b.id, b.aos, b.scale};
+                    b.px,    b.py,    b.pz, b.m,  b.radius, b.id, b.aos, b.scale, b.mass256};
     for (void *p : ptrs) dev_free(p, stream);
     b = DeviceBodies();
 }
 
-int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, cudaStream_t stream)
+int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, bool with_scale,
+                   cudaStream_t stream)
 {
     size_t need = pad_bodies(n);
-    if (need <= b.cap && (!with_state || b.x)) {
+    if (need <= b.cap && (!with_state || b.x) && (!with_scale || b.scale)) {
         b.n = n;
         return PHYSIM_OK;
     }
@@ -483,8 +565,11 @@ int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, cudaStream_t stre
     PG_TRY(dev_alloc(b.fixed, need, stream));
     PG_TRY(dev_alloc(b.aos, need, stream));
     PG_TRY(dev_alloc(b.m, need, stream));
-    PG_TRY(dev_alloc(b.scale, 1, stream));
-    PG_CUDA(cudaMemsetAsync(b.scale, 0, sizeof(PairScale), stream));
+    if (with_scale) {
+        PG_TRY(dev_alloc(b.scale, 1, stream));
+        PG_CUDA(cudaMemsetAsync(b.scale, 0, sizeof(PairScale), stream));
+        PG_TRY(dev_alloc(b.mass256, need / kThreads, stream));
+    }
     if (with_state) {
         double **d[] = {&b.x, &b.y, &b.z, &b.vx, &b.vy, &b.vz, &b.px, &b.py, &b.pz, &b.radius};
         for (double **p : d) PG_TRY(dev_alloc(*p, need, stream));
@@ -493,16 +578,70 @@ int bodies_reserve(DeviceBodies &b, size_t n, bool with_state, cudaStream_t stre
     return PHYSIM_OK;
 }
 
+namespace {
+
+// The tracked halves of the largest |coordinate|; they change places once the
+// kernel is launched.
+Track next_extent(const DeviceBodies &b)
+{
+    if (!b.scale) return Track();
+    return {&b.scale->ext[b.ext_half ^ 1], &b.scale->ext[b.ext_half]};
+}
+
+__global__ void settle_kernel(uint32_t *ext, int eh, uint32_t *mass, int mh)
+{
+    ext[eh] = ext[eh ^ 1];
+    ext[eh ^ 1] = 0u;
+    if (mass) {
+        mass[mh] = mass[mh ^ 1];
+        mass[mh ^ 1] = 0u;
+    }
+}
+
+// After a kernel that filled the other halves: they are current from here on.
+// Inside a capture (the caller's, whose graph may be launched any number of
+// times) the values move instead, so that every launch finds them where this
+// one did.
+int swap_halves(DeviceBodies &b, bool mass_too, cudaStream_t stream)
+{
+    PG_CUDA(cudaGetLastError());
+    if (!b.scale) return PHYSIM_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PG_CUDA(cudaStreamIsCapturing(stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {
+        settle_kernel<<<1, 1, 0, stream>>>(b.scale->ext, b.ext_half,
+                                           mass_too ? b.scale->mass : nullptr, b.mass_half);
+        PG_CUDA(cudaGetLastError());
+        return PHYSIM_OK;
+    }
+    b.ext_half ^= 1;
+    if (mass_too) b.mass_half ^= 1;
+    return PHYSIM_OK;
+}
+
+// Threads per block of the integrators: small states in small blocks, over more
+// SMs (a block of 256 keeps one SM's f64 pipe busy for 3 us).
+int integrator_threads(size_t n) { return n <= 40000 ? 64 : kThreads; }
+
+int integrator_blocks(size_t n)
+{
+    const size_t t = (size_t)integrator_threads(n);
+    return (int)((n + t - 1) / t);
+}
+
+}  // namespace
+
 int launch_unpack(DeviceBodies &b, const Entity *aos, size_t n, bool full_state,
                   cudaStream_t stream)
 {
     size_t n_pad = pad_bodies(n);
     if (n_pad == 0) return PHYSIM_OK;
+    Track mass;
+    if (b.scale) mass = {&b.scale->mass[b.mass_half ^ 1], &b.scale->mass[b.mass_half]};
     unpack_kernel<<<blocks_for(n_pad), kThreads, 0, stream>>>(
         aos, (int)n, (int)n_pad, b.body4, b.fixed, full_state ? b.x : nullptr, b.y, b.z, b.vx,
-        b.vy, b.vz, b.m, b.radius, b.id);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+        b.vy, b.vz, b.m, b.radius, b.id, next_extent(b), mass, b.mass256);
+    return swap_halves(b, true, stream);
 }
 
 int launch_pack(DeviceBodies &b, cudaStream_t stream)
@@ -539,22 +678,20 @@ int launch_verlet(DeviceBodies &b, const double *partial, int splits, double dt,
                   cudaStream_t stream)
 {
     if (b.n == 0) return PHYSIM_OK;
-    verlet_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(
+    verlet_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
         b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.px, b.py,
-        b.pz, dt, initial ? 1 : 0);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+        b.pz, dt, initial ? 1 : 0, next_extent(b));
+    return swap_halves(b, false, stream);
 }
 
 int launch_euler(DeviceBodies &b, const double *partial, int splits, double dt,
                  cudaStream_t stream)
 {
     if (b.n == 0) return PHYSIM_OK;
-    euler_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(b.body4, b.m, b.fixed, partial, splits,
-                                                           (int)b.n, b.x, b.y, b.z, b.vx, b.vy,
-                                                           b.vz, dt);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+    euler_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
+        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, dt,
+        next_extent(b));
+    return swap_halves(b, false, stream);
 }
 
 int launch_rk4_stage(DeviceBodies &b, const double *partial, int splits, double dt, int stage,
@@ -562,11 +699,10 @@ int launch_rk4_stage(DeviceBodies &b, const double *partial, int splits, double 
 {
     if (b.n == 0) return PHYSIM_OK;
     PG_CHECK(stage >= 1 && stage <= 4, PHYSIM_ERR_ARGUMENT, "rk4 stage %d", stage);
-    rk4_stage_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(
+    rk4_stage_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
         b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, save,
-        ksum, dt, stage);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+        ksum, dt, stage, next_extent(b));
+    return swap_halves(b, false, stream);
 }
 
 int launch_euler_aos(const Entity *d_in, Entity *d_out, const Acceleration *d_acc, size_t n,

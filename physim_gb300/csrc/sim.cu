@@ -38,8 +38,10 @@ struct PhysimSim {
     // Barnes-Hut build is ~100 short kernels whose launch cost would
     // otherwise dominate at small N.
     bool use_graph = true;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    // one per current half of the pair-law maxima (PairScale), which the
+    // captured kernels read by address
+    cudaGraph_t graph[4] = {};
+    cudaGraphExec_t graph_exec[4] = {};
     double *diag = nullptr;  // 9 f64 diagnostics sums
     // rk4 (rk4.rs:24-178): the entity state saved at stage 1 and the running
     // sum of the k's, 6 x n f64 each
@@ -93,17 +95,31 @@ int sim_forces(PhysimSim *s, int *splits_out)
     const PhysimSimConfig &c = s->cfg;
     if (c.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO) {
         *splits_out = s->plan.splits;
-        return launch_direct(s->plan, s->b.body4, (float)c.e, s->b.scale, s->partial, s->stream,
-                             s->profiling ? s->ev[3] : nullptr);
+        return launch_direct(s->plan, s->b.body4, s->b.mass256, (float)c.e, s->b.scale_ref(),
+                             s->partial, s->stream, s->profiling ? s->ev[3] : nullptr);
     }
     *splits_out = 1;
     return bh_accelerations(s->bh, s->b, bh_params(c), s->partial, s->stream);
+}
+
+// The graph of the current halves.
+int graph_slot(const PhysimSim *s) { return s->b.ext_half | s->b.mass_half << 1; }
+
+void drop_graphs(PhysimSim *s)
+{
+    for (int k = 0; k < 4; ++k) {
+        if (s->graph_exec[k]) cudaGraphExecDestroy(s->graph_exec[k]);
+        if (s->graph[k]) cudaGraphDestroy(s->graph[k]);
+        s->graph_exec[k] = nullptr;
+        s->graph[k] = nullptr;
+    }
 }
 
 // Captures the gravity phase into a graph.  If the stream cannot be captured
 // (e.g. the caller is itself capturing), the simulation stays eager.
 int sim_capture(PhysimSim *s)
 {
+    const int k = graph_slot(s);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PG_CUDA(cudaStreamIsCapturing(s->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) {
@@ -124,14 +140,14 @@ int sim_capture(PhysimSim *s)
         s->use_graph = false;
         return PHYSIM_OK;
     }
-    if (cudaGraphInstantiate(&s->graph_exec, g, 0) != cudaSuccess) {
+    if (cudaGraphInstantiate(&s->graph_exec[k], g, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         cudaGraphDestroy(g);
-        s->graph_exec = nullptr;
+        s->graph_exec[k] = nullptr;
         s->use_graph = false;
         return PHYSIM_OK;
     }
-    s->graph = g;
+    s->graph[k] = g;
     return PHYSIM_OK;
 }
 
@@ -188,7 +204,7 @@ int physim_gpu_sim_create(const PhysimSimConfig *cfg, size_t n, PhysimSim **out)
         }
         s->own_stream = true;
     }
-    rc = bodies_reserve(s->b, n, true, s->stream);
+    rc = bodies_reserve(s->b, n, true, cfg->gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO, s->stream);
     size_t partial_elems = 3 * (n ? n : 1);
     if (rc == PHYSIM_OK && cfg->gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO) {
         s->plan = plan_direct((int)n, cfg->device, cfg->compensated != 0);
@@ -279,9 +295,10 @@ int generate_host(int kind, const void *params, Entity *out, size_t n, int32_t d
 // kernels themselves when the stream cannot be captured.
 int sim_gravity(PhysimSim *s, int *splits)
 {
-    if (s->use_graph && !s->graph_exec) PG_TRY(sim_capture(s));
-    if (s->graph_exec) {
-        PG_CUDA(cudaGraphLaunch(s->graph_exec, s->stream));
+    const int k = graph_slot(s);
+    if (s->use_graph && !s->graph_exec[k]) PG_TRY(sim_capture(s));
+    if (s->graph_exec[k]) {
+        PG_CUDA(cudaGraphLaunch(s->graph_exec[k], s->stream));
         *splits = s->cfg.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO ? s->plan.splits : 1;
         return PHYSIM_OK;
     }
@@ -375,8 +392,8 @@ int physim_gpu_sim_autotune(PhysimSim *s, PhysimDirectTuning *out)
         for (int rep = 0; rep < 3 && rc == PHYSIM_OK; ++rep) {
             if (cudaEventRecord(a, s->stream) != cudaSuccess) rc = PHYSIM_ERR_CUDA;
             if (rc == PHYSIM_OK)
-                rc = launch_direct(cand[c], s->b.body4, (float)s->cfg.e, s->b.scale, s->partial,
-                                   s->stream);
+                rc = launch_direct(cand[c], s->b.body4, s->b.mass256, (float)s->cfg.e,
+                                   s->b.scale_ref(), s->partial, s->stream);
             if (rc == PHYSIM_OK && (cudaEventRecord(b, s->stream) != cudaSuccess ||
                                     cudaEventSynchronize(b) != cudaSuccess))
                 rc = PHYSIM_ERR_CUDA;
@@ -398,10 +415,7 @@ int physim_gpu_sim_autotune(PhysimSim *s, PhysimDirectTuning *out)
     if (best >= 0) {
         s->plan = cand[best];
         // the captured gravity phase used the old plan
-        if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-        if (s->graph) cudaGraphDestroy(s->graph);
-        s->graph_exec = nullptr;
-        s->graph = nullptr;
+        drop_graphs(s);
     }
     if (out) {
         out->block = (uint32_t)s->plan.block;
@@ -488,10 +502,7 @@ int physim_gpu_sim_set_plan(PhysimSim *s, const PhysimDirectTuning *plan)
     }
     s->plan = p;
     // the captured gravity phase used the old plan
-    if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
-    s->graph_exec = nullptr;
-    s->graph = nullptr;
+    drop_graphs(s);
     return PHYSIM_OK;
 }
 
@@ -505,10 +516,7 @@ int physim_gpu_sim_set_profiling(PhysimSim *s, int enable)
     if (s->bh) PG_TRY(bh_set_profiling(s->bh, s->profiling));
     // the captured gravity phase must be re-captured with (or without) the
     // traversal and pair-kernel events
-    if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
-    s->graph_exec = nullptr;
-    s->graph = nullptr;
+    drop_graphs(s);
     return PHYSIM_OK;
 }
 
@@ -657,8 +665,7 @@ void physim_gpu_sim_destroy(PhysimSim *s)
     cudaSetDevice(s->cfg.device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     // the graph references the buffers: destroy it before they are freed
-    if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
+    drop_graphs(s);
     bodies_free(s->b, s->stream);
     dev_free(s->partial, s->stream);
     dev_free(s->acc_soa, s->stream);

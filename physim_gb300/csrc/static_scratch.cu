@@ -112,14 +112,12 @@ extern "C" int physim_gpu_simple_astro_accumulate_static(const Entity *state, si
     view.m = (double *)(base + kOffMass);
     view.fixed = (uint8_t *)(base + kOffFixed);
     double *partial = (double *)(base + kOffPartial);
-    PairScale *scale = (PairScale *)(base + kOffScale);
+    view.scale = (PairScale *)(base + kOffScale);
 
     // The f32 copy is rewritten for all padded slots (zero mass past n), and
-    // every partial sum is overwritten by the pair kernel.  The scale pass's
-    // arrival count must start at zero: it is left at zero by every completed
-    // pass, and cleared here as well (a memset, not an allocation), so a call
-    // after an interrupted one still starts clean.
-    PG_CUDA(cudaMemsetAsync(&scale->arrivals, 0, sizeof(uint32_t), st));
+    // every partial sum is overwritten by the pair kernel.  The maxima that
+    // unpack adds to start at zero.
+    PG_CUDA(cudaMemsetAsync(view.scale, 0, sizeof(PairScale), st));
     PG_TRY(launch_unpack(view, state, n, false, st));
     const int sms = device_sm_count(device);
     const int block = 128, ipt = 4;
@@ -129,7 +127,7 @@ extern "C" int physim_gpu_simple_astro_accumulate_static(const Entity *state, si
     const DirectPlan plan = make_direct_plan((int)n, block, ipt, splits, true);
     PG_CHECK(plan.splits <= kStaticMaxSplits, PHYSIM_ERR_ARGUMENT, "internal: %d splits",
              plan.splits);
-    PG_TRY(launch_direct(plan, view.body4, (float)fabs(e), scale, partial, st));
+    PG_TRY(launch_direct(plan, view.body4, nullptr, (float)fabs(e), view.scale_ref(), partial, st));
     PG_TRY(launch_accumulate_aos(view, partial, plan.splits, acc, st));
     return PHYSIM_OK;
 }
