@@ -2867,12 +2867,13 @@ namespace {
 std::atomic<uint32_t> g_wait_limit{0};  // 0: kLookbackSpins
 std::atomic<int32_t> g_stall_tile{-1};
 std::atomic<int> g_sort_single{1};
+}  // namespace
+
 int wait_limit()
 {
     const uint32_t v = g_wait_limit.load();
     return v == 0u ? kLookbackSpins : (int)std::min<uint32_t>(v, (uint32_t)INT32_MAX);
 }
-}  // namespace
 
 // Extent, keys and sort of a state whose tiles are all resident.
 static int launch_tree_sort(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, int n,

@@ -116,8 +116,8 @@ static double wave_efficiency(long units, long slots)
     return (double)units / (double)(waves * slots);
 }
 
-// Bodies from which the heuristic plan evaluates each unordered pair once.
-// Measured on GB300 (step of the best one-pair plan vs the symmetric plan):
+// Bodies from which the heuristic plan evaluates each unordered pair once (below
+// kDirectSmallMax bodies compensated states take direct_small.cu).  Measured on GB300 (step of the best one-pair plan vs the symmetric plan):
 // 4,098 bodies 25 vs 37 us, 6,000 31 vs 39, 8,192 49 vs 38, 12,289 87 vs 73,
 // 16,387 139 vs 96, 65,536 1.81 vs 1.05 ms.
 constexpr int kSymmetricMinBodies = 7168;
@@ -175,8 +175,18 @@ DirectPlan plan_direct_one_pair(int n, int device, bool compensated)
     return best;
 }
 
+// Small states: blocks that own their bodies, with the one-pair plan's fields.
+static DirectPlan small_plan(int n, int device)
+{
+    DirectPlan p = plan_direct_one_pair(n, device, true);
+    p.small = true;
+    return p;
+}
+
 DirectPlan plan_direct(int n, int device, bool compensated)
 {
+    // (times on both sides of the line: direct_small.cu)
+    if (compensated && n <= direct_small_limit(device)) return small_plan(n, device);
     if (compensated && n >= kSymmetricMinBodies && symmetric_fits(n, device))
         return make_symmetric_plan(n);
     return plan_direct_one_pair(n, device, compensated);
@@ -214,6 +224,7 @@ int direct_candidates(int n, int device, bool compensated, DirectPlan *out, int 
     }
     if (compensated && n >= kSymmetricCandidateBodies && k < cap && symmetric_fits(n, device))
         out[k++] = make_symmetric_plan(n);
+    if (compensated && n <= direct_small_limit(device) && k < cap) out[k++] = small_plan(n, device);
     return k;
 }
 
@@ -264,6 +275,10 @@ int launch_direct(const DirectPlan &plan, const float4 *body4, const float *mass
 {
     if (plan.n <= 0) return PHYSIM_OK;
     PG_CHECK(scale.ext, PHYSIM_ERR_ARGUMENT, "no pair-scale workspace");
+    if (plan.small) {
+        PG_TRY(launch_direct_small(body4, plan.n, e, scale, partial, stream));
+        return pairs_done ? record_event(pairs_done, stream) : PHYSIM_OK;
+    }
     if (plan.symmetric)
         return launch_direct_symmetric(plan, body4, mass256, e, scale, partial, stream,
                                        pairs_done);

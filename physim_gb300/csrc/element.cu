@@ -74,7 +74,7 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
             rc = ensure_doubles(el->partial, el->partial_cap, direct_partial_doubles(el->plan), st);
         }
         PG_TRY(rc);
-        splits = el->plan.splits;
+        splits = el->plan.out_splits();
         PG_TRY(launch_direct(el->plan, el->bodies.body4, el->bodies.mass256, (float)el->e,
                              el->bodies.scale_ref(), el->partial, st));
     } else {

@@ -118,6 +118,10 @@ struct DirectPlan {
     bool symmetric = false;
     int tiles = 0;
     bool clusters = false;
+    // Blocks that own their bodies (direct_small.cu) run instead of the one-pair
+    // kernels that the fields above describe; the sums come out as one split.
+    bool small = false;
+    int out_splits() const { return small ? 1 : splits; }
 };
 
 // Heuristic plan that fills the GPU: picks the i-tile shape and the number of
@@ -152,6 +156,31 @@ int launch_direct(const DirectPlan &plan, const float4 *body4, const float *mass
 int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const float *mass256,
                             float e, ScaleRef scale, double *partial, cudaStream_t stream,
                             cudaEvent_t pairs_done);
+// Largest state of the blocks that own their bodies (compensated sums), by the
+// measured steps against the next best plan: see plan_direct.
+constexpr int kDirectSmallMax = 12500;
+int direct_small_limit(int device);
+// One force pass; partial: 3 n doubles, one split.
+int launch_direct_small(const float4 *body4, int n, float e, ScaleRef scale, double *partial,
+                        cudaStream_t stream);
+// Whole verlet steps in one launch: the other body array and the barrier's and
+// maxima's words.  Nothing is reserved on a device without cooperative launches.
+struct SmallWork {
+    uint32_t *words = nullptr;
+    float4 *body4 = nullptr;
+    bool unchecked = false;  // launches since the last check
+};
+struct DeviceBodies;
+int reserve_small(SmallWork &w, const DeviceBodies &b, int device, cudaStream_t stream);
+void free_small(SmallWork &w, cudaStream_t stream);
+int small_steps_per_launch(int n);
+int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int steps, bool initial,
+                       cudaStream_t stream);
+// Waits for the stream if steps were launched since the last check, then reports
+// a wait between two of them that gave up.
+int check_small_steps(SmallWork &w, cudaStream_t stream);
+// Polls after which a kernel's wait gives up (physim_gpu_set_wait_limit).
+int wait_limit();
 // Records `ev` on `stream`; inside a stream capture as an external event node.
 int record_event(cudaEvent_t ev, cudaStream_t stream);
 

@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "verlet_axis.cuh"
 
 namespace pg {
 
@@ -218,25 +219,6 @@ __global__ void combine_soa_kernel(const double *__restrict__ mass, const uint8_
     acc[i] = ax;
     acc[n + i] = ay;
     acc[2 * (size_t)n + i] = az;
-}
-
-// verlet.rs:33-39 (initial, Taylor step) and verlet.rs:64-70 (regular).
-__device__ __forceinline__ void verlet_axis(double &x, double &v, double &p, double a, double dt,
-                                            double dt2, bool initial)
-{
-    double xn, vn;
-    if (initial) {
-        // x + vx*dt + 0.5*a*dt^2 ; vx + a*dt
-        xn = __dadd_rn(__dadd_rn(x, __dmul_rn(v, dt)), __dmul_rn(__dmul_rn(0.5, a), dt2));
-        vn = __dadd_rn(v, __dmul_rn(a, dt));
-    } else {
-        // 2*x - prev + a*dt^2 ; (x' - x)/dt
-        xn = __dadd_rn(__dsub_rn(__dmul_rn(2.0, x), p), __dmul_rn(a, dt2));
-        vn = __ddiv_rn(__dsub_rn(xn, x), dt);
-    }
-    p = x;
-    x = xn;
-    v = vn;
 }
 
 __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *fixed,

@@ -27,6 +27,7 @@ struct PhysimSim {
     double *acc_soa = nullptr;
     pg::DirectPlan plan;
     pg::BhWorkspace *bh = nullptr;
+    pg::SmallWork small;   // whole verlet steps of a small direct sum
     bool history = false;  // verlet previous_state is valid
     bool uploaded = false;
     // Optional per-step timing: events around the gravity kernels and the
@@ -94,7 +95,7 @@ int sim_forces(PhysimSim *s, int *splits_out)
 {
     const PhysimSimConfig &c = s->cfg;
     if (c.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO) {
-        *splits_out = s->plan.splits;
+        *splits_out = s->plan.out_splits();
         return launch_direct(s->plan, s->b.body4, s->b.mass256, (float)c.e, s->b.scale_ref(),
                              s->partial, s->stream, s->profiling ? s->ev[3] : nullptr);
     }
@@ -221,6 +222,8 @@ int physim_gpu_sim_create(const PhysimSimConfig *cfg, size_t n, PhysimSim **out)
         rc = dev_alloc(s->partial, partial_elems, s->stream);
     }
     s->partial_cap = partial_elems;
+    if (rc == PHYSIM_OK && s->plan.small && cfg->integrator == PHYSIM_INTEGRATOR_VERLET)
+        rc = reserve_small(s->small, s->b, cfg->device, s->stream);
     if (rc == PHYSIM_OK && cfg->integrator == PHYSIM_INTEGRATOR_RK4) {
         const size_t m = 6 * (n ? n : 1);
         rc = dev_alloc(s->rk4_save, m, s->stream);
@@ -299,7 +302,7 @@ int sim_gravity(PhysimSim *s, int *splits)
     if (s->use_graph && !s->graph_exec[k]) PG_TRY(sim_capture(s));
     if (s->graph_exec[k]) {
         PG_CUDA(cudaGraphLaunch(s->graph_exec[k], s->stream));
-        *splits = s->cfg.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO ? s->plan.splits : 1;
+        *splits = s->cfg.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO ? s->plan.out_splits() : 1;
         return PHYSIM_OK;
     }
     return sim_forces(s, splits);
@@ -333,6 +336,18 @@ int physim_gpu_sim_step(PhysimSim *s, uint32_t steps)
     PG_CHECK(s, PHYSIM_ERR_ARGUMENT, "null simulation");
     PG_CHECK(s->uploaded, PHYSIM_ERR_ARGUMENT, "step before upload");
     PG_CUDA(cudaSetDevice(s->cfg.device));
+    if (s->n && s->plan.small && s->small.words && !s->profiling) {
+        // a small direct sum: many steps per launch
+        const uint32_t most = (uint32_t)small_steps_per_launch((int)s->n);
+        while (steps > 0) {
+            const uint32_t k = std::min(steps, most);
+            PG_TRY(launch_small_steps(s->b, s->small, (float)s->cfg.e, s->cfg.dt, (int)k,
+                                      !s->history, s->stream));
+            s->history = true;
+            steps -= k;
+        }
+        return PHYSIM_OK;
+    }
     for (uint32_t k = 0; k < steps; ++k) {
         if (s->n == 0) break;
         int splits = 1;
@@ -560,6 +575,7 @@ int physim_gpu_sim_download(PhysimSim *s, Entity *state, size_t n)
                                 s->stream));
     }
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    PG_TRY(check_small_steps(s->small, s->stream));
     return bh_check(s->bh, s->stream);
 }
 
@@ -578,6 +594,7 @@ int physim_gpu_sim_accelerations(PhysimSim *s, Acceleration *acc, size_t n)
     PG_CUDA(cudaMemcpyAsync(h.data(), s->acc_soa, 3 * n * sizeof(double), cudaMemcpyDeviceToHost,
                             s->stream));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    PG_TRY(check_small_steps(s->small, s->stream));
     PG_TRY(bh_check(s->bh, s->stream));
     for (size_t i = 0; i < n; ++i) {
         acc[i].x = h[i];
@@ -644,6 +661,7 @@ int physim_gpu_sim_synchronize(PhysimSim *s)
     PG_CHECK(s, PHYSIM_ERR_ARGUMENT, "null simulation");
     PG_CUDA(cudaSetDevice(s->cfg.device));
     PG_CUDA(cudaStreamSynchronize(s->stream));
+    PG_TRY(check_small_steps(s->small, s->stream));
     return bh_check(s->bh, s->stream);
 }
 
@@ -652,6 +670,7 @@ void *physim_gpu_sim_stream(PhysimSim *s) { return s ? (void *)s->stream : nullp
 int physim_gpu_sim_launches_per_step(PhysimSim *s)
 {
     if (!s) return 0;
+    if (s->plan.small && s->small.words && !s->profiling) return 1;  // or fewer: many steps in one
     // gravity launches + the integrator's kernel
     const int per_eval = s->cfg.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO
                              ? (s->plan.symmetric ? 2 : 1) + 1
@@ -673,6 +692,7 @@ void physim_gpu_sim_destroy(PhysimSim *s)
     dev_free(s->rk4_save, s->stream);
     dev_free(s->rk4_ksum, s->stream);
     bh_free(s->bh);
+    free_small(s->small, s->stream);
     for (cudaEvent_t e : s->ev)
         if (e) cudaEventDestroy(e);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
