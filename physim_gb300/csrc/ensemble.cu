@@ -14,7 +14,9 @@
 // Members from a plan's size threshold up evaluate each unordered pair once
 // (direct_sym_tile.cuh): a second persistent kernel pulls their 1,024-body
 // tile pairs, writing per-member f32 slot sums that the verlet kernel adds
-// with TwoSum; smaller members keep the one-pair units.
+// with TwoSum; smaller members keep the one-pair units.  The two kernels run side
+// by side, and both kinds of units are cut finer where a batch has few of them
+// (plan_ensemble): 30 members of 256 to 14,671 bodies 1.51 -> 0.33 ms a step.
 // One step is captured once (per work plan) into a CUDA graph and replayed
 // for every step.  Members can be resized in place (a finished member's slot
 // takes the next job; the work plan is rebuilt).  The autotuner times the candidate kernel shapes (threads x bodies per thread)
@@ -91,14 +93,25 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
                     const SymUnit *__restrict__ units, int n_units,
                     const unsigned long long *__restrict__ remaining, int *__restrict__ counter,
                     const int32_t *__restrict__ member_kx, const int32_t *__restrict__ member_km,
-                    float *__restrict__ slots)
+                    float *__restrict__ slots, int parts)
 {
+    // with parts > 1 a cluster of that many blocks shares out each unit
+    // (sym_tile_pair); its first block draws the units
     __shared__ float smem[kSymWarps * kSymTile * 3];
     __shared__ int next;
+    const int rank = parts > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0;
     for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(counter, 1);
-        __syncthreads();
-        const int u = next;
+        if (threadIdx.x == 0 && rank == 0) next = atomicAdd(counter, 1);
+        int u;
+        if (parts > 1) {
+            cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+            cluster.sync();
+            u = *cluster.map_shared_rank(&next, 0);
+            cluster.sync();  // every block has read it
+        } else {
+            __syncthreads();
+            u = next;
+        }
         if (u >= n_units) return;
         const SymUnit w = units[u];
         if (remaining[w.member] != 0) {
@@ -106,10 +119,10 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
             const int sk = pair_scale_from(member_kx[w.member], m.e), skm = member_km[w.member];
             if (w.I == w.J)
                 sym_tile_pair<true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                    skm, slots + m.soff, smem);
+                                    skm, slots + m.soff, smem, rank, parts);
             else
                 sym_tile_pair<false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                     skm, slots + m.soff, smem);
+                                     skm, slots + m.soff, smem, rank, parts);
         }
         __syncthreads();
     }
@@ -149,24 +162,47 @@ __global__ void ensemble_verlet_kernel(float4 *body4, const double *__restrict__
                 const size_t n3 = 3 * (size_t)m.n;
                 const float *p = slot_sums + m.soff + i;
                 float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
-                for (int t = 0; t < m.sym_tiles; ++t)
-                    for (int c = 0; c < 3; ++c) {
-                        float sum, err;
-                        two_sum(h[c], p[(size_t)t * n3 + (size_t)c * m.n], sum, err);
-                        h[c] = sum;
-                        l[c] += err;
-                    }
+                // four slots' loads in flight together
+                for (int t0 = 0; t0 < m.sym_tiles; t0 += 4) {
+                    float v[4][3];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (t0 + u < m.sym_tiles)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+                                v[u][c] = p[(size_t)(t0 + u) * n3 + (size_t)c * m.n];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (t0 + u < m.sym_tiles)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                float sum, err;
+                                two_sum(h[c], v[u][c], sum, err);
+                                h[c] = sum;
+                                l[c] += err;
+                            }
+                }
                 const double unsc =
                     pow2d(member_km[k] - 2 * pair_scale_from(member_kx[k], m.e));
                 ax = ((double)h[0] + (double)l[0]) * unsc;
                 ay = ((double)h[1] + (double)l[1]) * unsc;
                 az = ((double)h[2] + (double)l[2]) * unsc;
             } else {
-                for (int sp = 0; sp < m.splits; ++sp) {
-                    const double *p = partial + m.poff + (size_t)sp * 3 * m.n;
-                    ax += p[i];
-                    ay += p[m.n + i];
-                    az += p[2 * (size_t)m.n + i];
+                for (int s0 = 0; s0 < m.splits; s0 += 4) {
+                    double v[4][3];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (s0 + u < m.splits)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+                                v[u][c] = partial[m.poff + (size_t)((s0 + u) * 3 + c) * m.n + i];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (s0 + u < m.splits) {
+                            ax += v[u][0];
+                            ay += v[u][1];
+                            az += v[u][2];
+                        }
                 }
             }
             if (mass[s] == 0.0) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
@@ -291,10 +327,11 @@ struct Shape {
 };
 constexpr Shape kShapes[] = {{128, 2}, {128, 4}, {256, 4}, {256, 2}, {128, 8}};
 constexpr int kChunks[] = {4096, 8192, 16384, 65536};
-constexpr int kMinChunk = 4096;  // smallest j chunk any plan uses (sizes the partial sums)
+// Most j chunks a member of n bodies is split into (sizes the partial sums).
+inline int max_splits(int n) { return std::max((n + 4095) / 4096, std::min(8, (n + 255) / 256)); }
 // Default size from which members use the symmetric units, and the thresholds
 // the autotuner compares (INT32_MAX: none).
-constexpr int kEnsembleSymMin = 16384;
+constexpr int kEnsembleSymMin = 8192;
 constexpr int kSymMins[] = {8192, 16384, 32768, INT32_MAX};
 
 template <int BLOCK, int IPT>
@@ -326,6 +363,8 @@ struct PhysimEnsemble {
     int device = 0;
     bool own_stream = false;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;  // the one-pair units beside the tile pairs
+    cudaEvent_t forked = nullptr, joined = nullptr;
     std::vector<size_t> sizes;
     std::vector<size_t> caps;  // bodies each member's slot was created for
     std::vector<int32_t> offsets;
@@ -354,11 +393,11 @@ struct PhysimEnsemble {
     size_t sym_units_cap = 0;
     float *slot_sums = nullptr;  // f32 slot sums of the symmetric members
     size_t slot_cap = 0;
-    int sym_grid = 0;
+    int sym_grid = 0, sym_parts = 1;
     Entity *staging = nullptr;
     size_t staging_cap = 0;
     // plan
-    int block = 128, ipt = 4, chunk = 16384;
+    int block = 128, ipt = 2, chunk = 16384;
     int sym_min = kEnsembleSymMin;  // members from this many bodies use the symmetric units
     int grid = 0;
     bool tuned = false;
@@ -390,7 +429,6 @@ void drop_graph(PhysimEnsemble *E)
 // Builds member tiling and the work list for (block, ipt, chunk) and uploads them.
 int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
 {
-    const int chunk_tiles = std::max(1, chunk / block);
     {
         // the members' slot sums grow as n^2 (12 B per body and 1,024-body
         // tile); above a quarter of the device's memory every member takes
@@ -403,6 +441,19 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
             (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || slot_bytes > total_b / 4))
             sym_min = INT32_MAX;
     }
+    int per_sm = 1;
+    PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, ens_kernel(block, ipt, E->cfg.compensated != 0), block, 0));
+    E->grid = std::max(1, per_sm) * device_sm_count(E->device);
+    // The chunk is cut so that the one-pair units are at least four times the
+    // blocks that draw them: with fewer, one unit's blocks outlast the rest
+    // (30 members of 256 to 14,671 bodies: 135 units of up to 16,384 bodies for
+    // 456 blocks, 1.42 ms a step for 0.25 ms of pair arithmetic).
+    long long jbodies = 0;
+    for (const MemberInfo &mi : E->members)
+        if (mi.n < sym_min || E->cfg.compensated == 0)
+            jbodies += (long long)cdiv(mi.n, block * ipt) * mi.n;
+    const long long even = jbodies / (4ll * E->grid);
     std::vector<WorkUnit> units;
     std::vector<SymUnit> sym_units;
     std::vector<long long> cost;
@@ -410,6 +461,9 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     for (size_t k = 0; k < E->members.size(); ++k) {
         MemberInfo &mi = E->members[k];
         mi.n_jtiles = cdiv(mi.n, block);
+        const int chunk_k = std::max((int)std::min<long long>(chunk, even),
+                                     cdiv(mi.n, max_splits(mi.n)));
+        const int chunk_tiles = std::max(1, cdiv(chunk_k, block));
         mi.chunk_tiles = chunk_tiles;
         mi.splits = std::max(1, cdiv(mi.n_jtiles, chunk_tiles));
         mi.poff = poff;
@@ -474,10 +528,11 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     E->ipt = ipt;
     E->chunk = chunk;
     E->sym_min = sym_min;
-    int per_sm = 1;
-    PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, ens_kernel(block, ipt, E->cfg.compensated != 0), block, 0));
-    E->grid = std::max(1, per_sm) * device_sm_count(E->device);
+    // few tile pairs: each shared out over a cluster until there are about eight
+    // for every resident block
+    E->sym_parts = 1;
+    while (E->sym_parts < 8 && (long long)E->n_sym_units * E->sym_parts < 8ll * 4 * device_sm_count(E->device))
+        E->sym_parts *= 2;
     int sym_per_sm = 1;
     PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sym_per_sm, ensemble_sym_kernel,
                                                           kSymThreads, 0));
@@ -486,13 +541,33 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     return PHYSIM_OK;
 }
 
+// Both kinds of units, side by side where there are both: the one-pair blocks
+// fill the SMs that the tile pairs' last blocks leave.
 int launch_forces(PhysimEnsemble *E)
 {
+    const bool fork = E->n_sym_units > 0 && E->n_units > 0;
+    if (fork) {
+        PG_CUDA(cudaEventRecord(E->forked, E->stream));
+        PG_CUDA(cudaStreamWaitEvent(E->side, E->forked, 0));
+    }
     if (E->n_sym_units > 0) {
-        ensemble_sym_kernel<<<std::min(E->sym_grid, E->n_sym_units), kSymThreads, 0, E->stream>>>(
-            E->body4, E->mass256, E->d_members, E->d_sym_units, E->n_sym_units, E->remaining, E->counter + 1,
-            E->member_kx, E->member_km, E->slot_sums);
-        PG_CUDA(cudaGetLastError());
+        const int parts = E->sym_parts;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)std::min<long long>(E->sym_grid / parts, E->n_sym_units) * parts);
+        cfg.blockDim = dim3(kSymThreads);
+        cfg.stream = E->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)parts;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = parts > 1 ? 1 : 0;
+        PG_CUDA(cudaLaunchKernelEx(&cfg, ensemble_sym_kernel, (const float4 *)E->body4,
+                                   (const float *)E->mass256, (const MemberInfo *)E->d_members,
+                                   (const SymUnit *)E->d_sym_units, E->n_sym_units,
+                                   (const unsigned long long *)E->remaining, E->counter + 1,
+                                   (const int32_t *)E->member_kx, (const int32_t *)E->member_km,
+                                   E->slot_sums, parts));
     }
     if (E->n_units == 0) return PHYSIM_OK;
     void *fn = ens_kernel(E->block, E->ipt, E->cfg.compensated != 0);
@@ -500,14 +575,19 @@ int launch_forces(PhysimEnsemble *E)
     void *args[] = {(void *)&E->body4, (void *)&E->d_members, (void *)&E->d_units,
                     (void *)&E->n_units, (void *)&E->remaining, (void *)&E->counter,
                     (void *)&E->member_kx, (void *)&E->member_km, (void *)&E->partial};
-    PG_CUDA(cudaLaunchKernel(fn, dim3(E->grid), dim3(E->block), args, 0, E->stream));
+    PG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::min(E->grid, E->n_units)), dim3(E->block), args,
+                             0, fork ? E->side : E->stream));
+    if (fork) {
+        PG_CUDA(cudaEventRecord(E->joined, E->side));
+        PG_CUDA(cudaStreamWaitEvent(E->stream, E->joined, 0));
+    }
     return PHYSIM_OK;
 }
 
 int enqueue_step(PhysimEnsemble *E)
 {
     PG_TRY(launch_forces(E));
-    const int t = 256;
+    const int t = E->slots <= 40000 ? 64 : 256;  // small states over more SMs' f64 pipes
     ensemble_verlet_kernel<<<cdiv(E->slots, t), t, 0, E->stream>>>(
         E->body4, E->m, E->fixed, E->slot_member, E->d_members, E->remaining, E->done, E->partial,
         E->slot_sums, E->slots, E->x, E->y, E->z, E->vx, E->vy, E->vz, E->px, E->py, E->pz,
@@ -527,6 +607,9 @@ void free_ensemble(PhysimEnsemble *E)
                  E->d_sym_units, E->slot_sums, E->member_kx, E->member_km, E->member_ext};
     for (void *q : p) dev_free(q, E->stream);
     if (E->stream) cudaStreamSynchronize(E->stream);
+    if (E->forked) cudaEventDestroy(E->forked);
+    if (E->joined) cudaEventDestroy(E->joined);
+    if (E->side) cudaStreamDestroy(E->side);
 }
 
 }  // namespace
@@ -565,7 +648,7 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
         mi.dt = E->cfg.dt;
         E->members[k] = mi;
         slots += (long long)pad_bodies(sizes[k]);
-        partial_elems += 3LL * (long long)sizes[k] * cdiv((long long)sizes[k], kMinChunk);
+        partial_elems += 3LL * (long long)sizes[k] * max_splits((int)sizes[k]);
     }
     if (slots >= (1LL << 31)) {
         delete E;
@@ -579,6 +662,13 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
     } else if (cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking) == cudaSuccess) {
         E->own_stream = true;
     } else {
+        rc = PHYSIM_ERR_CUDA;
+    }
+    if (rc == PHYSIM_OK &&
+        (cudaStreamCreateWithFlags(&E->side, cudaStreamNonBlocking) != cudaSuccess ||
+         cudaEventCreateWithFlags(&E->forked, cudaEventDisableTiming) != cudaSuccess ||
+         cudaEventCreateWithFlags(&E->joined, cudaEventDisableTiming) != cudaSuccess)) {
+        set_error("stream or event creation failed");
         rc = PHYSIM_ERR_CUDA;
     }
 #define EA(ptr, cnt)                                                                        \
@@ -632,7 +722,7 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
             rc = PHYSIM_ERR_CUDA;
         }
     }
-    if (rc == PHYSIM_OK) rc = plan_ensemble(E, 128, 4, 16384, kEnsembleSymMin);
+    if (rc == PHYSIM_OK) rc = plan_ensemble(E, 128, 2, 16384, kEnsembleSymMin);
     if (rc != PHYSIM_OK) {
         free_ensemble(E);
         if (E->own_stream) cudaStreamDestroy(E->stream);
