@@ -244,7 +244,7 @@ struct SmallSteps {
     double *x[3], *v[3], *p[3];
     int n, steps, initial;
     float e;
-    double dt;
+    Divisor dt;
     uint32_t *ext;         // the state's largest |coordinate|: in and out
     const uint32_t *mass_max;
     uint32_t *ring;        // three maxima in turn
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_steps_kernel(SmallStep
     }
     uint32_t target = gridDim.x;
     bool ok = steps_barrier(a, target, &sh.ok);  // the ring is clear
-    const double dt2 = __dmul_rn(a.dt, a.dt);
+    const double dt2 = __dmul_rn(a.dt.value, a.dt.value);
     int cur = 0;
     for (int s = 0; ok && s < a.steps; ++s) {
         const int sk = pair_scale_exp(__uint_as_float(ext), a.e);
@@ -424,7 +424,7 @@ int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int st
     a.steps = steps;
     a.initial = initial ? 1 : 0;
     a.e = e;
-    a.dt = dt;
+    a.dt = make_divisor(dt);
     a.ext = &b.scale->ext[b.ext_half];
     a.mass_max = &b.scale->mass[b.mass_half];
     a.ring = w.words;

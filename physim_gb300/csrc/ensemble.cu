@@ -31,6 +31,7 @@
 #include "direct_sym_tile.cuh"
 #include "direct_tile.cuh"
 #include "engine.h"
+#include "verlet_axis.cuh"
 
 namespace pg {
 namespace {
@@ -43,7 +44,7 @@ struct MemberInfo {
     int64_t poff;         // first partial sum of the member
     int32_t splits;
     float e;
-    double dt;
+    Divisor dt;
     int32_t sym_tiles;    // > 0: tiles of the symmetric units, slot sums at soff
     int32_t pad;
     int64_t soff;         // first f32 slot sum of the member
@@ -208,24 +209,11 @@ __global__ void ensemble_verlet_kernel(float4 *body4, const double *__restrict__
             if (mass[s] == 0.0) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
         }
         const bool initial = done[k] == 0;
-        const double dt = m.dt, dt2 = __dmul_rn(dt, dt);
+        const double dt2 = __dmul_rn(m.dt.value, m.dt.value);
         double q[3] = {x[s], y[s], z[s]}, v[3] = {vx[s], vy[s], vz[s]},
                pr[3] = {px[s], py[s], pz[s]};
         const double a[3] = {ax, ay, az};
-        for (int c = 0; c < 3; ++c) {
-            double xn, vn;
-            if (initial) {
-                xn = __dadd_rn(__dadd_rn(q[c], __dmul_rn(v[c], dt)),
-                               __dmul_rn(__dmul_rn(0.5, a[c]), dt2));
-                vn = __dadd_rn(v[c], __dmul_rn(a[c], dt));
-            } else {
-                xn = __dadd_rn(__dsub_rn(__dmul_rn(2.0, q[c]), pr[c]), __dmul_rn(a[c], dt2));
-                vn = __ddiv_rn(__dsub_rn(xn, q[c]), dt);
-            }
-            pr[c] = q[c];
-            q[c] = xn;
-            v[c] = vn;
-        }
+        for (int c = 0; c < 3; ++c) verlet_axis(q[c], v[c], pr[c], a[c], m.dt, dt2, initial);
         x[s] = q[0]; y[s] = q[1]; z[s] = q[2];
         vx[s] = v[0]; vy[s] = v[1]; vz[s] = v[2];
         px[s] = pr[0]; py[s] = pr[1]; pz[s] = pr[2];
@@ -645,7 +633,7 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
         mi.off = (int32_t)slots;
         mi.n = (int32_t)sizes[k];
         mi.e = (float)E->cfg.e;
-        mi.dt = E->cfg.dt;
+        mi.dt = make_divisor(E->cfg.dt);
         E->members[k] = mi;
         slots += (long long)pad_bodies(sizes[k]);
         partial_elems += 3LL * (long long)sizes[k] * max_splits((int)sizes[k]);
@@ -779,7 +767,7 @@ int physim_gpu_ensemble_set_member(PhysimEnsemble *E, size_t index, double e, do
     PG_CHECK(index < E->members.size(), PHYSIM_ERR_ARGUMENT, "member %zu out of range", index);
     PG_CUDA(cudaSetDevice(E->device));
     E->members[index].e = (float)fabs(e);
-    E->members[index].dt = dt;
+    E->members[index].dt = make_divisor(dt);
     PG_CUDA(cudaMemcpyAsync(E->d_members + index, &E->members[index], sizeof(MemberInfo),
                             cudaMemcpyHostToDevice, E->stream));
     const unsigned long long r = steps_remaining;

@@ -161,6 +161,17 @@ __device__ __forceinline__ void body_acc(const double *partial, int splits, int 
 {
     ax = ay = az = 0.0;
     if (fixed) return;
+    if (splits == 1) {
+        // 0 + p without an f64 operation: p, and +0 for -0
+        auto plus_zero = [](double p) {
+            return __double_as_longlong(p) == (long long)(1ull << 63) ? 0.0 : p;
+        };
+        ax = plus_zero(partial[i]);
+        ay = plus_zero(partial[(size_t)n + i]);
+        az = plus_zero(partial[2 * (size_t)n + i]);
+        if (mass == 0.0) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
+        return;
+    }
     // four splits' loads in flight together (summed in split order): one after
     // another they were a chain of L2 round trips, 6 of 11 us at 17 splits
     constexpr int kAhead = 4;
@@ -225,7 +236,7 @@ __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *
                               const double *partial,
                               int splits, int n, double *x, double *y, double *z, double *vx,
                               double *vy, double *vz, double *px, double *py, double *pz,
-                              double dt, int initial, Track ext)
+                              Divisor dt, int initial, Track ext)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
@@ -244,7 +255,7 @@ __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *
         }
         double ax, ay, az;
         body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
-        const double dt2 = __dmul_rn(dt, dt);
+        const double dt2 = __dmul_rn(dt.value, dt.value);
         verlet_axis(xi, vxi, pxi, ax, dt, dt2, initial);
         verlet_axis(yi, vyi, pyi, ay, dt, dt2, initial);
         verlet_axis(zi, vzi, pzi, az, dt, dt2, initial);
@@ -261,7 +272,7 @@ __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *
 }
 
 __global__ void verlet_aos_kernel(const Entity *in, const Entity *prev, Entity *out, Entity *keep,
-                                  const Acceleration *acc, int n, double dt, int initial)
+                                  const Acceleration *acc, int n, Divisor dt, int initial)
 {
     __shared__ __align__(16) Entity s_e[kThreads];
     __shared__ __align__(16) Acceleration s_a[kThreads];
@@ -282,7 +293,7 @@ __global__ void verlet_aos_kernel(const Entity *in, const Entity *prev, Entity *
         vy = en.vy;
         vz = en.vz;
         const Acceleration a = s_a[threadIdx.x];
-        const double dt2 = __dmul_rn(dt, dt);
+        const double dt2 = __dmul_rn(dt.value, dt.value);
         double px = 0.0, py = 0.0, pz = 0.0;
         if (!initial) {
             px = prev[i].x;
@@ -313,7 +324,7 @@ __global__ void verlet_aos_kernel(const Entity *in, const Entity *prev, Entity *
 // body has a = 0 (transforms skip it) and still drifts with its velocity.
 __global__ void euler_kernel(float4 *body4, const double *mass, const uint8_t *fixed,
                              const double *partial, int splits, int n, double *x, double *y,
-                             double *z, double *vx, double *vy, double *vz, double dt, Track ext)
+                             double *z, double *vx, double *vy, double *vz, Divisor dt, Track ext)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
@@ -321,7 +332,7 @@ __global__ void euler_kernel(float4 *body4, const double *mass, const uint8_t *f
         float4 b = body4[i];
         double ax, ay, az;
         body_acc(partial, splits, n, i, fixed[i] != 0, mass[i], ax, ay, az);
-        const double dt2 = __dmul_rn(dt, dt);
+        const double dt2 = __dmul_rn(dt.value, dt.value);
         double xi = x[i], yi = y[i], zi = z[i];
         double vxi = vx[i], vyi = vy[i], vzi = vz[i];
         double unused = 0.0;
@@ -348,7 +359,7 @@ __global__ void euler_kernel(float4 *body4, const double *mass, const uint8_t *f
 // body (rk4.rs:165-171).
 __device__ __forceinline__ void rk4_stage(int stage, const double q[6], const double a[3],
                                           const double e[6], double S[6], bool fixed, double dt,
-                                          double out[6])
+                                          const Divisor &six, double out[6])
 {
     double k[6];
     for (int c = 0; c < 3; ++c) {
@@ -368,7 +379,7 @@ __device__ __forceinline__ void rk4_stage(int stage, const double q[6], const do
     } else if (stage == 3) {
         for (int c = 0; c < 6; ++c) out[c] = __dadd_rn(e[c], k[c]);
     } else if (!fixed) {
-        for (int c = 0; c < 6; ++c) out[c] = __dadd_rn(e[c], __ddiv_rn(S[c], 6.0));
+        for (int c = 0; c < 6; ++c) out[c] = __dadd_rn(e[c], divide(S[c], six));
     } else {
         for (int c = 0; c < 3; ++c) {
             out[c] = e[c];
@@ -384,7 +395,7 @@ __device__ __forceinline__ void rk4_stage(int stage, const double q[6], const do
 __global__ void rk4_stage_kernel(float4 *body4, const double *mass, const uint8_t *fixed,
                                  const double *partial, int splits, int n, double *x, double *y,
                                  double *z, double *vx, double *vy, double *vz, double *save,
-                                 double *ksum, double dt, int stage, Track ext)
+                                 double *ksum, double dt, int stage, Divisor six, Track ext)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
@@ -406,7 +417,7 @@ __global__ void rk4_stage_kernel(float4 *body4, const double *mass, const uint8_
                 S[c] = ksum[(size_t)c * n + i];
             }
         }
-        rk4_stage(stage, q, a, e, S, fx, dt, out);
+        rk4_stage(stage, q, a, e, S, fx, dt, six, out);
         if (stage < 4)
             for (int c = 0; c < 6; ++c) ksum[(size_t)c * n + i] = S[c];
         for (int c = 0; c < 6; ++c) st[c][i] = out[c];
@@ -421,13 +432,13 @@ __global__ void rk4_stage_kernel(float4 *body4, const double *mass, const uint8_
 }
 
 __global__ void euler_aos_kernel(const Entity *in, Entity *out, const Acceleration *acc, int n,
-                                 double dt)
+                                 Divisor dt)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     Entity en = in[i];
     const Acceleration a = acc[i];
-    const double dt2 = __dmul_rn(dt, dt);
+    const double dt2 = __dmul_rn(dt.value, dt.value);
     double unused = 0.0;
     verlet_axis(en.x, en.vx, unused, a.x, dt, dt2, true);
     verlet_axis(en.y, en.vy, unused, a.y, dt, dt2, true);
@@ -441,7 +452,7 @@ __global__ void euler_aos_kernel(const Entity *in, Entity *out, const Accelerati
 // alias q.
 __global__ void rk4_aos_stage_kernel(const Entity *ent, const Entity *q_in,
                                      const Acceleration *f, double *ksum, Entity *out, int n,
-                                     double dt, int stage)
+                                     double dt, int stage, Divisor six)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -454,7 +465,7 @@ __global__ void rk4_aos_stage_kernel(const Entity *ent, const Entity *q_in,
     double S[6] = {0, 0, 0, 0, 0, 0}, r[6];
     if (stage > 1)
         for (int c = 0; c < 6; ++c) S[c] = ksum[(size_t)c * n + i];
-    rk4_stage(stage, q, a, e, S, en.fixed, dt, r);
+    rk4_stage(stage, q, a, e, S, en.fixed, dt, six, r);
     if (stage < 4)
         for (int c = 0; c < 6; ++c) ksum[(size_t)c * n + i] = S[c];
     Entity o = en;
@@ -662,7 +673,7 @@ int launch_verlet(DeviceBodies &b, const double *partial, int splits, double dt,
     if (b.n == 0) return PHYSIM_OK;
     verlet_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
         b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.px, b.py,
-        b.pz, dt, initial ? 1 : 0, next_extent(b));
+        b.pz, make_divisor(dt), initial ? 1 : 0, next_extent(b));
     return swap_halves(b, false, stream);
 }
 
@@ -671,8 +682,8 @@ int launch_euler(DeviceBodies &b, const double *partial, int splits, double dt,
 {
     if (b.n == 0) return PHYSIM_OK;
     euler_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
-        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, dt,
-        next_extent(b));
+        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz,
+        make_divisor(dt), next_extent(b));
     return swap_halves(b, false, stream);
 }
 
@@ -683,7 +694,7 @@ int launch_rk4_stage(DeviceBodies &b, const double *partial, int splits, double 
     PG_CHECK(stage >= 1 && stage <= 4, PHYSIM_ERR_ARGUMENT, "rk4 stage %d", stage);
     rk4_stage_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
         b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, save,
-        ksum, dt, stage, next_extent(b));
+        ksum, dt, stage, make_divisor(6.0), next_extent(b));
     return swap_halves(b, false, stream);
 }
 
@@ -691,7 +702,8 @@ int launch_euler_aos(const Entity *d_in, Entity *d_out, const Acceleration *d_ac
                      double dt, cudaStream_t stream)
 {
     if (n == 0) return PHYSIM_OK;
-    euler_aos_kernel<<<blocks_for(n), kThreads, 0, stream>>>(d_in, d_out, d_acc, (int)n, dt);
+    euler_aos_kernel<<<blocks_for(n), kThreads, 0, stream>>>(d_in, d_out, d_acc, (int)n,
+                                                             make_divisor(dt));
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }
@@ -703,7 +715,7 @@ int launch_rk4_aos_stage(const Entity *d_ent, const Entity *d_q, const Accelerat
     if (n == 0) return PHYSIM_OK;
     PG_CHECK(stage >= 1 && stage <= 4, PHYSIM_ERR_ARGUMENT, "rk4 stage %d", stage);
     rk4_aos_stage_kernel<<<blocks_for(n), kThreads, 0, stream>>>(d_ent, d_q, d_f, ksum, d_out,
-                                                                 (int)n, dt, stage);
+                                                                 (int)n, dt, stage, make_divisor(6.0));
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }
@@ -714,7 +726,7 @@ int launch_verlet_aos(const Entity *in, const Entity *d_prev, Entity *out, Entit
 {
     if (n == 0) return PHYSIM_OK;
     verlet_aos_kernel<<<blocks_for(n), kThreads, 0, stream>>>(in, d_prev, out, keep, acc, (int)n,
-                                                              dt, initial ? 1 : 0);
+                                                              make_divisor(dt), initial ? 1 : 0);
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }
