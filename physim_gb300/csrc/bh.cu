@@ -61,7 +61,7 @@ constexpr size_t kSortSmem = (size_t)kSortTile * (sizeof(uint64_t) + sizeof(uint
 constexpr int kMaxLevels = 31;
 
 constexpr int kTravWarps = 4;
-constexpr int kStack = 192;
+constexpr int kStack = 320;
 
 // flags[0]: node capacity exceeded (tree truncated; results stay exact)
 // flags[1]: traversal stack overflow (results of the affected warp invalid)
@@ -2042,18 +2042,29 @@ __device__ __forceinline__ void fold(float &hi, float &lo, float &t)
     t = 0.f;
 }
 
+// An opened cell: its children and the bodies that opened it.
 struct StackEntry {
-    int32_t node;
+    int32_t first, count;
     uint32_t mask;
 };
 
+// A warp walks its 32 bodies' own lists together: a stack of opened cells, each
+// with the mask of the bodies that opened it.  A turn takes up to 32 / nchild
+// opened cells and reads all their children at once, one lane each (geometry,
+// centre of mass, record), then tests child after child for the bodies of its
+// parent's mask.  Nothing is read inside that: an opened leaf of one body is its
+// own centre of mass, and the record of an opened cell goes on the stack.  (One
+// cell per turn, with its record, its leaves' bodies and its centres read when
+// they were needed, was three or four L2 round trips per cell: 71 us at 50,021
+// bodies, theta 0.5.)
 __global__ void __launch_bounds__(kTravWarps * 32)
 traverse_exact_kernel(TravArgs a_in)
 {
     __shared__ StackEntry stack[kTravWarps][kStack];
-    __shared__ float4 child_geo[kTravWarps][8];  // the children being tested
-    __shared__ float4 child_lo[kTravWarps][8];
-    __shared__ int4 child_meta[kTravWarps][8];
+    __shared__ float4 child_geo[kTravWarps][32];  // the children being tested
+    __shared__ float4 child_lo[kTravWarps][32];
+    __shared__ float4 child_com[kTravWarps][32];
+    __shared__ int4 child_meta[kTravWarps][32];
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
     TravArgs a = a_in;
@@ -2079,17 +2090,17 @@ traverse_exact_kernel(TravArgs a_in)
     // accepted lanes take the cell's monopole (and quadrupole); the lanes that
     // open a leaf take its bodies here; an internal cell opened by any lane
     // goes on the stack with those lanes, to have its children tested.
-    auto visit = [&](int node, uint32_t mask, float4 geo, float4 gl, int4 meta) {
+    auto visit = [&](int node, uint32_t mask, float4 geo, float4 gl, float4 com, int4 meta) {
         const bool in = (mask >> lane) & 1u;
         bool acc = false;
         if (in) {
             acc = accept_cell(a, node, geo, gl, q, ql, k);
-            if (acc && a.com_theta > 0.f) acc = com_guard(a, geo, a.nd.com[node], q.x, q.y, q.z);
+            if (acc && a.com_theta > 0.f) acc = com_guard(a, geo, com, q.x, q.y, q.z);
         }
         const uint32_t open = mask & ~__ballot_sync(0xffffffffu, acc);
         ++visits;
         if (acc) {
-            const float4 cm = scaled(a.nd.com[node], a.sc, a.msc);
+            const float4 cm = scaled(com, a.sc, a.msc);
             pair_acc(qs.x, qs.y, qs.z, cm, a.es, ax, ay, az);
             if (a.quad)
                 quad_acc(qs.x, qs.y, qs.z, cm, scaled2(a.nd.quad_a[node], sc2),
@@ -2101,14 +2112,18 @@ traverse_exact_kernel(TravArgs a_in)
         if (meta.y < 0) {
             const int b = meta.z, c = meta.w;
             const bool mine = (open >> lane) & 1u;
-            for (int j = b; j < b + c; ++j) {
-                const float4 bj = scaled(a.sbody[j], a.sc, a.msc);
-                if (mine) pair_acc(qs.x, qs.y, qs.z, bj, a.es, ax, ay, az);
+            if (c == 1) {  // the leaf's body is its centre of mass
+                if (mine) pair_acc(qs.x, qs.y, qs.z, scaled(com, a.sc, a.msc), a.es, ax, ay, az);
+            } else {
+                for (int j = b; j < b + c; ++j) {
+                    const float4 bj = scaled(a.sbody[j], a.sc, a.msc);
+                    if (mine) pair_acc(qs.x, qs.y, qs.z, bj, a.es, ax, ay, az);
+                }
             }
             if (mine) pairs += c;
             since_fold += c;
         } else if (sp < kStack) {
-            if (lane == 0) stack[warp][sp] = {node, open};
+            if (lane == 0) stack[warp][sp] = {meta.y, (int32_t)((uint32_t)meta.x >> 28), open};
             ++sp;
         } else {
             overflow = true;
@@ -2120,25 +2135,32 @@ traverse_exact_kernel(TravArgs a_in)
             since_fold = 0;
         }
     };
-    visit(0, active, a.nd.geo[0], a.nd.geo_lo[0], a.nd.meta[0]);
+    visit(0, active, a.nd.geo[0], a.nd.geo_lo[0], a.nd.com[0], a.nd.meta[0]);
+    const int slots = a.nchild;  // lanes per taken cell
+    const int slot = lane / slots, which = lane - slot * slots;
     while (sp > 0 && !overflow) {
+        // (one cell a turn where the stack is deep: each level then adds at most 7)
+        const int m = sp > kStack - 32 - 7 * kMaxLevels ? 1 : min(32 / slots, sp);
         __syncwarp();
-        const StackEntry top = stack[warp][sp - 1];
-        --sp;
-        __syncwarp();
-        const int4 pm = a.nd.meta[top.node];
-        const int fc = pm.y, nc = (int)((uint32_t)pm.x >> 28);
-        // the children's records, one lane each, loaded together
-        if (lane < nc) {
-            child_geo[warp][lane] = a.nd.geo[fc + lane];
-            child_lo[warp][lane] = a.nd.geo_lo[fc + lane];
-            child_meta[warp][lane] = a.nd.meta[fc + lane];
+        StackEntry mine = {0, 0, 0u};
+        if (slot < m) mine = stack[warp][sp - 1 - slot];
+        sp -= m;
+        if (which < mine.count) {
+            const int x = mine.first + which;
+            child_geo[warp][lane] = a.nd.geo[x];
+            child_lo[warp][lane] = a.nd.geo_lo[x];
+            child_com[warp][lane] = a.nd.com[x];
+            child_meta[warp][lane] = a.nd.meta[x];
         }
-        __syncwarp();
-        // last child first, as the reference pops them (octree.rs:152-154)
+        __syncwarp();  // also: every lane has read the stack
 #pragma unroll 1
-        for (int c = nc - 1; c >= 0; --c)
-            visit(fc + c, top.mask, child_geo[warp][c], child_lo[warp][c], child_meta[warp][c]);
+        for (uint32_t todo = __ballot_sync(0xffffffffu, which < mine.count); todo;
+             todo &= todo - 1u) {
+            const int l = __ffs(todo) - 1;
+            visit(__shfl_sync(0xffffffffu, mine.first + which, l),
+                  __shfl_sync(0xffffffffu, mine.mask, l), child_geo[warp][l], child_lo[warp][l],
+                  child_com[warp][l], child_meta[warp][l]);
+        }
     }
     if (overflow && lane == 0) atomicOr(&a.flags[kFlagStack], 1u);
     fold(hx, lx, ax);
@@ -2212,8 +2234,12 @@ __device__ __forceinline__ int warp_exclusive_scan(int v, int lane, int &total)
 // kQuad: quadrupole corrections of accepted cells (the quadrupole tiles are
 // only sized in that instantiation, so the monopole kernel keeps its
 // registers and occupancy).
-template <bool kQuad, int S>
-__global__ void __launch_bounds__(S * 32, kQuad || S > 1 ? 1 : 28)
+// kGuard: the centre-of-mass guard may be on.  Its cells' centres are then read
+// with the cells, so neither the samples nor the per-body test below goes back to
+// memory (a broadcast load per asked cell was most of the quadrupole walk: 260
+// cells per group at 100,003 bodies).
+template <bool kQuad, bool kGuard, int S>
+__global__ void __launch_bounds__(S * 32, S > 1 ? (kGuard ? 6 : 7) : (kGuard ? 24 : 28))
 traverse_warp_kernel(TravArgs a_in)
 {
     using T = TeamSize<S>;
@@ -2278,6 +2304,7 @@ traverse_warp_kernel(TravArgs a_in)
     const float pmax = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
     const float theta = a.theta;
     const float need = (1.f + 2.8e-6f) / theta;
+    const float ct2 = a.com_theta * a.com_theta;
     if (tw == 0) {
         // four bodies spread over the group
 #pragma unroll
@@ -2411,10 +2438,21 @@ traverse_warp_kernel(TravArgs a_in)
         visits += m;
         int qref = 0, qcnt = 0, nchild = 0, first_child = 0;
         float4 geo = make_float4(0.f, 0.f, 0.f, 0.f);
+        float cx = 0.f, cy = 0.f, cz = 0.f, bm2 = 0.f;  // kGuard: centre of mass, b_max^2
         bool acc = false, maybe = false;
         if (tl < m) {
             geo = a.nd.geo[cell];
             const int4 meta = a.nd.meta[cell];
+            if (kGuard && ct2 > 0.f) {
+                const float4 cm = a.nd.com[cell];
+                cx = cm.x;
+                cy = cm.y;
+                cz = cm.z;
+                const float ox = cx - geo.x, oy = cy - geo.y, oz = cz - geo.z;
+                const float bm =
+                    fmaf(1.7320509f, geo.w, sqrtf(fmaf(ox, ox, fmaf(oy, oy, oz * oz))));
+                bm2 = bm * bm;
+            }
             const float cmax = fmaxf(fmaxf(fabsf(geo.x), fabsf(geo.y)), fabsf(geo.z));
             const float dx = fmaxf(fmaxf(lo_x - geo.x, geo.x - hi_x), 0.f);
             const float dy = fmaxf(fmaxf(lo_y - geo.y, geo.y - hi_y), 0.f);
@@ -2424,18 +2462,13 @@ traverse_warp_kernel(TravArgs a_in)
             // r - (2e-7 (bmax + cmax) + 5e-7 r) must exceed extent (1 + 2e-6) / theta
             const float t = fmaf(geo.w, need, 2.000002e-7f * (bmax + cmax));
             acc = theta > 0.f && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > t * t;
-            if (acc && a.com_theta > 0.f) {
+            if (kGuard && acc && ct2 > 0.f) {
                 // centre-of-mass guard against the whole box (distance from c
                 // to the box is a lower bound of every body's |x - c|)
-                const float4 cm = a.nd.com[cell];
-                const float ox = cm.x - geo.x, oy = cm.y - geo.y, oz = cm.z - geo.z;
-                const float bmax =
-                    fmaf(1.7320509f, geo.w, sqrtf(fmaf(ox, ox, fmaf(oy, oy, oz * oz))));
-                const float ex = fmaxf(fmaxf(lo_x - cm.x, cm.x - hi_x), 0.f);
-                const float ey = fmaxf(fmaxf(lo_y - cm.y, cm.y - hi_y), 0.f);
-                const float ez = fmaxf(fmaxf(lo_z - cm.z, cm.z - hi_z), 0.f);
-                const float rc2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-                acc = bmax * bmax < a.com_theta * a.com_theta * rc2;
+                const float ex = fmaxf(fmaxf(lo_x - cx, cx - hi_x), 0.f);
+                const float ey = fmaxf(fmaxf(lo_y - cy, cy - hi_y), 0.f);
+                const float ez = fmaxf(fmaxf(lo_z - cz, cz - hi_z), 0.f);
+                acc = bm2 < ct2 * fmaf(ex, ex, fmaf(ey, ey, ez * ez));
             }
             if (acc) {
                 qref = -cell - 1;
@@ -2465,6 +2498,13 @@ traverse_warp_kernel(TravArgs a_in)
                 const float2 dz = add2(sample_z[u], make_float2(geo.z, geo.z));
                 const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
                 maybe = maybe && !(t2 * r2.x <= w2) && !(t2 * r2.y <= w2);
+                if (kGuard && ct2 > 0.f) {
+                    const float2 ex = add2(make_float2(xy.x, xy.y), make_float2(cx, cx));
+                    const float2 ey = add2(make_float2(xy.z, xy.w), make_float2(cy, cy));
+                    const float2 ez = add2(sample_z[u], make_float2(cz, cz));
+                    const float2 c2 = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
+                    maybe = maybe && bm2 < ct2 * c2.x && bm2 < ct2 * c2.y;
+                }
             }
         }
         uint32_t pend = __ballot_sync(0xffffffffu, maybe);
@@ -2481,10 +2521,13 @@ traverse_warp_kernel(TravArgs a_in)
             const float cm = fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fabsf(gz));
             const float rl = r - (2e-7f * (pmax + cm) + 5e-7f * r);
             bool ok = !valid || (rl > 0.f && gw * (1.f + 2e-6f) < theta * rl);
-            if (a.com_theta > 0.f) {
-                const int src_cell = __shfl_sync(0xffffffffu, cell, src);
-                const float4 c4 = a.nd.com[src_cell];
-                ok = ok && (!valid || com_guard(a, make_float4(gx, gy, gz, gw), c4, q.x, q.y, q.z));
+            if (kGuard && ct2 > 0.f) {
+                // com_guard for this body
+                const float ex = __shfl_sync(0xffffffffu, cx, src) - q.x;
+                const float ey = __shfl_sync(0xffffffffu, cy, src) - q.y;
+                const float ez = __shfl_sync(0xffffffffu, cz, src) - q.z;
+                const float b2 = __shfl_sync(0xffffffffu, bm2, src);
+                ok = ok && (!valid || b2 < ct2 * fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
             }
             if (__all_sync(0xffffffffu, ok) && lane == src) {
                 qref = -cell - 1;
@@ -3028,14 +3071,14 @@ static int bh_team(int n, const BhParams &p, int sms)
     return p.theta < 0.8 && groups_per_sm < 8 ? 4 : 1;
 }
 
-template <bool kQuad>
+template <bool kQuad, bool kGuard>
 static void launch_traverse_warp(const TravArgs &a, int team, cudaStream_t st)
 {
     const int groups = cdiv(a.n, 32);
     if (team == 4)
-        traverse_warp_kernel<kQuad, 4><<<groups, 128, 0, st>>>(a);
+        traverse_warp_kernel<kQuad, kGuard, 4><<<groups, 128, 0, st>>>(a);
     else
-        traverse_warp_kernel<kQuad, 1><<<groups, 32, 0, st>>>(a);
+        traverse_warp_kernel<kQuad, kGuard, 1><<<groups, 32, 0, st>>>(a);
 }
 
 int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, double *partial,
@@ -3080,9 +3123,11 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
     if (p.traversal == PHYSIM_TRAVERSAL_WARP) {
         const int team = bh_team(n, p, device_sm_count(ws->device));
         if (a.quad)
-            launch_traverse_warp<true>(a, team, st);
+            launch_traverse_warp<true, true>(a, team, st);
+        else if (a.com_theta > 0.f)
+            launch_traverse_warp<false, true>(a, team, st);
         else
-            launch_traverse_warp<false>(a, team, st);
+            launch_traverse_warp<false, false>(a, team, st);
     } else
         traverse_exact_kernel<<<blocks, kTravWarps * 32, 0, st>>>(a);
     PG_CUDA(cudaGetLastError());
