@@ -60,8 +60,6 @@ constexpr size_t kSortSmem = (size_t)kSortTile * (sizeof(uint64_t) + sizeof(uint
 
 constexpr int kMaxLevels = 31;
 
-constexpr int kTravWarps = 4;
-constexpr int kStack = 320;
 
 // flags[0]: node capacity exceeded (tree truncated; results stay exact)
 // flags[1]: traversal stack overflow (results of the affected warp invalid)
@@ -2057,14 +2055,21 @@ struct StackEntry {
 // cell per turn, with its record, its leaves' bodies and its centres read when
 // they were needed, was three or four L2 round trips per cell: 71 us at 50,021
 // bodies, theta 0.5.)
-__global__ void __launch_bounds__(kTravWarps * 32)
+// As in the warp traversal a team of S warps walks for one group, sharing the
+// stack: each warp takes its share of a turn's cells and keeps its opened ones
+// aside until the team puts them on the stack, in warp order.
+template <int S>
+__global__ void __launch_bounds__(S * 32, S > 1 ? 24 / S : 24)
 traverse_exact_kernel(TravArgs a_in)
 {
-    __shared__ StackEntry stack[kTravWarps][kStack];
-    __shared__ float4 child_geo[kTravWarps][32];  // the children being tested
-    __shared__ float4 child_lo[kTravWarps][32];
-    __shared__ float4 child_com[kTravWarps][32];
-    __shared__ int4 child_meta[kTravWarps][32];
+    constexpr int kCap = S == 1 ? 320 : 192 * S;
+    __shared__ StackEntry stack[kCap];
+    __shared__ StackEntry aside[S > 1 ? S : 1][S > 1 ? 32 : 1];
+    __shared__ int aside_count[S];
+    __shared__ float4 child_geo[S][32];  // the children being tested
+    __shared__ float4 child_lo[S][32];
+    __shared__ float4 child_com[S][32];
+    __shared__ int4 child_meta[S][32];
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
     TravArgs a = a_in;
@@ -2073,8 +2078,7 @@ traverse_exact_kernel(TravArgs a_in)
     const float sc2 = a.sc * a.sc * a.msc;
     unsigned long long visits = 0, pairs = 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k0 = (blockIdx.x * kTravWarps + warp) * 32;
-    if (k0 >= a.n) return;
+    const int k0 = blockIdx.x * 32;
     const int k = k0 + lane;
     const bool valid = k < a.n;
     const uint32_t active = __ballot_sync(0xffffffffu, valid);
@@ -2083,6 +2087,7 @@ traverse_exact_kernel(TravArgs a_in)
     const float4 qs = scaled(q, a.sc, a.msc);
     float ax = 0.f, ay = 0.f, az = 0.f, hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
     int sp = 0;
+    int put = 0;  // S > 1: cells kept aside this turn
     int since_fold = 0;
     bool overflow = false;
     // Tests cell `node` (geometry `geo`, record `meta`) for the lanes of
@@ -2122,8 +2127,12 @@ traverse_exact_kernel(TravArgs a_in)
             }
             if (mine) pairs += c;
             since_fold += c;
-        } else if (sp < kStack) {
-            if (lane == 0) stack[warp][sp] = {meta.y, (int32_t)((uint32_t)meta.x >> 28), open};
+        } else if (S > 1) {  // at most 32 per turn
+            if (lane == 0)
+                aside[warp][put] = {meta.y, (int32_t)((uint32_t)meta.x >> 28), open};
+            ++put;
+        } else if (sp < kCap) {
+            if (lane == 0) stack[sp] = {meta.y, (int32_t)((uint32_t)meta.x >> 28), open};
             ++sp;
         } else {
             overflow = true;
@@ -2135,15 +2144,40 @@ traverse_exact_kernel(TravArgs a_in)
             since_fold = 0;
         }
     };
-    visit(0, active, a.nd.geo[0], a.nd.geo_lo[0], a.nd.com[0], a.nd.meta[0]);
+    // the cells kept aside go on the stack, in warp order
+    auto settle = [&]() {
+        if (S == 1) return;
+        if (lane == 0) aside_count[warp] = put;
+        __syncthreads();  // also: every warp has taken its cells
+        int at = sp, total = 0;
+#pragma unroll
+        for (int w = 0; w < S; ++w) {
+            const int c = aside_count[w];
+            if (w < warp) at += c;
+            total += c;
+        }
+        if (sp + total > kCap)
+            overflow = true;
+        else if (lane < put)
+            stack[at + lane] = aside[warp][lane];
+        sp += total;
+        put = 0;
+        __syncthreads();
+    };
+    if (warp == 0)
+        visit(0, active, a.nd.geo[0], a.nd.geo_lo[0], a.nd.com[0], a.nd.meta[0]);
+    settle();
     const int slots = a.nchild;  // lanes per taken cell
+    const int per_warp = 32 / slots;
     const int slot = lane / slots, which = lane - slot * slots;
     while (sp > 0 && !overflow) {
         // (one cell a turn where the stack is deep: each level then adds at most 7)
-        const int m = sp > kStack - 32 - 7 * kMaxLevels ? 1 : min(32 / slots, sp);
+        const int m = sp > kCap - S * 32 - 7 * kMaxLevels ? 1 : min(S * per_warp, sp);
         __syncwarp();
         StackEntry mine = {0, 0, 0u};
-        if (slot < m) mine = stack[warp][sp - 1 - slot];
+        // dealt to the warps in turn
+        const int take = slot * S + warp;
+        if (slot < per_warp && take < m) mine = stack[sp - 1 - take];
         sp -= m;
         if (which < mine.count) {
             const int x = mine.first + which;
@@ -2161,6 +2195,7 @@ traverse_exact_kernel(TravArgs a_in)
                   __shfl_sync(0xffffffffu, mine.mask, l), child_geo[warp][l], child_lo[warp][l],
                   child_com[warp][l], child_meta[warp][l]);
         }
+        settle();
     }
     if (overflow && lane == 0) atomicOr(&a.flags[kFlagStack], 1u);
     fold(hx, lx, ax);
@@ -2170,6 +2205,33 @@ traverse_exact_kernel(TravArgs a_in)
     if (lane == 0) {
         atomicAdd(&a.stats[0], visits);
         atomicAdd(&a.stats[1], pairs);
+    }
+    if (S > 1) {
+        // the warps' sums, added in warp order (child_geo is free)
+        __syncthreads();
+        float *part = reinterpret_cast<float *>(&child_geo[0][0]);  // [S][3][32], then lows
+        float *low = reinterpret_cast<float *>(&child_com[0][0]);
+        part[(warp * 3 + 0) * 32 + lane] = hx;
+        part[(warp * 3 + 1) * 32 + lane] = hy;
+        part[(warp * 3 + 2) * 32 + lane] = hz;
+        low[(warp * 3 + 0) * 32 + lane] = lx;
+        low[(warp * 3 + 1) * 32 + lane] = ly;
+        low[(warp * 3 + 2) * 32 + lane] = lz;
+        __syncthreads();
+        if (warp > 0) return;
+        for (int w = 1; w < S; ++w) {
+            const int o = w * 3 * 32 + lane;
+            float sum, err;
+            two_sum(hx, part[o], sum, err);
+            hx = sum;
+            lx += err + low[o];
+            two_sum(hy, part[o + 32], sum, err);
+            hy = sum;
+            ly += err + low[o + 32];
+            two_sum(hz, part[o + 64], sum, err);
+            hz = sum;
+            lz += err + low[o + 64];
+        }
     }
     if (valid) {
         const uint32_t i = a.order[k];
@@ -3071,6 +3133,19 @@ static int bh_team(int n, const BhParams &p, int sms)
     return p.theta < 0.8 && groups_per_sm < 8 ? 4 : 1;
 }
 
+// Warps per group of the exact traversal, by the same trade.  Step times with
+// one / four / eight warps (us), leaf 1, Plummer: theta 0.3, 1,003 bodies 282 /
+// 145 / 119, 20,011 605 / 277 / 273, 250,007 2,015 / 2,009; theta 0.5, 1,003
+// bodies 190 / 114 / 103, 10,007 - / 148 / 127, 20,011 291 / 164 / 177, 50,021
+// 335 / 257 / 277, 100,003 406 / 413; quadtree, theta 0.5, 50,021 bodies 160 /
+// 153, 100,003 183 / 203; theta 1.0, 20,011 bodies 88 / 91 / 93.
+static int exact_team(int n, const BhParams &p, int sms)
+{
+    const double groups_per_sm = n / 32.0 / sms;
+    if (p.theta >= 0.8 || groups_per_sm > 16.0) return 1;
+    return groups_per_sm > 2.5 ? 4 : 8;
+}
+
 template <bool kQuad, bool kGuard>
 static void launch_traverse_warp(const TravArgs &a, int team, cudaStream_t st)
 {
@@ -3116,7 +3191,6 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
     a.sc = a.msc = 1.f;
     a.es = a.e;
     PG_CUDA(cudaMemsetAsync(ws->stats, 0, 2 * sizeof(unsigned long long), st));
-    const int blocks = cdiv(cdiv(n, 32), kTravWarps);
     // external records, so they also time the kernel when replayed from a graph
     if (ws->profiling)
         PG_CUDA(cudaEventRecordWithFlags(ws->trav_ev[0], st, cudaEventRecordExternal));
@@ -3129,7 +3203,15 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
         else
             launch_traverse_warp<false, false>(a, team, st);
     } else
-        traverse_exact_kernel<<<blocks, kTravWarps * 32, 0, st>>>(a);
+    {
+        const int team = exact_team(n, p, device_sm_count(ws->device)), groups = cdiv(n, 32);
+        if (team == 8)
+            traverse_exact_kernel<8><<<groups, 256, 0, st>>>(a);
+        else if (team == 4)
+            traverse_exact_kernel<4><<<groups, 128, 0, st>>>(a);
+        else
+            traverse_exact_kernel<1><<<groups, 32, 0, st>>>(a);
+    }
     PG_CUDA(cudaGetLastError());
     if (ws->profiling)
         PG_CUDA(cudaEventRecordWithFlags(ws->trav_ev[1], st, cudaEventRecordExternal));
