@@ -1152,6 +1152,12 @@ __device__ __forceinline__ float4 shfl_down4(float4 v, int o)
                        __shfl_down_sync(0xffffffffu, v.w, o));
 }
 
+__device__ __forceinline__ float4 shfl_xor4(float4 v, int o)
+{
+    return make_float4(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o),
+                       __shfl_xor_sync(0xffffffffu, v.z, o), __shfl_xor_sync(0xffffffffu, v.w, o));
+}
+
 // Sums of the next levels over the block's threads (thread t holds group
 // first + t of `level`, complete where first + t < groups(level)), by shuffles
 // within a warp and then over the warps' sums in shared memory; each complete
@@ -1221,6 +1227,7 @@ boundary_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ 
                 uint8_t *__restrict__ lcp, Segments sg, const uint32_t *__restrict__ flags)
 {
     static_assert(kSegBase == 4, "a thread's bodies are one 16-byte word of the order");
+    pdl_wait();
     if (sort_failed(flags)) return;
     __shared__ GroupSum warp_sum[kSegBlock / kSegBase / 32];
     __shared__ float4 warp_com[kSegBlock / kSegBase / 32];
@@ -1358,6 +1365,7 @@ mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, 
             int nchild, int leaf, uint32_t *__restrict__ mask, uint32_t *__restrict__ blk_cnt,
             int nblk, uint8_t *__restrict__ leafcnt, const uint32_t *__restrict__ flags)
 {
+    pdl_wait();
     if (sort_failed(flags)) return;
     // sM[p][t]: minimum of L over boundaries t .. t + 2^p - 1 of the tile
     // (clipped at the tile's end; every query below stays inside it)
@@ -1467,6 +1475,7 @@ level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
                   uint32_t *__restrict__ blk_off, LevelInfo *lv, int cap,
                   uint32_t *__restrict__ flags, Segments sg, int quad)
 {
+    pdl_wait();
     if (sort_failed(flags)) return;
     if (blockIdx.x == 1) {
         if (quad)
@@ -1536,6 +1545,7 @@ node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafc
             int n, int nchild, NodeArrays nd, const LevelInfo *__restrict__ lv,
             const uint32_t *__restrict__ flags)
 {
+    pdl_wait();
     if (sort_failed(flags)) return;
     __shared__ uint32_t sbal[kTreeBlock / 32][32];  // per warp and level: lanes with that bit
     __shared__ uint32_t woff[kTreeBlock / 32][32];  // ... and the level's nodes before the warp
@@ -1640,7 +1650,7 @@ __device__ __forceinline__ uint32_t compact2(uint64_t x)
 // to arrive) took 37 us at 8,195 bodies, 45 at 1,048,580 (leaf 16) and 124 at
 // 250,007 with one body per leaf: three dependent round trips to L2 per level of
 // the tree, whatever the size, after a centre pass of 6, 12 and 70 (the f64
-// chain of every centre).  This takes 14, 23 and 24 for both, and the group
+// chain of every centre).  This takes 9, 23 and 24 for both, and the group
 // sums add 1, 3 and 5 to the boundary pass.
 //
 // Each product m x is taken exactly (TwoProduct by FMA) and summed as
@@ -1692,48 +1702,59 @@ __global__ void snapshot_centre_kernel(const uint64_t *__restrict__ keys, NodeAr
     for (int p = 0; p < 4; ++p) out[(size_t)p * m + x] = c[p];
 }
 
-// Calls body(p) for the bodies of [b, e) outside complete groups and
-// group(a, left, z, right) for the groups, each once; loads go out together,
-// three bodies or two groups at a time.
-template <typename Body, typename Group>
-__device__ __forceinline__ void range_pieces(const Segments &sg, const float4 *__restrict__ sbody,
-                                             int b, int e, Body body, Group group)
-{
-    auto bodies = [&](int from, int to) {
-        for (int j = from; j < to; j += 3) {
-            float4 p[3];
-#pragma unroll
-            for (int u = 0; u < 3; ++u) p[u] = sbody[min(j + u, to - 1)];
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                if (j + u < to) body(p[u]);
+// The bodies [b, e) as pieces: at most three bodies before and three after the
+// complete groups, and per level k of the groups the one at its lower end if
+// that is odd and the one at its upper end if that is odd, where groups remain
+// (lo(k) < hi(k)).
+struct RangePieces {
+    int b, lo, hi, head, bodies;  // `bodies` loose ones, `head` of them before
+    __device__ __forceinline__ RangePieces(int begin, int end)
+    {
+        b = begin;
+        lo = (begin + kSegBase - 1) / kSegBase;
+        hi = end / kSegBase;
+        if (lo < hi) {
+            head = lo * kSegBase - begin;
+            bodies = head + end - hi * kSegBase;
+        } else {
+            head = bodies = end - begin;
         }
-    };
-    int lo = (b + kSegBase - 1) / kSegBase, hi = e / kSegBase;
-    bodies(b, lo < hi ? lo * kSegBase : e);
-    if (lo >= hi) return;
-    bodies(hi * kSegBase, e);
-    for (int k = 0; lo < hi; ++k, lo >>= 1, hi >>= 1) {
-        const bool left = lo & 1, right = hi & 1;
-        group(sg.off[k] + lo, left, sg.off[k] + hi - 1, right);
-        lo += left;
-        hi -= right;
     }
-}
+    __device__ __forceinline__ int body(int t) const
+    {
+        return t < head ? b + t : hi * kSegBase + t - head;
+    }
+    __device__ __forceinline__ int lo_at(int k) const { return (lo + (1 << k) - 1) >> k; }
+    __device__ __forceinline__ int hi_at(int k) const { return hi >> k; }
+};
 
-template <bool kQuad, bool kExact>
+// One lane per node, or eight: they share out the loose bodies and the groups'
+// levels, so that all of a node's reads are in flight together, and add their
+// sums by shuffles; the first three take an axis each for the geometry (f64) and
+// the quotients.  launch_cells picks.
+template <bool kQuad, bool kExact, int kLanes>
 __global__ void __launch_bounds__(256)
 cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody, NodeArrays nd,
             const LevelInfo *__restrict__ lv, int nchild, Segments sg,
             const unsigned long long *__restrict__ extent_bits,
             const uint32_t *__restrict__ flags)
 {
+    pdl_wait();
     if (sort_failed(flags)) return;
     const int total = lv->total;
     const int D = tree_levels(nchild), B = level_bits(nchild);
     const double X = __longlong_as_double((long long)*extent_bits);
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += gridDim.x * blockDim.x) {
-        const int l = nd.level[x], b = nd.begin[x], fc = nd.child[x];
+    constexpr int kBatch = kLanes == 1 ? 3 : 1;  // loose bodies read at a time
+    const int l = threadIdx.x & (kLanes - 1);  // lane of the node
+    const unsigned full = 0xffffffffu;
+    const int shift = (int)(threadIdx.x & 31) & ~(kLanes - 1);
+    const int per_grid = gridDim.x * (blockDim.x / kLanes);
+    const int first = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+    // (whole warps take part in the shuffles: the last turn repeats the last node)
+    for (int x0 = first - (threadIdx.x & 31) / kLanes; x0 < total; x0 += per_grid) {
+        const bool live = x0 + shift / kLanes < total;
+        const int x = live ? x0 + shift / kLanes : total - 1;
+        const int level = nd.level[x], b = nd.begin[x], fc = nd.child[x];
         const uint64_t key = keys[b];
         int e;
         if (fc < 0) {
@@ -1753,74 +1774,138 @@ cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody,
                 s = par;
                 par = nd.parent[s];
             }
-            int nc = 1;  // the nodes from fc on whose parent this is
+        }
+        // children: the nodes from fc on whose parent this is
+        int nc = 0;
 #pragma unroll
-            for (int k = 1; k < 8; ++k)
-                nc += k < nchild && fc + k < total && nd.parent[fc + k] == x;
-            nd.count[x] = e - b;
-            nd.nchild[x] = (uint8_t)nc;
-            nd.meta[x] = make_int4(x | (nc << 28), fc, b, e - b);
+        for (int k = 0; k < 8; k += kLanes) {
+            const bool mine = fc >= 0 && k + l < nchild && fc + k + l < total &&
+                              nd.parent[fc + k + l] == x;
+            if constexpr (kLanes == 1)
+                nc += mine;
+            else
+                nc += __popc((__ballot_sync(full, mine) >> shift) & ((1u << kLanes) - 1u));
+        }
+        // moments
+        const RangePieces pc(b, e);
+        GroupSum g = group_zero();
+        for (int t = l; t < pc.bodies; t += kLanes * kBatch) {
+            float4 p[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) p[u] = sbody[pc.body(min(t + u, pc.bodies - 1))];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (t + u < pc.bodies) df_add_body(g, p[u]);
+        }
+        for (int k = l; pc.lo_at(k) < pc.hi_at(k); k += kLanes) {
+            const int lo = pc.lo_at(k), hi = pc.hi_at(k);
+            GroupSum p = group_zero(), r = p;
+            if (lo & 1) {
+                p.h = sg.hi[sg.off[k] + lo];
+                p.l = sg.lo[sg.off[k] + lo];
+            }
+            if (hi & 1) {
+                r.h = sg.hi[sg.off[k] + hi - 1];
+                r.l = sg.lo[sg.off[k] + hi - 1];
+            }
+            if (lo & 1) df_add4(g, p);
+            if (hi & 1) df_add4(g, r);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = 1; o < kLanes; o <<= 1) {
+            GroupSum p;
+            p.h = shfl_xor4(g.h, o);
+            p.l = shfl_xor4(g.l, o);
+            df_add4(g, p);
         }
         // geometry
-        const uint64_t pre = l == 0 ? 0ull : key >> (B * (D - l));
-        const double h = X * pow2d(-l);  // the half-width, exact
-        const long long span = 1ll << l;
-        const uint32_t qx = nchild == 8 ? compact3(pre) : compact2(pre);
-        const uint32_t qy = nchild == 8 ? compact3(pre >> 1) : compact2(pre >> 1);
-        const double dx = h * (double)(2ll * qx + 1 - span);
-        const double dy = h * (double)(2ll * qy + 1 - span);
-        const double dz =
-            nchild == 8 ? h * (double)(2ll * compact3(pre >> 2) + 1 - span) : 0.0;
-        const float4 geo = make_float4((float)dx, (float)dy, (float)dz, (float)h);
-        nd.geo[x] = geo;
-        if (kExact)
-            nd.geo_lo[x] = make_float4((float)(dx - (double)geo.x), (float)(dy - (double)geo.y),
-                                       (float)(dz - (double)geo.z), 0.f);
-        // moments
-        GroupSum g = group_zero();
-        range_pieces(
-            sg, sbody, b, e, [&](float4 p) { df_add_body(g, p); },
-            [&](int a, bool left, int z, bool right) {
-                GroupSum p = group_zero(), r = p;
-                if (left) {
-                    p.h = sg.hi[a];
-                    p.l = sg.lo[a];
-                }
-                if (right) {
-                    r.h = sg.hi[z];
-                    r.l = sg.lo[z];
-                }
-                if (left) df_add4(g, p);
-                if (right) df_add4(g, r);
-            });
+        const uint64_t pre = level == 0 ? 0ull : key >> (B * (D - level));
+        const double h = X * pow2d(-level);  // the half-width, exact
+        const long long span = 1ll << level;
+        auto axis = [&](int c) {
+            const uint32_t q = nchild == 8 ? compact3(pre >> c) : compact2(pre >> c);
+            return c == 2 && nchild != 8 ? 0.0 : h * (double)(2ll * q + 1 - span);
+        };
+        float4 geo, low = make_float4(0.f, 0.f, 0.f, 0.f);
+        geo.w = (float)h;
+        if constexpr (kLanes == 1) {
+            const double dx = axis(0), dy = axis(1), dz = axis(2);
+            geo.x = (float)dx;
+            geo.y = (float)dy;
+            geo.z = (float)dz;
+            if (kExact)
+                low = make_float4((float)(dx - (double)geo.x), (float)(dy - (double)geo.y),
+                                  (float)(dz - (double)geo.z), 0.f);
+        } else {  // an axis per lane
+            const double d = axis(l < 3 ? l : 0);
+            const float df = (float)d;
+            geo.x = __shfl_sync(full, df, shift);
+            geo.y = __shfl_sync(full, df, shift + 1);
+            geo.z = __shfl_sync(full, df, shift + 2);
+            if (kExact) {
+                const float dl = (float)(d - (double)df);
+                low = make_float4(__shfl_sync(full, dl, shift), __shfl_sync(full, dl, shift + 1),
+                                  __shfl_sync(full, dl, shift + 2), 0.f);
+            }
+        }
         bool same = fc < 0;  // a leaf's bodies all at one position
         const float4 p0 = sbody[b];
         for (int j = b + 1; same && j < e; ++j) {
             const float4 p = sbody[j];
             same = p.x == p0.x && p.y == p0.y && p.z == p0.z;
         }
-        const float4 com = same ? make_float4(p0.x, p0.y, p0.z, g.h.x + g.l.x)
-                                : df_com(g.h, g.l, geo);
-        nd.com[x] = com;
+        __syncwarp();
+        float4 com;
+        if constexpr (kLanes == 1) {
+            com = df_com(g.h, g.l, geo);
+        } else {  // df_com, a quotient per lane
+            const float qh = l == 1 ? g.h.z : l == 2 ? g.h.w : g.h.y;
+            const float ql = l == 1 ? g.l.z : l == 2 ? g.l.w : g.l.y;
+            const float quot = df_div(qh, ql, g.h.x, g.l.x);
+            com = make_float4(__shfl_sync(full, quot, shift), __shfl_sync(full, quot, shift + 1),
+                              __shfl_sync(full, quot, shift + 2), g.h.x + g.l.x);
+            if (g.h.x == 0.f && g.l.x == 0.f) com = make_float4(geo.x, geo.y, geo.z, 0.f);
+        }
+        if (same) com = make_float4(p0.x, p0.y, p0.z, g.h.x + g.l.x);
+        if (live && l == 0) {
+            if (fc >= 0) {
+                nd.count[x] = e - b;
+                nd.nchild[x] = (uint8_t)nc;
+                nd.meta[x] = make_int4(x | (nc << 28), fc, b, e - b);
+            }
+            nd.geo[x] = geo;
+            if (kExact) nd.geo_lo[x] = low;
+            nd.com[x] = com;
+        }
         if (kQuad) {
             Quad6 q = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
-            if (!same)
-                range_pieces(
-                    sg, sbody, b, e, [&](float4 p) { quad_body_add(q, p, com); },
-                    [&](int a, bool left, int z, bool right) {
-                        if (left) {
-                            const float4 c = sg.com[a];
-                            quad_shift_add(q, quad_load(sg, a), c.w, c.x - com.x, c.y - com.y,
-                                           c.z - com.z);
-                        }
-                        if (right) {
-                            const float4 c = sg.com[z];
-                            quad_shift_add(q, quad_load(sg, z), c.w, c.x - com.x, c.y - com.y,
-                                           c.z - com.z);
-                        }
-                    });
-            nd.quad_a[x] = make_float4(q.v[0], q.v[1], q.v[2], q.v[0] + q.v[1] + q.v[2]);
-            nd.quad_b[x] = make_float4(q.v[3], q.v[4], q.v[5], 0.f);
+            if (!same) {
+                for (int t = l; t < pc.bodies; t += kLanes)
+                    quad_body_add(q, sbody[pc.body(t)], com);
+                for (int k = l; pc.lo_at(k) < pc.hi_at(k); k += kLanes) {
+                    const int lo = pc.lo_at(k), hi = pc.hi_at(k);
+                    if (lo & 1) {
+                        const float4 c = sg.com[sg.off[k] + lo];
+                        quad_shift_add(q, quad_load(sg, sg.off[k] + lo), c.w, c.x - com.x,
+                                       c.y - com.y, c.z - com.z);
+                    }
+                    if (hi & 1) {
+                        const float4 c = sg.com[sg.off[k] + hi - 1];
+                        quad_shift_add(q, quad_load(sg, sg.off[k] + hi - 1), c.w, c.x - com.x,
+                                       c.y - com.y, c.z - com.z);
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 1; o < kLanes; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < 6; ++c) q.v[c] += __shfl_xor_sync(full, q.v[c], o);
+            if (live && l == 0) {
+                nd.quad_a[x] = make_float4(q.v[0], q.v[1], q.v[2], q.v[0] + q.v[1] + q.v[2]);
+                nd.quad_b[x] = make_float4(q.v[3], q.v[4], q.v[5], 0.f);
+            }
         }
     }
 }
@@ -2070,6 +2155,7 @@ traverse_exact_kernel(TravArgs a_in)
     __shared__ float4 child_lo[S][32];
     __shared__ float4 child_com[S][32];
     __shared__ int4 child_meta[S][32];
+    pdl_wait();
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
     TravArgs a = a_in;
@@ -2313,6 +2399,7 @@ traverse_warp_kernel(TravArgs a_in)
     __shared__ float4 sample_xy[kSamples / 2];  // negated (x, x', y, y')
     __shared__ float2 sample_z[kSamples / 2];
     __shared__ int warp_total[2][S];
+    pdl_wait();
     // a failed sort left no tree to walk (the node arrays may hold anything)
     if (sort_failed(a_in.flags)) return;
     TravArgs a = a_in;
@@ -3062,6 +3149,33 @@ static int launch_split_sort(BhWorkspace *ws, const DeviceBodies &b, const BhPar
     return PHYSIM_OK;
 }
 
+template <int kLanes>
+static int launch_cells_lanes(const uint64_t *keys, BhWorkspace *ws, const BhParams &p,
+                              const Segments &sg, bool quad, bool exact, int blocks,
+                              cudaStream_t st)
+{
+    auto cells = quad ? (exact ? cell_kernel<true, true, kLanes> : cell_kernel<true, false, kLanes>)
+                      : (exact ? cell_kernel<false, true, kLanes>
+                               : cell_kernel<false, false, kLanes>);
+    return launch_pdl(cells, blocks, 256, st, keys, (const float4 *)ws->sbody, ws->nd,
+                      (const LevelInfo *)ws->lv, p.nchild, sg,
+                      (const unsigned long long *)ws->extent_bits, (const uint32_t *)ws->flags);
+}
+
+static int launch_cells(const uint64_t *keys, BhWorkspace *ws, int n, const BhParams &p,
+                        const Segments &sg, bool quad, bool exact, int sms, cudaStream_t st)
+{
+    // Eight lanes while the nodes (about 1.5 per body with one body per leaf, an
+    // eighth per body with 16) leave the SMs idle.  One lane vs eight (us): leaf
+    // 16, 2,003 bodies 12.0 / 7.9, 100,003 15.1 / 9.4, 200,003 15.9 / 13.8,
+    // 400,009 17.2 / 23.4; with quadrupoles 100,003 25.0 / 11.4, 400,009 28.7 /
+    // 29.4; leaf 1, 2,003 bodies 12.3 / 8.5, 20,011 13.5 / 12.9, 50,021 15.1 / 19.0.
+    const double leaf = std::max(1.0, 0.625 * p.leaf_size);
+    if (n <= (quad ? 30000.0 : 20000.0) * leaf)
+        return launch_cells_lanes<8>(keys, ws, p, sg, quad, exact, sms * 8, st);
+    return launch_cells_lanes<1>(keys, ws, p, sg, quad, exact, sms * 8, st);
+}
+
 static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, cudaStream_t st)
 {
     const int n = (int)b.n;
@@ -3091,24 +3205,22 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
     }
     auto boundary = quad ? (exact ? boundary_kernel<true, true> : boundary_kernel<true, false>)
                          : (exact ? boundary_kernel<false, true> : boundary_kernel<false, false>);
-    boundary<<<cdiv(n, kSegBlock), kSegBlock / kSegBase, 0, st>>>(
-        keys, ws->vals[cur], n, p.nchild, b.body4, b.x, b.y, b.z, ws->sbody, ws->sbody_lo, ws->lcp,
-        sg, ws->flags);
+    PG_TRY(launch_pdl(boundary, cdiv(n, kSegBlock), kSegBlock / kSegBase, st, keys,
+                      (const uint32_t *)ws->vals[cur], n, p.nchild, (const float4 *)b.body4,
+                      (const double *)b.x, (const double *)b.y, (const double *)b.z, ws->sbody,
+                      ws->sbody_lo, ws->lcp, sg, (const uint32_t *)ws->flags));
     const int tree_blocks = cdiv(n, kTreeBlock);
     PG_CHECK(p.leaf_size >= 1 && p.leaf_size <= kMaxLeaf, PHYSIM_ERR_ARGUMENT,
              "leaf size %d outside 1..%d", p.leaf_size, kMaxLeaf);
-    mask_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(keys, ws->lcp, n, p.nchild, p.leaf_size,
-                                                    ws->mask, ws->blk_cnt, tree_blocks,
-                                                    ws->leafcnt, ws->flags);
-    level_scan_kernel<<<2, 1024, 0, st>>>(ws->blk_cnt, tree_blocks, p.nchild, ws->blk_off, ws->lv,
-                                          ws->nd.cap, ws->flags, sg, quad ? 1 : 0);
-    node_kernel<<<tree_blocks, kTreeBlock, 0, st>>>(keys, ws->leafcnt, ws->mask, ws->blk_off,
-                                                    tree_blocks, n, p.nchild, ws->nd, ws->lv,
-                                                    ws->flags);
-    auto cells = quad ? (exact ? cell_kernel<true, true> : cell_kernel<true, false>)
-                      : (exact ? cell_kernel<false, true> : cell_kernel<false, false>);
-    cells<<<sms * 8, 256, 0, st>>>(keys, ws->sbody, ws->nd, ws->lv, p.nchild, sg, ws->extent_bits,
-                                   ws->flags);
+    PG_TRY(launch_pdl(mask_kernel, tree_blocks, kTreeBlock, st, keys, (const uint8_t *)ws->lcp, n,
+                      p.nchild, p.leaf_size, ws->mask, ws->blk_cnt, tree_blocks, ws->leafcnt,
+                      (const uint32_t *)ws->flags));
+    PG_TRY(launch_pdl(level_scan_kernel, 2, 1024, st, (const uint32_t *)ws->blk_cnt, tree_blocks,
+                      p.nchild, ws->blk_off, ws->lv, ws->nd.cap, ws->flags, sg, quad ? 1 : 0));
+    PG_TRY(launch_pdl(node_kernel, tree_blocks, kTreeBlock, st, keys, (const uint8_t *)ws->leafcnt,
+                      (const uint32_t *)ws->mask, (const uint32_t *)ws->blk_off, tree_blocks, n,
+                      p.nchild, ws->nd, (const LevelInfo *)ws->lv, (const uint32_t *)ws->flags));
+    PG_TRY(launch_cells(keys, ws, n, p, sg, quad, exact, sms, st));
     launches += 5;
     ws->nchild = p.nchild;
     ws->exact = exact;
@@ -3147,13 +3259,12 @@ static int exact_team(int n, const BhParams &p, int sms)
 }
 
 template <bool kQuad, bool kGuard>
-static void launch_traverse_warp(const TravArgs &a, int team, cudaStream_t st)
+static int launch_traverse_warp(const TravArgs &a, int team, cudaStream_t st)
 {
     const int groups = cdiv(a.n, 32);
     if (team == 4)
-        traverse_warp_kernel<kQuad, kGuard, 4><<<groups, 128, 0, st>>>(a);
-    else
-        traverse_warp_kernel<kQuad, kGuard, 1><<<groups, 32, 0, st>>>(a);
+        return launch_pdl(traverse_warp_kernel<kQuad, kGuard, 4>, groups, 128, st, a);
+    return launch_pdl(traverse_warp_kernel<kQuad, kGuard, 1>, groups, 32, st, a);
 }
 
 int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, double *partial,
@@ -3197,20 +3308,20 @@ int bh_accelerations(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, 
     if (p.traversal == PHYSIM_TRAVERSAL_WARP) {
         const int team = bh_team(n, p, device_sm_count(ws->device));
         if (a.quad)
-            launch_traverse_warp<true, true>(a, team, st);
+            PG_TRY((launch_traverse_warp<true, true>(a, team, st)));
         else if (a.com_theta > 0.f)
-            launch_traverse_warp<false, true>(a, team, st);
+            PG_TRY((launch_traverse_warp<false, true>(a, team, st)));
         else
-            launch_traverse_warp<false, false>(a, team, st);
+            PG_TRY((launch_traverse_warp<false, false>(a, team, st)));
     } else
     {
         const int team = exact_team(n, p, device_sm_count(ws->device)), groups = cdiv(n, 32);
         if (team == 8)
-            traverse_exact_kernel<8><<<groups, 256, 0, st>>>(a);
+            PG_TRY(launch_pdl(traverse_exact_kernel<8>, groups, 256, st, a));
         else if (team == 4)
-            traverse_exact_kernel<4><<<groups, 128, 0, st>>>(a);
+            PG_TRY(launch_pdl(traverse_exact_kernel<4>, groups, 128, st, a));
         else
-            traverse_exact_kernel<1><<<groups, 32, 0, st>>>(a);
+            PG_TRY(launch_pdl(traverse_exact_kernel<1>, groups, 32, st, a));
     }
     PG_CUDA(cudaGetLastError());
     if (ws->profiling)

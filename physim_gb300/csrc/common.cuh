@@ -84,5 +84,33 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &err)
     err = (a - ap) + (b - bp);
 }
 
+// Programmatic dependent launch (PTX griddepcontrol): a kernel launched by
+// launch_pdl may be set up, and its blocks start, while the kernel before it on
+// the stream still runs; pdl_wait, the first thing it does, returns when that one
+// has ended and its writes are visible.  It takes the launch latency (1 to 2 us)
+// out of a chain of short kernels.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+inline int launch_pdl(void (*kernel)(Params...), int grid, int block, cudaStream_t stream,
+                      Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PG_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+    return PHYSIM_OK;
+}
+
 }  // namespace pg
 #endif
