@@ -2452,7 +2452,7 @@ traverse_warp_kernel(TravArgs a_in)
                              fmaxf(fabsf(lo_z), fabsf(hi_z)));
     const float pmax = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
     const float theta = a.theta;
-    const float need = (1.f + 2.8e-6f) / theta;
+    const float need = (1.f + 2.5e-6f) / theta;
     const float ct2 = a.com_theta * a.com_theta;
     if (tw == 0) {
         // four bodies spread over the group
@@ -2608,9 +2608,17 @@ traverse_warp_kernel(TravArgs a_in)
             const float dz = fmaxf(fmaxf(lo_z - geo.z, geo.z - hi_z), 0.f);
             // f32 rounding of positions and centre moves r by at most
             // 1.1e-7 (|p| + |c|) + 3.5e-7 r against the reference's f64 value:
-            // r - (2e-7 (bmax + cmax) + 5e-7 r) must exceed extent (1 + 2e-6) / theta
-            const float t = fmaf(geo.w, need, 2.000002e-7f * (bmax + cmax));
-            acc = theta > 0.f && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > t * t;
+            // rmin = r - (2e-7 (bmax + cmax) + 5e-7 r) must exceed extent (1 + 2e-6) /
+            // theta.  Squared, for a root less; what is as near as the rounding of
+            // the squares (1e-6, one cell in a million) is decided by rmin itself.
+            const float t = fmaf(geo.w, need, 2.000001e-7f * (bmax + cmax));
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), t2 = t * t;
+            acc = theta > 0.f && r2 > t2;
+            if (fabsf(r2 - t2) <= 1e-6f * t2) {
+                const float r = sqrtf(r2);
+                const float rmin = r - (2e-7f * (bmax + cmax) + 5e-7f * r);
+                acc = theta > 0.f && rmin > 0.f && geo.w * (1.f + 2e-6f) < theta * rmin;
+            }
             if (kGuard && acc && ct2 > 0.f) {
                 // centre-of-mass guard against the whole box (distance from c
                 // to the box is a lower bound of every body's |x - c|)
