@@ -607,23 +607,21 @@ struct TreeSortArgs {
     int spin_limit, stall_tile;
 };
 
-// Grid barrier of the resident sort: the count must reach `target`.  A wait
+// Grid barrier of the resident kernels: the count must reach `want`.  A wait
 // that exceeds the limit raises the sort's error flag and sets the poison bit,
 // which ends every other wait.  False: some wait gave up.
-__device__ __forceinline__ bool tree_sort_barrier(const TreeSortArgs &a, uint32_t target,
-                                                  int *s_ok)
+__device__ __forceinline__ bool grid_barrier(uint32_t *count, uint32_t *flags, int spin_limit,
+                                             uint32_t want, int *s_ok)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> bar(*a.bar);
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> bar(*count);
         bar.fetch_add(1u, cuda::memory_order_release);
-        // the test hook's tile waits for a count that nothing reaches
-        const uint32_t want = (int)blockIdx.x == a.stall_tile ? kBarPoison : target;
         int spins = 0;
         uint32_t v;
         while ((v = bar.load(cuda::memory_order_acquire)) < want) {
-            if (++spins > a.spin_limit) {
-                atomicOr(&a.flags[kFlagSort], 1u);
+            if (++spins > spin_limit) {
+                atomicOr(&flags[kFlagSort], 1u);
                 v = bar.fetch_or(kBarPoison, cuda::memory_order_relaxed) | kBarPoison;
                 break;
             }
@@ -632,6 +630,14 @@ __device__ __forceinline__ bool tree_sort_barrier(const TreeSortArgs &a, uint32_
     }
     __syncthreads();
     return *s_ok != 0;
+}
+
+__device__ __forceinline__ bool tree_sort_barrier(const TreeSortArgs &a, uint32_t target,
+                                                  int *s_ok)
+{
+    // the test hook's tile waits for a count that nothing reaches
+    return grid_barrier(a.bar, a.flags, a.spin_limit,
+                        (int)blockIdx.x == a.stall_tile ? kBarPoison : target, s_ok);
 }
 
 template <int ITEMS>
@@ -1162,7 +1168,18 @@ __device__ __forceinline__ float4 shfl_xor4(float4 v, int o)
 // first + t of `level`, complete where first + t < groups(level)), by shuffles
 // within a warp and then over the warps' sums in shared memory; each complete
 // group is stored.
-template <bool kQuad>
+// kThreads threads take part, the block's first; fewer than the whole block
+// (kShare) meet at a named barrier.
+template <int kThreads, bool kShare>
+__device__ __forceinline__ void share_sync()
+{
+    if (kShare)
+        asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+    else
+        __syncthreads();
+}
+
+template <bool kQuad, int kThreads, bool kShare>
 __device__ __forceinline__ void block_groups(const Segments &sg, int level, int first,
                                              GroupSum g, float4 com, Quad6 q,
                                              GroupSum *warp_sum, float4 *warp_com,
@@ -1200,8 +1217,8 @@ __device__ __forceinline__ void block_groups(const Segments &sg, int level, int 
             warp_quad[warp] = q;
         }
     }
-    __syncthreads();
-    const int warps = (int)(blockDim.x >> 5);
+    share_sync<kThreads, kShare>();
+    constexpr int warps = kThreads / 32;
     if (warp == 0) {
         const int w = lane < warps ? lane : 0;
         g = warp_sum[w];
@@ -1213,72 +1230,91 @@ __device__ __forceinline__ void block_groups(const Segments &sg, int level, int 
     }
 }
 
-// L(k) for k >= 1 (the number of leading digits keys[k-1] and keys[k] share,
-// D for equal keys), the sorted f32 bodies (with kExact what f32 dropped of
-// their f64 positions), and the group sums of up to kSegBlock bodies.  Four
-// bodies a thread: the keys and the order come as 16-byte words and a thread's
-// bodies are its first group.
-template <bool kQuad, bool kExact>
-__global__ void __launch_bounds__(kSegBlock / kSegBase)
-boundary_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ order, int n,
-                int nchild, const float4 *__restrict__ body4, const double *__restrict__ bx,
-                const double *__restrict__ by, const double *__restrict__ bz,
-                float4 *__restrict__ sbody, float4 *__restrict__ sbody_lo,
-                uint8_t *__restrict__ lcp, Segments sg, const uint32_t *__restrict__ flags)
+// L(k) for k >= 1: the number of leading digits that a and b (keys k - 1 and k)
+// share, D for equal keys.
+__device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b, int nchild)
+{
+    const int D = tree_levels(nchild), B = level_bits(nchild);
+    const uint64_t x = a ^ b;
+    // keys use the low B * D bits: 64 - B * D leading bits are always 0
+    return x == 0 ? D : (__clzll((long long)x) - (64 - B * D)) / B;
+}
+
+struct GatherArgs {
+    const uint64_t *keys;
+    const uint32_t *order;
+    int n, nchild;
+    const float4 *body4;
+    const double *bx, *by, *bz;
+    float4 *sbody, *sbody_lo;
+    uint8_t *lcp;  // null: not kept
+    Segments sg;
+};
+
+template <int kThreads>
+struct GatherShared {
+    GroupSum sum[kThreads / 32];
+    float4 com[kThreads / 32];
+    Quad6 quad[kThreads / 32];
+};
+
+// The sorted f32 bodies (with kExact what f32 dropped of their f64 positions),
+// the L of lcp, and the group sums of kThreads * kSegBase bodies from group
+// `first` on, by the block's first kThreads threads.  Four bodies a thread: the
+// keys and the order come as 16-byte words and a thread's bodies are its first
+// group.
+template <bool kQuad, bool kExact, int kThreads, bool kShare>
+__device__ __forceinline__ void gather_groups(const GatherArgs &a, int first,
+                                              GatherShared<kThreads> &sh)
 {
     static_assert(kSegBase == 4, "a thread's bodies are one 16-byte word of the order");
-    pdl_wait();
-    if (sort_failed(flags)) return;
-    __shared__ GroupSum warp_sum[kSegBlock / kSegBase / 32];
-    __shared__ float4 warp_com[kSegBlock / kSegBase / 32];
-    __shared__ Quad6 warp_quad[kSegBlock / kSegBase / 32];
-    const int first = blockIdx.x * (kSegBlock / kSegBase);
     const int g0 = first + (int)threadIdx.x;  // this thread's group
     const int k0 = g0 * kSegBase;
-    const int D = tree_levels(nchild), B = level_bits(nchild);
-    const int cnt = max(0, min(kSegBase, n - k0));
+    const int cnt = max(0, min(kSegBase, a.n - k0));
     uint64_t key[kSegBase] = {0, 0, 0, 0};
     uint32_t ord[kSegBase] = {0, 0, 0, 0};
     if (cnt == kSegBase) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(keys + k0);
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(keys + k0 + 2);
-        const uint4 o = *reinterpret_cast<const uint4 *>(order + k0);
-        key[0] = a.x;
-        key[1] = a.y;
-        key[2] = b.x;
-        key[3] = b.y;
+        const uint4 o = *reinterpret_cast<const uint4 *>(a.order + k0);
         ord[0] = o.x;
         ord[1] = o.y;
         ord[2] = o.z;
         ord[3] = o.w;
+        if (a.lcp) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(a.keys + k0);
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(a.keys + k0 + 2);
+            key[0] = u.x;
+            key[1] = u.y;
+            key[2] = v.x;
+            key[3] = v.y;
+        }
     } else {
 #pragma unroll
         for (int u = 0; u < kSegBase; ++u)
             if (u < cnt) {
-                key[u] = keys[k0 + u];
-                ord[u] = order[k0 + u];
+                ord[u] = a.order[k0 + u];
+                if (a.lcp) key[u] = a.keys[k0 + u];
             }
     }
-    uint64_t prev = k0 > 0 && cnt > 0 ? keys[k0 - 1] : 0ull;
+    uint64_t prev = a.lcp && k0 > 0 && cnt > 0 ? a.keys[k0 - 1] : 0ull;
     float4 p[kSegBase];
 #pragma unroll
     for (int u = 0; u < kSegBase; ++u)
-        p[u] = u < cnt ? body4[ord[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        p[u] = u < cnt ? a.body4[ord[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
     GroupSum g = group_zero();
 #pragma unroll
     for (int u = 0; u < kSegBase; ++u) {
         if (u >= cnt) continue;
-        const uint64_t x = prev ^ key[u];
-        prev = key[u];
-        // keys use the low B * D bits: 64 - B * D leading bits are always 0
-        const int L = x == 0 ? D : (__clzll((long long)x) - (64 - B * D)) / B;
-        lcp[k0 + u] = (uint8_t)(k0 + u == 0 ? 0 : L);
-        sbody[k0 + u] = p[u];
+        if (a.lcp) {
+            const int L = shared_digits(prev, key[u], a.nchild);
+            prev = key[u];
+            a.lcp[k0 + u] = (uint8_t)(k0 + u == 0 ? 0 : L);
+        }
+        a.sbody[k0 + u] = p[u];
         if (kExact) {
             const uint32_t i = ord[u];
-            sbody_lo[k0 + u] = make_float4((float)(bx[i] - (double)p[u].x),
-                                           (float)(by[i] - (double)p[u].y),
-                                           (float)(bz[i] - (double)p[u].z), 0.f);
+            a.sbody_lo[k0 + u] = make_float4((float)(a.bx[i] - (double)p[u].x),
+                                             (float)(a.by[i] - (double)p[u].y),
+                                             (float)(a.bz[i] - (double)p[u].z), 0.f);
         }
         df_add_body(g, p[u]);
     }
@@ -1290,24 +1326,35 @@ boundary_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ 
         for (int u = 0; u < kSegBase; ++u)
             if (u < cnt) quad_body_add(q, p[u], com);
     }
-    if (g0 < sg.groups(0)) {
-        group_store(sg, sg.off[0] + g0, g);
-        if (kQuad) group_store_quad(sg, sg.off[0] + g0, com, q);
+    if (g0 < a.sg.groups(0)) {
+        group_store(a.sg, a.sg.off[0] + g0, g);
+        if (kQuad) group_store_quad(a.sg, a.sg.off[0] + g0, com, q);
     }
-    block_groups<kQuad>(sg, 0, first, g, com, q, warp_sum, warp_com, warp_quad);
+    block_groups<kQuad, kThreads, kShare>(a.sg, 0, first, g, com, q, sh.sum, sh.com, sh.quad);
 }
 
-// The group sums of more than kSegBlock bodies, by one block of 1,024 threads
-// (ten levels per round).
-template <bool kQuad>
-__device__ __forceinline__ void top_groups(const Segments &sg)
+template <bool kQuad, bool kExact>
+__global__ void __launch_bounds__(kSegBlock / kSegBase)
+boundary_kernel(GatherArgs a, const uint32_t *__restrict__ flags)
 {
-    __shared__ GroupSum warp_sum[32];
-    __shared__ float4 warp_com[32];
-    __shared__ Quad6 warp_quad[32];
-    for (int level = kSegBlockLevel; level < kSegLevels && sg.groups(level) > 1; level += 10) {
+    pdl_wait();
+    if (sort_failed(flags)) return;
+    constexpr int kThreads = kSegBlock / kSegBase;
+    __shared__ GatherShared<kThreads> sh;
+    gather_groups<kQuad, kExact, kThreads, false>(a, blockIdx.x * kThreads, sh);
+}
+
+// The group sums above level `from`, by one block of kThreads threads
+// (log2(kThreads) levels per round).
+template <bool kQuad, int kThreads>
+__device__ __forceinline__ void top_groups(const Segments &sg, int from)
+{
+    constexpr int kLevels = kThreads == 1024 ? 10 : 9;
+    static_assert(kThreads == 1 << kLevels, "512 or 1,024 threads");
+    __shared__ GatherShared<kThreads> sh;
+    for (int level = from; level < kSegLevels && sg.groups(level) > 1; level += kLevels) {
         const int m = sg.groups(level);
-        for (int first = 0; first < m; first += 1024) {
+        for (int first = 0; first < m; first += kThreads) {
             const int at = first + (int)threadIdx.x;
             GroupSum g = group_zero();
             float4 com = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1322,7 +1369,8 @@ __device__ __forceinline__ void top_groups(const Segments &sg)
                     q = {{a.x, a.y, a.z, b.x, b.y, b.z}};
                 }
             }
-            block_groups<kQuad>(sg, level, first, g, com, q, warp_sum, warp_com, warp_quad);
+            block_groups<kQuad, kThreads, false>(sg, level, first, g, com, q, sh.sum, sh.com,
+                                                 sh.quad);
             __syncthreads();  // the warps' sums serve the next chunk, the groups the next round
         }
     }
@@ -1355,43 +1403,49 @@ __device__ __forceinline__ int next_key_change(const uint64_t *__restrict__ keys
 // length by binary lifting (the longest run is the sum of the powers of two
 // whose windows, taken largest first, stay at or below the level), so every
 // body takes the same few steps instead of a loop of data-dependent length.
-constexpr int kTreeTile = kTreeBlock + 2 * kTreeHalo;
 constexpr int kMinTables = 7;  // windows of 2^0 .. 2^6 boundaries
 static_assert(kMaxLeaf <= (1 << (kMinTables - 1)) && kMaxLeaf + 1 < kTreeHalo,
               "leaf windows fit the tables and the halo");
 
-__global__ void __launch_bounds__(kTreeBlock)
-mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, int n,
-            int nchild, int leaf, uint32_t *__restrict__ mask, uint32_t *__restrict__ blk_cnt,
-            int nblk, uint8_t *__restrict__ leafcnt, const uint32_t *__restrict__ flags)
-{
-    pdl_wait();
-    if (sort_failed(flags)) return;
-    // sM[p][t]: minimum of L over boundaries t .. t + 2^p - 1 of the tile
+template <int kBlock>
+struct MaskShared {
+    // m[p][t]: minimum of L over boundaries t .. t + 2^p - 1 of the tile
     // (clipped at the tile's end; every query below stays inside it)
-    __shared__ int8_t sM[kMinTables][kTreeTile];
-    __shared__ uint32_t cnt[32];
+    int8_t m[kMinTables][kBlock + 2 * kTreeHalo];
+    uint32_t cnt[32];
+};
+
+// One tile of kBlock bodies, one thread each: its body's mask m and leaf count
+// lc, and the tile's counts to blk_cnt; shared(j) gives L(j).
+template <int kBlock, typename Shared>
+__device__ __forceinline__ void level_masks(const uint64_t *__restrict__ keys, Shared shared,
+                                            int tile, int n, int nchild, int leaf,
+                                            uint32_t *__restrict__ blk_cnt, int nblk,
+                                            MaskShared<kBlock> &sh, uint32_t &m, uint8_t &lc)
+{
+    constexpr int kTile = kBlock + 2 * kTreeHalo;
     const int D = tree_levels(nchild);
-    const int base = blockIdx.x * kTreeBlock;
+    const int base = tile * kBlock;
     // boundaries base - halo .. base + block + halo; -1 marks "no boundary
     // beyond here" (index 0 starts every run, indices >= n end them)
-    for (int t = threadIdx.x; t < kTreeTile; t += blockDim.x) {
+    for (int t = threadIdx.x; t < kTile; t += blockDim.x) {
         const int j = base - kTreeHalo + t;
-        sM[0][t] = (j >= 1 && j < n) ? (int8_t)lcp[j] : (int8_t)-1;
+        sh.m[0][t] = (j >= 1 && j < n) ? (int8_t)shared(j) : (int8_t)-1;
     }
-    if (threadIdx.x < 32) cnt[threadIdx.x] = 0u;
+    if (threadIdx.x < 32) sh.cnt[threadIdx.x] = 0u;
     __syncthreads();
     for (int q = 1; q < kMinTables; ++q) {
         const int h = 1 << (q - 1);
-        for (int t = threadIdx.x; t < kTreeTile; t += blockDim.x) {
-            const int a = sM[q - 1][t];
-            sM[q][t] = (int8_t)(t + h < kTreeTile ? min(a, (int)sM[q - 1][t + h]) : a);
+        for (int t = threadIdx.x; t < kTile; t += blockDim.x) {
+            const int a = sh.m[q - 1][t];
+            sh.m[q][t] = (int8_t)(t + h < kTile ? min(a, (int)sh.m[q - 1][t + h]) : a);
         }
         __syncthreads();
     }
-    const int8_t *sL = sM[0];
+    const int8_t *sL = sh.m[0];
     const int i = base + threadIdx.x;
-    uint32_t m = 0u;
+    m = 0u;
+    lc = 0;
     if (i < n) {
         const int s = threadIdx.x + kTreeHalo;  // i's slot in the tile
         const int Li = i == 0 ? -1 : sL[s];
@@ -1399,18 +1453,18 @@ mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, 
         int mi = -1;
         if (i + leaf <= n - 1) {
             const int q = 31 - __clz(leaf);
-            mi = min((int)sM[q][s + 1], (int)sM[q][s + leaf + 1 - (1 << q)]);
+            mi = min((int)sh.m[q][s + 1], (int)sh.m[q][s + leaf + 1 - (1 << q)]);
         }
         // u(i): the next body with another key; L(u(i)), -1 if none
         int Lu = -1;
         {
             int j = i + 1, t = s + 1;
-            while (j < n && t < kTreeTile && sL[t] == D) {
+            while (j < n && t < kTile && sL[t] == D) {
                 ++j;
                 ++t;
             }
-            if (j < n && t >= kTreeTile) j = next_key_change(keys, i, j, n);
-            if (j < n) Lu = lcp[j];
+            if (j < n && t >= kTile) j = next_key_change(keys, i, j, n);
+            if (j < n) Lu = shared(j);
         }
         const int c = min(min(mi, Lu), D - 1);
         if (i == 0) {
@@ -1424,33 +1478,30 @@ mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, 
 #pragma unroll
             for (int q = kMinTables - 1; q >= 0; --q) {
                 const int k = 1 << q;
-                if (lft + k <= leaf && sM[q][s - lft - k] >= Li) lft += k;
-                if (rgt + k <= leaf && sM[q][s + rgt + 1] >= Li) rgt += k;
+                if (lft + k <= leaf && sh.m[q][s - lft - k] >= Li) lft += k;
+                if (rgt + k <= leaf && sh.m[q][s + rgt + 1] >= Li) rgt += k;
             }
             if (lft + rgt + 2 > leaf) {
                 m |= 1u << (Li + 1);
                 for (int l = Li + 2; l <= c + 1; ++l) m |= 1u << l;
             }
         }
-        mask[i] = m;
         // the leaf starting here (the deepest run; unless the capacity stops
         // the tree above it) runs to the next boundary below its level
-        uint8_t lc = 0;
         if (m != 0u) {
             const int lf = 31 - __clz(m);
-            const int room = kTreeTile - 1 - s;  // boundaries after i in the tile
+            const int room = kTile - 1 - s;  // boundaries after i in the tile
             int run = 0;
-            while (run + 64 <= room && sM[6][s + 1 + run] >= lf) run += 64;
+            while (run + 64 <= room && sh.m[6][s + 1 + run] >= lf) run += 64;
 #pragma unroll
             for (int q = kMinTables - 2; q >= 0; --q) {
                 const int k = 1 << q;
-                if (run + k <= room && sM[q][s + 1 + run] >= lf) run += k;
+                if (run + k <= room && sh.m[q][s + 1 + run] >= lf) run += k;
             }
             const int e = i + 1 + run, t = s + 1 + run;
-            lc = (e < n && t >= kTreeTile) || e - i >= (int)kLongLeaf ? kLongLeaf
+            lc = (e < n && t >= kTile) || e - i >= (int)kLongLeaf ? kLongLeaf
                                                                       : (uint8_t)(e - i);
         }
-        leafcnt[i] = lc;
     }
     // per-level counts: only the levels some lane of the warp starts
     uint32_t present = __reduce_or_sync(0xffffffffu, m);
@@ -1458,18 +1509,65 @@ mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, 
         const int l = __ffs(present) - 1;
         present &= present - 1u;
         const uint32_t b = __ballot_sync(0xffffffffu, (m >> l) & 1u);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&cnt[l], (uint32_t)__popc(b));
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sh.cnt[l], (uint32_t)__popc(b));
     }
     __syncthreads();
-    if (threadIdx.x < 32) blk_cnt[(size_t)threadIdx.x * nblk + blockIdx.x] = cnt[threadIdx.x];
+    if (threadIdx.x < 32) blk_cnt[(size_t)threadIdx.x * nblk + tile] = sh.cnt[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(kTreeBlock)
+mask_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ lcp, int n,
+            int nchild, int leaf, uint32_t *__restrict__ mask, uint32_t *__restrict__ blk_cnt,
+            int nblk, uint8_t *__restrict__ leafcnt, const uint32_t *__restrict__ flags)
+{
+    pdl_wait();
+    if (sort_failed(flags)) return;
+    __shared__ MaskShared<kTreeBlock> sh;
+    uint32_t m;
+    uint8_t lc;
+    level_masks<kTreeBlock>(
+        keys, [&](int j) { return (int)lcp[j]; }, blockIdx.x, n, nchild, leaf, blk_cnt, nblk, sh,
+        m, lc);
+    const int i = blockIdx.x * kTreeBlock + threadIdx.x;
+    if (i < n) {
+        mask[i] = m;
+        leafcnt[i] = lc;
+    }
+}
+
+// The levels' first nodes and counts from their totals, by one warp.  If the
+// nodes do not fit the node arrays, the tree stops at the deepest level that
+// fits (its nodes become leaves: results stay exact, slower) and
+// flags[kFlagNodes] is raised.
+__device__ __forceinline__ void level_starts(const uint32_t *total_of, int D, int cap,
+                                             LevelInfo &lv, uint32_t *flags)
+{
+    static_assert(kMaxLevels <= 32, "a level per lane");
+    const int q = threadIdx.x & 31;
+    const long long c = q <= D ? (long long)total_of[q] : 0;
+    long long end = c;  // of level q's nodes
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, end, o);
+        if (q >= o) end += t;
+    }
+    const uint32_t over = __ballot_sync(0xffffffffu, end > cap);
+    const int max_level = over ? min(D, __ffs(over) - 2) : D;
+    const int total = max_level < 0 ? 0 : (int)__shfl_sync(0xffffffffu, end, max_level & 31);
+    for (int l = q; l < kMaxLevels + 2; l += 32) {
+        const bool built = l == q && l <= max_level;
+        lv.begin[l] = built ? (int32_t)(end - c) : total;
+        lv.count[l] = built ? (int32_t)c : 0;
+    }
+    if (q == 0) {
+        lv.total = total;
+        lv.max_level = max_level;
+        if (over) atomicOr(&flags[kFlagNodes], 1u);
+    }
 }
 
 // Block 0: per level, the exclusive scan of the block counts (blk_off,
 // same layout as blk_cnt) and the level's first node; block 1: the group sums
-// of over kSegBlock bodies.  Warp l scans row l,
-// 32 blocks per step.  If the nodes do not fit the node arrays, the tree
-// stops at the deepest level that fits (its nodes become leaves: results
-// stay exact, slower) and flags[kFlagNodes] is raised.
+// of over kSegBlock bodies.  Warp l scans row l, 32 blocks per step.
 __global__ void __launch_bounds__(1024)
 level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
                   uint32_t *__restrict__ blk_off, LevelInfo *lv, int cap,
@@ -1479,9 +1577,9 @@ level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
     if (sort_failed(flags)) return;
     if (blockIdx.x == 1) {
         if (quad)
-            top_groups<true>(sg);
+            top_groups<true, 1024>(sg, kSegBlockLevel);
         else
-            top_groups<false>(sg);
+            top_groups<false, 1024>(sg, kSegBlockLevel);
         return;
     }
     __shared__ uint32_t total_of[32];
@@ -1512,97 +1610,77 @@ level_scan_kernel(const uint32_t *__restrict__ blk_cnt, int nblk, int nchild,
     }
     if (lane == 0) total_of[l] = carry;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        long long at = 0;
-        int max_level = D;
-        for (int q = 0; q <= D; ++q) {
-            const long long c = total_of[q];
-            if (at + c > cap) {
-                max_level = q - 1;
-                atomicOr(&flags[kFlagNodes], 1u);
-                break;
-            }
-            at += c;
-        }
-        at = 0;
-        for (int q = 0; q < kMaxLevels + 2; ++q) {
-            const int c = q <= max_level ? (int)total_of[q] : 0;
-            lv->begin[q] = (int32_t)at;
-            lv->count[q] = c;
-            at += c;
-        }
-        lv->total = (int32_t)at;
-        lv->max_level = max_level;
-    }
+    if (threadIdx.x < 32) level_starts(total_of, D, cap, *lv, flags);
 }
 
 // Node records: per body, one node per set bit of its mask.  Leaves get
 // their body count here; an internal node's count, its child count and its
 // traversal metadata, and every node's geometry and moments, are cell_kernel's.
-__global__ void __launch_bounds__(kTreeBlock)
-node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafcnt,
-            const uint32_t *__restrict__ mask, const uint32_t *__restrict__ blk_off, int nblk,
-            int n, int nchild, NodeArrays nd, const LevelInfo *__restrict__ lv,
-            const uint32_t *__restrict__ flags)
+template <int kBlock>
+struct NodeShared {
+    uint32_t bal[kBlock / 32][32];  // per warp and level: lanes with that bit
+    uint32_t off[kBlock / 32][32];  // ... and the level's nodes before the warp
+};
+
+// One tile of kBlock bodies, one thread each, with its body's mask m and leaf
+// count lc; before(l): the nodes of level l in the tiles before it.
+template <int kBlock, typename Before>
+__device__ __forceinline__ void node_records(const uint64_t *__restrict__ keys, uint32_t m,
+                                             uint8_t lc, Before before, int tile, int n,
+                                             int nchild, const NodeArrays &nd,
+                                             const LevelInfo &lv, NodeShared<kBlock> &sh)
 {
-    pdl_wait();
-    if (sort_failed(flags)) return;
-    __shared__ uint32_t sbal[kTreeBlock / 32][32];  // per warp and level: lanes with that bit
-    __shared__ uint32_t woff[kTreeBlock / 32][32];  // ... and the level's nodes before the warp
-    __shared__ int32_t lbeg[kMaxLevels + 2];
     const int D = tree_levels(nchild), B = level_bits(nchild);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * kTreeBlock + threadIdx.x;
-    const uint32_t m = i < n ? mask[i] : 0u;
+    const int i = tile * kBlock + threadIdx.x;
     for (int l = 0; l < 32; ++l) {
         const uint32_t b = __ballot_sync(0xffffffffu, (m >> l) & 1u);
         if (lane == 0) {
-            sbal[warp][l] = b;
-            woff[warp][l] = (uint32_t)__popc(b);
+            sh.bal[warp][l] = b;
+            sh.off[warp][l] = (uint32_t)__popc(b);
         }
     }
-    if (threadIdx.x < kMaxLevels + 2) lbeg[threadIdx.x] = lv->begin[threadIdx.x];
     __syncthreads();
     if (threadIdx.x < 32) {
-        uint32_t run = blk_off[(size_t)threadIdx.x * nblk + blockIdx.x];
-        for (int w = 0; w < kTreeBlock / 32; ++w) {
-            const uint32_t v = woff[w][threadIdx.x];
-            woff[w][threadIdx.x] = run;
+        uint32_t run = before(threadIdx.x);
+        for (int w = 0; w < kBlock / 32; ++w) {
+            const uint32_t v = sh.off[w][threadIdx.x];
+            sh.off[w][threadIdx.x] = run;
             run += v;
         }
     }
     __syncthreads();
     if (m == 0u) return;
-    const int max_level = lv->max_level;
+    const int max_level = lv.max_level;
     const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
     const int top = min(31 - __clz(m), max_level);
     for (int l = __ffs(m) - 1; l <= top; ++l) {
         if (!((m >> l) & 1u)) continue;
-        const int x = lbeg[l] + (int)woff[warp][l] + __popc(sbal[warp][l] & lt);
+        const int x = lv.begin[l] + (int)sh.off[warp][l] + __popc(sh.bal[warp][l] & lt);
         int parent = -1;
         if (l > 0) {
             // the last node of level l - 1 starting at or before body i
-            parent = lbeg[l - 1] + (int)woff[warp][l - 1] + __popc(sbal[warp][l - 1] & le) - 1;
+            parent = lv.begin[l - 1] + (int)sh.off[warp][l - 1] + __popc(sh.bal[warp][l - 1] & le) - 1;
         }
         const bool splits = l + 1 <= max_level && ((m >> (l + 1)) & 1u);
         const int first_child =
-            splits ? lbeg[l + 1] + (int)woff[warp][l + 1] + __popc(sbal[warp][l + 1] & lt) : -1;
+            splits ? lv.begin[l + 1] + (int)sh.off[warp][l + 1] + __popc(sh.bal[warp][l + 1] & lt) : -1;
         nd.begin[x] = i;
         nd.level[x] = (uint8_t)l;
         nd.parent[x] = parent;
         nd.child[x] = first_child;
         if (!splits) {
             // a leaf: its bodies run to the next boundary below level l
-            int cnt = leafcnt[i];
+            int cnt = lc;
             if (cnt == kLongLeaf || l != 31 - __clz(m)) {
                 // a long run (equal keys, or a node the capacity kept from
                 // splitting): the end of its level-l key prefix
-                const int sh = B * (D - l);
-                const uint64_t p = keys[i] >> sh;
+                const int shift = B * (D - l);
+                const uint64_t p = keys[i] >> shift;
                 int lo = i + 1, hi = n;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if ((keys[mid] >> sh) == p)
+                    if ((keys[mid] >> shift) == p)
                         lo = mid + 1;
                     else
                         hi = mid;
@@ -1614,6 +1692,26 @@ node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafc
             nd.meta[x] = make_int4(x, -1, i, cnt);
         }
     }
+}
+
+__global__ void __launch_bounds__(kTreeBlock)
+node_kernel(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ leafcnt,
+            const uint32_t *__restrict__ mask, const uint32_t *__restrict__ blk_off, int nblk,
+            int n, int nchild, NodeArrays nd, const LevelInfo *__restrict__ lv,
+            const uint32_t *__restrict__ flags)
+{
+    pdl_wait();
+    if (sort_failed(flags)) return;
+    __shared__ NodeShared<kTreeBlock> sh;
+    __shared__ LevelInfo s_lv;
+    if (threadIdx.x < kMaxLevels + 2) s_lv.begin[threadIdx.x] = lv->begin[threadIdx.x];
+    if (threadIdx.x == 0) s_lv.max_level = lv->max_level;
+    // (node_records synchronises before it reads the levels)
+    const int i = blockIdx.x * kTreeBlock + threadIdx.x;
+    node_records<kTreeBlock>(
+        keys, i < n ? mask[i] : 0u, i < n ? leafcnt[i] : (uint8_t)0,
+        [&](int l) { return blk_off[(size_t)l * nblk + blockIdx.x]; }, blockIdx.x, n, nchild, nd,
+        s_lv, sh);
 }
 
 __device__ __forceinline__ uint32_t compact3(uint64_t x)
@@ -1731,17 +1829,13 @@ struct RangePieces {
 // One lane per node, or eight: they share out the loose bodies and the groups'
 // levels, so that all of a node's reads are in flight together, and add their
 // sums by shuffles; the first three take an axis each for the geometry (f64) and
-// the quotients.  launch_cells picks.
+// the quotients.  cell_lanes picks.
 template <bool kQuad, bool kExact, int kLanes>
-__global__ void __launch_bounds__(256)
-cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody, NodeArrays nd,
-            const LevelInfo *__restrict__ lv, int nchild, Segments sg,
-            const unsigned long long *__restrict__ extent_bits,
-            const uint32_t *__restrict__ flags)
+__device__ __forceinline__ void cell_nodes(const uint64_t *__restrict__ keys,
+                                           const float4 *sbody, const NodeArrays &nd, int total,
+                                           int nchild, const Segments &sg,
+                                           const unsigned long long *__restrict__ extent_bits)
 {
-    pdl_wait();
-    if (sort_failed(flags)) return;
-    const int total = lv->total;
     const int D = tree_levels(nchild), B = level_bits(nchild);
     const double X = __longlong_as_double((long long)*extent_bits);
     constexpr int kBatch = kLanes == 1 ? 3 : 1;  // loose bodies read at a time
@@ -1906,6 +2000,127 @@ cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody,
                 nd.quad_a[x] = make_float4(q.v[0], q.v[1], q.v[2], q.v[0] + q.v[1] + q.v[2]);
                 nd.quad_b[x] = make_float4(q.v[3], q.v[4], q.v[5], 0.f);
             }
+        }
+    }
+}
+
+template <bool kQuad, bool kExact, int kLanes>
+__global__ void __launch_bounds__(256)
+cell_kernel(const uint64_t *__restrict__ keys, const float4 *__restrict__ sbody, NodeArrays nd,
+            const LevelInfo *__restrict__ lv, int nchild, Segments sg,
+            const unsigned long long *__restrict__ extent_bits,
+            const uint32_t *__restrict__ flags)
+{
+    pdl_wait();
+    if (sort_failed(flags)) return;
+    cell_nodes<kQuad, kExact, kLanes>(keys, sbody, nd, lv->total, nchild, sg, extent_bits);
+}
+
+// ---------------------------------------------------------------------------
+// The tree of few bodies in one launch
+// ---------------------------------------------------------------------------
+// The five kernels above take 6 + 7 + 5 + 7 + 9 us for 8,195 bodies and hardly
+// less for 300: their beginnings and ends and the round trips to L2 in each.
+// Where an SM's block of kBuildBlock threads has no more than one tile of bodies,
+// this takes the same stages in 23 us, with a grid barrier (1.2 us) between
+// them: sorted bodies,
+// group sums and level masks; node records (each block adds up the level counts
+// of the tiles before its own, so there is no scan kernel, and the last block
+// makes the top group sums); cells.  Masks and leaf counts stay in registers.
+// What other blocks of the launch wrote is never read through the read-only
+// cache.
+constexpr int kBuildBlock = 512;
+
+struct BuildArgs {
+    GatherArgs gather;
+    int leaf;
+    uint32_t *blk_cnt;
+    NodeArrays nd;
+    LevelInfo *lv;
+    const unsigned long long *extent_bits;
+    uint32_t *bar;  // [0] barrier count, [1] blocks that left
+    uint32_t *flags;
+    int spin_limit;
+};
+
+template <bool kQuad, bool kExact, int kLanes>
+__global__ void __launch_bounds__(kBuildBlock, 1) tree_build_kernel(BuildArgs a)
+{
+    constexpr int kGather = kBuildBlock / kSegBase;  // threads of the gather
+    constexpr int kGatherLevel = 7;                  // its last level of group sums
+    static_assert(kSegBase << kGatherLevel == kBuildBlock, "a group of all the tile's bodies");
+    __shared__ union {
+        struct {
+            GatherShared<kGather> gather;
+            MaskShared<kBuildBlock> mask;
+        } first;
+        NodeShared<kBuildBlock> node;
+    } sh;
+    __shared__ uint32_t total_of[32], before_of[32];
+    __shared__ LevelInfo lv;
+    __shared__ int s_ok;
+    if (threadIdx.x == 0) s_ok = !sort_failed(a.flags);
+    __syncthreads();
+    const int n = a.gather.n, nchild = a.gather.nchild;
+    const uint64_t *keys = a.gather.keys;
+    const int tiles = (n + kBuildBlock - 1) / kBuildBlock;  // at most gridDim.x
+    const int tile = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t m = 0u;
+    uint8_t lc = 0;
+    bool ok = s_ok != 0;  // (else an earlier kernel gave up: there is no order to read)
+    if (ok) {
+        if (tile < tiles) {
+            if (threadIdx.x < kGather)
+                gather_groups<kQuad, kExact, kGather, true>(a.gather, tile * kGather,
+                                                            sh.first.gather);
+            level_masks<kBuildBlock>(
+                keys, [&](int j) { return shared_digits(keys[j - 1], keys[j], nchild); }, tile, n,
+                nchild, a.leaf, a.blk_cnt, tiles, sh.first.mask, m, lc);
+        }
+        ok = grid_barrier(a.bar, a.flags, a.spin_limit, gridDim.x, &s_ok);
+    }
+    if (ok) {
+        // the levels' totals and starts, the same in every block, and the nodes
+        // of the tiles before this block's
+        for (int l = warp; l < 32; l += kBuildBlock / 32) {
+            uint32_t sum = 0, before = 0;
+            for (int t = lane; t < tiles; t += 32) {
+                const uint32_t v = __ldcg(&a.blk_cnt[(size_t)l * tiles + t]);
+                sum += v;
+                before += t < tile ? v : 0u;
+            }
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            before = __reduce_add_sync(0xffffffffu, before);
+            if (lane == 0) {
+                total_of[l] = sum;
+                before_of[l] = before;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) level_starts(total_of, tree_levels(nchild), a.nd.cap, lv, a.flags);
+        __syncthreads();
+        if (blockIdx.x == 0 && threadIdx.x < sizeof lv / sizeof(int32_t))
+            reinterpret_cast<int32_t *>(a.lv)[threadIdx.x] =
+                reinterpret_cast<const int32_t *>(&lv)[threadIdx.x];
+        if (tile < tiles)
+            node_records<kBuildBlock>(
+                keys, m, lc, [&](int l) { return before_of[l]; }, tile, n, nchild, a.nd, lv,
+                sh.node);
+        if (blockIdx.x == gridDim.x - 1)
+            top_groups<kQuad, kBuildBlock>(a.gather.sg, kGatherLevel);
+        ok = grid_barrier(a.bar, a.flags, a.spin_limit, 2u * gridDim.x, &s_ok);
+    }
+    if (ok)
+        cell_nodes<kQuad, kExact, kLanes>(keys, a.gather.sbody, a.nd, lv.total, nchild,
+                                          a.gather.sg, a.extent_bits);
+    // the last block to leave resets the barrier for the next build
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {
+            a.bar[0] = 0u;
+            a.bar[1] = 0u;
         }
     }
 }
@@ -2949,7 +3164,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaSt
     PG_WA(w->tile_cnt, rtiles * kRadixBuckets);
     PG_WA(w->tile_grp, 2 * ((rtiles + kSortGroup - 1) / kSortGroup) * kRadixBuckets);
     PG_WA(w->blockmax, rtiles);
-    PG_WA(w->tree_bar, 4);
+    PG_WA(w->tree_bar, 8);
     PG_WA(w->sbody, cap);
     PG_WA(w->lcp, cap);
     PG_WA(w->mask, cap);
@@ -2986,7 +3201,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaSt
     if (rc == PHYSIM_OK &&
         (cudaMemsetAsync(w->flags, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->lv, 0, sizeof(LevelInfo), stream) != cudaSuccess ||
-         cudaMemsetAsync(w->tree_bar, 0, 4 * sizeof(uint32_t), stream) != cudaSuccess ||
+         cudaMemsetAsync(w->tree_bar, 0, 8 * sizeof(uint32_t), stream) != cudaSuccess ||
          cudaMemsetAsync(w->sort_meta, 0,
                          ((size_t)kSortPasses * kRadixBuckets + kSortPasses + 2) * sizeof(uint32_t),
                          stream) != cudaSuccess ||
@@ -3170,18 +3385,64 @@ static int launch_cells_lanes(const uint64_t *keys, BhWorkspace *ws, const BhPar
                       (const unsigned long long *)ws->extent_bits, (const uint32_t *)ws->flags);
 }
 
-static int launch_cells(const uint64_t *keys, BhWorkspace *ws, int n, const BhParams &p,
-                        const Segments &sg, bool quad, bool exact, int sms, cudaStream_t st)
+// Lanes per node of the cells: eight while the nodes (about 1.5 per body with
+// one body per leaf, an eighth per body with 16) leave the SMs idle.  One lane
+// vs eight (us): leaf 16, 2,003 bodies 12.0 / 7.9, 100,003 15.1 / 9.4, 200,003
+// 15.9 / 13.8, 400,009 17.2 / 23.4; with quadrupoles 100,003 25.0 / 11.4, 400,009
+// 28.7 / 29.4; leaf 1, 2,003 bodies 12.3 / 8.5, 20,011 13.5 / 12.9, 50,021 15.1 /
+// 19.0.
+static int cell_lanes(int n, const BhParams &p)
 {
-    // Eight lanes while the nodes (about 1.5 per body with one body per leaf, an
-    // eighth per body with 16) leave the SMs idle.  One lane vs eight (us): leaf
-    // 16, 2,003 bodies 12.0 / 7.9, 100,003 15.1 / 9.4, 200,003 15.9 / 13.8,
-    // 400,009 17.2 / 23.4; with quadrupoles 100,003 25.0 / 11.4, 400,009 28.7 /
-    // 29.4; leaf 1, 2,003 bodies 12.3 / 8.5, 20,011 13.5 / 12.9, 50,021 15.1 / 19.0.
     const double leaf = std::max(1.0, 0.625 * p.leaf_size);
-    if (n <= (quad ? 30000.0 : 20000.0) * leaf)
-        return launch_cells_lanes<8>(keys, ws, p, sg, quad, exact, sms * 8, st);
-    return launch_cells_lanes<1>(keys, ws, p, sg, quad, exact, sms * 8, st);
+    const bool quad = p.multipole == kMultipoleQuadrupole;
+    return n <= (quad ? 30000.0 : 20000.0) * leaf ? 8 : 1;
+}
+
+// Whether the tree is built in one launch: a tile per SM.  Step times, separate
+// launches vs one (us): theta 1.0, leaf 16, 303 bodies 54.3 / 52.6, 8,195 77.6 /
+// 73.9, 50,021 83.5 / 79.5, and with several tiles per block 100,003 97.0 /
+// 100.5, 300,007 139.6 / 149.0; leaf 1, 8,195 80.4 / 75.9, 250,007 150.5 / 175.8;
+// quadrupoles, 8,195 104.5 / 98.8, 100,003 242.4 / 246.0.
+static bool resident_build(int n, int per_sm, int sms)
+{
+    return g_sort_single.load() && per_sm > 0 && n <= sms * kBuildBlock;
+}
+
+template <int kLanes>
+static const void *tree_build_fn(bool quad, bool exact)
+{
+    auto f = quad ? (exact ? tree_build_kernel<true, true, kLanes>
+                           : tree_build_kernel<true, false, kLanes>)
+                  : (exact ? tree_build_kernel<false, true, kLanes>
+                           : tree_build_kernel<false, false, kLanes>);
+    return (const void *)f;
+}
+
+static int launch_build(BhWorkspace *ws, const GatherArgs &ga, const BhParams &p, bool quad,
+                        bool exact, int sms, cudaStream_t st)
+{
+    BuildArgs a;
+    a.gather = ga;
+    a.gather.lcp = nullptr;
+    a.leaf = p.leaf_size;
+    a.blk_cnt = ws->blk_cnt;
+    a.nd = ws->nd;
+    a.lv = ws->lv;
+    a.extent_bits = ws->extent_bits;
+    a.bar = ws->tree_bar + 4;
+    a.flags = ws->flags;
+    a.spin_limit = wait_limit();
+    // blocks for the tiles, one for the top group sums, and more if the cells
+    // are more than those blocks' threads
+    const int lanes = cell_lanes(ga.n, p);
+    const int nodes = (int)(1.6 * ga.n / std::max(1.0, 0.625 * p.leaf_size)) + 1;
+    const int blocks = std::min(
+        sms, std::max(cdiv(ga.n, kBuildBlock) + 1, cdiv(nodes * lanes, kBuildBlock)));
+    void *args[] = {&a};
+    PG_CUDA(cudaLaunchCooperativeKernel(
+        lanes == 8 ? tree_build_fn<8>(quad, exact) : tree_build_fn<1>(quad, exact),
+        dim3((unsigned)blocks), dim3(kBuildBlock), args, 0, st));
+    return PHYSIM_OK;
 }
 
 static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, cudaStream_t st)
@@ -3211,15 +3472,33 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
         sg.off[k] = at;
         at += sg.groups(k);
     }
-    auto boundary = quad ? (exact ? boundary_kernel<true, true> : boundary_kernel<true, false>)
-                         : (exact ? boundary_kernel<false, true> : boundary_kernel<false, false>);
-    PG_TRY(launch_pdl(boundary, cdiv(n, kSegBlock), kSegBlock / kSegBase, st, keys,
-                      (const uint32_t *)ws->vals[cur], n, p.nchild, (const float4 *)b.body4,
-                      (const double *)b.x, (const double *)b.y, (const double *)b.z, ws->sbody,
-                      ws->sbody_lo, ws->lcp, sg, (const uint32_t *)ws->flags));
-    const int tree_blocks = cdiv(n, kTreeBlock);
     PG_CHECK(p.leaf_size >= 1 && p.leaf_size <= kMaxLeaf, PHYSIM_ERR_ARGUMENT,
              "leaf size %d outside 1..%d", p.leaf_size, kMaxLeaf);
+    GatherArgs ga;
+    ga.keys = keys;
+    ga.order = ws->vals[cur];
+    ga.n = n;
+    ga.nchild = p.nchild;
+    ga.body4 = (const float4 *)b.body4;
+    ga.bx = b.x;
+    ga.by = b.y;
+    ga.bz = b.z;
+    ga.sbody = ws->sbody;
+    ga.sbody_lo = ws->sbody_lo;
+    ga.lcp = ws->lcp;
+    ga.sg = sg;
+    ws->nchild = p.nchild;
+    ws->exact = exact;
+    if (resident_build(n, per_sm, sms)) {
+        PG_TRY(launch_build(ws, ga, p, quad, exact, sms, st));
+        ws->launches = launches + 1;
+        return PHYSIM_OK;
+    }
+    auto boundary = quad ? (exact ? boundary_kernel<true, true> : boundary_kernel<true, false>)
+                         : (exact ? boundary_kernel<false, true> : boundary_kernel<false, false>);
+    PG_TRY(launch_pdl(boundary, cdiv(n, kSegBlock), kSegBlock / kSegBase, st, ga,
+                      (const uint32_t *)ws->flags));
+    const int tree_blocks = cdiv(n, kTreeBlock);
     PG_TRY(launch_pdl(mask_kernel, tree_blocks, kTreeBlock, st, keys, (const uint8_t *)ws->lcp, n,
                       p.nchild, p.leaf_size, ws->mask, ws->blk_cnt, tree_blocks, ws->leafcnt,
                       (const uint32_t *)ws->flags));
@@ -3228,10 +3507,10 @@ static int bh_build(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, c
     PG_TRY(launch_pdl(node_kernel, tree_blocks, kTreeBlock, st, keys, (const uint8_t *)ws->leafcnt,
                       (const uint32_t *)ws->mask, (const uint32_t *)ws->blk_off, tree_blocks, n,
                       p.nchild, ws->nd, (const LevelInfo *)ws->lv, (const uint32_t *)ws->flags));
-    PG_TRY(launch_cells(keys, ws, n, p, sg, quad, exact, sms, st));
+    PG_TRY(cell_lanes(n, p) == 8
+               ? launch_cells_lanes<8>(keys, ws, p, sg, quad, exact, sms * 8, st)
+               : launch_cells_lanes<1>(keys, ws, p, sg, quad, exact, sms * 8, st));
     launches += 5;
-    ws->nchild = p.nchild;
-    ws->exact = exact;
     PG_CUDA(cudaGetLastError());
     ws->launches = launches;
     return PHYSIM_OK;
