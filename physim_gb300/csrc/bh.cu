@@ -3169,7 +3169,9 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaSt
     PG_WA(w->lcp, cap);
     PG_WA(w->mask, cap);
     PG_WA(w->leafcnt, cap);
-    PG_WA(w->blk_cnt, 32 * tree_blocks);
+    // (tree_build_kernel counts tiles of kBuildBlock, mask_kernel of kTreeBlock)
+    static_assert(kBuildBlock <= kTreeBlock, "the finer tiles");
+    PG_WA(w->blk_cnt, (size_t)32 * cdiv((long long)cap, kBuildBlock));
     PG_WA(w->blk_off, 32 * tree_blocks);
     if (exact) PG_WA(w->sbody_lo, cap);
     const size_t groups = cap / 2 + kSegLevels;  // all levels of cap / 4, cap / 8, ...
