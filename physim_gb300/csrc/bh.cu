@@ -640,6 +640,58 @@ __device__ __forceinline__ bool tree_sort_barrier(const TreeSortArgs &a, uint32_
                         (int)blockIdx.x == a.stall_tile ? kBarPoison : target, s_ok);
 }
 
+// The extent (bits of the largest |coordinate|) in wm[0] of every block, from
+// each thread's maximum m, and to extent_bits; one barrier.
+template <int kWarps>
+__device__ __forceinline__ bool grid_extent(const TreeSortArgs &a, unsigned long long m,
+                                            unsigned long long *wm, uint32_t &target, int *s_ok)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto block_max = [&]() {  // m of thread 0
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) wm[warp] = m;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < kWarps; ++w) m = max(m, wm[w]);
+    };
+    block_max();
+    if (threadIdx.x == 0) a.blockmax[blockIdx.x] = m;
+    target += gridDim.x;
+    if (!tree_sort_barrier(a, target, s_ok)) return false;
+    m = 0;
+    for (int t = threadIdx.x; t < (int)gridDim.x; t += kWarps * 32)
+        m = max(m, __ldcg(&a.blockmax[t]));
+    block_max();
+    if (threadIdx.x == 0) {
+        wm[0] = m;
+        if (blockIdx.x == 0) *a.extent_bits = m;
+    }
+    __syncthreads();
+    return true;
+}
+
+// 2^(D - 1) / X, one thread's division.
+__device__ __forceinline__ double key_scale(double X, int nchild, double *s_scale)
+{
+    if (threadIdx.x == 0)
+        *s_scale = X > 0.0 ? __ddiv_rn(ldexp(1.0, tree_levels(nchild) - 1), X) : 0.0;
+    __syncthreads();
+    return *s_scale;
+}
+
+// The last block to leave resets the barrier for the next build.
+__device__ __forceinline__ void leave_grid(uint32_t *bar)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&bar[1], 1u) == gridDim.x - 1) {
+            bar[0] = 0u;
+            bar[1] = 0u;
+        }
+    }
+}
+
 template <int ITEMS>
 struct TreeSortShared {
     uint32_t h[kSortWarps][kRadixBuckets];
@@ -790,39 +842,14 @@ __device__ __forceinline__ void tree_sort_body(const TreeSortArgs &a, TreeSortSh
             for (int r = 0; r < kBatch; ++r)
                 m = max(max(m, abs_bits(px[r])), max(abs_bits(py[r]), abs_bits(pz[r])));
         }
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) sh.wm[warp] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < kSortWarps; ++w) m = max(m, sh.wm[w]);
-            a.blockmax[tile] = m;
-        }
-    }
-    target += tiles;
-    if (!tree_sort_barrier(a, target, &sh.ok)) return;
-    {
-        unsigned long long m = 0;
-        for (int t = threadIdx.x; t < tiles; t += kSortThreads)
-            m = max(m, __ldcg(&a.blockmax[t]));
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) sh.wm[warp] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < kSortWarps; ++w) m = max(m, sh.wm[w]);
-            sh.wm[0] = m;
-            if (tile == 0) *a.extent_bits = m;
-        }
-        __syncthreads();
+        if (!grid_extent<kSortWarps>(a, m, sh.wm, target, &sh.ok)) return;
     }
     const double X = __longlong_as_double((long long)sh.wm[0]);
     uint64_t kk[ITEMS];
     uint32_t vv[ITEMS];
     {
-        const int D = tree_levels(a.nchild);
         __shared__ double s_scale;
-        if (threadIdx.x == 0) s_scale = X > 0.0 ? __ddiv_rn(ldexp(1.0, D - 1), X) : 0.0;
-        __syncthreads();
-        const double scale = s_scale;
+        const double scale = key_scale(X, a.nchild, &s_scale);
         // through shared memory: the loop stays rolled (unrolled over all keys
         // its code outgrows the instruction cache) and the keys in registers
 #pragma unroll 1
@@ -933,15 +960,108 @@ __global__ void __launch_bounds__(kSortThreads, 1) tree_sort_kernel(TreeSortArgs
     __shared__ TreeSortShared<ITEMS> sh;
     extern __shared__ uint64_t skeys_dyn[];
     tree_sort_body<ITEMS>(a, sh, skeys_dyn);
-    // the last block to leave resets the barrier for the next build
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {
-            a.bar[0] = 0u;
-            a.bar[1] = 0u;
+    leave_grid(a.bar);
+}
+
+// The same for few bodies, by ranks instead of digits: each block sorts a tile of
+// kRankTile keys (a bitonic network), then every key's place is its place in its
+// own tile plus the keys below it in each other tile, by binary search over all
+// the tiles' keys in shared memory.  Keys compare whole and equal ones keep the
+// order of their tiles and places, so any state takes the same time, with two
+// barriers where the digit passes take ten.  A key's searches and the keys each
+// block reads grow with n.  Step times by digits / by ranks (us), theta 1.0, leaf
+// 16, Plummer and cube: 255 bodies 50 / 42 and 53 / 41, 2,003 67 / 51 and 67 / 51,
+// 8,195 74 / 62 and 73 / 58, 16,384 74 / 70 and 74 / 67, 20,011 76 / 77 and 73 /
+// 73, 24,576 77 / 81 and 77 / 79.
+constexpr int kRankTile = 256;
+constexpr int kRankMax = 18432;
+
+__device__ __forceinline__ void rank_sort_body(const TreeSortArgs &a, uint64_t *all)
+{
+    __shared__ unsigned long long wm[kRankTile / 32];
+    __shared__ double s_scale;
+    __shared__ int s_ok;
+    const int t = threadIdx.x, tile = blockIdx.x, tiles = gridDim.x;
+    const int i = tile * kRankTile + t;
+    uint32_t target = 0;
+    double x = 0.0, y = 0.0, z = 0.0;
+    if (i < a.n) {
+        x = a.x[i];
+        y = a.y[i];
+        z = a.z[i];
+    }
+    if (!grid_extent<kRankTile / 32>(a, max(abs_bits(x), max(abs_bits(y), abs_bits(z))), wm, target,
+                                     &s_ok))
+        return;
+    const double X = __longlong_as_double((long long)wm[0]);
+    const double scale = key_scale(X, a.nchild, &s_scale);
+    // (no key has bit 63: the places after the last body sort to the end)
+    uint64_t k = i >= a.n ? ~0ull : X > 0.0 ? body_key(x, y, z, X, scale, a.nchild) : 0ull;
+    uint32_t v = t;
+    // the tile, by (key, place)
+    {
+        uint32_t *sv = reinterpret_cast<uint32_t *>(all + 2 * kRankTile);
+        int buf = 0;
+#pragma unroll 1
+        for (int size = 2; size <= kRankTile; size <<= 1) {
+#pragma unroll 1
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                uint64_t pk;
+                uint32_t pv;
+                if (stride >= 32) {
+                    all[buf + t] = k;
+                    sv[buf + t] = v;
+                    __syncthreads();
+                    pk = all[buf + (t ^ stride)];
+                    pv = sv[buf + (t ^ stride)];
+                    buf ^= kRankTile;  // (read again only after the next barrier)
+                } else {
+                    pk = __shfl_xor_sync(0xffffffffu, k, stride);
+                    pv = __shfl_xor_sync(0xffffffffu, v, stride);
+                }
+                const bool less = k < pk || (k == pk && v < pv);
+                if (less != (((t & stride) == 0) == ((t & size) == 0))) {
+                    k = pk;
+                    v = pv;
+                }
+            }
         }
     }
+    if (i < a.n) a.k0[i] = k;
+    target += tiles;
+    if (!tree_sort_barrier(a, target, &s_ok)) return;
+    // all keys, 16 bytes at a time; no key is below the places after the last
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(all);
+    for (int p = t; p < a.n / 2; p += kRankTile)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * p),
+                     "l"(a.k0 + 2 * p)
+                     : "memory");
+    for (int p = (a.n & ~1) + t; p < tiles * kRankTile; p += kRankTile)
+        all[p] = p < a.n ? __ldcg(&a.k0[p]) : ~0ull;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (i >= a.n) return;
+    int to = t;
+#pragma unroll 4
+    for (int o = 0; o < tiles; ++o) {
+        if (o == tile) continue;
+        const uint64_t *q = all + o * kRankTile;
+        const uint64_t below = k + (o < tile);  // equal keys of earlier tiles come first
+        int at = 0;
+#pragma unroll
+        for (int step = kRankTile / 2; step > 0; step >>= 1)
+            at += q[at + step - 1] < below ? step : 0;
+        to += at + (q[at] < below);
+    }
+    a.k1[to] = k;
+    a.v1[to] = (uint32_t)(tile * kRankTile) + v;
+}
+
+__global__ void __launch_bounds__(kRankTile, 1) rank_sort_kernel(TreeSortArgs a)
+{
+    extern __shared__ uint64_t skeys_dyn[];
+    rank_sort_body(a, skeys_dyn);
+    leave_grid(a.bar);
 }
 
 // ---------------------------------------------------------------------------
@@ -2114,15 +2234,7 @@ __global__ void __launch_bounds__(kBuildBlock, 1) tree_build_kernel(BuildArgs a)
     if (ok)
         cell_nodes<kQuad, kExact, kLanes>(keys, a.gather.sbody, a.nd, lv.total, nchild,
                                           a.gather.sg, a.extent_bits);
-    // the last block to leave resets the barrier for the next build
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {
-            a.bar[0] = 0u;
-            a.bar[1] = 0u;
-        }
-    }
+    leave_grid(a.bar);
 }
 
 // ---------------------------------------------------------------------------
@@ -3020,8 +3132,18 @@ size_t tree_sort_smem(int items)
            2 * kFixRun * sizeof(uint64_t);
 }
 
+size_t rank_sort_smem(int n)
+{
+    // all keys; the tile's two buffers of keys and places before them
+    const size_t keys = (size_t)cdiv(n, kRankTile) * kRankTile * sizeof(uint64_t);
+    return std::max(keys, (size_t)2 * kRankTile * (sizeof(uint64_t) + sizeof(uint32_t)));
+}
+
 int tree_sort_attributes()
 {
+    PG_CUDA(cudaFuncSetAttribute((const void *)rank_sort_kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)rank_sort_smem(kRankMax)));
     for (int items : kTreeSortItems)
         PG_CUDA(cudaFuncSetAttribute(tree_sort_fn(items),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3163,7 +3285,7 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaSt
     const size_t rtiles = (size_t)resident_tiles(cap, resident_blocks);
     PG_WA(w->tile_cnt, rtiles * kRadixBuckets);
     PG_WA(w->tile_grp, 2 * ((rtiles + kSortGroup - 1) / kSortGroup) * kRadixBuckets);
-    PG_WA(w->blockmax, rtiles);
+    PG_WA(w->blockmax, 2 * rtiles);  // (a rank tile is half a sort tile)
     PG_WA(w->tree_bar, 8);
     PG_WA(w->sbody, cap);
     PG_WA(w->lcp, cap);
@@ -3292,6 +3414,8 @@ int wait_limit()
     return v == 0u ? kLookbackSpins : (int)std::min<uint32_t>(v, (uint32_t)INT32_MAX);
 }
 
+static bool rank_sort(int n, int sms) { return n <= std::min(kRankMax, sms * kRankTile); }
+
 // Extent, keys and sort of a state whose tiles are all resident.
 static int launch_tree_sort(BhWorkspace *ws, const DeviceBodies &b, const BhParams &p, int n,
                             int items, cudaStream_t st)
@@ -3315,6 +3439,12 @@ static int launch_tree_sort(BhWorkspace *ws, const DeviceBodies &b, const BhPara
     a.spin_limit = wait_limit();
     a.stall_tile = (int)g_stall_tile.load();
     void *args[] = {&a};
+    if (rank_sort(n, device_sm_count(ws->device))) {
+        PG_CUDA(cudaLaunchCooperativeKernel((const void *)rank_sort_kernel,
+                                            dim3((unsigned)cdiv(n, kRankTile)), dim3(kRankTile),
+                                            args, rank_sort_smem(n), st));
+        return PHYSIM_OK;
+    }
     PG_CUDA(cudaLaunchCooperativeKernel(tree_sort_fn(items),
                                         dim3((unsigned)cdiv(n, kSortThreads * items)),
                                         dim3(kSortThreads), args, tree_sort_smem(items), st));
