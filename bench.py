@@ -110,7 +110,7 @@ def parse():
                    help="bodies whose accelerations are checked against the f64 reference law")
     p.add_argument("--sym-pairs-limit", type=int, default=0,
                    help="slot bytes up to which the each-pair-once plan runs one block per tile "
-                        "pair (0: the library's 4 GiB; 1: thread-block clusters at any size)")
+                        "pair (0: the library's 4 GiB; 1: runs of tiles at any size)")
     p.add_argument("--bodies", type=int, default=N_CUBE,
                    help="cube bodies (profiling of smaller cases; the reported workload is "
                         "the default 1,048,576)")
@@ -966,7 +966,7 @@ def measure_tour(args, dist: Dist, device: int) -> dict:
         sim.accelerations_f64(np.arange(64))
         sim.download()
     paths.append("simple_astro 65,536 each pair once + verlet, diagnostics, f64 sample")
-    # the same sum in thread-block clusters (the schedule of large states)
+    # the same sum in runs of tiles (the schedule of large states)
     pg.set_symmetric_pairs_limit(1)
     try:
         with pg.Simulation(cube, pg.SimConfig(gravity="simple_astro", e=E, dt=DT,
@@ -974,7 +974,7 @@ def measure_tour(args, dist: Dist, device: int) -> dict:
             sim.step(2)
     finally:
         pg.set_symmetric_pairs_limit(0)
-    paths.append("simple_astro 65,536 each pair once in thread-block clusters")
+    paths.append("simple_astro 65,536 each pair once in runs of tiles")
     for integ in ("euler", "rk4"):
         with pg.Simulation(small, pg.SimConfig(gravity="simple_astro", e=E, dt=DT,
                                                integrator=integ, device=device)) as sim:

@@ -29,32 +29,29 @@
 // body's T slots.  That keeps every SM busy at any size and is the faster of
 // the two, but its slots grow as 12 T n bytes (12.9 GB at 1,048,580 bodies),
 // so once they would exceed kSymPairsSlotBytes (4 GiB, about 600,000 bodies)
-// the cluster schedule below takes over.
+// the group schedule below takes over.
 //
-// Blocks work in thread-block clusters of kSymCluster (8) blocks: a cluster
-// takes the I tiles g*8 .. g*8+7 (one per block) and a run of kSymRun (16) J
-// tiles r*16 .. r*16+15, the pairs with I <= J.  A block's a_i accumulates
-// over the whole run and is written once, to slot r of its tile's i-side
-// slots: after each J tile a thread folds its register sums into its bodies'
-// compensated (TwoSum) sums in shared memory (high part f32, low part bf16:
-// the low part only carries rounding errors), so every tile's contribution
-// is compensated as when each tile pair had a slot of its own.  A block's
-// two warps add their reactions to tile J into one shared buffer; the
-// cluster then adds its blocks' buffers (read through distributed shared
-// memory, ranks in a fixed order, TwoSum-compensated, each block summing an
-// eighth of the tile) and writes them once, to slot g of tile J's j-side
-// slots.  Per cluster of up to 8 x 16 tile pairs that is 8 + 16 slot writes
-// of 12 KB instead of 2 per tile pair.
-// The cluster barrier is split: a block arrives when its reactions to tile
-// J are in shared memory and waits for the others only after it has
-// evaluated tile J + 1, so a block that is behind by up to a tile holds no
-// other block up.  Three reaction buffers make that safe: the buffer of tile
-// J + 1 was last read (for tile J - 2) before every block arrived for tile
-// J - 1, which this block waited for before starting tile J + 1.  Every
-// block of a cluster takes the same arrivals and waits (its run's length
-// plus one), and a last arrive-and-wait keeps each block's shared memory
-// alive until the others have read it.
-// Cluster schedule output.  Tile K has Rn - floor(K / 16) i-side slots (the runs r whose last
+// Group schedule.  A block of four teams (of two warps) holds an SM.  It takes
+// the I tiles g*8 .. g*8+7 and a run of kSymRun (16) J tiles r*16 .. r*16+15,
+// the pairs with I <= J: for each J tile first I tiles 0..3 of the group, one
+// per team, then 4..7.  A tile's a_i accumulates over the whole run and is
+// written once, to slot r of its tile's i-side slots: after each J tile a thread
+// folds its register sums into its bodies' compensated (TwoSum) sums in shared
+// memory (high part f32, low part bf16: the low part only carries rounding
+// errors), so every tile's contribution is compensated as when each tile pair
+// had a slot of its own.  A team's two warps add their reactions to tile J into
+// the team's buffer; the block adds the buffers (I tiles in order,
+// TwoSum-compensated) and writes the sums of all eight once, to slot g of tile
+// J's j-side slots.  Per unit of up to 8 x 16 tile pairs that is 8 + 16 slot
+// writes of 12 KB instead of 2 per tile pair.  All of it stays on one SM: the
+// same units as clusters of eight blocks of two warps, adding through
+// distributed shared memory, took 293 ms for the 1,048,580-body force pass where
+// this takes 257 (tile pairs with a slot each: 248); a cluster waits for the
+// slowest of its blocks at every J tile, and an SM that is left over in its
+// group of SMs holds none.
+// The units on the diagonal are half as long and come last, where the SMs run
+// out of units.
+// Group schedule output.  Tile K has Rn - floor(K / 16) i-side slots (the runs r whose last
 // J tile is >= K) and floor(K / 8) + 1 j-side slots (the groups g with
 // 8 g <= K), each [3][1024] f32, packed tile after tile (offsets in closed
 // form, sym_iside_base / sym_jside_base): 1.2 GB at 1,048,580 bodies,
@@ -65,7 +62,6 @@
 // sums act as the per-tile compensation of the one-pair kernels.
 #include <math.h>
 
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <atomic>
@@ -76,8 +72,6 @@
 
 namespace pg {
 
-namespace cg = cooperative_groups;
-
 namespace {
 
 // The tile-pair schedule while its slot buffer (12 B per body per tile) fits
@@ -85,7 +79,8 @@ namespace {
 constexpr size_t kSymPairsSlotBytes = size_t(4) << 30;
 std::atomic<uint64_t> g_pairs_limit{0};
 
-constexpr int kSymCluster = 8;  // I tiles per thread-block cluster (a portable size)
+constexpr int kSymTeams = 4;    // I tiles in registers at a time, two warps each
+constexpr int kSymGroup = 8;    // I tiles per unit
 constexpr int kSymRun = 16;     // J tiles per run
 
 // Slots of tile K (see the file comment), in units of one [3][1024] slot.
@@ -102,180 +97,148 @@ __host__ __device__ inline long long sym_iside_base(int K, int runs)
 
 __host__ __device__ inline long long sym_jside_base(int K)
 {
-    const long long q = K / kSymCluster, rem = K - q * kSymCluster;
-    return (long long)K + kSymCluster * q * (q - 1) / 2 + q * rem;
+    const long long q = K / kSymGroup, rem = K - q * kSymGroup;
+    return (long long)K + kSymGroup * q * (q - 1) / 2 + q * rem;
 }
 
 constexpr int kSlot = 3 * kSymTile;  // floats per slot
 
-// Clusters: I group g (tiles 8g .. 8g+7) with the J runs r >= floor(8g / 16).
-__host__ __device__ inline long long sym_clusters(int T)
+// Units: I group g (tiles 8g .. 8g+7) with the J runs r >= floor(8g / 16).
+__host__ __device__ inline long long sym_units(int T)
 {
-    const int groups = (T + kSymCluster - 1) / kSymCluster;
+    const int groups = (T + kSymGroup - 1) / kSymGroup;
     const int runs = (T + kSymRun - 1) / kSymRun;
     long long c = 0;
-    for (int g = 0; g < groups; ++g) c += runs - (g * kSymCluster) / kSymRun;
+    for (int g = 0; g < groups; ++g) c += runs - (g * kSymGroup) / kSymRun;
     return c;
 }
 
-// Dynamic shared memory of the pair kernel: three reaction buffers
-// (jacc[3][1024][3] f32), then the compensated i-side sums of the run
-// (hi[3][1024] f32, lo[3][1024] bf16): 54 KB, four blocks per SM.
-constexpr int kSymBufs = 3;
-constexpr size_t kSymJacc = (size_t)kSymBufs * kSymTile * 3;  // floats
-constexpr size_t kSymSmem =
-    kSymJacc * sizeof(float) + 3 * kSymTile * (sizeof(float) + sizeof(__nv_bfloat16));
-
-// The cluster barrier in two halves (PTX barrier.cluster): arrive publishes
-// this thread's earlier shared-memory writes to the cluster, wait returns
-// once every thread of the cluster has arrived and makes their writes
-// visible.  Arrivals and waits alternate.
-__device__ __forceinline__ void cluster_arrive()
+// Unit u: those past the diagonal, group by group, then the groups' first runs.
+__device__ __forceinline__ void sym_unit(int u, int T, int &g, int &r)
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void cluster_wait()
-{
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Tile J's reactions from this cluster's I tiles (those <= J): this block
-// sums bodies rank*128 .. rank*128+127 over the ranks' buffers, in rank
-// order with TwoSum, and writes them to slot g of tile J's j-side slots.
-__device__ __forceinline__ void sym_reduce_tile(cg::cluster_group &cluster, int rank, int g,
-                                                int J, int n, const float (*jw)[3],
-                                                float *__restrict__ Pj)
-{
-    if (g * kSymCluster > J) return;  // no I tile of this cluster reaches tile J
-    constexpr int per = kSymTile / kSymCluster;
-    float *dst = Pj + (sym_jside_base(J) + g) * kSlot;
-    const float *own = &jw[0][0];
-    for (int t = threadIdx.x; t < per * 3; t += kSymThreads) {
-        const int at = rank * per * 3 + t;  // = 3 jj + c
-        float v[kSymCluster];
-#pragma unroll
-        for (int src = 0; src < kSymCluster; ++src) v[src] = cluster.map_shared_rank(own, src)[at];
-        float hi = 0.f, lo = 0.f;
-#pragma unroll
-        for (int src = 0; src < kSymCluster; ++src) {
-            float sum, err;
-            two_sum(hi, v[src], sum, err);
-            hi = sum;
-            lo += err;
+    const int groups = (T + kSymGroup - 1) / kSymGroup;
+    const int runs = (T + kSymRun - 1) / kSymRun;
+    for (g = 0; g < groups; ++g) {
+        const int first = (g * kSymGroup) / kSymRun, c = runs - first - 1;
+        if (u < c) {
+            r = first + 1 + u;
+            return;
         }
-        const int jj = at / 3, c = at - 3 * jj;
-        if (J * kSymTile + jj < n) dst[c * kSymTile + jj] = hi + lo;
+        u -= c;
     }
+    g = u;
+    r = (g * kSymGroup) / kSymRun;
 }
 
-// 64 threads of up to 255 registers (about 245 used), 54 KB of shared
-// memory: four blocks per SM.
-__global__ void __cluster_dims__(kSymCluster, 1, 1) __launch_bounds__(kSymThreads, 4)
+// Dynamic shared memory of the pair kernel: the teams' reaction buffers
+// ([4][1024][3] f32), the reactions' sums over the I tiles so far (high and low
+// part), then the compensated i-side sums of the run ([8] x hi[3][1024] f32,
+// lo[3][1024] bf16): 216 KB, one block per SM.
+constexpr int kSymBlock = kSymTeams * kSymThreads;
+constexpr size_t kSymSmem = ((kSymTeams + 2) * sizeof(float) +
+                             kSymGroup * (sizeof(float) + sizeof(__nv_bfloat16))) * kSlot;
+
+// 256 threads of up to 255 registers (about 245 used).
+__global__ void __launch_bounds__(kSymBlock, 1)
 direct_sym_kernel(const float4 *__restrict__ body, const float *__restrict__ mass256, int n, int T,
                   float e, ScaleRef scale, float *__restrict__ Pi, float *__restrict__ Pj)
 {
     extern __shared__ float4 smem4[];
-    float *smem = reinterpret_cast<float *>(smem4);
-    float (*jacc)[kSymTile][3] = reinterpret_cast<float (*)[kSymTile][3]>(smem);
-    float *ihi = smem + kSymJacc;
-    __nv_bfloat16 *ilo = reinterpret_cast<__nv_bfloat16 *>(ihi + 3 * kSymTile);
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int runs = (T + kSymRun - 1) / kSymRun;
-    // this cluster's (g, r)
-    int u = (int)(blockIdx.x / kSymCluster), g = 0;
-    for (;;) {
-        const int c = runs - (g * kSymCluster) / kSymRun;
-        if (u < c) break;
-        u -= c;
-        ++g;
-    }
-    const int r = (g * kSymCluster) / kSymRun + u;
-    const int I = g * kSymCluster + rank;
+    float *jacc = reinterpret_cast<float *>(smem4);  // [team][1024][3]
+    float *jhi = jacc + kSymTeams * kSlot, *jlo = jhi + kSlot;
+    float *ihi = jlo + kSlot;  // [I tile of the group][3][1024]
+    __nv_bfloat16 *ilo = reinterpret_cast<__nv_bfloat16 *>(ihi + kSymGroup * kSlot);
+    const int team = threadIdx.x / kSymThreads;
+    const int ib = threadIdx.x & (kSymThreads - 1);  // this thread's first body of its tile
+    int g, r;
+    sym_unit((int)blockIdx.x, T, g, r);
     const int J0 = r * kSymRun, nJ = min(J0 + kSymRun, T) - J0;
-    const bool have_i = I < T;
-    const int warp = threadIdx.x >> 5;
-    const int ib = warp * 32 + (threadIdx.x & 31);  // this thread's first body of tile I
     const int sk = pair_scale_exp(__uint_as_float(*scale.ext), e);
     const int skm = mass_scale_exp(__uint_as_float(*scale.mass));
     const float sc = pow2f(-sk), msc = pow2f(-skm);
     const float es = e * pow2f(-2 * sk);
     const float2 e2 = make_float2(es, es);
-    float mi = 0.f;
-    const bool uni_i = have_i && common_mass(mass256, I * 4, I * 4 + 4, mi);
-    float2 nx[kSymQ], ny[kSymQ], nz[kSymQ], nm[kSymQ], ax[kSymQ], ay[kSymQ], az[kSymQ];
-#pragma unroll
-    for (int q = 0; q < kSymQ; ++q) {
-        ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                ihi[c * kSymTile + ib + (2 * q + h) * kSymThreads] = 0.f;
-                ilo[c * kSymTile + ib + (2 * q + h) * kSymThreads] = __float2bfloat16_rn(0.f);
-            }
+    for (int x = threadIdx.x; x < kSymTeams * kSlot; x += kSymBlock) jacc[x] = 0.f;
+    for (int x = threadIdx.x; x < kSymGroup * kSlot; x += kSymBlock) {
+        ihi[x] = 0.f;
+        ilo[x] = __float2bfloat16_rn(0.f);
     }
-    if (have_i) sym_load_i(body, I, sc, msc, nx, ny, nz, nm);
+    __syncthreads();
     for (int t = 0; t < nJ; ++t) {
         const int J = J0 + t;
-        float (*jw)[3] = jacc[t % kSymBufs];
-        // free: every block has read it (tile J - 3) before arriving for tile J - 2
-        for (int x = threadIdx.x; x < 3 * kSymTile; x += kSymThreads) (&jw[0][0])[x] = 0.f;
-        __syncthreads();
-        float mj = 0.f;
-        const bool uni = uni_i && common_mass(mass256, J * 4, J * 4 + 4, mj);
-        if (have_i && I < J)
-            sym_pair<false, true>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc, msc, e2, nx,
-                                  ny, nz, nm, ax, ay, az, jw);
-        else if (have_i && I == J)
-            sym_pair<true, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc, msc, e2, nx,
-                                  ny, nz, nm, ax, ay, az, jw);
-        if (have_i && I <= J) {
-            // this tile's partial sums into the compensated run sums
+        if (g * kSymGroup > J) continue;  // no I tile of the group reaches tile J
+#pragma unroll 1
+        for (int half = 0; half < kSymGroup / kSymTeams; ++half) {
+            const int slot = half * kSymTeams + team;
+            const int I = g * kSymGroup + slot;
+            if (I < T && I <= J) {
+                float2 nx[kSymQ], ny[kSymQ], nz[kSymQ], nm[kSymQ];
+                float2 ax[kSymQ], ay[kSymQ], az[kSymQ];
+                sym_load_i(body, I, sc, msc, nx, ny, nz, nm);
 #pragma unroll
-            for (int q = 0; q < kSymQ; ++q) {
-                const float v[2][3] = {{ax[q].x, ay[q].x, az[q].x}, {ax[q].y, ay[q].y, az[q].y}};
+                for (int q = 0; q < kSymQ; ++q) ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
+                float mi = 0.f, mj = 0.f;
+                bool uni = common_mass(mass256, I * 4, I * 4 + 4, mi);
+                uni = common_mass(mass256, J * 4, J * 4 + 4, mj) && uni;
+                float (*jw)[3] = reinterpret_cast<float (*)[3]>(jacc + team * kSlot);
+                if (I < J)
+                    sym_pair<false, true>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
+                                          msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
+                else
+                    sym_pair<true, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
+                                          msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
+                // this tile's partial sums into the compensated run sums
+                float *hi = ihi + slot * kSlot;
+                __nv_bfloat16 *lo = ilo + slot * kSlot;
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int q = 0; q < kSymQ; ++q) {
+                    const float v[2][3] = {{ax[q].x, ay[q].x, az[q].x},
+                                           {ax[q].y, ay[q].y, az[q].y}};
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int at = c * kSymTile + ib + (2 * q + h) * kSymThreads;
-                        float sum, err;
-                        two_sum(ihi[at], v[h][c], sum, err);
-                        ihi[at] = sum;
-                        ilo[at] = __float2bfloat16_rn(__bfloat162float(ilo[at]) + err);
-                    }
-                ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const int at = c * kSymTile + ib + (2 * q + h) * kSymThreads;
+                            float sum, err;
+                            two_sum(hi[at], v[h][c], sum, err);
+                            hi[at] = sum;
+                            lo[at] = __float2bfloat16_rn(__bfloat162float(lo[at]) + err);
+                        }
+                }
             }
-        }
-        if (t > 0) {
-            cluster_wait();  // every block's reactions to tile J - 1
-            sym_reduce_tile(cluster, rank, g, J - 1, n, jacc[(t - 1) % kSymBufs], Pj);
-        }
-        cluster_arrive();  // this block's reactions to tile J
-    }
-    cluster_wait();
-    sym_reduce_tile(cluster, rank, g, J0 + nJ - 1, n, jacc[(nJ - 1) % kSymBufs], Pj);
-    if (have_i && J0 + nJ - 1 >= I) {
-        // tile I's sums over the run: i-side slot r
-        float *dst = Pi + (sym_iside_base(I, runs) + (r - I / kSymRun)) * kSlot;
+            __syncthreads();
+            // tile J's reactions, I tiles in order; the buffers are zero again
+            float *dst = Pj + (sym_jside_base(J) + g) * kSlot;
+            for (int x = threadIdx.x; x < kSlot; x += kSymBlock) {  // x = 3 jj + c
+                float hi = half == 0 ? 0.f : jhi[x], lo = half == 0 ? 0.f : jlo[x];
 #pragma unroll
-        for (int q = 0; q < kSymQ; ++q)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int b = ib + (2 * q + h) * kSymThreads;
-                if (I * kSymTile + b < n)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int at = c * kSymTile + b;
-                        dst[at] = ihi[at] + __bfloat162float(ilo[at]);
-                    }
+                for (int w = 0; w < kSymTeams; ++w) {
+                    float sum, err;
+                    two_sum(hi, jacc[w * kSlot + x], sum, err);
+                    hi = sum;
+                    lo += err;
+                    jacc[w * kSlot + x] = 0.f;
+                }
+                if (half == 0) {
+                    jhi[x] = hi;
+                    jlo[x] = lo;
+                } else {
+                    const int jj = x / 3, c = x - 3 * jj;
+                    if (J * kSymTile + jj < n) dst[c * kSymTile + jj] = hi + lo;
+                }
             }
+            __syncthreads();
+        }
     }
-    // every block's shared memory stays until the others have read it
-    cluster_arrive();
-    cluster_wait();
+    // the I tiles' sums over the run: i-side slot r
+    for (int k = 0; k < kSymGroup; ++k) {
+        const int I = g * kSymGroup + k;
+        if (I >= T || J0 + nJ - 1 < I) break;
+        float *dst = Pi + (sym_iside_base(I, (T + kSymRun - 1) / kSymRun) + (r - I / kSymRun)) * kSlot;
+        for (int x = threadIdx.x; x < kSlot; x += kSymBlock)
+            if (I * kSymTile + x % kSymTile < n)
+                dst[x] = ihi[k * kSlot + x] + __bfloat162float(ilo[k * kSlot + x]);
+    }
 }
 
 // The factor that takes the scaled sums back: 2^(km - 2k).
@@ -308,7 +271,7 @@ __global__ void sym_reduce_kernel(const float *__restrict__ Pi, const float *__r
         lo += err;
     }
     p = Pj + sym_jside_base(K) * kSlot + c * kSymTile + local;
-    const int nj = K / kSymCluster + 1;
+    const int nj = K / kSymGroup + 1;
     for (int t = 0; t < nj; ++t) {
         const float v = __ldcs(p + (size_t)t * kSlot);
         float s, err;
@@ -361,8 +324,7 @@ __global__ void sym_pairs_reduce_kernel(const float *__restrict__ P, long long n
 
 DirectPlan make_symmetric_plan(int n)
 {
-    // 54 KB of dynamic shared memory per block, and the largest carveout to keep four
-    // resident.  Set here, when a plan is made (never inside a stream capture), per device.
+    // 216 KB of dynamic shared memory per block, and the largest carveout.  Set here, when a plan is made (never inside a stream capture), per device.
     static std::atomic<bool> attrs_set[64];
     int device = 0;
     if (cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64 &&
@@ -392,7 +354,7 @@ DirectPlan make_symmetric_plan(int n)
     p.n_jtiles = p.tiles;
     p.chunk_tiles = p.tiles;
     const uint64_t limit = g_pairs_limit.load();
-    p.clusters = (size_t)p.tiles * 12 * (size_t)(n > 0 ? n : 1) >
+    p.grouped = (size_t)p.tiles * 12 * (size_t)(n > 0 ? n : 1) >
                  (limit ? (size_t)limit : kSymPairsSlotBytes);
     return p;
 }
@@ -412,7 +374,7 @@ size_t direct_partial_doubles(const DirectPlan &p)
     const size_t n3 = 3 * (size_t)(p.n > 0 ? p.n : 1);
     if (!p.symmetric) return (size_t)p.splits * n3;
     // f64 sums, then the f32 slots carved after them
-    if (!p.clusters) return n3 + ((size_t)p.tiles * n3 + 1) / 2;
+    if (!p.grouped) return n3 + ((size_t)p.tiles * n3 + 1) / 2;
     return n3 + (sym_slot_floats(p.tiles, nullptr) + 1) / 2;
 }
 
@@ -424,7 +386,8 @@ size_t direct_partial_doubles(const DirectPlan &p)
 // (the cluster's exchange).  Force passes at 1 / 2 / 4 / 8 parts (us): 12,289
 // bodies 171 / 101 / 96 / 73, 16,387 169 / 100 / 96 / 101, 24,000 173 / 175 /
 // 187 / 181, 30,011 319 / 264 / 266 / 264, 50,000 731 / 690 / 668 / 679, 65,537
-// 1,053 / 1,073 / 1,109 / 1,125.
+// 1,053 / 1,073 / 1,109 / 1,125 (with the pair loop unrolled by two; 2 to 3% less
+// each since it is not).
 static int pair_parts(int n, int sms)
 {
     const double tiles = (double)n / kSymTile;
@@ -450,7 +413,7 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const f
                             cudaEvent_t pairs_done)
 {
     if (plan.n <= 0) return PHYSIM_OK;
-    if (!plan.clusters) {
+    if (!plan.grouped) {
         const long long T = plan.tiles;
         const long long units = T * (T + 1) / 2;
         PG_CHECK(units < (1ll << 31), PHYSIM_ERR_ARGUMENT, "too many bodies for one pass: %d",
@@ -479,7 +442,7 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const f
         return PHYSIM_OK;
     }
     const int T = plan.tiles;
-    const long long blocks = sym_clusters(T) * kSymCluster;
+    const long long blocks = sym_units(T);
     PG_CHECK(blocks < (1ll << 31), PHYSIM_ERR_ARGUMENT, "too many bodies for one pass: %d",
              plan.n);
     const long long n3 = 3ll * plan.n;
@@ -487,7 +450,7 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const f
     sym_slot_floats(T, &jside_at);
     float *Pi = (float *)(partial + n3);
     float *Pj = Pi + jside_at;
-    direct_sym_kernel<<<(unsigned)blocks, kSymThreads, kSymSmem, stream>>>(
+    direct_sym_kernel<<<(unsigned)blocks, kSymBlock, kSymSmem, stream>>>(
         body4, mass256, plan.n, T, e, scale, Pi, Pj);
     PG_CUDA(cudaGetLastError());
     if (pairs_done) PG_TRY(record_event(pairs_done, stream));

@@ -31,14 +31,15 @@ __device__ __forceinline__ void unit_tiles(long long u, int &I, int &J)
 
 // Tile I's bodies in registers: positions (negated) scaled by sc, masses
 // (negated) by msc (PairScale in engine.h).  Thread layout: bodies
-// I*1024 + p*128 + warp*32 + lane, p = 2q (x half) and 2q+1 (y half).
+// I*1024 + p*64 + t, p = 2q (x half) and 2q+1 (y half), t = 0..63 within the
+// two warps that hold the tile.
 constexpr int kSymQ = kSymIpt / 2;
 
 __device__ __forceinline__ void sym_load_i(const float4 *__restrict__ body, int I, float sc,
                                            float msc, float2 (&nx)[kSymQ], float2 (&ny)[kSymQ],
                                            float2 (&nz)[kSymQ], float2 (&nm)[kSymQ])
 {
-    const int ib = I * kSymTile + (threadIdx.x >> 5) * 32 + (threadIdx.x & 31);
+    const int ib = I * kSymTile + (threadIdx.x & (kSymThreads - 1));
 #pragma unroll
     for (int q = 0; q < kSymQ; ++q) {
         const float4 b0 = body[ib + (2 * q) * kSymThreads];
@@ -97,6 +98,11 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
     const float2 g2 = make_float2(kPairGuard, kPairGuard);
     const unsigned full = 0xffffffffu;
     const int src = (lane + 1) & 31;
+    // steps per turn of the loop, by what the registers' rotation costs in moves:
+    // ADD (131,072 bodies by groups) 1 / 2 / 4 / 8 / 16: - / 9.90 / 9.59 / 9.35 / 9.37
+    // ms; else (524,288 bodies by tile pairs) 1 / 2 / 4: 62.4 / 64.0 / 64.3 ms, with
+    // masses of their own 69.2 / 70.0 / -
+    constexpr int kUnroll = ADD ? 8 : 1;
 
     float4 next = body[J * kSymTile + g0 * 32 + lane];
     for (int g = g0; g < g1; ++g) {
@@ -105,7 +111,7 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
         if (g + 1 < g1) next = body[J * kSymTile + (g + 1) * 32 + lane];
         float xj = bj.x * sc, yj = bj.y * sc, zj = bj.z * sc, mj = bj.w * msc;
         float2 jx = make_float2(0.f, 0.f), jy = jx, jz = jx;
-#pragma unroll 2
+#pragma unroll kUnroll
         for (int k = 0; k < 32; ++k) {
             const float2 xj2 = make_float2(xj, xj);
             const float2 yj2 = make_float2(yj, yj);

@@ -112,12 +112,12 @@ struct DirectPlan {
     bool compensated = true;
     // Every unordered pair evaluated once (direct_sym.cu): `tiles` body tiles
     // of 1,024; the partial sums come out as one split, after f32 slot sums
-    // the same allocation holds.  clusters: thread-block clusters over runs of
-    // tiles (3T^2/32 slots of 3 x 1,024 floats); otherwise one block per tile
-    // pair (one [3][n] slot per tile).
+    // the same allocation holds.  grouped: a block takes 8 I tiles and a
+    // run of 16 J tiles (3T^2/32 slots of 3 x 1,024 floats); otherwise one block
+    // per tile pair (one [3][n] slot per tile).
     bool symmetric = false;
     int tiles = 0;
-    bool clusters = false;
+    bool grouped = false;
     // Blocks that own their bodies (direct_small.cu) run instead of the one-pair
     // kernels that the fields above describe; the sums come out as one split.
     bool small = false;

@@ -53,8 +53,8 @@ SYMMETRIC_CAP_BYTES = 284_208 * (1 << 20) // 4
 #   * in an ensemble (GpuExecutor): one [3][n] f32 slot per 1,024-body tile
 #     for each member from the threshold up (csrc/ensemble.cu, plan_ensemble);
 #   * as its own simulation (PlainExecutor): the same while those stay within
-#     4 GiB (one block per tile pair), else thread-block clusters of 8 I tiles
-#     over runs of 16 J tiles with [3][1,024] slots in a triangular layout
+#     4 GiB (one block per tile pair), else one block per 8 I tiles and
+#     run of 16 J tiles with [3][1,024] slots in a triangular layout
 #     (csrc/direct_sym.cu, make_symmetric_plan and direct_partial_doubles)
 SYM_TILE = 1024
 SYM_PAIRS_SLOT_BYTES = 4 << 30
