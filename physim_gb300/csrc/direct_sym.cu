@@ -382,12 +382,12 @@ size_t direct_partial_doubles(const DirectPlan &p)
 // schedulers, so an SM's time is that of its blocks rounded up to an even
 // number, each 1 / parts of a tile pair; while more blocks than are resident at
 // once (four per SM) follow one another, the last ones run beside idle slots,
-// about one block's time more; and each doubling of the parts costs some 3%
-// (the cluster's exchange).  Force passes at 1 / 2 / 4 / 8 parts (us): 12,289
-// bodies 171 / 101 / 96 / 73, 16,387 169 / 100 / 96 / 101, 24,000 173 / 175 /
-// 187 / 181, 30,011 319 / 264 / 266 / 264, 50,000 731 / 690 / 668 / 679, 65,537
-// 1,053 / 1,073 / 1,109 / 1,125 (with the pair loop unrolled by two; 2 to 3% less
-// each since it is not).
+// about one block's time more; up to two per SM leave a scheduler one warp, 3%;
+// and each doubling of the parts costs some 3% (the cluster's exchange).  Steps
+// at 1 / 2 / 4 / 8 parts (us): 12,600 bodies 164 / 96 / 92 / 70, 16,387 164 / 96 /
+// 92 / 99, 22,000 166 / 170 / 160 / 150, 24,000 164 / 169 / 180 / 175, 30,011 310 /
+// 254 / 258 / 256, 50,000 703 / 667 / 650 / 663, 65,537 1,032 / 1,051 / 1,086 /
+// 1,103.
 static int pair_parts(int n, int sms)
 {
     const double tiles = (double)n / kSymTile;
@@ -399,6 +399,7 @@ static int pair_parts(int n, int sms)
         const double blocks = pairs * parts;
         double time = 2.0 * ceil(blocks / sms / 2.0);
         if (blocks > 4.0 * sms) time += 1.0;
+        if (blocks <= 2.0 * sms) time *= 1.03;
         time *= (1.0 + 0.03 * step) / parts;
         if (time < best_time) {
             best_time = time;
