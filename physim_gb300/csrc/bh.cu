@@ -3372,13 +3372,17 @@ int bh_traversal_ms(BhWorkspace *ws, double *ms)
 
 int bh_launches(const BhWorkspace *ws) { return ws ? ws->launches : 0; }
 
+const uint32_t *bh_flags(const BhWorkspace *ws) { return ws->flags; }
+
+bool bh_failed(const uint32_t f[4]) { return f[kFlagStack] != 0 || f[kFlagSort] != 0; }
+
 int bh_check(BhWorkspace *ws, cudaStream_t st)
 {
     if (!ws) return PHYSIM_OK;
     uint32_t f[4];
     PG_CUDA(cudaMemcpyAsync(f, ws->flags, sizeof f, cudaMemcpyDeviceToHost, st));
     PG_CUDA(cudaStreamSynchronize(st));
-    if (f[kFlagStack] == 0 && f[kFlagSort] == 0) return PHYSIM_OK;
+    if (!bh_failed(f)) return PHYSIM_OK;
     PG_CUDA(cudaMemsetAsync(ws->flags + kFlagStack, 0, 2 * sizeof(uint32_t), st));
     PG_CUDA(cudaStreamSynchronize(st));
     if (f[kFlagSort]) {

@@ -43,7 +43,6 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
     const Entity *state_in = state;
     if (direct) {
         host_prefault(state, n * sizeof(Entity), false);
-        host_prefault(acc, n * sizeof(Acceleration), true);
     } else {
         if (el->acc_cap < n) {
             dev_free(el->d_acc, st);
@@ -90,12 +89,16 @@ static int accumulate_locked(ElementState *el, const Entity *state, size_t n, Ac
         PG_TRY(bh_reserve(el->bh, n, el->device, p, st));
         PG_TRY(bh_accelerations(el->bh, el->bodies, p, el->partial, st));
     }
-    PG_TRY(launch_accumulate_aos(el->bodies, el->partial, splits, acc_io, st));
+    // only the last kernel touches acc: its pages are mapped while the others run
+    if (direct) host_prefault(acc, n * sizeof(Acceleration), true);
+    const bool direct_flags = tree && direct;
+    PG_TRY(launch_accumulate_aos(el->bodies, el->partial, splits, acc_io, st,
+                                 direct_flags ? bh_flags(el->bh) : nullptr, el->flags));
     if (!direct)
         PG_CUDA(cudaMemcpyAsync(acc, el->d_acc, n * sizeof(Acceleration), cudaMemcpyDeviceToHost,
                                 st));
     PG_CUDA(cudaStreamSynchronize(st));
-    if (tree) PG_TRY(bh_check(el->bh, st));
+    if (tree && (!direct_flags || bh_failed(el->flags))) PG_TRY(bh_check(el->bh, st));
     return PHYSIM_OK;
 }
 

@@ -251,7 +251,8 @@ int launch_pack(DeviceBodies &b, cudaStream_t stream);
 // acc[i] += a_i (f64) for each non-fixed body, a_i = sum over splits of the
 // partial sums; NaN for a massless body (the reference divides F by m_i).
 int launch_accumulate_aos(const DeviceBodies &b, const double *partial, int splits,
-                          Acceleration *d_acc, cudaStream_t stream);
+                          Acceleration *d_acc, cudaStream_t stream, const uint32_t *flags = nullptr,
+                          uint32_t *flags_out = nullptr);
 // acc_soa[c*n + i] = a_i (f64).
 int launch_combine_soa(const DeviceBodies &b, const double *partial, int splits,
                        double *acc_soa, cudaStream_t stream);

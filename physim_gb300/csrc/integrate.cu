@@ -196,10 +196,14 @@ __device__ __forceinline__ void body_acc(const double *partial, int splits, int 
 
 // The block's accelerations are read and written back as one contiguous run;
 // a fixed body's entry is written back with the bits it was read with.
+// flags: four words that the kernels before this one may have raised, copied to
+// host memory (flags_out) on the way.
 __global__ void accumulate_aos_kernel(const double *__restrict__ mass, const uint8_t *fixed,
                                       const double *partial, int splits, int n,
-                                      Acceleration *acc)
+                                      Acceleration *acc, const uint32_t *flags,
+                                      uint32_t *flags_out)
 {
+    if (flags && blockIdx.x == 0 && threadIdx.x < 4) flags_out[threadIdx.x] = flags[threadIdx.x];
     __shared__ __align__(16) Acceleration s_acc[kThreads];
     const int base = blockIdx.x * kThreads;
     const int count = min(kThreads, n - base);
@@ -648,11 +652,12 @@ int launch_pack(DeviceBodies &b, cudaStream_t stream)
 }
 
 int launch_accumulate_aos(const DeviceBodies &b, const double *partial, int splits,
-                          Acceleration *d_acc, cudaStream_t stream)
+                          Acceleration *d_acc, cudaStream_t stream, const uint32_t *flags,
+                          uint32_t *flags_out)
 {
     if (b.n == 0) return PHYSIM_OK;
-    accumulate_aos_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(b.m, b.fixed, partial,
-                                                                      splits, (int)b.n, d_acc);
+    accumulate_aos_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(
+        b.m, b.fixed, partial, splits, (int)b.n, d_acc, flags, flags_out);
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }

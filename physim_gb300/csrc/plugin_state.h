@@ -36,6 +36,7 @@ struct ElementState {
     DirectPlan plan;
     int plan_n = -1;
     BhWorkspace *bh = nullptr;
+    uint32_t flags[4] = {};  // the last call's copy of bh's error flags
 };
 
 // acc[i] += a_i on host arrays (host->device copies, kernels, device->host).
@@ -67,6 +68,9 @@ int bh_reserve(BhWorkspace *&ws, size_t n, int device, const BhParams &p, cudaSt
 // raise: PHYSIM_ERR_TREE for a traversal stack overflow, PHYSIM_ERR_TIMEOUT
 // for a radix-sort look-back wait that gave up.
 int bh_check(BhWorkspace *ws, cudaStream_t st);
+// The four error flags on the device, and whether a copy of them holds an error.
+const uint32_t *bh_flags(const BhWorkspace *ws);
+bool bh_failed(const uint32_t flags[4]);
 void bh_free(BhWorkspace *ws);
 // Accelerations of the bodies in b (f64 positions and f32 copies must be
 // current) into partial[c*n + i] (one split).
