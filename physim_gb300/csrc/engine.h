@@ -200,6 +200,7 @@ struct DeviceBodies {
     Entity *aos = nullptr;  // staging for host<->device copies
     PairScale *scale = nullptr;  // pair-law maxima of the direct-sum kernels
     int ext_half = 0, mass_half = 0;  // the current halves of *scale
+    bool swap_in_capture = false;     // the capture is the owner's, which keeps count
     // the mass that all of each 256 bodies have, as f32; NaN where they differ
     // or padding is among them (direct-sum states only)
     float *mass256 = nullptr;

@@ -605,7 +605,7 @@ int swap_halves(DeviceBodies &b, bool mass_too, cudaStream_t stream)
     if (!b.scale) return PHYSIM_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PG_CUDA(cudaStreamIsCapturing(stream, &cs));
-    if (cs != cudaStreamCaptureStatusNone) {
+    if (cs != cudaStreamCaptureStatusNone && !b.swap_in_capture) {
         settle_kernel<<<1, 1, 0, stream>>>(b.scale->ext, b.ext_half,
                                            mass_too ? b.scale->mass : nullptr, b.mass_half);
         PG_CUDA(cudaGetLastError());

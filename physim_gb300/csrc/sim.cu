@@ -43,6 +43,14 @@ struct PhysimSim {
     // captured kernels read by address
     cudaGraph_t graph[4] = {};
     cudaGraphExec_t graph_exec[4] = {};
+    // The same for two whole steps (after which the halves are the same again):
+    // a graph's first kernel starts about 2 us after the kernel before the graph,
+    // where a kernel of the same graph starts after 1.  Steps, gravity's graph and
+    // the integrator / pairs of steps (us): 8,195 bodies Barnes-Hut 77.2 / 74.1, rk4
+    // of 16,387 382 / 367, 100,003 with quadrupoles 508 / 501 (four or eight steps
+    // per graph: under 1% more).
+    cudaGraph_t steps_graph[4] = {};
+    cudaGraphExec_t steps_exec[4] = {};
     double *diag = nullptr;  // 9 f64 diagnostics sums
     // rk4 (rk4.rs:24-178): the entity state saved at stage 1 and the running
     // sum of the k's, 6 x n f64 each
@@ -111,25 +119,31 @@ void drop_graphs(PhysimSim *s)
     for (int k = 0; k < 4; ++k) {
         if (s->graph_exec[k]) cudaGraphExecDestroy(s->graph_exec[k]);
         if (s->graph[k]) cudaGraphDestroy(s->graph[k]);
-        s->graph_exec[k] = nullptr;
-        s->graph[k] = nullptr;
+        if (s->steps_exec[k]) cudaGraphExecDestroy(s->steps_exec[k]);
+        if (s->steps_graph[k]) cudaGraphDestroy(s->steps_graph[k]);
+        s->graph_exec[k] = s->steps_exec[k] = nullptr;
+        s->graph[k] = s->steps_graph[k] = nullptr;
     }
 }
 
-// Captures the gravity phase into a graph.  If the stream cannot be captured
+// Captures what `work` enqueues into a graph.  If the stream cannot be captured
 // (e.g. the caller is itself capturing), the simulation stays eager.
-int sim_capture(PhysimSim *s)
+template <typename Work>
+int sim_capture(PhysimSim *s, cudaGraph_t &graph, cudaGraphExec_t &exec, Work work)
 {
-    const int k = graph_slot(s);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PG_CUDA(cudaStreamIsCapturing(s->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) {
         s->use_graph = false;
         return PHYSIM_OK;
     }
+    const int ext_half = s->b.ext_half, mass_half = s->b.mass_half;
     PG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    int splits = 1;
-    int rc = sim_forces(s, &splits);
+    s->b.swap_in_capture = true;
+    const int rc = work();
+    s->b.swap_in_capture = false;
+    s->b.ext_half = ext_half;
+    s->b.mass_half = mass_half;
     cudaGraph_t g = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
     if (rc != PHYSIM_OK) {
@@ -141,14 +155,14 @@ int sim_capture(PhysimSim *s)
         s->use_graph = false;
         return PHYSIM_OK;
     }
-    if (cudaGraphInstantiate(&s->graph_exec[k], g, 0) != cudaSuccess) {
+    if (cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         cudaGraphDestroy(g);
-        s->graph_exec[k] = nullptr;
+        exec = nullptr;
         s->use_graph = false;
         return PHYSIM_OK;
     }
-    s->graph[k] = g;
+    graph = g;
     return PHYSIM_OK;
 }
 
@@ -295,17 +309,51 @@ int generate_host(int kind, const void *params, Entity *out, size_t n, int32_t d
 }
 
 // The gravity phase of one force evaluation: the captured graph, or the
-// kernels themselves when the stream cannot be captured.
-int sim_gravity(PhysimSim *s, int *splits)
+// kernels themselves when the stream cannot be captured (or, without `capture`,
+// has not been).
+int sim_gravity(PhysimSim *s, bool capture, int *splits)
 {
     const int k = graph_slot(s);
-    if (s->use_graph && !s->graph_exec[k]) PG_TRY(sim_capture(s));
+    int captured = 1;
+    if (capture && s->use_graph && !s->graph_exec[k])
+        PG_TRY(sim_capture(s, s->graph[k], s->graph_exec[k],
+                           [&] { return sim_forces(s, &captured); }));
     if (s->graph_exec[k]) {
         PG_CUDA(cudaGraphLaunch(s->graph_exec[k], s->stream));
         *splits = s->cfg.gravity == PHYSIM_GRAVITY_SIMPLE_ASTRO ? s->plan.out_splits() : 1;
         return PHYSIM_OK;
     }
     return sim_forces(s, splits);
+}
+
+// One step.  capturing: inside a capture of this simulation's own, where the
+// gravity phase enters as kernels.
+int sim_one_step(PhysimSim *s, bool capturing, bool capture_gravity)
+{
+    int splits = 1;
+    auto forces = [&](int *n) {
+        return capturing ? sim_forces(s, n) : sim_gravity(s, capture_gravity, n);
+    };
+    if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[0], s->stream));
+    if (s->cfg.integrator == PHYSIM_INTEGRATOR_RK4) {
+        // four force evaluations at the stage states (rk4.rs:33,57,82,108)
+        for (int stage = 1; stage <= 4; ++stage) {
+            PG_TRY(forces(&splits));
+            if (stage == 4 && s->profiling) PG_CUDA(cudaEventRecord(s->ev[1], s->stream));
+            PG_TRY(launch_rk4_stage(s->b, s->partial, splits, s->cfg.dt, stage, s->rk4_save,
+                                    s->rk4_ksum, s->stream));
+        }
+    } else {
+        PG_TRY(forces(&splits));
+        if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[1], s->stream));
+        if (s->cfg.integrator == PHYSIM_INTEGRATOR_EULER)
+            PG_TRY(launch_euler(s->b, s->partial, splits, s->cfg.dt, s->stream));
+        else
+            PG_TRY(launch_verlet(s->b, s->partial, splits, s->cfg.dt, !s->history, s->stream));
+    }
+    if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[2], s->stream));
+    s->history = true;
+    return PHYSIM_OK;
 }
 
 }  // namespace
@@ -348,29 +396,24 @@ int physim_gpu_sim_step(PhysimSim *s, uint32_t steps)
         }
         return PHYSIM_OK;
     }
+    if (s->n == 0) return PHYSIM_OK;
+    // three steps or more go by pairs, and the ones left over capture nothing
+    const bool pairs = steps >= 3 && s->use_graph && !s->profiling;
     for (uint32_t k = 0; k < steps; ++k) {
-        if (s->n == 0) break;
-        int splits = 1;
-        if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[0], s->stream));
-        if (s->cfg.integrator == PHYSIM_INTEGRATOR_RK4) {
-            // four force evaluations at the stage states (rk4.rs:33,57,82,108)
-            for (int stage = 1; stage <= 4; ++stage) {
-                PG_TRY(sim_gravity(s, &splits));
-                if (stage == 4 && s->profiling) PG_CUDA(cudaEventRecord(s->ev[1], s->stream));
-                PG_TRY(launch_rk4_stage(s->b, s->partial, splits, s->cfg.dt, stage, s->rk4_save,
-                                        s->rk4_ksum, s->stream));
+        if (pairs && s->use_graph && s->history && steps - k >= 2) {
+            const int slot = graph_slot(s);
+            if (!s->steps_exec[slot])
+                PG_TRY(sim_capture(s, s->steps_graph[slot], s->steps_exec[slot], [&] {
+                    PG_TRY(sim_one_step(s, true, false));
+                    return sim_one_step(s, true, false);
+                }));
+            if (s->steps_exec[slot]) {
+                PG_CUDA(cudaGraphLaunch(s->steps_exec[slot], s->stream));
+                ++k;
+                continue;
             }
-        } else {
-            PG_TRY(sim_gravity(s, &splits));
-            if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[1], s->stream));
-            if (s->cfg.integrator == PHYSIM_INTEGRATOR_EULER)
-                PG_TRY(launch_euler(s->b, s->partial, splits, s->cfg.dt, s->stream));
-            else
-                PG_TRY(launch_verlet(s->b, s->partial, splits, s->cfg.dt, !s->history,
-                                     s->stream));
         }
-        if (s->profiling) PG_CUDA(cudaEventRecord(s->ev[2], s->stream));
-        s->history = true;
+        PG_TRY(sim_one_step(s, false, !pairs));
     }
     return PHYSIM_OK;
 }
