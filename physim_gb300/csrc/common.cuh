@@ -87,11 +87,17 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &err)
 // Programmatic dependent launch (PTX griddepcontrol): a kernel launched by
 // launch_pdl may be set up, and its blocks start, while the kernel before it on
 // the stream still runs; pdl_wait, the first thing it does, returns when that one
-// has ended and its writes are visible.  It takes the launch latency (1 to 2 us)
+// has ended and its writes are visible (pdl_trigger: the next one may do so beside
+// this one).  It takes the launch latency (1 to 2 us)
 // out of a chain of short kernels.
-__device__ __forceinline__ void pdl_wait()
+__device__ __forceinline__ void pdl_trigger()
 {
     asm volatile("griddepcontrol.launch_dependents;");
+}
+
+__device__ __forceinline__ void pdl_wait()
+{
+    pdl_trigger();
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 

@@ -242,6 +242,7 @@ __global__ void verlet_kernel(float4 *body4, const double *mass, const uint8_t *
                               double *vy, double *vz, double *px, double *py, double *pz,
                               Divisor dt, int initial, Track ext)
 {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
     if (i < n) {
@@ -330,6 +331,7 @@ __global__ void euler_kernel(float4 *body4, const double *mass, const uint8_t *f
                              const double *partial, int splits, int n, double *x, double *y,
                              double *z, double *vx, double *vy, double *vz, Divisor dt, Track ext)
 {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
     if (i < n) {
@@ -401,6 +403,7 @@ __global__ void rk4_stage_kernel(float4 *body4, const double *mass, const uint8_
                                  double *z, double *vx, double *vy, double *vz, double *save,
                                  double *ksum, double dt, int stage, Divisor six, Track ext)
 {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t top = 0;
     if (i < n) {
@@ -676,9 +679,9 @@ int launch_verlet(DeviceBodies &b, const double *partial, int splits, double dt,
                   cudaStream_t stream)
 {
     if (b.n == 0) return PHYSIM_OK;
-    verlet_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
-        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.px, b.py,
-        b.pz, make_divisor(dt), initial ? 1 : 0, next_extent(b));
+    PG_TRY(launch_pdl(verlet_kernel, integrator_blocks(b.n), integrator_threads(b.n), stream,
+                      b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy,
+                      b.vz, b.px, b.py, b.pz, make_divisor(dt), initial ? 1 : 0, next_extent(b)));
     return swap_halves(b, false, stream);
 }
 
@@ -686,9 +689,9 @@ int launch_euler(DeviceBodies &b, const double *partial, int splits, double dt,
                  cudaStream_t stream)
 {
     if (b.n == 0) return PHYSIM_OK;
-    euler_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
-        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz,
-        make_divisor(dt), next_extent(b));
+    PG_TRY(launch_pdl(euler_kernel, integrator_blocks(b.n), integrator_threads(b.n), stream,
+                      b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy,
+                      b.vz, make_divisor(dt), next_extent(b)));
     return swap_halves(b, false, stream);
 }
 
@@ -697,9 +700,9 @@ int launch_rk4_stage(DeviceBodies &b, const double *partial, int splits, double 
 {
     if (b.n == 0) return PHYSIM_OK;
     PG_CHECK(stage >= 1 && stage <= 4, PHYSIM_ERR_ARGUMENT, "rk4 stage %d", stage);
-    rk4_stage_kernel<<<integrator_blocks(b.n), integrator_threads(b.n), 0, stream>>>(
-        b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy, b.vz, save,
-        ksum, dt, stage, make_divisor(6.0), next_extent(b));
+    PG_TRY(launch_pdl(rk4_stage_kernel, integrator_blocks(b.n), integrator_threads(b.n), stream,
+                      b.body4, b.m, b.fixed, partial, splits, (int)b.n, b.x, b.y, b.z, b.vx, b.vy,
+                      b.vz, save, ksum, dt, stage, make_divisor(6.0), next_extent(b)));
     return swap_halves(b, false, stream);
 }
 
