@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
 small_forces_kernel(const float4 *__restrict__ body, int n, float e, ScaleRef scale,
                     double *__restrict__ out)
 {
+    pdl_wait();
     __shared__ SmallShared sh;
     const int i0 = (int)((long long)blockIdx.x * n / gridDim.x);
     const int m = (int)((long long)(blockIdx.x + 1) * n / gridDim.x) - i0;
@@ -378,10 +379,8 @@ int launch_direct_small(const float4 *body4, int n, float e, ScaleRef scale, dou
 {
     int device = 0;
     PG_CUDA(cudaGetDevice(&device));
-    small_forces_kernel<<<small_grid(n, device_sm_count(device)), kSmallThreads, 0, stream>>>(
-        body4, n, e, scale, partial);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+    return launch_pdl(small_forces_kernel, small_grid(n, device_sm_count(device)), kSmallThreads,
+                      stream, body4, n, e, scale, partial);
 }
 
 int reserve_small(SmallWork &w, const DeviceBodies &b, int device, cudaStream_t stream)

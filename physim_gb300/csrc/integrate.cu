@@ -94,6 +94,7 @@ __global__ void unpack_kernel(const Entity *__restrict__ in, int n, int n_pad, f
                               double *vy, double *vz, double *m, double *radius, uint64_t *id,
                               Track ext, Track mass, float *mass256)
 {
+    pdl_trigger();
     static_assert(kThreads == 256, "a block fills one entry of mass256");
     __shared__ __align__(16) Entity s_in[kThreads];
     const int base = blockIdx.x * kThreads;
@@ -203,6 +204,7 @@ __global__ void accumulate_aos_kernel(const double *__restrict__ mass, const uin
                                       Acceleration *acc, const uint32_t *flags,
                                       uint32_t *flags_out)
 {
+    pdl_wait();
     if (flags && blockIdx.x == 0 && threadIdx.x < 4) flags_out[threadIdx.x] = flags[threadIdx.x];
     __shared__ __align__(16) Acceleration s_acc[kThreads];
     const int base = blockIdx.x * kThreads;
@@ -659,10 +661,11 @@ int launch_accumulate_aos(const DeviceBodies &b, const double *partial, int spli
                           uint32_t *flags_out)
 {
     if (b.n == 0) return PHYSIM_OK;
-    accumulate_aos_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(
-        b.m, b.fixed, partial, splits, (int)b.n, d_acc, flags, flags_out);
-    PG_CUDA(cudaGetLastError());
-    return PHYSIM_OK;
+    // (as dependent launches, this and the small force kernel: 1,002 bodies 57 -> 51 us
+    // per pipeline step, 50,021 by quadtree 271 -> 264; the pair sums' reduction gains
+    // nothing by it, rk4 of 16,387 1,804 -> 1,824)
+    return launch_pdl(accumulate_aos_kernel, blocks_for(b.n), kThreads, stream, b.m, b.fixed,
+                      partial, splits, (int)b.n, d_acc, flags, flags_out);
 }
 
 int launch_combine_soa(const DeviceBodies &b, const double *partial, int splits,
