@@ -231,6 +231,13 @@ void bodies_free(DeviceBodies &b, cudaStream_t stream);
 // memory access through the host's page tables); false when they copy.
 // Fails if DIRECT is requested on a device that cannot.
 int host_direct(int device, bool *direct);
+// Whether a download of `bytes` to `p` is packed straight into the caller's array:
+// host access is direct, p is aligned for it, and the array is small enough to come
+// from mapped pages of the allocator (above 32 MB each allocation is fresh pages,
+// which a copy maps while it moves others: 1,048,580 bodies 3.7 ms by copy, 3.9 in
+// place; 8,195 23 / 20 us and 262,147 139 / 133, in a Barnes-Hut simulation, whose
+// error flags come along, 34 / 18 and 151 / 145; 30 members 636 / 495).
+int download_direct(int device, const void *p, size_t bytes, bool *direct);
 // Before kernels touch a host array in place: maps every page of
 // [p, p + bytes) into the process (writable if `write`), without changing its
 // contents, so the GPU meets no page that was never touched.  A GPU access to
@@ -246,8 +253,10 @@ void host_prefault(const void *p, size_t bytes, bool write);
 // its 256 entities as one contiguous run.
 int launch_unpack(DeviceBodies &b, const Entity *aos, size_t n, bool full_state,
                   cudaStream_t stream);
-// Packs the SoA state back into b.aos.
-int launch_pack(DeviceBodies &b, cudaStream_t stream);
+// Packs the SoA state into out, device memory or (host_direct) host memory, and
+// copies four words from flags, if given, to flags_out.
+int launch_pack(DeviceBodies &b, Entity *out, cudaStream_t stream, const uint32_t *flags = nullptr,
+                uint32_t *flags_out = nullptr);
 
 // acc[i] += a_i (f64) for each non-fixed body, a_i = sum over splits of the
 // partial sums; NaN for a massless body (the reference divides F by m_i).

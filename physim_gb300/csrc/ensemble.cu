@@ -273,23 +273,38 @@ __global__ void ensemble_unpack_kernel(const Entity *__restrict__ in, int n, int
     id[s] = (uint64_t)en.id;
 }
 
-__global__ void ensemble_pack_kernel(Entity *out, int n, int off, const uint8_t *fixed,
-                                     const double *x, const double *y, const double *z,
-                                     const double *vx, const double *vy, const double *vz,
-                                     const double *m, const double *radius, const uint64_t *id)
+// A block's records leave as one contiguous run: out may be host memory.
+__global__ void __launch_bounds__(256)
+ensemble_pack_kernel(Entity *out, int n, int off, const uint8_t *fixed, const double *x,
+                     const double *y, const double *z, const double *vx, const double *vy,
+                     const double *vz, const double *m, const double *radius, const uint64_t *id)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int s = off + i;
-    Entity en;
-    memset(&en, 0, sizeof en);
-    en.x = x[s]; en.y = y[s]; en.z = z[s];
-    en.vx = vx[s]; en.vy = vy[s]; en.vz = vz[s];
-    en.radius = radius[s];
-    en.mass = m[s];
-    en.id = (uintptr_t)id[s];
-    en.fixed = fixed[s] != 0;
-    out[i] = en;
+    __shared__ __align__(16) Entity s_out[256];
+    const int base = blockIdx.x * 256, i = base + threadIdx.x;
+    if (i < n) {
+        const int s = off + i;
+        Entity en;
+        memset(&en, 0, sizeof en);
+        en.x = x[s]; en.y = y[s]; en.z = z[s];
+        en.vx = vx[s]; en.vy = vy[s]; en.vz = vz[s];
+        en.radius = radius[s];
+        en.mass = m[s];
+        en.id = (uintptr_t)id[s];
+        en.fixed = fixed[s] != 0;
+        s_out[threadIdx.x] = en;
+    }
+    __syncthreads();
+    // 16-byte words (80 B records) where the array allows
+    const int bytes = min(256, n - base) * (int)sizeof(Entity);
+    if (((uintptr_t)out & 15) == 0) {
+        const int4 *src = reinterpret_cast<const int4 *>(s_out);
+        int4 *dst = reinterpret_cast<int4 *>(out + base);
+        for (int w = threadIdx.x; w < bytes / 16; w += 256) dst[w] = src[w];
+    } else {
+        const long long *src = reinterpret_cast<const long long *>(s_out);
+        long long *dst = reinterpret_cast<long long *>(out + base);
+        for (int w = threadIdx.x; w < bytes / 8; w += 256) dst[w] = src[w];
+    }
 }
 
 // A member's slot range [off, off + slot_len): the first n slots belong to
@@ -916,7 +931,12 @@ int physim_gpu_ensemble_download(PhysimEnsemble *E, size_t index, Entity *state,
     PG_CHECK(n == E->sizes[index], PHYSIM_ERR_ARGUMENT, "member %zu holds %zu bodies, not %zu",
              index, E->sizes[index], n);
     PG_CUDA(cudaSetDevice(E->device));
-    if (n > E->staging_cap) {
+    bool direct = false;
+    PG_TRY(download_direct(E->device, state, n * sizeof(Entity), &direct));
+    if (direct) {
+        // written in place; the pages are mapped while the steps still run
+        host_prefault(state, n * sizeof(Entity), true);
+    } else if (n > E->staging_cap) {
         dev_free(E->staging, E->stream);
         E->staging = nullptr;
         PG_TRY(ealloc(E, E->staging, n));
@@ -924,11 +944,12 @@ int physim_gpu_ensemble_download(PhysimEnsemble *E, size_t index, Entity *state,
     }
     const int off = E->members[index].off;
     ensemble_pack_kernel<<<cdiv((long long)n, 256), 256, 0, E->stream>>>(
-        E->staging, (int)n, off, E->fixed, E->x, E->y, E->z, E->vx, E->vy, E->vz, E->m, E->radius,
-        E->id);
+        direct ? state : E->staging, (int)n, off, E->fixed, E->x, E->y, E->z, E->vx, E->vy, E->vz,
+        E->m, E->radius, E->id);
     PG_CUDA(cudaGetLastError());
-    PG_CUDA(cudaMemcpyAsync(state, E->staging, n * sizeof(Entity), cudaMemcpyDeviceToHost,
-                            E->stream));
+    if (!direct)
+        PG_CUDA(cudaMemcpyAsync(state, E->staging, n * sizeof(Entity), cudaMemcpyDeviceToHost,
+                                E->stream));
     PG_CUDA(cudaStreamSynchronize(E->stream));
     return PHYSIM_OK;
 }

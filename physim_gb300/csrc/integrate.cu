@@ -132,26 +132,35 @@ __global__ void unpack_kernel(const Entity *__restrict__ in, int n, int n_pad, f
     }
 }
 
+// A block's records leave as one contiguous run: out may be host memory.  flags:
+// see accumulate_aos_kernel.
 __global__ void pack_kernel(Entity *out, int n, const uint8_t *fixed, const double *x,
                             const double *y, const double *z, const double *vx, const double *vy,
                             const double *vz, const double *m, const double *radius,
-                            const uint64_t *id)
+                            const uint64_t *id, const uint32_t *flags, uint32_t *flags_out)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Entity en;
-    memset(&en, 0, sizeof en);
-    en.x = x[i];
-    en.y = y[i];
-    en.z = z[i];
-    en.vx = vx[i];
-    en.vy = vy[i];
-    en.vz = vz[i];
-    en.radius = radius[i];
-    en.mass = m[i];
-    en.id = (uintptr_t)id[i];
-    en.fixed = fixed[i] != 0;
-    out[i] = en;
+    __shared__ __align__(16) Entity s_out[kThreads];
+    if (flags && blockIdx.x == 0 && threadIdx.x < 4) flags_out[threadIdx.x] = flags[threadIdx.x];
+    const int base = blockIdx.x * kThreads;
+    const int count = min(kThreads, n - base);
+    const int i = base + threadIdx.x;
+    if (i < n) {
+        Entity en;
+        memset(&en, 0, sizeof en);
+        en.x = x[i];
+        en.y = y[i];
+        en.z = z[i];
+        en.vx = vx[i];
+        en.vy = vy[i];
+        en.vz = vz[i];
+        en.radius = radius[i];
+        en.mass = m[i];
+        en.id = (uintptr_t)id[i];
+        en.fixed = fixed[i] != 0;
+        s_out[threadIdx.x] = en;
+    }
+    __syncthreads();
+    block_copy(out + base, s_out, count * (int)sizeof(Entity));
 }
 
 // a_i from the partial sums; zero for fixed bodies (never accumulated);
@@ -544,6 +553,13 @@ int host_direct(int device, bool *direct)
     return PHYSIM_OK;
 }
 
+int download_direct(int device, const void *p, size_t bytes, bool *direct)
+{
+    PG_TRY(host_direct(device, direct));
+    *direct = *direct && ((uintptr_t)p & 7) == 0 && bytes <= (size_t(32) << 20);
+    return PHYSIM_OK;
+}
+
 void bodies_free(DeviceBodies &b, cudaStream_t stream)
 {
     void *ptrs[] = {b.body4, b.fixed, b.x,  b.y,  b.z,      b.vx, b.vy,    b.vz,
@@ -646,12 +662,13 @@ int launch_unpack(DeviceBodies &b, const Entity *aos, size_t n, bool full_state,
     return swap_halves(b, true, stream);
 }
 
-int launch_pack(DeviceBodies &b, cudaStream_t stream)
+int launch_pack(DeviceBodies &b, Entity *out, cudaStream_t stream, const uint32_t *flags,
+                uint32_t *flags_out)
 {
     if (b.n == 0) return PHYSIM_OK;
-    pack_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(b.aos, (int)b.n, b.fixed, b.x, b.y,
-                                                            b.z, b.vx, b.vy, b.vz, b.m,
-                                                            b.radius, b.id);
+    pack_kernel<<<blocks_for(b.n), kThreads, 0, stream>>>(out, (int)b.n, b.fixed, b.x, b.y, b.z,
+                                                            b.vx, b.vy, b.vz, b.m, b.radius, b.id,
+                                                            flags, flags_out);
     PG_CUDA(cudaGetLastError());
     return PHYSIM_OK;
 }
