@@ -330,7 +330,7 @@ int physim_gpu_generate_plummer(const PhysimPlummerParams *p, Entity *out, size_
 
 /* Waits for the stream, then copies the current state out.  This call, sim_accelerations
  * and sim_synchronize report a Barnes-Hut traversal stack overflow
- * (PHYSIM_ERR_TREE) or a radix-sort wait that gave up (PHYSIM_ERR_TIMEOUT) raised by
+ * (PHYSIM_ERR_TREE) or a device-side wait that gave up (PHYSIM_ERR_TIMEOUT) raised by
  * the kernels since the last check. */
 int physim_gpu_sim_download(PhysimSim *sim, Entity *state, size_t n);
 /* Waits, then writes the accelerations of the current state (not +=). */
@@ -392,26 +392,29 @@ int physim_gpu_set_symmetric_cap(uint64_t bytes);
  * is made.  No reference counterpart (simple_astro, transformers.rs:219-244,
  * has no plans). */
 int physim_gpu_set_symmetric_pairs_limit(uint64_t bytes);
-/* Barnes-Hut builds wait on other thread blocks only in the radix sort: its
- * decoupled look-back and, when its passes run as one launch, the barrier
- * between passes.  Every such wait gives up after `polls` polls that saw no
+/* Thread blocks wait on others in the sort and the one-launch tree build of
+ * Barnes-Hut builds (grid barriers; the decoupled look-back of the sort of large
+ * states) and between the whole steps of a small direct sum (a grid barrier).
+ * Every such wait gives up after `polls` polls that saw no
  * progress (0 restores the default, 2^20), raising an error flag: later
- * kernels of the build and the traversal then return at once and the next
+ * kernels of the build and the traversal, or the remaining steps, then return at once and the next
  * synchronising call (physim_gpu_sim_synchronize / _download, the transform)
  * reports PHYSIM_ERR_TIMEOUT.  Process-wide, read when a build is enqueued or
  * captured.  No reference counterpart (the reference builds its tree on one
  * CPU thread, octree.rs:27-128). */
 int physim_gpu_set_wait_limit(uint32_t polls);
-/* How the Barnes-Hut build runs its 7-pass radix sort: `on` != 0 (default)
- * runs every pass in one cooperative launch where the device supports
- * cooperative launches (a grid barrier between passes, bounded by the wait
- * limit above), 0 runs one launch per pass.  The sorted order, and so every
+/* How the Barnes-Hut build runs: `on` != 0 (default) runs extent, keys and sort
+ * in one cooperative launch up to 1.2M bodies (beyond, the radix sort's passes),
+ * and the tree of up to 512 bodies per SM in another, where the device supports
+ * cooperative launches (grid barriers, bounded by the wait limit above); 0 runs
+ * separate launches, one per radix pass.  The sorted order, and so every
  * result, is the same either way.  Process-wide, read when a build is enqueued
  * or captured.  No reference counterpart (octree.rs:27-128 sorts on one CPU
  * thread). */
 int physim_gpu_set_sort_single_launch(int32_t on);
 /* Test hook for the path above: tile `tile` (>= 0; -1 turns it off) of each
- * radix pass sees no predecessor word, so its wait always runs out.
+ * radix pass sees no predecessor word (of the resident sorts, waits for a count
+ * that nothing reaches), so its wait always runs out.
  * Process-wide, read when a build is enqueued or captured. */
 int physim_gpu_test_stall_sort(int32_t tile);
 /* The current pair-kernel plan of a simple_astro simulation (block, ipt,
