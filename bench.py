@@ -772,7 +772,7 @@ def measure_ensemble(args, dist: Dist, device: int) -> dict:
                                     "seconds": plain_s,
                                     "path": "physim_gpu_sim_step per member, members in turn, "
                                             "each with its heuristic plan (each pair once "
-                                            "above 12,500 bodies)"},
+                                            "above 7,400 bodies)"},
             "plain_one_pair_kernels": {"value": one_pair_rate, "unit": "member-steps/s",
                                        "seconds": one_pair_s,
                                        "path": "the same, one-pair kernels only (every ordered "

@@ -351,7 +351,7 @@ void *physim_gpu_sim_stream(PhysimSim *sim);
 /* Pair-kernel plan of a simple_astro simulation: threads per block, bodies
  * per thread, j-range splits, candidates timed, whether every unordered pair
  * is evaluated once (and in how many body tiles of 1,024), time of one force
- * pass.  States of up to 12,500 bodies whose plan is the heuristic or the tuned
+ * pass.  States of up to 7,400 bodies whose plan is the heuristic or the tuned
  * one may run in blocks that own their bodies instead (many verlet steps per
  * launch); block, ipt and splits then describe the one-pair kernels that
  * physim_gpu_sim_set_plan would give them. */

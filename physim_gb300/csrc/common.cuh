@@ -95,9 +95,10 @@ __device__ __forceinline__ void pdl_trigger()
     asm volatile("griddepcontrol.launch_dependents;");
 }
 
-__device__ __forceinline__ void pdl_wait()
+// early: the kernel after this one may come in at once, as pdl_trigger.
+__device__ __forceinline__ void pdl_wait(bool early = true)
 {
-    pdl_trigger();
+    if (early) pdl_trigger();
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 

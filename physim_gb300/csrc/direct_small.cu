@@ -25,8 +25,9 @@
 //     arrays, and one grid barrier per step (1.2 us, every block resident by a
 //     cooperative launch) lets the next step read them.
 // Step times against the best tiled or each-pair-once plan (us): 300 bodies 14.4
-// -> 3.7, 1,002 16.5 -> 4.1, 4,098 24.7 -> 11.8, 8,192 37.8 -> 37.6, 12,000 82
-// -> 74; at 14,000 the each-pair-once plan takes 77.  Bound by the FMA pipe (60%
+// -> 3.7, 1,002 16.5 -> 4.1, 4,098 24.7 -> 11.7, and against the each-pair-once
+// plan as it is now 6,500 32.8 -> 25.8, 7,400 31.3 -> 31.6, 8,192 32.3 -> 37.5,
+// 10,000 52 -> 57, 12,000 60 -> 75: the line is at 7,400.  Bound by the FMA pipe (60%
 // busy) from about 6,000 bodies, below by the barrier and one pass of latency.
 // Eight warps of 255 registers, four bodies i at a time: sixteen of 128, two at a
 // time, left the pipe waiting on each chain (4,098 bodies 14.1).  A wait at the barrier that exceeds the wait limit raises an
@@ -50,6 +51,7 @@ constexpr int kMaxPacks = 8;     // units every warp holds at a time (some one m
 constexpr int kMaxOwned = 84;    // bodies per block (a thread per coordinate)
 constexpr int kTurn = 4;         // owned bodies per turn of the pair loop
 constexpr int kUnit = 64;        // bodies of a unit
+constexpr int kSmallOwned = 16;  // bodies per block until every SM has one
 constexpr uint32_t kPoison = 0x40000000u;
 
 struct SmallShared {
@@ -218,10 +220,10 @@ __device__ __forceinline__ void put_owned(SmallShared &sh, int t, float4 p, floa
 
 // One force pass: out[c * n + i], f64 and unscaled.
 __global__ void __launch_bounds__(kSmallThreads, 1)
-small_forces_kernel(const float4 *__restrict__ body, int n, float e, ScaleRef scale,
+small_forces_kernel(const float4 *__restrict__ body, int n, float e, ScaleRef scale, int early,
                     double *__restrict__ out)
 {
-    pdl_wait();
+    pdl_wait(early != 0);
     __shared__ SmallShared sh;
     const int i0 = (int)((long long)blockIdx.x * n / gridDim.x);
     const int m = (int)((long long)(blockIdx.x + 1) * n / gridDim.x) - i0;
@@ -365,7 +367,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_steps_kernel(SmallStep
 // Blocks: sixteen bodies each until every SM has one, then n / SMs.  (Fewer per
 // block would shorten the smallest steps by 0.4 us, but a block takes a whole
 // SM's registers, and several such simulations side by side would queue.)
-int small_grid(int n, int sms) { return std::max(1, std::min(sms, (n + 15) / 16)); }
+int small_grid(int n, int sms)
+{
+    return std::max(1, std::min(sms, (n + kSmallOwned - 1) / kSmallOwned));
+}
 
 }  // namespace
 
@@ -379,8 +384,12 @@ int launch_direct_small(const float4 *body4, int n, float e, ScaleRef scale, dou
 {
     int device = 0;
     PG_CUDA(cudaGetDevice(&device));
-    return launch_pdl(small_forces_kernel, small_grid(n, device_sm_count(device)), kSmallThreads,
-                      stream, body4, n, e, scale, partial);
+    // Where this kernel fills every SM's registers, the next one must not be let in
+    // early: it finds no room, and a force pass and integrator of 3,000 bodies take
+    // 17.6 us instead of 10.4.
+    const int sms = device_sm_count(device), grid = small_grid(n, sms);
+    return launch_pdl(small_forces_kernel, grid, kSmallThreads, stream, body4, n, e, scale,
+                      grid < sms ? 1 : 0, partial);
 }
 
 int reserve_small(SmallWork &w, const DeviceBodies &b, int device, cudaStream_t stream)

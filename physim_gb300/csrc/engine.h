@@ -158,7 +158,7 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const f
                             cudaEvent_t pairs_done);
 // Largest state of the blocks that own their bodies (compensated sums), by the
 // measured steps against the next best plan: see plan_direct.
-constexpr int kDirectSmallMax = 12500;
+constexpr int kDirectSmallMax = 7400;
 int direct_small_limit(int device);
 // One force pass; partial: 3 n doubles, one split.
 int launch_direct_small(const float4 *body4, int n, float e, ScaleRef scale, double *partial,
