@@ -2164,6 +2164,7 @@ struct BuildArgs {
     uint32_t *bar;  // [0] barrier count, [1] blocks that left
     uint32_t *flags;
     int spin_limit;
+    bool early;  // SMs are free for the next kernel's blocks
 };
 
 template <bool kQuad, bool kExact, int kLanes>
@@ -2237,7 +2238,9 @@ __global__ void __launch_bounds__(kBuildBlock, 1) tree_build_kernel(BuildArgs a)
     // the traversal's blocks may come in beside the cells; with the counts it adds to
     // cleared by the sort instead of a memset between the two, and the integrator as
     // dependent launch after it, a step of 8,195 bodies takes 67.3 us instead of 74.1
-    pdl_trigger();
+    // (not where this grid holds every SM, 50,021 bodies with one per leaf 80.1
+    // instead of 77.9 us)
+    if (a.early) pdl_trigger();
     if (ok)
         cell_nodes<kQuad, kExact, kLanes>(keys, a.gather.sbody, a.nd, lv.total, nchild,
                                           a.gather.sg, a.extent_bits);
@@ -3583,6 +3586,7 @@ static int launch_build(BhWorkspace *ws, const GatherArgs &ga, const BhParams &p
     const int nodes = (int)(1.6 * ga.n / std::max(1.0, 0.625 * p.leaf_size)) + 1;
     const int blocks = std::min(
         sms, std::max(cdiv(ga.n, kBuildBlock) + 1, cdiv(nodes * lanes, kBuildBlock)));
+    a.early = blocks < sms;
     void *args[] = {&a};
     PG_CUDA(cudaLaunchCooperativeKernel(
         lanes == 8 ? tree_build_fn<8>(quad, exact) : tree_build_fn<1>(quad, exact),
