@@ -327,8 +327,8 @@ int sim_gravity(PhysimSim *s, bool capture, int *splits)
     return sim_forces(s, splits);
 }
 
-// One step.  capturing: inside a capture of this simulation's own, where the
-// gravity phase enters as kernels.
+// One step.  capturing: inside a capture (of this simulation's own or the
+// caller's), where the gravity phase enters as kernels.
 int sim_one_step(PhysimSim *s, bool capturing, bool capture_gravity)
 {
     int splits = 1;
@@ -398,6 +398,14 @@ int physim_gpu_sim_step(PhysimSim *s, uint32_t steps)
         return PHYSIM_OK;
     }
     if (s->n == 0) return PHYSIM_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PG_CUDA(cudaStreamIsCapturing(s->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {
+        // the caller is capturing: the kernels themselves (a graph cannot be launched
+        // into a capture, whether or not earlier steps left one for this half)
+        for (; steps > 0; --steps) PG_TRY(sim_one_step(s, true, false));
+        return PHYSIM_OK;
+    }
     // three steps or more go by pairs, and the ones left over capture nothing
     const bool pairs = steps >= 3 && s->use_graph && !s->profiling;
     for (uint32_t k = 0; k < steps; ++k) {

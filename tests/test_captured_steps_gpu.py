@@ -1,0 +1,45 @@
+"""Steps that a caller captures."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(n, scale, seed):
+    from physim_gb300 import ics
+    s = ics.plummer(n, seed=seed)
+    for f in "xyz":
+        s[f] *= scale
+    for f in ("vx", "vy", "vz"):
+        s[f] = 0.0
+    s["mass"] *= np.random.default_rng(seed).uniform(0.5, 1.5, size=n)
+    s["fixed"][n // 2] = 1
+    return s
+
+
+@pytest.mark.parametrize("integrator", ["verlet", "euler", "rk4"])
+@pytest.mark.parametrize("gravity,n", [("simple_astro", 3000), ("simple_astro", 9001),
+                                       ("astro2", 3000)])
+def test_captured_after_any_number_of_steps(gravity, n, integrator):
+    """The simulation's own graphs are there by then, or not, for the current half of
+    the maxima: a step and a run of steps are captured all the same, and leave the
+    bits of steps that were never captured."""
+    torch = pytest.importorskip("torch")
+    import physim_gb300 as pg
+    stream = torch.cuda.Stream()
+    kw = dict(gravity=gravity, theta=0.8, e=0.01, dt=1e-4, integrator=integrator)
+    first = _state(n, 1.0, 1)
+    with pg.Simulation(first, pg.SimConfig(stream=stream.cuda_stream, **kw)) as sim, \
+            pg.Simulation(first, pg.SimConfig(**kw)) as ref:
+        for before, captured in ((1, 1), (1, 1), (2, 2), (5, 4)):
+            sim.step(before)
+            sim.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                sim.step(captured)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            ref.step(before + captured)
+            assert sim.download().tobytes() == ref.download().tobytes(), (before, captured)
