@@ -417,6 +417,10 @@ int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int st
     int device = 0;
     PG_CUDA(cudaGetDevice(&device));
     PG_CHECK(w.words && w.body4, PHYSIM_ERR_ARGUMENT, "no workspace for whole steps");
+    // a caller's graph keeps the addresses of the maxima (PairScale)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PG_CUDA(cudaStreamIsCapturing(stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) b.halves_fixed = true;
     SmallSteps a;
     a.body[0] = b.body4;
     a.body[1] = w.body4;

@@ -48,7 +48,10 @@ constexpr float kPairGuard = 1.17549435e-38f;
 // bodies).  Each maximum has two halves: the kernel that writes a state adds its
 // bodies' maxima to the half that is not current, which is zero, and clears the
 // current one, which no later kernel on the stream reads; then the halves change
-// places (DeviceBodies::ext_half, mass_half).
+// places (DeviceBodies::ext_half, mass_half).  A graph that a caller captured keeps
+// the addresses of the halves that were current then, and may be launched at any
+// time after: from the first such capture on the halves stay where they are, and
+// the values move instead (swap_halves), also after steps and uploads outside it.
 struct PairScale {
     uint32_t ext[2];   // largest |coordinate|
     uint32_t mass[2];  // largest |mass| (unpack only: integrators keep masses)
@@ -201,6 +204,7 @@ struct DeviceBodies {
     PairScale *scale = nullptr;  // pair-law maxima of the direct-sum kernels
     int ext_half = 0, mass_half = 0;  // the current halves of *scale
     bool swap_in_capture = false;     // the capture is the owner's, which keeps count
+    bool halves_fixed = false;        // a caller's graph reads the current halves
     // the mass that all of each 256 bodies have, as f32; NaN where they differ
     // or padding is among them (direct-sum states only)
     float *mass256 = nullptr;

@@ -616,21 +616,24 @@ __global__ void settle_kernel(uint32_t *ext, int eh, uint32_t *mass, int mh)
     }
 }
 
-// After a kernel that filled the other halves: they are current from here on.
-// Inside a capture (the caller's, whose graph may be launched any number of
-// times) the values move instead, so that every launch finds them where this
-// one did.
+// After a kernel that filled the other halves: they are current from here on, or,
+// once a caller has captured such a kernel (its graph may be launched any number of
+// times, between other steps and uploads), the values move back into the halves
+// that its kernels read.
 int swap_halves(DeviceBodies &b, bool mass_too, cudaStream_t stream)
 {
     PG_CUDA(cudaGetLastError());
     if (!b.scale) return PHYSIM_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PG_CUDA(cudaStreamIsCapturing(stream, &cs));
-    if (cs != cudaStreamCaptureStatusNone && !b.swap_in_capture) {
-        settle_kernel<<<1, 1, 0, stream>>>(b.scale->ext, b.ext_half,
-                                           mass_too ? b.scale->mass : nullptr, b.mass_half);
-        PG_CUDA(cudaGetLastError());
-        return PHYSIM_OK;
+    if (!b.swap_in_capture) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        PG_CUDA(cudaStreamIsCapturing(stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) b.halves_fixed = true;
+        if (b.halves_fixed) {
+            settle_kernel<<<1, 1, 0, stream>>>(b.scale->ext, b.ext_half,
+                                               mass_too ? b.scale->mass : nullptr, b.mass_half);
+            PG_CUDA(cudaGetLastError());
+            return PHYSIM_OK;
+        }
     }
     b.ext_half ^= 1;
     if (mass_too) b.mass_half ^= 1;

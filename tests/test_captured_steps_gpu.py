@@ -43,3 +43,66 @@ def test_captured_after_any_number_of_steps(gravity, n, integrator):
                 graph.replay()
             ref.step(before + captured)
             assert sim.download().tobytes() == ref.download().tobytes(), (before, captured)
+
+
+@pytest.mark.parametrize("integrator", ["verlet", "euler", "rk4"])
+@pytest.mark.parametrize("n", [3000, 9001])
+@pytest.mark.parametrize("scale,e,dt", [(1e7, 0.01, 1e4), (1e-7, 0.0, 1e-13)])
+def test_between_other_steps_and_uploads(n, scale, e, dt, integrator):
+    """A captured step launched between steps and uploads outside its graph
+    (csrc/integrate.cu: swap_halves): every state and its accelerations are, bit for
+    bit, those of a simulation that was never captured.  At these coordinates
+    accelerations are lost without the pair law's scale, so a graph or a later step
+    that misses the current maxima shows."""
+    torch = pytest.importorskip("torch")
+    import physim_gb300 as pg
+    stream = torch.cuda.Stream()
+    kw = dict(gravity="simple_astro", e=e, dt=dt, integrator=integrator)
+    first, second = _state(n, scale, 1), _state(n, 3.0 * scale, 2)
+    second["mass"] *= 1e6
+    with pg.Simulation(first, pg.SimConfig(stream=stream.cuda_stream, **kw)) as sim, \
+            pg.Simulation(first, pg.SimConfig(**kw)) as ref:
+        sim.step(1)
+        sim.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            sim.step(1)
+        ref.step(1)
+
+        def check(what):
+            got, want = sim.accelerations(), ref.accelerations()
+            assert np.count_nonzero(want["x"]) == n - 1, what  # one body is fixed
+            assert got.tobytes() == want.tobytes(), what
+            assert sim.download().tobytes() == ref.download().tobytes(), what
+
+        def replay():
+            with torch.cuda.stream(stream):
+                graph.replay()
+            ref.step(1)
+
+        check("capture")
+        replay()
+        check("graph")
+        sim.step(1)
+        ref.step(1)
+        check("step")
+        replay()
+        check("graph after a step")
+        sim.step(5)
+        ref.step(5)
+        check("steps")
+        replay()
+        replay()
+        check("graph twice")
+        for s in (sim, ref):
+            s.upload(second)
+        if integrator == "verlet":  # the graph's step is not the first of a state
+            sim.step(1)
+            ref.step(1)
+        check("upload")
+        replay()
+        check("graph after an upload")
+        sim.step(1)
+        ref.step(1)
+        replay()
+        check("step and graph after an upload")
