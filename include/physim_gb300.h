@@ -397,9 +397,10 @@ int physim_gpu_set_symmetric_pairs_limit(uint64_t bytes);
  * states) and between the whole steps of a small direct sum (a grid barrier).
  * Every such wait gives up after `polls` polls that saw no
  * progress (0 restores the default, 2^20), raising an error flag: later
- * kernels of the build and the traversal, or the remaining steps, then return at once and the next
+ * kernels of the build and the traversal, or the launch's remaining steps, then return at
+ * once and the next
  * synchronising call (physim_gpu_sim_synchronize / _download, the transform)
- * reports PHYSIM_ERR_TIMEOUT.  Process-wide, read when a build is enqueued or
+ * reports PHYSIM_ERR_TIMEOUT; the state is invalid until the next upload.  Process-wide, read when a build is enqueued or
  * captured.  No reference counterpart (the reference builds its tree on one
  * CPU thread, octree.rs:27-128). */
 int physim_gpu_set_wait_limit(uint32_t polls);

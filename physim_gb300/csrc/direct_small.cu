@@ -420,7 +420,7 @@ int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int st
     // a caller's graph keeps the addresses of the maxima (PairScale)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PG_CUDA(cudaStreamIsCapturing(stream, &cs));
-    if (cs != cudaStreamCaptureStatusNone) b.halves_fixed = true;
+    if (cs != cudaStreamCaptureStatusNone) b.halves_fixed = w.captured = true;
     SmallSteps a;
     a.body[0] = b.body4;
     a.body[1] = w.body4;
@@ -453,7 +453,7 @@ int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int st
 
 int check_small_steps(SmallWork &w, cudaStream_t stream)
 {
-    if (!w.unchecked) return PHYSIM_OK;
+    if (!w.unchecked && !w.captured) return PHYSIM_OK;
     w.unchecked = false;
     uint32_t f = 0;
     PG_CUDA(cudaMemcpyAsync(&f, w.words + 6, sizeof f, cudaMemcpyDeviceToHost, stream));

@@ -172,6 +172,7 @@ struct SmallWork {
     uint32_t *words = nullptr;
     float4 *body4 = nullptr;
     bool unchecked = false;  // launches since the last check
+    bool captured = false;   // a caller's graph may launch at any time
 };
 struct DeviceBodies;
 int reserve_small(SmallWork &w, const DeviceBodies &b, int device, cudaStream_t stream);
@@ -179,8 +180,9 @@ void free_small(SmallWork &w, cudaStream_t stream);
 int small_steps_per_launch(int n);
 int launch_small_steps(DeviceBodies &b, SmallWork &w, float e, double dt, int steps, bool initial,
                        cudaStream_t stream);
-// Waits for the stream if steps were launched since the last check, then reports
-// a wait between two of them that gave up.
+// Waits for the stream if steps were launched since the last check, or may have
+// been by a graph of the caller's, then reports a wait between two of them that
+// gave up.
 int check_small_steps(SmallWork &w, cudaStream_t stream);
 // Polls after which a kernel's wait gives up (physim_gpu_set_wait_limit).
 int wait_limit();

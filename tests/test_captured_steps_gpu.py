@@ -106,3 +106,38 @@ def test_between_other_steps_and_uploads(n, scale, e, dt, integrator):
         ref.step(1)
         replay()
         check("step and graph after an upload")
+
+
+def test_every_launch_that_gives_up_is_reported():
+    """Whole steps of a small direct sum, captured with a wait limit of one poll:
+    each launch of the graph is reported by the next synchronising call, not only the
+    one that the capture itself announced.  (The state is invalid from the first on,
+    until the next upload.)"""
+    torch = pytest.importorskip("torch")
+    import physim_gb300 as pg
+    stream = torch.cuda.Stream()
+    s = _state(4098, 1.0, 3)
+    cfg = pg.SimConfig(gravity="simple_astro", e=0.01, dt=1e-4, stream=stream.cuda_stream)
+    with pg.Simulation(s, cfg) as sim:
+        sim.step(1)
+        sim.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        pg.lib.physim_gpu_set_wait_limit(1)
+        try:
+            with torch.cuda.graph(graph, stream=stream):
+                sim.step(50)
+        finally:
+            pg.lib.physim_gpu_set_wait_limit(0)
+        for call in (sim.synchronize, sim.download, sim.accelerations):
+            with torch.cuda.stream(stream):
+                graph.replay()
+            with pytest.raises(pg.PhysimError) as err:
+                call()
+            assert err.value.code == 5  # PHYSIM_ERR_TIMEOUT
+        sim.synchronize()  # reported once each
+        sim.upload(s)
+        sim.step(3)
+        got = sim.download()
+    with pg.Simulation(s, pg.SimConfig(gravity="simple_astro", e=0.01, dt=1e-4)) as sim:
+        sim.step(3)
+        assert sim.download().tobytes() == got.tobytes()
