@@ -31,6 +31,7 @@
 #include "direct_sym_tile.cuh"
 #include "direct_tile.cuh"
 #include "engine.h"
+#include "ensemble_plan.h"
 #include "verlet_axis.cuh"
 
 namespace pg {
@@ -330,8 +331,6 @@ struct Shape {
 };
 constexpr Shape kShapes[] = {{128, 2}, {128, 4}, {256, 4}, {256, 2}, {128, 8}};
 constexpr int kChunks[] = {4096, 8192, 16384, 65536};
-// Most j chunks a member of n bodies is split into (sizes the partial sums).
-inline int max_splits(int n) { return std::max((n + 4095) / 4096, std::min(8, (n + 255) / 256)); }
 // Default size from which members use the symmetric units, and the thresholds
 // the autotuner compares (INT32_MAX: none).
 constexpr int kEnsembleSymMin = 8192;
@@ -463,12 +462,11 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     int64_t poff = 0, soff = 0;
     for (size_t k = 0; k < E->members.size(); ++k) {
         MemberInfo &mi = E->members[k];
-        mi.n_jtiles = cdiv(mi.n, block);
-        const int chunk_k = std::max((int)std::min<long long>(chunk, even),
-                                     cdiv(mi.n, max_splits(mi.n)));
-        const int chunk_tiles = std::max(1, cdiv(chunk_k, block));
+        const MemberCut cut = cut_member(mi.n, block, (int)std::min<long long>(chunk, even));
+        const int chunk_tiles = cut.chunk_tiles;
+        mi.n_jtiles = cut.n_jtiles;
         mi.chunk_tiles = chunk_tiles;
-        mi.splits = std::max(1, cdiv(mi.n_jtiles, chunk_tiles));
+        mi.splits = cut.splits;
         mi.poff = poff;
         mi.sym_tiles = 0;
         mi.soff = soff;
@@ -651,7 +649,7 @@ int physim_gpu_ensemble_create(const PhysimSimConfig *cfg, const size_t *sizes, 
         mi.dt = make_divisor(E->cfg.dt);
         E->members[k] = mi;
         slots += (long long)pad_bodies(sizes[k]);
-        partial_elems += 3LL * (long long)sizes[k] * max_splits((int)sizes[k]);
+        partial_elems += 3LL * (long long)sizes[k] * most_splits((int)sizes[k]);
     }
     if (slots >= (1LL << 31)) {
         delete E;
