@@ -117,9 +117,11 @@ static double wave_efficiency(long units, long slots)
 }
 
 // Bodies from which the heuristic plan evaluates each unordered pair once (below
-// kDirectSmallMax bodies compensated states take direct_small.cu).  Measured on GB300 (step of the best one-pair plan vs the symmetric plan):
-// 4,098 bodies 25 vs 37 us, 6,000 31 vs 39, 8,192 49 vs 38, 12,289 87 vs 73,
-// 16,387 139 vs 96, 65,536 1.81 vs 1.05 ms.
+// kDirectSmallMax bodies compensated states take direct_small.cu).  Measured on
+// GB300, step of the best one-pair plan vs the symmetric plan (us): 4,098 bodies 25
+// vs 38, 6,000 31 vs 40, 8,192 55 vs 33, 9,001 61 vs 57, 12,001 84 vs 69, 16,387
+// 154 vs 92, 65,536 1,810 vs 1,050; with different masses 8,192 55 vs 38, 9,001 61
+// vs 60, 16,387 154 vs 107.
 constexpr int kSymmetricMinBodies = 7168;
 // Smallest size at which the autotuner also times the symmetric plan.
 constexpr int kSymmetricCandidateBodies = 4096;

@@ -79,6 +79,16 @@ namespace {
 constexpr size_t kSymPairsSlotBytes = size_t(4) << 30;
 std::atomic<uint64_t> g_pairs_limit{0};
 
+// States below this many bodies, which the one-pair kernels would take otherwise,
+// are summed as exactly as those do (FINE, sym_pair_core), in slots of two f32, the
+// sum and what its rounding dropped.  RMS error against f64 at e = 0.01 (1e-8 of the
+// acceleration), one-pair kernels / chains of a tile and one f32 per slot / FINE:
+// Plummer 8,192 bodies 3.3 / 4.2 / 2.8, 16,387 4.8 / 4.9 / 4.0, 20,479 3.0 / 3.5 /
+// 2.9, cube with four heavy stars 8,192 5.7 / 8.7 / 5.7, 20,479 5.7 / 7.8 / 5.7.
+// FINE costs 2 to 6% of a step (16,387 bodies 89 -> 92 us, one-pair 154) and, where
+// masses differ, some 10% (97 -> 107).  From 20,480 on, plain chains as ever.
+constexpr int kSymFine = 20480;
+
 constexpr int kSymTeams = 4;    // I tiles in registers at a time, two warps each
 constexpr int kSymGroup = 8;    // I tiles per unit
 constexpr int kSymRun = 16;     // J tiles per run
@@ -182,10 +192,10 @@ direct_sym_kernel(const float4 *__restrict__ body, const float *__restrict__ mas
                 uni = common_mass(mass256, J * 4, J * 4 + 4, mj) && uni;
                 float (*jw)[3] = reinterpret_cast<float (*)[3]>(jacc + team * kSlot);
                 if (I < J)
-                    sym_pair<false, true>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
+                    sym_pair<false, true, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
                                           msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
                 else
-                    sym_pair<true, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
+                    sym_pair<true, false, false>(uni, mi * msc, mj * msc, body, J, 0, kSymGroups, sc,
                                           msc, e2, nx, ny, nz, nm, ax, ay, az, jw);
                 // this tile's partial sums into the compensated run sums
                 float *hi = ihi + slot * kSlot;
@@ -284,6 +294,7 @@ __global__ void sym_reduce_kernel(const float *__restrict__ Pi, const float *__r
 
 // The tile-pair schedule: `parts` consecutive blocks (a thread-block cluster)
 // take tile pair (I, J) (unit_tiles).
+template <bool FINE>
 __global__ void __launch_bounds__(kSymThreads, 4)
 direct_sym_pairs_kernel(const float4 *__restrict__ body, const float *__restrict__ mass256, int n,
                         float e, ScaleRef scale, float *__restrict__ P, int parts)
@@ -295,27 +306,33 @@ direct_sym_pairs_kernel(const float4 *__restrict__ body, const float *__restrict
     const int sk = pair_scale_exp(__uint_as_float(*scale.ext), e);
     const int skm = mass_scale_exp(__uint_as_float(*scale.mass));
     if (I == J)
-        sym_tile_pair<true>(body, mass256, n, I, J, e, sk, skm, P, smem, rank, parts);
+        sym_tile_pair<true, FINE>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
     else
-        sym_tile_pair<false>(body, mass256, n, I, J, e, sk, skm, P, smem, rank, parts);
+        sym_tile_pair<false, FINE>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
 }
 
 // out[idx] = the sum of entry idx of the T slots P[t][3][n], in slot order,
-// TwoSum-compensated, rounded once to f64 and unscaled (x 2^(km - 2k)).
+// TwoSum-compensated, rounded once to f64 and unscaled (x 2^(km - 2k)); FINE: the
+// slots are float2 (sym_tile_pair).
+template <bool FINE>
 __global__ void sym_pairs_reduce_kernel(const float *__restrict__ P, long long n3, int T,
                                         ScaleRef scale, float e, double *__restrict__ out)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n3) return;
     float hi = 0.f, lo = 0.f;
-    const float *p = P + idx;
 #pragma unroll 8
     for (int t = 0; t < T; ++t) {
-        const float v = __ldcs(p + (size_t)t * n3);
+        const size_t at = (size_t)t * n3 + idx;
+        float2 v = make_float2(0.f, 0.f);
+        if (FINE)
+            v = __ldcs(reinterpret_cast<const float2 *>(P) + at);
+        else
+            v.x = __ldcs(P + at);
         float s, err;
-        two_sum(hi, v, s, err);
+        two_sum(hi, v.x, s, err);
         hi = s;
-        lo += err;
+        lo += FINE ? err + v.y : err;
     }
     out[idx] = ((double)hi + (double)lo) * unscale(scale, e);
 }
@@ -337,10 +354,10 @@ DirectPlan make_symmetric_plan(int n)
         if (cudaFuncSetAttribute(direct_sym_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             (void)cudaGetLastError();  // a hint only: the kernel runs without it
-        if (cudaFuncSetAttribute(direct_sym_pairs_kernel,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            (void)cudaGetLastError();
+        for (auto *pairs : {direct_sym_pairs_kernel<false>, direct_sym_pairs_kernel<true>})
+            if (cudaFuncSetAttribute(pairs, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+                (void)cudaGetLastError();
     }
     DirectPlan p;
     p.symmetric = true;
@@ -374,7 +391,7 @@ size_t direct_partial_doubles(const DirectPlan &p)
     const size_t n3 = 3 * (size_t)(p.n > 0 ? p.n : 1);
     if (!p.symmetric) return (size_t)p.splits * n3;
     // f64 sums, then the f32 slots carved after them
-    if (!p.grouped) return n3 + ((size_t)p.tiles * n3 + 1) / 2;
+    if (!p.grouped) return n3 + ((p.n < kSymFine ? 2 : 1) * (size_t)p.tiles * n3 + 1) / 2;
     return n3 + (sym_slot_floats(p.tiles, nullptr) + 1) / 2;
 }
 
@@ -434,11 +451,13 @@ int launch_direct_symmetric(const DirectPlan &plan, const float4 *body4, const f
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = parts > 1 ? 1 : 0;
-        PG_CUDA(cudaLaunchKernelEx(&cfg, direct_sym_pairs_kernel, body4, mass256, plan.n, e, scale,
-                                   P, parts));
+        PG_CUDA(cudaLaunchKernelEx(
+            &cfg, plan.n < kSymFine ? direct_sym_pairs_kernel<true> : direct_sym_pairs_kernel<false>,
+            body4, mass256, plan.n, e, scale, P, parts));
         if (pairs_done) PG_TRY(record_event(pairs_done, stream));
-        sym_pairs_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(
-            P, n3, (int)T, scale, e, partial);
+        auto reduce = plan.n < kSymFine ? sym_pairs_reduce_kernel<true>
+                                        : sym_pairs_reduce_kernel<false>;
+        reduce<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(P, n3, (int)T, scale, e, partial);
         PG_CUDA(cudaGetLastError());
         return PHYSIM_OK;
     }

@@ -71,6 +71,16 @@ __device__ __forceinline__ bool common_mass(const float *__restrict__ mass256, i
     return same;
 }
 
+// a += g with what the addition drops in g (TwoSum).
+__device__ __forceinline__ void fold2(float2 &a, float2 &g)
+{
+    const float2 minus = make_float2(-1.f, -1.f);
+    const float2 s = add2(a, g);
+    const float2 gp = fma2(a, minus, s), ap = fma2(gp, minus, s);
+    g = add2(fma2(ap, minus, a), fma2(gp, minus, g));
+    a = s;
+}
+
 // Tile I (in registers) against groups [g0, g1) of 32 bodies of tile J: a_i +=
 // the pairs' terms (scaled, see sym_load_i); unless DIAG, tile J's reactions go
 // to shared memory, jw[j][c] for body j from group g0 on: stored (this warp's own slice), or with ADD added to
@@ -84,7 +94,13 @@ __device__ __forceinline__ bool common_mass(const float *__restrict__ mass256, i
 // instead of 17 and 10), the reactions leave multiplied by nmi (minus tile I's
 // scaled mass), and the caller multiplies a_i by tile J's.  One rounding per sum
 // takes the place of one per term.
-template <bool DIAG, bool ADD, bool UNI>
+// With FINE the sums are as exact as the one-pair kernels' (direct_tile.cuh: chains
+// of 128 terms, folded by TwoSum): a_i takes each group's 32 terms as one sum, and
+// a travelling body's reaction each step's eight, so that no chain is longer than
+// 32 (1,024 and 256 otherwise).  A group in which one body outweighs the others by
+// far is folded every four terms, by TwoSum: after such a body's term each plain add
+// rounds at its size.
+template <bool DIAG, bool ADD, bool UNI, bool FINE>
 __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, int J, int g0,
                                               int g1, float sc, float msc, float nmi, float2 e2,
                                               const float2 (&nx)[kSymQ],
@@ -104,6 +120,11 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
     // masses of their own 69.2 / 70.0 / -
     constexpr int kUnroll = ADD ? 8 : 1;
 
+    float2 gx[FINE ? kSymQ : 1], gy[FINE ? kSymQ : 1], gz[FINE ? kSymQ : 1];
+    if (FINE) {
+#pragma unroll
+        for (int q = 0; q < kSymQ; ++q) gx[q] = gy[q] = gz[q] = make_float2(0.f, 0.f);
+    }
     float4 next = body[J * kSymTile + g0 * 32 + lane];
     for (int g = g0; g < g1; ++g) {
         const float4 bj = next;
@@ -111,8 +132,15 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
         if (g + 1 < g1) next = body[J * kSymTile + (g + 1) * 32 + lane];
         float xj = bj.x * sc, yj = bj.y * sc, zj = bj.z * sc, mj = bj.w * msc;
         float2 jx = make_float2(0.f, 0.f), jy = jx, jz = jx;
-#pragma unroll kUnroll
-        for (int k = 0; k < 32; ++k) {
+        int run = 32;  // FINE: steps between two folds
+        if (FINE && !UNI) {
+            float sum = fabsf(mj);
+            const float most =
+                __uint_as_float(__reduce_max_sync(full, __float_as_uint(sum)));
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+            if (most > 0.125f * sum) run = 4;  // four times the mean
+        }
+        auto step = [&]() {
             const float2 xj2 = make_float2(xj, xj);
             const float2 yj2 = make_float2(yj, yj);
             const float2 zj2 = make_float2(zj, zj);
@@ -122,6 +150,7 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
             yj = __shfl_sync(full, yj, src);
             zj = __shfl_sync(full, zj, src);
             if (!UNI) mj = __shfl_sync(full, mj, src);
+            float2 rx, ry, rz;  // FINE: this step's reaction
 #pragma unroll
             for (int q = 0; q < kSymQ; ++q) {
                 const float2 dx = add2(xj2, nx[q]);
@@ -135,15 +164,32 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
                 const float2 qv = fma2(r2, ww, g2);
                 const float2 inv = make_float2(rsqrt_approx(qv.x), rsqrt_approx(qv.y));
                 const float2 fi = UNI ? inv : mul2(mj2, inv);
-                ax[q] = fma2(dx, fi, ax[q]);
-                ay[q] = fma2(dy, fi, ay[q]);
-                az[q] = fma2(dz, fi, az[q]);
+                if (FINE) {
+                    gx[q] = fma2(dx, fi, gx[q]);
+                    gy[q] = fma2(dy, fi, gy[q]);
+                    gz[q] = fma2(dz, fi, gz[q]);
+                } else {
+                    ax[q] = fma2(dx, fi, ax[q]);
+                    ay[q] = fma2(dy, fi, ay[q]);
+                    az[q] = fma2(dz, fi, az[q]);
+                }
                 if (!DIAG) {
                     const float2 fj = UNI ? inv : mul2(nm[q], inv);
-                    jx = fma2(dx, fj, jx);
-                    jy = fma2(dy, fj, jy);
-                    jz = fma2(dz, fj, jz);
+                    if (FINE) {
+                        rx = q == 0 ? mul2(dx, fj) : fma2(dx, fj, rx);
+                        ry = q == 0 ? mul2(dy, fj) : fma2(dy, fj, ry);
+                        rz = q == 0 ? mul2(dz, fj) : fma2(dz, fj, rz);
+                    } else {
+                        jx = fma2(dx, fj, jx);
+                        jy = fma2(dy, fj, jy);
+                        jz = fma2(dz, fj, jz);
+                    }
                 }
+            }
+            if (!DIAG && FINE) {
+                jx = add2(jx, rx);
+                jy = add2(jy, ry);
+                jz = add2(jz, rz);
             }
             if (!DIAG) {
                 jx.x = __shfl_sync(full, jx.x, src);
@@ -152,6 +198,32 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
                 jy.y = __shfl_sync(full, jy.y, src);
                 jz.x = __shfl_sync(full, jz.x, src);
                 jz.y = __shfl_sync(full, jz.y, src);
+            }
+        };
+        if (FINE && !UNI) {
+#pragma unroll 1
+            for (int k = 0; k < 32; k += run) {
+#pragma unroll 1
+                for (int u = 0; u < run; ++u) step();
+                if (run == 32) break;
+#pragma unroll
+                for (int q = 0; q < kSymQ; ++q) {
+                    fold2(ax[q], gx[q]);
+                    fold2(ay[q], gy[q]);
+                    fold2(az[q], gz[q]);
+                }
+            }
+        } else {
+#pragma unroll kUnroll
+            for (int k = 0; k < 32; ++k) step();
+        }
+        if (FINE) {
+#pragma unroll
+            for (int q = 0; q < kSymQ; ++q) {
+                ax[q] = add2(ax[q], gx[q]);
+                ay[q] = add2(ay[q], gy[q]);
+                az[q] = add2(az[q], gz[q]);
+                gx[q] = gy[q] = gz[q] = make_float2(0.f, 0.f);
             }
         }
         if (!DIAG) {
@@ -174,7 +246,7 @@ __device__ __forceinline__ void sym_pair_core(const float4 *__restrict__ body, i
 
 // sym_pair_core with the variant that the tiles' masses allow.  uni: tile I's
 // scaled mass mi and the groups' mj are common.  a_i must enter as zero.
-template <bool DIAG, bool ADD>
+template <bool DIAG, bool ADD, bool FINE>
 __device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
                                          const float4 *__restrict__ body, int J, int g0, int g1,
                                          float sc, float msc, float2 e2,
@@ -184,7 +256,7 @@ __device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
                                          float2 (&az)[kSymQ], float (*jw)[3])
 {
     if (uni) {
-        sym_pair_core<DIAG, ADD, true>(body, J, g0, g1, sc, msc, -mi, e2, nx, ny, nz, nm, ax, ay,
+        sym_pair_core<DIAG, ADD, true, FINE>(body, J, g0, g1, sc, msc, -mi, e2, nx, ny, nz, nm, ax, ay,
                                        az, jw);
         const float2 m2 = make_float2(mj, mj);
 #pragma unroll
@@ -194,7 +266,7 @@ __device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
             az[q] = mul2(az[q], m2);
         }
     } else {
-        sym_pair_core<DIAG, ADD, false>(body, J, g0, g1, sc, msc, 0.f, e2, nx, ny, nz, nm, ax, ay,
+        sym_pair_core<DIAG, ADD, false, FINE>(body, J, g0, g1, sc, msc, 0.f, e2, nx, ny, nz, nm, ax, ay,
                                         az, jw);
     }
 }
@@ -207,13 +279,14 @@ __device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
 // take the parts: their sums for tile I are added through distributed shared
 // memory, ranks in order with TwoSum, each block adding and writing its share
 // of the bodies, so there is one slot per tile pair whatever the parts.
+// pairs: the slots are float2, the sum and what its rounding to f32 dropped.
 // smem: 6 x 1,024 floats.
-template <bool DIAG>
+template <bool DIAG, bool FINE>
 __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
                                               const float *__restrict__ mass256, int n, int I,
                                               int J, float e, int sk, int skm,
-                                              float *__restrict__ P, float *smem, int rank = 0,
-                                              int parts = 1)
+                                              float *__restrict__ P, bool pairs, float *smem,
+                                              int rank = 0, int parts = 1)
 {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -235,25 +308,31 @@ __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
         float mi = 0.f, mj = 0.f;
         bool uni = common_mass(mass256, I * 4, I * 4 + 4, mi);
         uni = common_mass(mass256, J * 4 + g0 / 8, J * 4 + (g1 + 7) / 8, mj) && uni;
-        sym_pair<DIAG, false>(uni, mi * msc, mj * msc, body, J, g0, g1, sc, msc, e2, nx, ny, nz,
+        sym_pair<DIAG, false, FINE>(uni, mi * msc, mj * msc, body, J, g0, g1, sc, msc, e2, nx, ny, nz,
                               nm, ax, ay, az, jacc + warp * rows);
     }
+    auto put = [&](int slot, int c, int k, float hi, float lo) {
+        const size_t at = (size_t)slot * n3 + (size_t)c * n + k;
+        if (pairs)
+            reinterpret_cast<float2 *>(P)[at] = make_float2(hi, lo);
+        else
+            P[at] = hi + lo;
+    };
     // tile J's contribution to tile I's bodies: slot J
-    float *pi = P + (size_t)J * n3;
     if (parts == 1) {
 #pragma unroll
         for (int q = 0; q < kSymQ; ++q) {
             const int i0 = I * kSymTile + ib + (2 * q) * kSymThreads;
             const int i1 = i0 + kSymThreads;
             if (i0 < n) {
-                pi[i0] = ax[q].x;
-                pi[(size_t)n + i0] = ay[q].x;
-                pi[2 * (size_t)n + i0] = az[q].x;
+                put(J, 0, i0, ax[q].x, 0.f);
+                put(J, 1, i0, ay[q].x, 0.f);
+                put(J, 2, i0, az[q].x, 0.f);
             }
             if (i1 < n) {
-                pi[i1] = ax[q].y;
-                pi[(size_t)n + i1] = ay[q].y;
-                pi[2 * (size_t)n + i1] = az[q].y;
+                put(J, 0, i1, ax[q].y, 0.f);
+                put(J, 1, i1, ay[q].y, 0.f);
+                put(J, 2, i1, az[q].y, 0.f);
             }
         }
         if (!DIAG) __syncthreads();
@@ -290,21 +369,20 @@ __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
                 hi = s;
                 lo += err;
             }
-            pi[(size_t)c * n + i] = hi + lo;
+            put(J, c, i, hi, lo);
         }
     }
     if (!DIAG) {
         // tile I's contribution to tile J's bodies: slot I, warps added in order
-        float *pj = P + (size_t)I * n3;
+        static_assert(kSymWarps == 2, "one sum");
         for (int j = threadIdx.x; j < rows; j += kSymThreads) {
             const int k = J * kSymTile + g0 * 32 + j;
             if (k >= n) break;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                float s = jacc[j][c];
-#pragma unroll
-                for (int w = 1; w < kSymWarps; ++w) s += jacc[w * rows + j][c];
-                pj[(size_t)c * n + k] = s;
+                float s, err;
+                two_sum(jacc[j][c], jacc[rows + j][c], s, err);
+                put(I, c, k, s, pairs ? err : 0.f);
             }
         }
     }

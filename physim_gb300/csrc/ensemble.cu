@@ -120,11 +120,11 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
             const MemberInfo m = members[w.member];
             const int sk = pair_scale_from(member_kx[w.member], m.e), skm = member_km[w.member];
             if (w.I == w.J)
-                sym_tile_pair<true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                    skm, slots + m.soff, smem, rank, parts);
+                sym_tile_pair<true, false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
+                                    skm, slots + m.soff, false, smem, rank, parts);
             else
-                sym_tile_pair<false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                     skm, slots + m.soff, smem, rank, parts);
+                sym_tile_pair<false, false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
+                                     skm, slots + m.soff, false, smem, rank, parts);
         }
         __syncthreads();
     }
