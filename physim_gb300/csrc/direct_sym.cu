@@ -306,9 +306,9 @@ direct_sym_pairs_kernel(const float4 *__restrict__ body, const float *__restrict
     const int sk = pair_scale_exp(__uint_as_float(*scale.ext), e);
     const int skm = mass_scale_exp(__uint_as_float(*scale.mass));
     if (I == J)
-        sym_tile_pair<true, FINE>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
+        sym_tile_pair<true, FINE, false>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
     else
-        sym_tile_pair<false, FINE>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
+        sym_tile_pair<false, FINE, false>(body, mass256, n, I, J, e, sk, skm, P, FINE, smem, rank, parts);
 }
 
 // out[idx] = the sum of entry idx of the T slots P[t][3][n], in slot order,

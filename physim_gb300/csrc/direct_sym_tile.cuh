@@ -279,9 +279,12 @@ __device__ __forceinline__ void sym_pair(bool uni, float mi, float mj,
 // take the parts: their sums for tile I are added through distributed shared
 // memory, ranks in order with TwoSum, each block adding and writing its share
 // of the bodies, so there is one slot per tile pair whatever the parts.
+// EIGHTHS: the sums for tile I are those of eight parts whether eight blocks take one
+// each or one block takes all (parts 8 or 1), which adds them up in shared memory the
+// same way, so the result does not depend on the parts.
 // pairs: the slots are float2, the sum and what its rounding to f32 dropped.
-// smem: 6 x 1,024 floats.
-template <bool DIAG, bool FINE>
+// smem: 6 x 1,024 floats; EIGHTHS with one part 12 x 1,024.
+template <bool DIAG, bool FINE, bool EIGHTHS>
 __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
                                               const float *__restrict__ mass256, int n, int I,
                                               int J, float e, int sk, int skm,
@@ -297,19 +300,46 @@ __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
     const float2 e2 = make_float2(es, es);
     // the groups of tile J that hold bodies, shared out over the parts
     const int groups = min(kSymGroups, (n - J * kSymTile + 31) / 32);
-    const int g0 = rank * groups / parts, g1 = (rank + 1) * groups / parts;
+    const int shares = EIGHTHS ? 8 : parts;
+    const int s0 = rank * shares / parts, s1 = (rank + 1) * shares / parts;
+    const int g0 = s0 * groups / shares, g1 = s1 * groups / shares;
     const int rows = (g1 - g0) * 32;  // <= 512 with two parts or more
     float (*jacc)[3] = reinterpret_cast<float (*)[3]>(smem);  // [kSymWarps][rows][3]
     float2 nx[kSymQ], ny[kSymQ], nz[kSymQ], nm[kSymQ], ax[kSymQ], ay[kSymQ], az[kSymQ];
     sym_load_i(body, I, sc, msc, nx, ny, nz, nm);
+    float mi = 0.f;
+    const bool uni_i = common_mass(mass256, I * 4, I * 4 + 4, mi);
+    auto share = [&](int a, int b) {
 #pragma unroll
-    for (int q = 0; q < kSymQ; ++q) ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
-    if (rows > 0) {
-        float mi = 0.f, mj = 0.f;
-        bool uni = common_mass(mass256, I * 4, I * 4 + 4, mi);
-        uni = common_mass(mass256, J * 4 + g0 / 8, J * 4 + (g1 + 7) / 8, mj) && uni;
-        sym_pair<DIAG, false, FINE>(uni, mi * msc, mj * msc, body, J, g0, g1, sc, msc, e2, nx, ny, nz,
-                              nm, ax, ay, az, jacc + warp * rows);
+        for (int q = 0; q < kSymQ; ++q) ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
+        if (a == b) return;
+        float mj = 0.f;
+        const bool uni = common_mass(mass256, J * 4 + a / 8, J * 4 + (b + 7) / 8, mj) && uni_i;
+        sym_pair<DIAG, false, FINE>(uni, mi * msc, mj * msc, body, J, a, b, sc, msc, e2, nx, ny,
+                                    nz, nm, ax, ay, az, jacc + warp * rows + (a - g0) * 32);
+    };
+    float *ihi = smem + 2 * 3 * kSymTile, *ilo = ihi + 3 * kSymTile;  // [3][1,024]
+    if (EIGHTHS && parts == 1) {
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k) {
+            share(k * groups / 8, (k + 1) * groups / 8);
+#pragma unroll
+            for (int q = 0; q < kSymQ; ++q) {
+                const float v[2][3] = {{ax[q].x, ay[q].x, az[q].x}, {ax[q].y, ay[q].y, az[q].y}};
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const int at = c * kSymTile + ib + (2 * q + h) * kSymThreads;
+                        float sum, err;
+                        two_sum(k == 0 ? 0.f : ihi[at], v[h][c], sum, err);
+                        ihi[at] = sum;
+                        ilo[at] = k == 0 ? err : ilo[at] + err;
+                    }
+            }
+        }
+    } else {
+        share(g0, g1);
     }
     auto put = [&](int slot, int c, int k, float hi, float lo) {
         const size_t at = (size_t)slot * n3 + (size_t)c * n + k;
@@ -319,7 +349,16 @@ __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
             P[at] = hi + lo;
     };
     // tile J's contribution to tile I's bodies: slot J
-    if (parts == 1) {
+    if (EIGHTHS && parts == 1) {
+        for (int p = 0; p < kSymIpt; ++p) {  // (this thread's own sums)
+            const int b = ib + p * kSymThreads, i = I * kSymTile + b;
+            if (i >= n) break;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                put(J, c, i, ihi[c * kSymTile + b], ilo[c * kSymTile + b]);
+        }
+        if (!DIAG) __syncthreads();
+    } else if (parts == 1) {
 #pragma unroll
         for (int q = 0; q < kSymQ; ++q) {
             const int i0 = I * kSymTile + ib + (2 * q) * kSymThreads;
@@ -351,9 +390,9 @@ __device__ __forceinline__ void sym_tile_pair(const float4 *__restrict__ body,
             mine[2 * kSymTile + b1] = az[q].y;
         }
         cluster.sync();
-        const int share = kSymTile / parts, first = rank * share;
-        for (int t = threadIdx.x; t < 3 * share; t += kSymThreads) {
-            const int c = t / share, b = first + t - c * share;
+        const int own = kSymTile / parts, first = rank * own;
+        for (int t = threadIdx.x; t < 3 * own; t += kSymThreads) {
+            const int c = t / own, b = first + t - c * own;
             const int i = I * kSymTile + b;
             if (i >= n) continue;
             float v[8];

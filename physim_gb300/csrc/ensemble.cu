@@ -47,8 +47,8 @@ struct MemberInfo {
     float e;
     Divisor dt;
     int32_t sym_tiles;    // > 0: tiles of the symmetric units, slot sums at soff
-    int32_t pad;
-    int64_t soff;         // first f32 slot sum of the member
+    int32_t pairs;        // the slots are float2 (sym_tile_pair)
+    int64_t soff;         // first slot sum of the member, in floats
 };
 
 struct WorkUnit {
@@ -97,9 +97,10 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
                     const int32_t *__restrict__ member_kx, const int32_t *__restrict__ member_km,
                     float *__restrict__ slots, int parts)
 {
-    // with parts > 1 a cluster of that many blocks shares out each unit
-    // (sym_tile_pair); its first block draws the units
-    __shared__ float smem[kSymWarps * kSymTile * 3];
+    // eight blocks (a cluster) take a unit's eighths, or one block takes them all
+    // (sym_tile_pair, EIGHTHS: so that a member's bits do not depend on what else is
+    // in the batch); the cluster's first block draws the units
+    extern __shared__ float sym_smem[];
     __shared__ int next;
     const int rank = parts > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0;
     for (;;) {
@@ -120,11 +121,13 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
             const MemberInfo m = members[w.member];
             const int sk = pair_scale_from(member_kx[w.member], m.e), skm = member_km[w.member];
             if (w.I == w.J)
-                sym_tile_pair<true, false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                    skm, slots + m.soff, false, smem, rank, parts);
+                sym_tile_pair<true, true, true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I,
+                                                w.J, m.e, sk, skm, slots + m.soff, m.pairs != 0,
+                                                sym_smem, rank, parts);
             else
-                sym_tile_pair<false, false>(body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk,
-                                     skm, slots + m.soff, false, smem, rank, parts);
+                sym_tile_pair<false, true, true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I,
+                                                 w.J, m.e, sk, skm, slots + m.soff, m.pairs != 0,
+                                                 sym_smem, rank, parts);
         }
         __syncthreads();
     }
@@ -164,24 +167,27 @@ __global__ void ensemble_verlet_kernel(float4 *body4, const double *__restrict__
                 const size_t n3 = 3 * (size_t)m.n;
                 const float *p = slot_sums + m.soff + i;
                 float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
+                const float2 *p2 = reinterpret_cast<const float2 *>(slot_sums + m.soff) + i;
                 // four slots' loads in flight together
                 for (int t0 = 0; t0 < m.sym_tiles; t0 += 4) {
-                    float v[4][3];
+                    float2 v[4][3];
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (t0 + u < m.sym_tiles)
 #pragma unroll
-                            for (int c = 0; c < 3; ++c)
-                                v[u][c] = p[(size_t)(t0 + u) * n3 + (size_t)c * m.n];
+                            for (int c = 0; c < 3; ++c) {
+                                const size_t at = (size_t)(t0 + u) * n3 + (size_t)c * m.n;
+                                v[u][c] = m.pairs ? p2[at] : make_float2(p[at], 0.f);
+                            }
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (t0 + u < m.sym_tiles)
 #pragma unroll
                             for (int c = 0; c < 3; ++c) {
                                 float sum, err;
-                                two_sum(h[c], v[u][c], sum, err);
+                                two_sum(h[c], v[u][c].x, sum, err);
                                 h[c] = sum;
-                                l[c] += err;
+                                l[c] += err + v[u][c].y;
                             }
                 }
                 const double unsc =
@@ -334,6 +340,15 @@ constexpr int kChunks[] = {4096, 8192, 16384, 65536};
 // Default size from which members use the symmetric units, and the thresholds
 // the autotuner compares (INT32_MAX: none).
 constexpr int kEnsembleSymMin = 8192;
+// Members below this size (which took the one-pair units before each-pair-once was the
+// default for them) keep what their slots' rounding drops (kSymFine in direct_sym.cu).
+constexpr int kEnsemblePairs = 16384;
+// Tile pairs from which one block takes a whole pair instead of a cluster of eight:
+// about sixteen per SM, where the blocks' last turns no longer matter and the
+// cluster's exchange would cost 10%.
+constexpr int kUnitsPerSm = 16;
+constexpr size_t kSymUnitSmem = 12 * kSymTile * sizeof(float);  // one block per pair
+constexpr size_t kSymClusterSmem = 6 * kSymTile * sizeof(float);
 constexpr int kSymMins[] = {8192, 16384, 32768, INT32_MAX};
 
 template <int BLOCK, int IPT>
@@ -438,7 +453,8 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
         size_t slot_bytes = 0, free_b = 0, total_b = 0;
         for (const MemberInfo &mi : E->members)
             if (mi.n >= sym_min)
-                slot_bytes += (pad_bodies((size_t)mi.n) / kSymTile) * 12 * (size_t)mi.n;
+                slot_bytes += (pad_bodies((size_t)mi.n) / kSymTile) * 12 * (size_t)mi.n *
+                              (mi.n < kEnsemblePairs ? 2 : 1);
         if (slot_bytes > 0 &&
             (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || slot_bytes > total_b / 4))
             sym_min = INT32_MAX;
@@ -468,14 +484,15 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
         mi.chunk_tiles = chunk_tiles;
         mi.splits = cut.splits;
         mi.poff = poff;
-        mi.sym_tiles = 0;
+        mi.sym_tiles = mi.pairs = 0;
         mi.soff = soff;
         if (mi.n >= sym_min && E->cfg.compensated != 0) {
             // each unordered pair once: all tile pairs of the member
             const int T = (int)(pad_bodies((size_t)mi.n) / kSymTile);
             mi.sym_tiles = T;
             mi.splits = 0;
-            soff += (int64_t)T * 3 * mi.n;
+            mi.pairs = mi.n < kEnsemblePairs;
+            soff += ((int64_t)T * 3 * mi.n * (mi.pairs ? 2 : 1) + 1) / 2 * 2;  // (float2)
             for (int J = 0; J < T; ++J)
                 for (int I = 0; I <= J; ++I) sym_units.push_back({(int32_t)k, I, J, 0});
             continue;
@@ -529,14 +546,13 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     E->ipt = ipt;
     E->chunk = chunk;
     E->sym_min = sym_min;
-    // few tile pairs: each shared out over a cluster until there are about eight
-    // for every resident block
-    E->sym_parts = 1;
-    while (E->sym_parts < 8 && (long long)E->n_sym_units * E->sym_parts < 8ll * 4 * device_sm_count(E->device))
-        E->sym_parts *= 2;
+    E->sym_parts = E->n_sym_units < kUnitsPerSm * device_sm_count(E->device) ? 8 : 1;
     int sym_per_sm = 1;
-    PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sym_per_sm, ensemble_sym_kernel,
-                                                          kSymThreads, 0));
+    PG_CUDA(cudaFuncSetAttribute(ensemble_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSymUnitSmem));
+    PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &sym_per_sm, ensemble_sym_kernel, kSymThreads,
+        E->sym_parts > 1 ? kSymClusterSmem : kSymUnitSmem));
     E->sym_grid = std::max(1, sym_per_sm) * device_sm_count(E->device);
     drop_graph(E);
     return PHYSIM_OK;
@@ -556,6 +572,7 @@ int launch_forces(PhysimEnsemble *E)
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)std::min<long long>(E->sym_grid / parts, E->n_sym_units) * parts);
         cfg.blockDim = dim3(kSymThreads);
+        cfg.dynamicSmemBytes = parts > 1 ? kSymClusterSmem : kSymUnitSmem;
         cfg.stream = E->stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
