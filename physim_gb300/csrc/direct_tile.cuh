@@ -19,16 +19,21 @@
 #include "common.cuh"
 #include "engine.h"
 
+#include <type_traits>
+
 namespace pg {
 
 // One i tile of BLOCK*IPT bodies starting at i_base against the j tiles
 // [t0, t1) of `body` (n bodies, padded), writing this split's partial sums to
-// out[c*n + i].  `tile` is the block's shared staging buffer; sk and skm the
-// pair scale exponents.
-template <int BLOCK, int IPT, bool COMP>
+// out[c*n + i], f64 and unscaled.  Where Out is float2, each `chunk` tiles give a sum
+// of their own, 3 n apart: the compensated sum's two parts as they are (scaled; no f64
+// operation).  `tile` is the block's shared staging buffer; sk and skm the pair scale
+// exponents.
+template <int BLOCK, int IPT, bool COMP, typename Out>
 __device__ __forceinline__ void direct_tile(const float4 *__restrict__ body, int n, int i_base,
                                             int t0, int t1, float e, int sk, int skm,
-                                            double *__restrict__ out, float4 (*tile)[BLOCK][2])
+                                            Out *__restrict__ out, float4 (*tile)[BLOCK][2],
+                                            int chunk = 0)
 {
     static_assert(IPT % 2 == 0, "bodies per thread must be even (packed pairs)");
     constexpr int P = IPT / 2;
@@ -52,6 +57,35 @@ __device__ __forceinline__ void direct_tile(const float4 *__restrict__ body, int
         hx[p] = hy[p] = hz[p] = make_float2(0.f, 0.f);
         lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
     }
+    constexpr bool kChunks = std::is_same<Out, float2>::value;
+    auto put = [&](int c, int i, float hi, float lo) {
+        if constexpr (kChunks)
+            out[(size_t)c * n + i] = make_float2(hi, lo);
+        else
+            out[(size_t)c * n + i] = ((double)hi + (double)lo) * unsc;
+    };
+    auto emit = [&]() {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int i0 = i_base + tid + (2 * p) * BLOCK;
+            const int i1 = i0 + BLOCK;
+            if (!COMP) {
+                hx[p] = ax[p];
+                hy[p] = ay[p];
+                hz[p] = az[p];
+            }
+            if (i0 < n) {
+                put(0, i0, hx[p].x, lx[p].x);
+                put(1, i0, hy[p].x, ly[p].x);
+                put(2, i0, hz[p].x, lz[p].x);
+            }
+            if (i1 < n) {
+                put(0, i1, hx[p].y, lx[p].y);
+                put(1, i1, hy[p].y, ly[p].y);
+                put(2, i1, hz[p].y, lz[p].y);
+            }
+        }
+    };
     const float es = e * pow2f(-2 * sk);
     const float2 e2 = make_float2(es, es);
     const float2 g2 = make_float2(kPairGuard, kPairGuard);
@@ -105,34 +139,21 @@ __device__ __forceinline__ void direct_tile(const float4 *__restrict__ body, int
                     ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
                 }
             }
-        }
-    }
-    if (!COMP) {
+            if constexpr (kChunks) {
+                if (t + 1 < t1 && (t + 1 - t0) % chunk == 0) {
+                    emit();
+                    out += 3 * (size_t)n;
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            hx[p] = ax[p];
-            hy[p] = ay[p];
-            hz[p] = az[p];
+                    for (int p = 0; p < P; ++p) {
+                        ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
+                        hx[p] = hy[p] = hz[p] = make_float2(0.f, 0.f);
+                        lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
+                    }
+                }
+            }
         }
     }
-    double *px = out;
-    double *py = out + n;
-    double *pz = out + 2 * (size_t)n;
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-        const int i0 = i_base + tid + (2 * p) * BLOCK;
-        const int i1 = i0 + BLOCK;
-        if (i0 < n) {
-            px[i0] = ((double)hx[p].x + (double)lx[p].x) * unsc;
-            py[i0] = ((double)hy[p].x + (double)ly[p].x) * unsc;
-            pz[i0] = ((double)hz[p].x + (double)lz[p].x) * unsc;
-        }
-        if (i1 < n) {
-            px[i1] = ((double)hx[p].y + (double)lx[p].y) * unsc;
-            py[i1] = ((double)hy[p].y + (double)ly[p].y) * unsc;
-            pz[i1] = ((double)hz[p].y + (double)lz[p].y) * unsc;
-        }
-    }
+    emit();
 }
 
 }  // namespace pg

@@ -41,7 +41,7 @@ struct MemberInfo {
     int32_t off;          // first slot of the member in the concatenated arrays
     int32_t n;            // bodies
     int32_t n_jtiles;     // j tiles of the current shape
-    int32_t chunk_tiles;  // j tiles per work unit
+    int32_t chunk_tiles;  // j tiles per chunk
     int64_t poff;         // first partial sum of the member
     int32_t splits;
     float e;
@@ -51,8 +51,9 @@ struct MemberInfo {
     int64_t soff;         // first slot sum of the member, in floats
 };
 
+// An i tile of a member against `count` j chunks from `split` on.
 struct WorkUnit {
-    int32_t member, itile, split, pad;
+    int32_t member, itile, split, count;
 };
 
 // A tile pair (I, J), I <= J, of a member on the symmetric units.
@@ -66,7 +67,7 @@ ensemble_forces_kernel(const float4 *__restrict__ body4, const MemberInfo *__res
                        const WorkUnit *__restrict__ units, int n_units,
                        const unsigned long long *__restrict__ remaining, int *__restrict__ counter,
                        const int32_t *__restrict__ member_kx, const int32_t *__restrict__ member_km,
-                       double *__restrict__ partial)
+                       float2 *__restrict__ partial)
 {
     __shared__ float4 tile[2][BLOCK][2];
     __shared__ int next;
@@ -79,11 +80,12 @@ ensemble_forces_kernel(const float4 *__restrict__ body4, const MemberInfo *__res
         if (remaining[w.member] != 0) {
             const MemberInfo m = members[w.member];
             const int t0 = w.split * m.chunk_tiles;
-            const int t1 = min(t0 + m.chunk_tiles, m.n_jtiles);
+            const int t1 = min(t0 + w.count * m.chunk_tiles, m.n_jtiles);
             direct_tile<BLOCK, IPT, COMP>(body4 + m.off, m.n, w.itile * BLOCK * IPT, t0, t1, m.e,
                                           pair_scale_from(member_kx[w.member], m.e),
                                           member_km[w.member],
-                                          partial + m.poff + (size_t)w.split * 3 * m.n, tile);
+                                          partial + m.poff + (size_t)w.split * 3 * m.n, tile,
+                                          m.chunk_tiles);
         }
         __syncthreads();
     }
@@ -145,7 +147,7 @@ __global__ void ensemble_verlet_kernel(float4 *body4, const double *__restrict__
                                        const MemberInfo *__restrict__ members,
                                        const unsigned long long *__restrict__ remaining,
                                        const unsigned long long *__restrict__ done,
-                                       const double *__restrict__ partial,
+                                       const float2 *__restrict__ partial,
                                        const float *__restrict__ slot_sums, int slots, double *x,
                                        double *y, double *z, double *vx, double *vy, double *vz,
                                        double *px, double *py, double *pz,
@@ -162,57 +164,40 @@ __global__ void ensemble_verlet_kernel(float4 *body4, const double *__restrict__
         const int i = s - m.off;
         double ax = 0.0, ay = 0.0, az = 0.0;
         if (!fixed[s]) {
-            if (m.sym_tiles > 0) {
-                // the member's slot sums, TwoSum-compensated in slot order, unscaled
-                const size_t n3 = 3 * (size_t)m.n;
-                const float *p = slot_sums + m.soff + i;
-                float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
-                const float2 *p2 = reinterpret_cast<const float2 *>(slot_sums + m.soff) + i;
-                // four slots' loads in flight together
-                for (int t0 = 0; t0 < m.sym_tiles; t0 += 4) {
-                    float2 v[4][3];
+            // the member's slot or partial sums, TwoSum-compensated in order, unscaled
+            const bool sym = m.sym_tiles > 0, pairs = !sym || m.pairs != 0;
+            const int count = sym ? m.sym_tiles : m.splits;
+            const size_t n3 = 3 * (size_t)m.n;
+            const float *p = slot_sums + m.soff + i;
+            const float2 *p2 = (sym ? reinterpret_cast<const float2 *>(slot_sums + m.soff)
+                                    : partial + m.poff) + i;
+            float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
+            // four sums' loads in flight together
+            for (int t0 = 0; t0 < count; t0 += 4) {
+                float2 v[4][3];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (t0 + u < m.sym_tiles)
+                for (int u = 0; u < 4; ++u)
+                    if (t0 + u < count)
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                const size_t at = (size_t)(t0 + u) * n3 + (size_t)c * m.n;
-                                v[u][c] = m.pairs ? p2[at] : make_float2(p[at], 0.f);
-                            }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (t0 + u < m.sym_tiles)
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                float sum, err;
-                                two_sum(h[c], v[u][c].x, sum, err);
-                                h[c] = sum;
-                                l[c] += err + v[u][c].y;
-                            }
-                }
-                const double unsc =
-                    pow2d(member_km[k] - 2 * pair_scale_from(member_kx[k], m.e));
-                ax = ((double)h[0] + (double)l[0]) * unsc;
-                ay = ((double)h[1] + (double)l[1]) * unsc;
-                az = ((double)h[2] + (double)l[2]) * unsc;
-            } else {
-                for (int s0 = 0; s0 < m.splits; s0 += 4) {
-                    double v[4][3];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (s0 + u < m.splits)
-#pragma unroll
-                            for (int c = 0; c < 3; ++c)
-                                v[u][c] = partial[m.poff + (size_t)((s0 + u) * 3 + c) * m.n + i];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (s0 + u < m.splits) {
-                            ax += v[u][0];
-                            ay += v[u][1];
-                            az += v[u][2];
+                        for (int c = 0; c < 3; ++c) {
+                            const size_t at = (size_t)(t0 + u) * n3 + (size_t)c * m.n;
+                            v[u][c] = pairs ? p2[at] : make_float2(p[at], 0.f);
                         }
-                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (t0 + u < count)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            float sum, err;
+                            two_sum(h[c], v[u][c].x, sum, err);
+                            h[c] = sum;
+                            l[c] += err + v[u][c].y;
+                        }
             }
+            const double unsc = pow2d(member_km[k] - 2 * pair_scale_from(member_kx[k], m.e));
+            ax = ((double)h[0] + (double)l[0]) * unsc;
+            ay = ((double)h[1] + (double)l[1]) * unsc;
+            az = ((double)h[2] + (double)l[2]) * unsc;
             if (mass[s] == 0.0) ax = ay = az = __longlong_as_double(0x7ff8000000000000LL);
         }
         const bool initial = done[k] == 0;
@@ -404,7 +389,7 @@ struct PhysimEnsemble {
     int32_t *member_kx = nullptr;    // coordinate exponent of each member's pair scale
     int32_t *member_km = nullptr;    // mass scale exponent of each member
     uint32_t *member_ext = nullptr;  // largest |coordinate| of the new positions (f32 bits)
-    double *partial = nullptr;
+    float2 *partial = nullptr;  // one-pair sums (direct_tile)
     SymUnit *d_sym_units = nullptr;
     int n_sym_units = 0;
     size_t sym_units_cap = 0;
@@ -463,7 +448,7 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, ens_kernel(block, ipt, E->cfg.compensated != 0), block, 0));
     E->grid = std::max(1, per_sm) * device_sm_count(E->device);
-    // The chunk is cut so that the one-pair units are at least four times the
+    // Units take as many of a member's chunks as leave them at least eight times the
     // blocks that draw them: with fewer, one unit's blocks outlast the rest
     // (30 members of 256 to 14,671 bodies: 135 units of up to 16,384 bodies for
     // 456 blocks, 1.42 ms a step for 0.25 ms of pair arithmetic).
@@ -471,17 +456,16 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
     for (const MemberInfo &mi : E->members)
         if (mi.n < sym_min || E->cfg.compensated == 0)
             jbodies += (long long)cdiv(mi.n, block * ipt) * mi.n;
-    const long long even = jbodies / (4ll * E->grid);
+    const long long even = jbodies / (8ll * E->grid);
     std::vector<WorkUnit> units;
     std::vector<SymUnit> sym_units;
     std::vector<long long> cost;
     int64_t poff = 0, soff = 0;
     for (size_t k = 0; k < E->members.size(); ++k) {
         MemberInfo &mi = E->members[k];
-        const MemberCut cut = cut_member(mi.n, block, (int)std::min<long long>(chunk, even));
-        const int chunk_tiles = cut.chunk_tiles;
+        const MemberCut cut = cut_member(mi.n, block, chunk);
         mi.n_jtiles = cut.n_jtiles;
-        mi.chunk_tiles = chunk_tiles;
+        mi.chunk_tiles = cut.chunk_tiles;
         mi.splits = cut.splits;
         mi.poff = poff;
         mi.sym_tiles = mi.pairs = 0;
@@ -498,11 +482,12 @@ int plan_ensemble(PhysimEnsemble *E, int block, int ipt, int chunk, int sym_min)
             continue;
         }
         poff += (int64_t)mi.splits * 3 * mi.n;
-        const int n_itiles = cdiv(mi.n, block * ipt);
+        const int n_itiles = cdiv(mi.n, block * ipt), per = unit_chunks(cut, block, even);
         for (int it = 0; it < n_itiles; ++it)
-            for (int sp = 0; sp < mi.splits; ++sp) {
-                const int t0 = sp * chunk_tiles, t1 = std::min(t0 + chunk_tiles, mi.n_jtiles);
-                units.push_back({(int32_t)k, it, sp, 0});
+            for (int sp = 0; sp < mi.splits; sp += per) {
+                const int t0 = sp * cut.chunk_tiles;
+                const int t1 = std::min(t0 + per * cut.chunk_tiles, mi.n_jtiles);
+                units.push_back({(int32_t)k, it, sp, std::min(per, mi.splits - sp)});
                 cost.push_back((long long)(t1 - t0));
             }
     }
