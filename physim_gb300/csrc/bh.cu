@@ -1062,8 +1062,8 @@ __device__ __forceinline__ void rank_sort_body(const TreeSortArgs &a, uint64_t *
 
 __global__ void __launch_bounds__(kRankTile, 1) rank_sort_kernel(TreeSortArgs a)
 {
-    extern __shared__ uint64_t skeys_dyn[];
-    rank_sort_body(a, skeys_dyn);
+    extern __shared__ __align__(16) uint64_t rank_keys[];  // (16-byte asynchronous copies)
+    rank_sort_body(a, rank_keys);
     leave_grid(a.bar);
 }
 
