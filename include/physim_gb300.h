@@ -418,6 +418,9 @@ int physim_gpu_set_sort_single_launch(int32_t on);
  * that nothing reaches), so its wait always runs out.
  * Process-wide, read when a build is enqueued or captured. */
 int physim_gpu_test_stall_sort(int32_t tile);
+/* The same for the one-launch tree build: block `block` waits at its first barrier for a
+ * count that nothing reaches. */
+int physim_gpu_test_stall_build(int32_t block);
 /* The current pair-kernel plan of a simple_astro simulation (block, ipt,
  * splits, symmetric, tiles; the other fields 0); all zero for astro/astro2. */
 int physim_gpu_sim_plan(PhysimSim *sim, PhysimDirectTuning *out);

@@ -2163,7 +2163,7 @@ struct BuildArgs {
     const unsigned long long *extent_bits;
     uint32_t *bar;  // [0] barrier count, [1] blocks that left
     uint32_t *flags;
-    int spin_limit;
+    int spin_limit, stall_tile;
     bool early;  // SMs are free for the next kernel's blocks
 };
 
@@ -2202,7 +2202,9 @@ __global__ void __launch_bounds__(kBuildBlock, 1) tree_build_kernel(BuildArgs a)
                 keys, [&](int j) { return shared_digits(keys[j - 1], keys[j], nchild); }, tile, n,
                 nchild, a.leaf, a.blk_cnt, tiles, sh.first.mask, m, lc);
         }
-        ok = grid_barrier(a.bar, a.flags, a.spin_limit, gridDim.x, &s_ok);
+        // the test hook's block waits for a count that nothing reaches
+        ok = grid_barrier(a.bar, a.flags, a.spin_limit,
+                          (int)blockIdx.x == a.stall_tile ? kBarPoison : gridDim.x, &s_ok);
     }
     if (ok) {
         // the levels' totals and starts, the same in every block, and the nodes
@@ -3418,7 +3420,7 @@ int bh_stats(BhWorkspace *ws, cudaStream_t st, uint64_t out[2])
 
 namespace {
 std::atomic<uint32_t> g_wait_limit{0};  // 0: kLookbackSpins
-std::atomic<int32_t> g_stall_tile{-1};
+std::atomic<int32_t> g_stall_tile{-1}, g_stall_build{-1};
 std::atomic<int> g_sort_single{1};
 }  // namespace
 
@@ -3580,6 +3582,7 @@ static int launch_build(BhWorkspace *ws, const GatherArgs &ga, const BhParams &p
     a.bar = ws->tree_bar + 4;
     a.flags = ws->flags;
     a.spin_limit = wait_limit();
+    a.stall_tile = (int)g_stall_build.load();
     // blocks for the tiles, one for the top group sums, and more if the cells
     // are more than those blocks' threads
     const int lanes = cell_lanes(ga.n, p);
@@ -3829,5 +3832,11 @@ extern "C" int physim_gpu_set_sort_single_launch(int32_t on)
 extern "C" int physim_gpu_test_stall_sort(int32_t tile)
 {
     pg::g_stall_tile.store(tile < 0 ? -1 : tile);
+    return PHYSIM_OK;
+}
+
+extern "C" int physim_gpu_test_stall_build(int32_t block)
+{
+    pg::g_stall_build.store(block < 0 ? -1 : block);
     return PHYSIM_OK;
 }
