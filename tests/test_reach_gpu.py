@@ -5,8 +5,8 @@
     the largest state, against the separate launches, bit for bit; accelerations there
     against the oracle;
   * the resident sort by digits (csrc/bh.cu: tree_sort_kernel, from 18,433 bodies): its
-    smallest state, whole count groups of 16 tiles of 512 and one tile more, equal keys
-    and extent 0, against the separate radix passes, bit for bit;
+    smallest state, whole count groups of 16 tiles of 512 and one tile more, equal keys,
+    extent 0 and runs that every block finds too long, against the separate radix passes, bit for bit;
   * each pair once with one, two, four and eight blocks to a tile pair
     (csrc/direct_sym.cu: pair_parts), against the one-pair kernels to 2e-6, as plans of
     the direct sum agree, and repeated bit for bit."""
@@ -50,12 +50,14 @@ def test_small_accelerations(oracle_mod, n):
     assert np.all(rel_err(got[~bad], want[~bad]) < RTOL)
 
 
-@pytest.mark.parametrize("kind", ["uniform", "clumps", "one position", "origin"])
+@pytest.mark.parametrize("kind", ["uniform", "clumps", "one position", "origin", "far body"])
 @pytest.mark.parametrize("n", [18433, 32 * 512, 48 * 512, 48 * 512 + 1, 160001])
 def test_resident_sort(n, kind):
     from test_tree_sort_gpu import _check, _clumps, _uniform
     n = max(n, 18433)
     s = _clumps(n, seed=3) if kind == "clumps" else _uniform(n, seed=n % 97)
+    if kind == "far body":  # all others within a few cells of the top digits
+        s["x"][n // 3] = 1e4
     if kind in ("one position", "origin"):
         for f in "xyz":
             s[f] = 0.25 if kind == "one position" else 0.0
