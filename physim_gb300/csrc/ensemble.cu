@@ -122,14 +122,21 @@ ensemble_sym_kernel(const float4 *__restrict__ body4, const float *__restrict__ 
         if (remaining[w.member] != 0) {
             const MemberInfo m = members[w.member];
             const int sk = pair_scale_from(member_kx[w.member], m.e), skm = member_km[w.member];
-            if (w.I == w.J)
-                sym_tile_pair<true, true, true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I,
-                                                w.J, m.e, sk, skm, slots + m.soff, m.pairs != 0,
-                                                sym_smem, rank, parts);
-            else
-                sym_tile_pair<false, true, true>(body4 + m.off, mass256 + m.off / 256, m.n, w.I,
-                                                 w.J, m.e, sk, skm, slots + m.soff, m.pairs != 0,
-                                                 sym_smem, rank, parts);
+            auto pair = [&](auto diag, auto fine) {
+                sym_tile_pair<decltype(diag)::value, decltype(fine)::value, true>(
+                    body4 + m.off, mass256 + m.off / 256, m.n, w.I, w.J, m.e, sk, skm,
+                    slots + m.soff, m.pairs != 0, sym_smem, rank, parts);
+            };
+            if (m.pairs != 0) {
+                if (w.I == w.J)
+                    pair(std::true_type(), std::true_type());
+                else
+                    pair(std::false_type(), std::true_type());
+            } else if (w.I == w.J) {
+                pair(std::true_type(), std::false_type());
+            } else {
+                pair(std::false_type(), std::false_type());
+            }
         }
         __syncthreads();
     }
@@ -325,8 +332,10 @@ constexpr int kChunks[] = {4096, 8192, 16384, 65536};
 // Default size from which members use the symmetric units, and the thresholds
 // the autotuner compares (INT32_MAX: none).
 constexpr int kEnsembleSymMin = 8192;
-// Members below this size (which took the one-pair units before each-pair-once was the
-// default for them) keep what their slots' rounding drops (kSymFine in direct_sym.cu).
+// Members below this size, which the one-pair units would take otherwise, are summed as
+// exactly as those do (kSymFine in direct_sym.cu), with slots that keep what rounding
+// drops: RMS error against f64 of 8,192 and 16,383 bodies, Plummer, 1e-8, one-pair / FINE
+// 3.3 / 2.8 and 2.9 / 2.6.  Larger members' chains are 128 terms, by the eighths.
 constexpr int kEnsemblePairs = 16384;
 // Tile pairs from which one block takes a whole pair instead of a cluster of eight:
 // about sixteen per SM, where the blocks' last turns no longer matter and the
