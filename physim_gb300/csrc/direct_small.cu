@@ -13,26 +13,34 @@
 //
 //   * j bodies in units of 64 (one packed pair per lane), units dealt to the
 //     8 warps in turn, up to kMaxPacks units per warp in registers at a time;
-//   * per two bodies i: the pair loop (13 FMA-pipe operations and one MUFU per
-//     pair, as direct_tile), then six sums over the lanes by a transposing
-//     butterfly (8 shuffles instead of 30), one partial per warp in shared
-//     memory; the 16 warps' partials are added with TwoSum in warp order.  The
-//     chains of plain FP32 adds are at most 16 long (128 and 256 in the tiled
-//     kernels);
+//   * per four bodies i: the pair loop (13 FMA-pipe operations and one MUFU per
+//     pair, as direct_tile), then for each two of them six sums over the lanes by
+//     a transposing butterfly (8 shuffles instead of 30), one partial per warp in
+//     shared memory; the eight warps' partials are added with TwoSum in warp
+//     order.  The chains of plain FP32 adds are at most 16 long: nine units, the
+//     two halves of a lane, five steps over the lanes, and above 4,608 bodies the
+//     second pass (128 and 256 in the tiled kernels).  RMS error against f64 at
+//     e = 0.01, against the tiled kernels' plan of the same size: Plummer 0.2 (300
+//     bodies) to 0.95 of it, a cube with heavy stars 0.4 to 0.7 in any order of the
+//     bodies but the stars last, where the tiled chains end, and then 0.3 to 1.1;
 //   * whole steps: the owned bodies' f64 state stays in registers, one thread
 //     per coordinate, which applies verlet as integrate.cu does (same
 //     operations, same order); the f32 positions go to the other of two body
 //     arrays, and one grid barrier per step (1.2 us, every block resident by a
 //     cooperative launch) lets the next step read them.
-// Step times against the best tiled or each-pair-once plan (us): 300 bodies 14.4
-// -> 3.7, 1,002 16.5 -> 4.1, 4,098 24.7 -> 11.7, and against the each-pair-once
-// plan as it is now 6,500 32.8 -> 25.8, 7,400 31.3 -> 31.6, 8,192 32.3 -> 37.5,
-// 10,000 52 -> 57, 12,000 60 -> 75: the line is at 7,400.  Bound by the FMA pipe (60%
-// busy) from about 6,000 bodies, below by the barrier and one pass of latency.
-// Eight warps of 255 registers, four bodies i at a time: sixteen of 128, two at a
-// time, left the pipe waiting on each chain (4,098 bodies 14.1).  A wait at the barrier that exceeds the wait limit raises an
+// Step times against the best tiled plan (us): 300 bodies 14.4 -> 3.7, 1,002 16.5
+// -> 4.1, 4,098 24.7 -> 11.7, 7,400 49 -> 31.6, and each pair once / here: 7,401
+// 32 / 32, with masses that differ 39 / 32, 8,192 33 / 38 and 39 / 38, 9,001 58 /
+// 47 and 60 / 47, 10,240 52 / 57 and 61 / 58, 12,001 70 / 74 and 73 / 74.  The line
+// is at 7,400: above it the other plan's error is no larger in any order of the
+// bodies (kSymFine in direct_sym.cu), for up to 20% of a step between 8,200 and
+// 9,800 bodies.  Bound by the FMA pipe (60% busy) from about 6,000 bodies, below by
+// the barrier and one pass of latency.  Eight warps of 255 registers, four bodies i
+// at a time: sixteen of 128, two at a time, left the pipe waiting on each chain
+// (4,098 bodies 14.1).  A wait at the barrier that exceeds the wait limit raises an
 // error flag and ends the launch in every block; the next synchronising call
-// reports PHYSIM_ERR_TIMEOUT.
+// reports PHYSIM_ERR_TIMEOUT, and the state is invalid until the next upload (the
+// blocks may have given up at different steps).
 #include <cuda/atomic>
 
 #include <algorithm>
@@ -48,7 +56,8 @@ namespace {
 constexpr int kSmallThreads = 256;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kMaxPacks = 8;     // units every warp holds at a time (some one more)
-constexpr int kMaxOwned = 84;    // bodies per block (a thread per coordinate)
+constexpr int kMaxOwned = 84;    // bodies per block at most (a thread per coordinate; 49
+                                 // of 7,400 on 152 SMs)
 constexpr int kTurn = 4;         // owned bodies per turn of the pair loop
 constexpr int kUnit = 64;        // bodies of a unit
 constexpr int kSmallOwned = 16;  // bodies per block until every SM has one
@@ -87,7 +96,7 @@ __device__ __forceinline__ float reduce6(float (&v)[6], int lane)
     return a;
 }
 
-// The owned bodies against P units per warp from unit u0 on (u0 + warp, + 16, ...)
+// The owned bodies against P units per warp from unit u0 on (u0 + warp, + 8, ...)
 // and, with `extra`, one more; `first`: sh.part is written, else added to.  The
 // P units are straight-line code, so their chains overlap (with a branch per
 // unit this loop ran at half the FMA pipe).

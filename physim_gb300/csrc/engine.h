@@ -117,7 +117,7 @@ struct DirectPlan {
     // of 1,024; the partial sums come out as one split, after f32 slot sums
     // the same allocation holds.  grouped: a block takes 8 I tiles and a
     // run of 16 J tiles (3T^2/32 slots of 3 x 1,024 floats); otherwise one block
-    // per tile pair (one [3][n] slot per tile).
+    // per tile pair (one [3][n] slot per tile, of two f32 below 20,480 bodies).
     bool symmetric = false;
     int tiles = 0;
     bool grouped = false;

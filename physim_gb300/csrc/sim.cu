@@ -37,8 +37,8 @@ struct PhysimSim {
     // step start, gravity done, step done, pair kernel done (simple_astro)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // The gravity phase of a step, captured once and replayed: the
-    // Barnes-Hut build is ~100 short kernels whose launch cost would
-    // otherwise dominate at small N.
+    // Barnes-Hut step is three to eight short kernels whose launches would otherwise
+    // cost 2 to 4 us.
     bool use_graph = true;
     // one per current half of the pair-law maxima (PairScale), which the
     // captured kernels read by address

@@ -43,9 +43,11 @@ import numpy as np
 BYTES_PER_BODY_DIRECT = 200
 BYTES_PER_BODY_TREE = 700
 BYTES_FIXED = 4 << 20
-# Smallest direct-sum job that may evaluate each unordered pair once (the
-# lowest size threshold the ensemble autotuner picks), and the largest slot
-# buffer the library gives that evaluation (a quarter of a GB300's 284,208
+# Smallest direct-sum job whose slot sums are counted: the size from which ensemble
+# members may evaluate each unordered pair once (the lowest threshold their autotuner
+# picks; a simulation does from 7,401 bodies, and below 16,384 in an ensemble and
+# 20,480 in a simulation a slot takes twice the bytes, 5 MB at most, which BYTES_FIXED
+# leaves room for), and the largest slot buffer the library gives that evaluation (a quarter of a GB300's 284,208
 # MiB; above it the library takes one-pair kernels, which keep no slot sums)
 SYMMETRIC_FROM = 8192
 SYMMETRIC_CAP_BYTES = 284_208 * (1 << 20) // 4
@@ -58,7 +60,7 @@ SYMMETRIC_CAP_BYTES = 284_208 * (1 << 20) // 4
 #     (csrc/direct_sym.cu, make_symmetric_plan and direct_partial_doubles)
 SYM_TILE = 1024
 SYM_PAIRS_SLOT_BYTES = 4 << 30
-SYM_CLUSTER, SYM_RUN = 8, 16
+SYM_GROUP, SYM_RUN = 8, 16
 
 
 def tile_slot_bytes(n: int) -> int:
@@ -76,8 +78,8 @@ def symmetric_slot_bytes(n: int) -> int:
     runs = -(-t // SYM_RUN)
     q, rem = divmod(t, SYM_RUN)
     iside = t * runs - (SYM_RUN * q * (q - 1) // 2 + q * rem)
-    q, rem = divmod(t, SYM_CLUSTER)
-    jside = t + SYM_CLUSTER * q * (q - 1) // 2 + q * rem
+    q, rem = divmod(t, SYM_GROUP)
+    jside = t + SYM_GROUP * q * (q - 1) // 2 + q * rem
     return (iside + jside) * 3 * SYM_TILE * 4
 
 
@@ -116,8 +118,9 @@ class JobSpec:
 
     def step_seconds(self) -> float:
         """Rough device seconds per step on one GB300 (scheduling estimates
-        only): N^2 pairs at 2.3e12 pairs/s for the direct sum, 1.4 us per
-        1,000 bodies plus launch latency for Barnes-Hut."""
+        only; what matters is how jobs compare): N^2 pairs at 2.3e12 pairs/s for
+        the direct sum, 1.4 us per 1,000 bodies plus launch latency for Barnes-Hut.
+        A large job alone on the GPU takes about half of either."""
         if self.gravity == "simple_astro":
             return self.n * self.n / 2.3e12 + 5e-6
         return self.n * 1.4e-9 + 6e-5
