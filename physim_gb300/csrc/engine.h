@@ -242,7 +242,10 @@ int host_direct(int device, bool *direct);
 // from mapped pages of the allocator (above 32 MB each allocation is fresh pages,
 // which a copy maps while it moves others: 1,048,580 bodies 3.7 ms by copy, 3.9 in
 // place; 8,195 23 / 20 us and 262,147 139 / 133, in a Barnes-Hut simulation, whose
-// error flags come along, 34 / 18 and 151 / 145; 30 members 636 / 495).
+// error flags come along, 34 / 18 and 151 / 145; 30 members 636 / 495).  Its pages are
+// mapped here, while the work before the download still runs; where they cannot be (an
+// array that may not be written to its end, which a kernel's write would fault on), the
+// answer is a copy.
 int download_direct(int device, const void *p, size_t bytes, bool *direct);
 // Before kernels touch a host array in place: maps every page of
 // [p, p + bytes) into the process (writable if `write`), without changing its

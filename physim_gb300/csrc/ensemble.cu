@@ -948,10 +948,7 @@ int physim_gpu_ensemble_download(PhysimEnsemble *E, size_t index, Entity *state,
     PG_CUDA(cudaSetDevice(E->device));
     bool direct = false;
     PG_TRY(download_direct(E->device, state, n * sizeof(Entity), &direct));
-    if (direct) {
-        // written in place; the pages are mapped while the steps still run
-        host_prefault(state, n * sizeof(Entity), true);
-    } else if (n > E->staging_cap) {
+    if (!direct && n > E->staging_cap) {
         dev_free(E->staging, E->stream);
         E->staging = nullptr;
         PG_TRY(ealloc(E, E->staging, n));

@@ -9,21 +9,12 @@
 // The same kernel combines the pair kernel's partial sums, so one launch
 // does combine + kick + drift + refresh of the f32 body copy.
 #include <string.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <atomic>
 
-// madvise advice values of Linux 5.14+ (absent from older headers)
-#ifndef MADV_POPULATE_READ
-#define MADV_POPULATE_READ 22
-#endif
-#ifndef MADV_POPULATE_WRITE
-#define MADV_POPULATE_WRITE 23
-#endif
-
 #include "common.cuh"
 #include "engine.h"
+#include "host_pages.h"
 #include "verlet_axis.cuh"
 
 namespace pg {
@@ -556,7 +547,8 @@ int host_direct(int device, bool *direct)
 int download_direct(int device, const void *p, size_t bytes, bool *direct)
 {
     PG_TRY(host_direct(device, direct));
-    *direct = *direct && ((uintptr_t)p & 7) == 0 && bytes <= (size_t(32) << 20);
+    *direct = *direct && ((uintptr_t)p & 7) == 0 && bytes <= (size_t(32) << 20) &&
+              populate_pages(p, bytes, true);
     return PHYSIM_OK;
 }
 
@@ -769,11 +761,7 @@ int launch_verlet_aos(const Entity *in, const Entity *d_prev, Entity *out, Entit
 
 void pg::host_prefault(const void *p, size_t bytes, bool write)
 {
-    if (!p || !bytes) return;
-    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    const uintptr_t lo = (uintptr_t)p & ~(page - 1);
-    const uintptr_t hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
-    (void)madvise((void *)lo, hi - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+    (void)populate_pages(p, bytes, write);
 }
 
 extern "C" int physim_gpu_set_host_access(uint32_t mode)

@@ -625,9 +625,7 @@ int physim_gpu_sim_download(PhysimSim *s, Entity *state, size_t n)
     PG_TRY(download_direct(s->cfg.device, state, n * sizeof(Entity), &direct));
     const bool direct_flags = direct && n && s->bh;
     if (n && direct) {
-        // the kernel writes the caller's array in place; its pages are mapped while
-        // the steps still run
-        host_prefault(state, n * sizeof(Entity), true);
+        // the kernel writes the caller's array in place
         PG_TRY(launch_pack(s->b, state, s->stream, direct_flags ? bh_flags(s->bh) : nullptr,
                            s->flags));
     } else if (n) {
